@@ -22,7 +22,7 @@
 //
 // What bounds it: instruction issue, and a chain of a dozen short dependent phases per head whose latencies the warps of
 // an SM hide for each other.  Four warps per chunk (24 per SM), code that fits the 32 KB instruction cache, two fp32
-// values per instruction (add / mul / fma .f32x2) where a phase is elementwise, exponents that carry beta and the
+// values per instruction (add / mul / fma .f32x2) where a phase is elementwise, exponents that carry |beta| and the
 // norms (three instructions per pair of entries of L besides the two ex2), and no causal mask: what lies on or above
 // the diagonal of L is never read.
 #include "chunk_params.cuh"
@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(kKktThreads, 3) kkt_solve_kernel(const __grid_
   uint8_t* sAst = sAw + 16384;                       // 16 KiB [128 tokens][64] staging tile of A for the TMA store (SW128)
   uint8_t* sW = sAw;                                 // 32 KiB staging tile of w (two [128][64] halves, SW128), once both are consumed
   __shared__ __align__(16) float s_bg[128];          // -beta * gamma per token
-  // exponents (log2) of L: -L[c][d] = -(k_c . k_d) 2^(s_row[c] + s_col[d])
-  __shared__ __align__(16) float s_row[128];         // g log2(e) + log2(beta / |k_c|)
+  // exponents (log2) of L: -L[c][d] = -sign(beta_c) (k_c . k_d) 2^(s_row[c] + s_col[d]); the sign is that of s_bg[c]
+  __shared__ __align__(16) float s_row[128];         // g log2(e) + log2(|beta| / |k_c|)
   __shared__ __align__(16) float s_col[128];         // -(g log2(e)) - log2 |k_d|     (|k| = 1 without in-kernel norm)
   __shared__ float s_norm[2][128][2];                // [column half][token][k | q]: partial squared norms
   __shared__ float s_part[kKktThreads / 32];
@@ -315,10 +315,10 @@ __global__ void __launch_bounds__(kKktThreads, 3) kkt_solve_kernel(const __grid_
       if (p.A_in != nullptr) gcs = gin;  // gates are cumulative already
       else if (valid) p.g_cumsum[tok * p.num_v_heads + hv] = gcs;
       const float gc2 = gcs * 1.4426950408889634f;  // exponents are formed in the log2 domain
-      const float er = gc2 + (ptx::lg2(bv) + lrk);  // (beta = 0: -inf, every power below is 0)
+      const float er = gc2 + (ptx::lg2(fabsf(bv)) + lrk);  // (beta = 0: -inf, every power below is 0)
       s_row[row] = er;
       s_col[row] = lrk - gc2;
-      s_bg[row] = -ptx::ex2(er);
+      s_bg[row] = copysignf(ptx::ex2(er), -bv);
     }
     ok = __syncthreads_and(warp != 0 || ptx::mbar_wait_addr(a_mma, mma_uses & 1)) != 0;  // (one warp polls)
     ++mma_uses;
@@ -341,7 +341,8 @@ __global__ void __launch_bounds__(kKktThreads, 3) kkt_solve_kernel(const __grid_
       // columns 32..63.
       if (ch == 0 || (warp & 1)) {
         const float er = s_row[row];
-        const F2 er2 = f2(er, er), minus = f2(-1.f, -1.f);
+        const float sign = copysignf(1.f, s_bg[row]);  // -sign(beta)
+        const F2 er2 = f2(er, er), sign2 = f2(sign, sign);
 #pragma unroll 1
         for (int d16 = ch * 32; d16 < ch * 32 + 32; d16 += 16) {
           uint32_t kk[16];
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(kKktThreads, 3) kkt_solve_kernel(const __grid_
           for (int j = 0; j < 8; ++j) {
             float lo, hi;
             unpack(e[j], lo, hi);
-            e[j] = mul2(f2(ptx::ex2(lo), ptx::ex2(hi)), minus);
+            e[j] = mul2(f2(ptx::ex2(lo), ptx::ex2(hi)), sign2);
           }
           ptx::tmem_wait_ld();
           ulonglong2* dst = reinterpret_cast<ulonglong2*>(Lc + c * kLStride + d16);

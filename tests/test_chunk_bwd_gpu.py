@@ -188,3 +188,18 @@ def test_backward_context_parallel_varlen_transposed(fq):
     gt = dict(zip(GRADS, res))
     gt["dh0"] = gt["dh0"].transpose(-1, -2)
     _report(gt, ref)
+
+
+@pytest.mark.parametrize("T", [200, 2048 + 37])  # uncut, and cut into context-parallel segments
+def test_beta_of_any_sign(fq, T):
+    """Forward and backward are linear in beta: negative values and exact zeros are ordinary inputs."""
+    inp = orc.make_prefill_inputs(1, T, 2, 4, seed=43, with_h0=True, with_grads=True)
+    inp["beta"] = 2 * inp["beta"] - 1
+    inp["beta"][:, ::7] = 0
+    c = _cuda(inp)
+    _, _, o, _, fs = fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], initial_state=c["h0"])
+    got = _raw_bwd(fq, c)
+    ref = orc.chunk_gdr_bwd(inp["q"], inp["k"], inp["v"], inp["g"], inp["beta"], inp["do"], dht=inp["dht"], h0=inp["h0"])
+    for x, n in ((o, "o"), (fs, "final_state")):
+        assert orc.rel_rms(x.float().cpu(), ref[n]) <= RMS_TOL, n
+    _report(got, ref)
