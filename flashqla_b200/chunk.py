@@ -212,6 +212,12 @@ def chunk_gated_delta_rule_fwd(
     row ``n``), and it is what the call returns as final state.  Pools may be fp32 or bf16 (both the same);
     the kernels index the slots themselves, nothing is gathered or scattered around the call.
 
+    ``cu_seqlens``: the kernels take the boundaries from what the tensor holds when they run.  Its lengths are also read
+    on the host, once per tensor and content version, for the context-parallel plan, the extent of ``h`` and the check
+    of the token count.  A write that the version counter does not see (a graph replay, a raw kernel, ``.data``) may
+    move boundaries as long as the numbers of sequences, tokens and, with ``output_h``, chunks stay the same and the
+    call is not cut into segments (``cp.plan_segments``); for anything else pass a new tensor or write through torch.
+
     Output norm (the gated RMS norm that follows the op in a GDN layer): with ``out_norm_gate`` ``z``
     ``[B,T,Hv,128]`` (q/k/v dtype) and ``out_norm_weight`` ``[128]`` the returned ``o`` is
     ``o * rsqrt(mean(o^2, -1) + out_norm_eps) * weight * silu(z)``, applied to the output tile inside the scan
@@ -228,20 +234,22 @@ def chunk_gated_delta_rule_fwd(
 
 
 def _lengths(q, v, cu_seqlens, auto_cp):
-    """``(plan | None, chunk tables | None, start order | None, number of chunks)`` of a call's sequences."""
+    """``(plan | None, start order | None, number of chunks)`` of a call's sequences."""
     B, T, Hv = q.shape[0], q.shape[1], v.shape[2]
     if cu_seqlens is None:
         plan = cp.get_plan([T] * B, Hv, q.device) if auto_cp and q.is_cuda else None
-        return (plan.native if plan is not None else None), None, None, B * ((T + CHUNK - 1) // CHUNK)
-    if host_seqlens(cu_seqlens, total_tokens=B * T) is None or not q.is_cuda:
-        return None, None, None, 0
+        return (plan.native if plan is not None else None), None, B * ((T + CHUNK - 1) // CHUNK)
+    host_seqlens(cu_seqlens, total_tokens=B * T)
+    if not q.is_cuda:
+        return None, None, 0
     batch = packed_batch(cu_seqlens, q.device)
     plan = None
     if auto_cp:
         plan = batch.plans.get(Hv)
         if plan is None:
             plan = batch.plans[Hv] = cp.get_plan(batch.lens, Hv, q.device)
-    return (plan.native if plan is not None else None), batch.tables, batch.order, batch.chunks
+    native = plan.native if plan is not None else None
+    return native, batch.order if native is None else None, batch.chunks
 
 
 def _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_state, output_h, auto_cp, output_v_new,
@@ -251,9 +259,9 @@ def _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_st
     not asked for)."""
     host = _cabi.host()
     host.chunk_check(q, k, v, g, beta, None if h0_indices is not None else initial_state, cu_seqlens, transposed)
-    plan, tables, order, chunks = _lengths(q, v, cu_seqlens, auto_cp)
-    return host.chunk_fwd(q, k, v, g, beta, scale, initial_state, h0_indices, cu_seqlens, tables, order, chunks,
-                          output_final_state, output_h, output_v_new, transposed, l2norm, A_log, dt_bias, beta_is_logit,
+    plan, order, chunks = _lengths(q, v, cu_seqlens, auto_cp)
+    return host.chunk_fwd(q, k, v, g, beta, scale, initial_state, h0_indices, cu_seqlens, order, chunks, output_final_state,
+                          output_h, output_v_new, transposed, l2norm, A_log, dt_bias, beta_is_logit,
                           fs_out, fs_indices, norm_gate, norm_weight, norm_eps, plan, cp.INLINE_WARMUP)
 
 
@@ -282,8 +290,8 @@ def chunk_gated_delta_rule_bwd(
     oracle's convention, tests/ref_gdr.py:378)."""
     host = _cabi.host()
     host.chunk_check(q, k, v, g, beta, initial_state, cu_seqlens, transpose_state_layout)
-    plan, tables, _, chunks = _lengths(q, v, cu_seqlens, auto_cp)
-    return host.chunk_bwd(q, k, v, g, beta, A, do, dht, scale, initial_state, cu_seqlens, tables, chunks, h, v_new,
+    plan, _, chunks = _lengths(q, v, cu_seqlens, auto_cp)
+    return host.chunk_bwd(q, k, v, g, beta, A, do, dht, scale, initial_state, cu_seqlens, chunks, h, v_new,
                           transpose_state_layout, w, plan, cp.INLINE_WARMUP)
 
 

@@ -12,6 +12,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/types.h>
 
+#include <algorithm>
 #include <array>
 
 #include "../../include/flashqla_b200.h"
@@ -243,6 +244,11 @@ py::tuple chunk_check_py(const Tensor& q, const Tensor& k, const Tensor& v, cons
 }
 
 int64_t chunks_of(int64_t tokens) { return (tokens + 63) / 64; }
+// Chunk states of a packed batch.  The storage has room for as many chunks as any `seqs` intervals of `tokens` can have:
+// the scan numbers chunks by what cu_seqlens holds when it runs, `n_chunks` is what it held when its lengths were read.
+Tensor new_h(int64_t n_chunks, int64_t tokens, int64_t seqs, int64_t heads, at::ScalarType dtype, const at::Device& dev) {
+  return new_tensor({std::max(n_chunks, tokens / 64 + seqs), heads, 128, 128}, dtype, dev).narrow(0, 0, n_chunks);
+}
 
 // Plan (+ start states) -> warm-up and transition passes (one launch) -> chaining, on the segments of `plan`; `a` is
 // filled for the main scan.  The scratch holds, per segment and head, the two limits and the warm-up lengths, the
@@ -284,29 +290,22 @@ void use_tables(QlaChunkFwdArgs& a, const Tensor& tables) {
   a.workspace_bytes = tables.nbytes();
   a.flags |= QLA_CHUNK_TABLES_READY;
 }
-// The chunk tables of the caller's cu_seqlens: the ready ones, except in a captured graph, where a launch of the graph
-// derives them from what cu_seqlens holds at each replay.  The returned tensor keeps the workspace alive.
-bool capturing(void* stream) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
-}
-Tensor set_tables(QlaChunkFwdArgs& a, const OptTensor& tables, const at::Device& dev, void* stream) {
-  if (!tables.has_value()) return Tensor();
-  if (!capturing(stream)) {
-    use_tables(a, *tables);
-    return *tables;
-  }
+// Workspace for the chunk tables of the caller's cu_seqlens, which a launch of the call derives from what the tensor holds
+// then: a table kept from an earlier call would be stale after a write that no version counter sees (a graph replay, a raw
+// kernel).  The returned tensor keeps the workspace alive.
+Tensor table_workspace(QlaChunkFwdArgs& a, const at::Device& dev) {
+  if (a.cu_seqlens == nullptr) return Tensor();
   Tensor ws = new_tensor({static_cast<int64_t>(qla_chunk_fwd_workspace_bytes(&a))}, at::kByte, dev);
   a.workspace = ws.data_ptr();
   a.workspace_bytes = ws.nbytes();
   return ws;
 }
 
-// The raw forward (chunk.chunk_gated_delta_rule_fwd says what the arguments mean).  `tables` are the ready chunk
-// tables of cu_seqlens, `order` the order in which its sequences are started, `plan` the context-parallel plan or None.
+// The raw forward (chunk.chunk_gated_delta_rule_fwd says what the arguments mean).  `order` is the order in which the
+// sequences of cu_seqlens are started, `plan` the context-parallel plan or None.
 py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_,
                     std::optional<double> scale, const OptTensor& initial_state, const OptTensor& initial_state_indices,
-                    const OptTensor& cu_seqlens, const OptTensor& tables, const OptTensor& order, int64_t n_chunks,
+                    const OptTensor& cu_seqlens, const OptTensor& order, int64_t n_chunks,
                     bool output_final_state, bool output_h, bool output_v_new, bool transposed, bool l2norm,
                     const OptTensor& A_log_, const OptTensor& dt_bias_, bool beta_is_logit, const OptTensor& final_state_out,
                     const OptTensor& final_state_indices, const OptTensor& norm_gate, const OptTensor& norm_weight,
@@ -373,7 +372,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   const Tensor w = new_tensor({B, T, Hv, 128}, dtype, dev), o = at::empty_like(v);
   Tensor h, v_new, rnorm, beta_act, final_state, A_log, dt_bias;
   if (output_h)
-    h = cu.defined() ? new_tensor({1, n_chunks, Hv, 128, 128}, dtype, dev) : new_tensor({B, chunks_of(T), Hv, 128, 128}, dtype, dev);
+    h = cu.defined() ? new_h(n_chunks, T, N, Hv, dtype, dev).unsqueeze(0) : new_tensor({B, chunks_of(T), Hv, 128, 128}, dtype, dev);
   if (output_v_new) v_new = at::empty_like(v);
   if (l2norm) rnorm = new_tensor({B, T, Hk, 2}, at::kFloat, dev);
   if (final_state_out.has_value()) final_state = *final_state_out;
@@ -402,7 +401,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     // g_cumsum, A and w on the original sequences, then per-segment initial states, then the scan over segments
     // (segments are whole chunks, so chunk numbering is unchanged)
     a.flags = QLA_CHUNK_PREPARE_ONLY | norm_flag | act_flags;
-    const Tensor ws = set_tables(a, tables, dev, stream);
+    const Tensor ws = table_workspace(a, dev);
     check(qla_chunk_fwd(&a, stream), "qla_chunk_fwd");
     if (beta_is_logit) {  // every later stage reads the activated values
       a.beta = a.beta_out;
@@ -431,7 +430,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     check(qla_chunk_fwd(&b, stream), "qla_chunk_fwd");
   } else {
     a.flags = layout | norm_flag | act_flags | out_flag;
-    const Tensor ws = set_tables(a, tables, dev, stream);
+    const Tensor ws = table_workspace(a, dev);
     a.seq_order = ptr<int32_t>(order);  // packed batches of unequal lengths: the longest sequences start first
     a.h0 = ptr(h0); a.h0_map = ptr<int32_t>(h0_map); a.seq_map = ptr<int32_t>(fs_map);
     a.o = ptr(o); a.h = ptr(h); a.v_new = ptr(v_new); a.final_state = ptr(final_state);
@@ -445,7 +444,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
 // The raw backward (chunk.chunk_gated_delta_rule_bwd): `g_` is the cumulative gate of the forward.
 py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, const Tensor& A_,
                     const Tensor& do_, const OptTensor& dht_, std::optional<double> scale_, const OptTensor& initial_state,
-                    const OptTensor& cu_seqlens, const OptTensor& tables, int64_t n_chunks, const OptTensor& h_,
+                    const OptTensor& cu_seqlens, int64_t n_chunks, const OptTensor& h_,
                     const OptTensor& v_new_, bool transposed, const OptTensor& w_, const Plan* plan, bool inline_warmup) {
   const Sizes s = chunk_check(q_, k_, v_, g_, beta_, initial_state, cu_seqlens, transposed);
   const at::Device dev = q_.device();
@@ -468,7 +467,7 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     QlaChunkFwdArgs a{};
     const bool scan = !h.defined() || !v_new.defined(), have_w = w.defined();
     if (scan) {
-      h = new_tensor({n_chunks, Hv, 128, 128}, dtype, dev);
+      h = cu.defined() ? new_h(n_chunks, T, s.N, Hv, dtype, dev) : new_tensor({n_chunks, Hv, 128, 128}, dtype, dev);
       v_new = at::empty_like(v);
     }
     if (!have_w) w = new_tensor({B, T, Hv, 128}, dtype, dev);
@@ -484,7 +483,7 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     } else {
       a.flags |= QLA_CHUNK_PREPARE_ONLY;
     }
-    const Tensor ws = set_tables(a, tables, dev, stream);
+    const Tensor ws = table_workspace(a, dev);
     check(qla_chunk_fwd(&a, stream), "qla_chunk_fwd");
   }
   w = contiguous(w); h = contiguous(h); v_new = contiguous(v_new);
@@ -500,7 +499,6 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   a.v_new = ptr(v_new); a.w = ptr(w); a.d_o = ptr(d_o); a.dht = ptr<float>(dht); a.cu_seqlens = ptr<int32_t>(cu);
   a.dq = ptr(dq); a.dk = ptr(dk); a.dv = ptr(dv); a.dbeta = ptr<float>(db); a.dg = ptr<float>(dg); a.dh0 = ptr<float>(dh0);
   a.status = status_word(dev);
-  if (tables.has_value() && !capturing(stream)) a.tables = ptr<int32_t>(*tables);
   SegmentScratch sc;
   if (plan != nullptr) {
     // Long sequences on few heads: the reverse scan runs over the same segments as the forward's.  Plan (reverse:

@@ -187,29 +187,31 @@ def host_seqlens(cu_seqlens: torch.Tensor, total_tokens: Optional[int] = None) -
 
 
 class PackedBatch:
-    """What the chunked op needs to know about one ``cu_seqlens``, derived once: the lengths, the number of 64-token
-    chunks, and on ``device`` (one upload) the chunk tables and the order in which the sequences are started."""
-    __slots__ = ("lens", "chunks", "tables", "order", "plans")
+    """What the host needs to know about one ``cu_seqlens``, derived once: the lengths, the number of 64-token chunks and
+    the order in which the sequences are started.  The chunk tables are not among it: the kernels read the boundaries
+    from the live tensor, and tables of an older content would send chunks to the wrong sequences, so every call derives
+    them on the device."""
+    __slots__ = ("lens", "chunks", "plans", "device", "_order")
 
     def __init__(self, cu_seqlens: torch.Tensor, device: torch.device):
-        self.lens = lens = host_seqlens(cu_seqlens)
+        self.lens = host_seqlens(cu_seqlens)
+        self.chunks = sum((n + 63) // 64 for n in self.lens)
         self.plans = {}  # context-parallel plan per head count (cp.get_plan), so that a call does not hash the lengths
-        pair, chunk = [0], [0]
-        for n in lens:
-            pair.append(pair[-1] + (n + 127) // 128)
-            chunk.append(chunk[-1] + (n + 63) // 64)
-        self.chunks = chunk[-1]
-        pad = [0] * (-len(pair) % 4)  # [n + 1] int32 tables, each padded to 16 bytes: qla_chunk_fwd's workspace
-        host = pair + pad + chunk + pad
-        size = len(host)
-        # Packed batches of unequal lengths: the longest chains start first instead of forming the tail.
-        unequal = len(lens) > 1 and min(lens) != max(lens)
-        if unequal:
-            host = host + sorted(range(len(lens)), key=lambda i: -lens[i])
-        # a blocking copy: the tables are complete before any stream can use them
-        dev = torch.tensor(host, dtype=torch.int32).to(device)
-        self.tables = dev[:size]
-        self.order = dev[size:] if unequal else None
+        self.device = device
+        self._order = False  # not asked for yet
+
+    @property
+    def order(self) -> Optional[torch.Tensor]:
+        """Int32 permutation on the device that lists the sequences longest first (the longest chains then start first
+        instead of forming the tail), or ``None`` when that changes nothing (one sequence, equal lengths)."""
+        if self._order is False:
+            lens = self.lens
+            self._order = None
+            if len(lens) > 1 and min(lens) != max(lens):
+                idx = sorted(range(len(lens)), key=lambda i: -lens[i])
+                # a blocking copy: complete before any stream can use it
+                self._order = torch.tensor(idx, dtype=torch.int32).to(self.device)
+        return self._order
 
 
 def packed_batch(cu_seqlens: torch.Tensor, device: torch.device) -> PackedBatch:

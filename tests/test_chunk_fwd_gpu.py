@@ -378,3 +378,25 @@ def test_cp_warmup_inside_the_scan_equals_the_separate_pass(fq, gate_div, zero_g
     ref = orc.chunk_gdr_fwd(inp["q"], inp["k"], inp["v"], inp["g"], inp["beta"], h0=inp["h0"])
     _check("o", a[2], ref["o"])
     _check("h", a[3], ref["h"])
+
+
+def test_boundaries_are_those_cu_seqlens_holds_at_the_call(fq):
+    """A persistent cu_seqlens rewritten by something its version counter does not see (a graph replay, a raw kernel; here
+    through ``.data``), same number of sequences and tokens, two chunks more: forward and backward follow what it holds."""
+    c = _cuda(orc.make_prefill_inputs(1, 900, 2, 4, seed=71, with_h0=True, n_states=3, with_grads=True))
+    old, new = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, 192, 832, 900], [0, 65, 450, 900]))
+    leaves = [c[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")]
+
+    def run(cu):
+        o, fs = fq.chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True, cu_seqlens=cu)
+        with torch.no_grad():
+            plain = fq.chunk_gated_delta_rule(*leaves[:5], initial_state=leaves[5], output_final_state=True, cu_seqlens=cu)
+        return [o, fs, *plain, *torch.autograd.grad([o, fs], leaves, [c["do"], c["dht"]])]
+
+    run(old)
+    version = old._version
+    old.data.copy_(new)
+    assert old._version == version
+    for x, y in zip(run(old), run(new)):
+        assert torch.equal(x, y)
+    fq.check_device_status()
