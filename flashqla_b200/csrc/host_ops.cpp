@@ -7,6 +7,7 @@
 // messages) are those of the Python functions that call this module.
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/utils/pybind.h>
@@ -83,6 +84,11 @@ void check(int code, const char* what) {
   raise(py::module_::import("flashqla_b200._cabi").attr("QlaError").ptr(), msg);
 }
 void* current_stream(const at::Device& dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
+// A tensor of this package that is kept between calls (start order, plan) was allocated on the stream of the call that made
+// it: its memory must not go back to that stream while a kernel of this one may still read it.
+void used_here(const Tensor& t) {
+  c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(t.get_device()));
+}
 
 // ------------------------------------------------------------------------------------------------ recurrent op
 Tensor recurrent_update(const OptTensor& A_log_, const Tensor& a_, const OptTensor& dt_bias_, const Tensor& q_, const Tensor& k_,
@@ -398,6 +404,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   if (final_state.defined() || h0.has_value()) a.state_dtype = dtype_code(final_state.defined() ? final_state : *h0);
 
   if (plan != nullptr) {
+    used_here(plan->cu);  // (every table of a plan lies in one allocation)
     // g_cumsum, A and w on the original sequences, then per-segment initial states, then the scan over segments
     // (segments are whole chunks, so chunk numbering is unchanged)
     a.flags = QLA_CHUNK_PREPARE_ONLY | norm_flag | act_flags;
@@ -431,6 +438,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   } else {
     a.flags = layout | norm_flag | act_flags | out_flag;
     const Tensor ws = table_workspace(a, dev);
+    if (order.has_value()) used_here(*order);
     a.seq_order = ptr<int32_t>(order);  // packed batches of unequal lengths: the longest sequences start first
     a.h0 = ptr(h0); a.h0_map = ptr<int32_t>(h0_map); a.seq_map = ptr<int32_t>(fs_map);
     a.o = ptr(o); a.h = ptr(h); a.v_new = ptr(v_new); a.final_state = ptr(final_state);
@@ -505,6 +513,7 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     // decay accumulated from a segment's START; rows of the last segments take the caller's dht) -> one launch of
     // the scan in state-only mode over the leading chunks of every segment together with the transition matrices
     // -> reverse chaining.
+    used_here(plan->cu);
     sc = segment_scratch(*plan, Hv, dev, inline_warmup);
     segment_plan(*plan, sc, Hv, a.g_cumsum, dht, nullptr, transposed, true, stream);
     QlaChunkBwdArgs b{};

@@ -400,3 +400,33 @@ def test_boundaries_are_those_cu_seqlens_holds_at_the_call(fq):
     for x, y in zip(run(old), run(new)):
         assert torch.equal(x, y)
     fq.check_device_status()
+
+
+@pytest.mark.parametrize("cut", [False, True])
+def test_kept_tables_are_not_reused_under_another_stream(fq, monkeypatch, cut):
+    """The start order and the plan of a packed batch belong to the stream that made them.  Dropped while a call on another
+    stream has still to run, their memory does not go back to the first stream's next allocations."""
+    from flashqla_b200 import cp, utils
+    lens = [3000, 100] if cut else [500, 100, 300]
+    bounds = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    c = _cuda(orc.make_prefill_inputs(1, bounds[-1], 1, 2, seed=72))
+    monkeypatch.setattr(cp, "_PLAN_CACHE", {i: None for i in range(256)})  # full: only the batch keeps its plan
+    monkeypatch.setattr(utils, "_BATCH_CACHE", {})
+    cu = torch.tensor(bounds, dtype=torch.int32, device="cuda")
+    run = lambda: fq.chunk_gated_delta_rule(c["q"], c["k"], c["v"], c["g"], c["beta"], cu_seqlens=cu)
+    run()
+    batch = utils.packed_batch(cu, cu.device)
+    kept = batch.plans[2].dev["tables"] if cut else batch.order
+    ptr, size = kept.data_ptr(), kept.untyped_storage().nbytes()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(int(1e9))
+        run()
+    del kept, batch, cu
+    utils._BATCH_CACHE.clear()
+    new = [torch.empty(size, dtype=torch.uint8, device="cuda") for _ in range(5000)]
+    waiting = not side.query()
+    torch.cuda.synchronize()
+    assert waiting and ptr not in [t.data_ptr() for t in new]
+    fq.check_device_status()
