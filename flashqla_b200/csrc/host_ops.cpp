@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 
 #include "../../include/flashqla_b200.h"
 
@@ -24,7 +25,11 @@ using OptTensor = std::optional<Tensor>;
 
 namespace {
 
+// The entry points release the GIL (py::gil_scoped_release): torch's allocator and launches may block, and a host callback
+// or another Python thread may be what they wait for.  What needs the interpreter takes it back: exceptions, the first look
+// at a device's status word, and the result tuple.
 [[noreturn]] void raise(PyObject* type, const std::string& msg) {
+  py::gil_scoped_acquire gil;
   PyErr_SetString(type, msg.c_str());
   throw py::error_already_set();
 }
@@ -68,12 +73,16 @@ Tensor new_tensor(at::IntArrayRef size, at::ScalarType dtype, const at::Device& 
 // The int32 word the kernels of a device report faults to.  It belongs to flashqla_b200.utils, which also reads it;
 // the reference kept here is never dropped, so that nothing touches the device when the process ends.
 int32_t* status_word(const at::Device& dev) {
-  static Tensor* words[64] = {};
+  static std::atomic<int32_t*> words[64];
   const int i = dev.index();
   TORCH_CHECK(i >= 0 && i < 64, "device index out of range");
-  if (words[i] == nullptr)
-    words[i] = new Tensor(py::module_::import("flashqla_b200.utils").attr("device_status")(py::cast(dev)).cast<Tensor>());
-  return words[i]->data_ptr<int32_t>();
+  int32_t* word = words[i].load();
+  if (word == nullptr) {
+    py::gil_scoped_acquire gil;
+    word = (new Tensor(py::module_::import("flashqla_b200.utils").attr("device_status")(py::cast(dev)).cast<Tensor>()))->data_ptr<int32_t>();
+    words[i].store(word);
+  }
+  return word;
 }
 
 void check(int code, const char* what) {
@@ -81,6 +90,7 @@ void check(int code, const char* what) {
   const std::string msg = std::string(what) + ": " + qla_status_string(code) + ": " + qla_last_error();
   if (code == QLA_ERR_INVALID_ARG) value_error(msg);
   if (code == QLA_ERR_UNSUPPORTED) raise(PyExc_NotImplementedError, msg);
+  py::gil_scoped_acquire gil;
   raise(py::module_::import("flashqla_b200._cabi").attr("QlaError").ptr(), msg);
 }
 void* current_stream(const at::Device& dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
@@ -97,6 +107,7 @@ Tensor recurrent_update(const OptTensor& A_log_, const Tensor& a_, const OptTens
                         const OptTensor& cu_seqlens, bool disable_state_update, const OptTensor& inter,
                         const OptTensor& inter_indices, std::optional<int64_t> cache_steps, const OptTensor& parent_token,
                         std::optional<int64_t> block_dv, bool assume_regular, bool b_is_beta, bool a_is_log_decay) {
+  py::gil_scoped_release nogil;
   const Tensor q = contiguous(q_), k = contiguous(k_), v = contiguous(v_), a = contiguous(a_);
   Tensor b = contiguous(b_);
   const int64_t NT = q.size(1), Hk = q.size(2), K = q.size(3), Hv = v.size(2), V = v.size(3);
@@ -185,6 +196,7 @@ Tensor recurrent_update(const OptTensor& A_log_, const Tensor& a_, const OptTens
 
 void state_commit(const Tensor& state, const Tensor& inter, const Tensor& num_accepted, const OptTensor& state_indices,
                   const OptTensor& inter_indices) {
+  py::gil_scoped_release nogil;
   if (inter.dim() != 5 || inter.size(3) != 128 || inter.size(4) != 128)
     value_error("intermediate_states_buffer must be [slots, steps, HV, 128, 128]");
   const int64_t Hv = inter.size(2), elems = Hv * 128 * 128;
@@ -316,6 +328,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
                     const OptTensor& A_log_, const OptTensor& dt_bias_, bool beta_is_logit, const OptTensor& final_state_out,
                     const OptTensor& final_state_indices, const OptTensor& norm_gate, const OptTensor& norm_weight,
                     double norm_eps, const Plan* plan, bool inline_warmup) {
+  py::gil_scoped_release nogil;
   const Sizes s = chunk_check(q_, k_, v_, g_, beta_, initial_state_indices.has_value() ? OptTensor() : initial_state, cu_seqlens,
                               transposed);
   if (A_log_.has_value() != dt_bias_.has_value()) value_error("A_log and dt_bias go together");
@@ -445,6 +458,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     a.norm_gate = ptr(gate); a.norm_weight = ptr<float>(weight); a.norm_eps = norm_eps;
     check(qla_chunk_fwd(&a, stream), "qla_chunk_fwd");
   }
+  py::gil_scoped_acquire gil;
   auto opt = [](const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); };
   return py::make_tuple(g_cumsum, A, o, opt(h), opt(final_state), opt(v_new), w, opt(rnorm), opt(beta_act));
 }
@@ -454,7 +468,9 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
                     const Tensor& do_, const OptTensor& dht_, std::optional<double> scale_, const OptTensor& initial_state,
                     const OptTensor& cu_seqlens, int64_t n_chunks, const OptTensor& h_,
                     const OptTensor& v_new_, bool transposed, const OptTensor& w_, const Plan* plan, bool inline_warmup) {
+  py::gil_scoped_release nogil;
   const Sizes s = chunk_check(q_, k_, v_, g_, beta_, initial_state, cu_seqlens, transposed);
+  if (!q_.is_cuda()) value_error("flashqla_b200 requires CUDA tensors");
   const at::Device dev = q_.device();
   const auto dtype = q_.scalar_type();
   const Tensor q = contiguous(q_), k = contiguous(k_), v = contiguous(v_), beta = contiguous(beta_), A = contiguous(A_);
@@ -533,12 +549,14 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   a.workspace = ws.data_ptr();
   a.workspace_bytes = bytes;
   check(qla_chunk_bwd(&a, stream), "qla_chunk_bwd");
+  py::gil_scoped_acquire gil;
   return py::make_tuple(dq, dk, dv, db, dg, dh0.defined() ? py::cast(dh0) : py::none());
 }
 
 // ------------------------------------------------------------------------------------------------ layer prologue, backward
 // Normalised q and k (16-bit, as l2norm gives them) for the backward of a forward that folded the norm in.
 py::tuple l2norm_pair(const Tensor& q_, const Tensor& k_) {
+  py::gil_scoped_release nogil;
   const Tensor q = contiguous(q_), k = contiguous(k_);
   c10::cuda::OptionalCUDAGuard guard(q.device());
   const Tensor qn = at::empty_like(q), kn = at::empty_like(k);
@@ -546,6 +564,7 @@ py::tuple l2norm_pair(const Tensor& q_, const Tensor& k_) {
   a.rows = q.numel() / 128; a.qkv_dtype = dtype_code(q); a.eps = 1e-6f;
   a.q = ptr(q); a.k = ptr(k); a.qn = ptr(qn); a.kn = ptr(kn);
   check(qla_layer_bwd(&a, current_stream(q.device())), "qla_layer_bwd");
+  py::gil_scoped_acquire gil;
   return py::make_tuple(qn, kn);
 }
 
@@ -554,6 +573,7 @@ py::tuple l2norm_pair(const Tensor& q_, const Tensor& k_) {
 py::tuple layer_bwd(const OptTensor& q_, const OptTensor& k_, const OptTensor& dq, const OptTensor& dk, const OptTensor& a_in_,
                     const OptTensor& A_log_, const OptTensor& dt_bias_, const Tensor& dg, const OptTensor& b_in,
                     const OptTensor& beta_act, const Tensor& db) {
+  py::gil_scoped_release nogil;
   const at::Device dev = dg.device();
   c10::cuda::OptionalCUDAGuard guard(dev);
   QlaLayerBwdArgs a{};
@@ -585,6 +605,7 @@ py::tuple layer_bwd(const OptTensor& q_, const OptTensor& k_, const OptTensor& d
     a.beta_dtype = dtype_code(dbr); a.beta = ptr<float>(beta_act); a.db = ptr<float>(db); a.db_raw = ptr(dbr);
   }
   check(qla_layer_bwd(&a, current_stream(dev)), "qla_layer_bwd");
+  py::gil_scoped_acquire gil;
   auto opt = [](const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); };
   return py::make_tuple(opt(da), opt(dA), opt(ddt), opt(dbr));
 }

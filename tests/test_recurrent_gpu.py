@@ -424,3 +424,37 @@ def test_against_the_reference_kernel_on_this_gpu(fq, mode):
         assert torch.equal(pool_m, c["state"]) and torch.equal(pool_r, c["state"])
         tol = STATE_TOL if inter_dt == torch.float32 else 8e-3  # two bf16 roundings of |S| ~ 1
         assert float((inter_r.float() - inter_m.float()).abs().max()) <= tol
+
+
+def test_other_threads_run_while_a_launch_waits(fq):
+    """A call whose launch has to wait (the stream's queue is full behind a long kernel) does not hold the interpreter."""
+    import threading
+    import time
+    q, k, v = (torch.randn(1, 1, h, 128, device="cuda", dtype=torch.bfloat16) for h in (2, 2, 4))
+    gate, pool = torch.rand(1, 1, 4, device="cuda"), torch.zeros(1, 4, 128, 128, device="cuda")
+    run = lambda: fq.fused_sigmoid_gating_delta_rule_update(None, -gate, None, q, k, v, gate, pool, a_is_log_decay=True,
+                                                            b_is_beta=True)
+    run()
+    torch.cuda.synchronize()
+    done, gap = threading.Event(), [0.0]
+
+    def beat():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gap[0] = max(gap[0], now - last)
+            last = now
+
+    other = threading.Thread(target=beat)
+    other.start()
+    torch.cuda._sleep(int(1.5e9))
+    start = time.perf_counter()
+    for _ in range(3000):  # more than a stream queues
+        run()
+    waited = time.perf_counter() - start
+    done.set()
+    other.join()
+    torch.cuda.synchronize()
+    fq.check_device_status()
+    assert waited > 0.4 and gap[0] < 0.25 * waited, (waited, gap)
