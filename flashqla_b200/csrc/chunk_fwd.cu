@@ -897,8 +897,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::tc_fence_before_sync();
         warp_arrive(&bars[kVdReady], lane);
         if (warp == 0) trace(1, i, 3);
-        // off the critical path: Vd itself, 16 bit, into the other 16 columns of its half (A operand of MMA4)
-        if (!kStateOnly || kAux) {
+        // off the critical path: Vd itself, 16 bit, into the other 16 columns of its half (A operand of MMA4, source of
+        // v_new).  Only where one of them waits for it: MMAu of the next chunk, which overwrites D2, is held back by them.
+        if (!kStateOnly || (kAux && p.v_new != nullptr)) {
           uint32_t vd[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) vd[j] = pack2<T>(__uint_as_float(d[2 * j]), __uint_as_float(d[2 * j + 1]));

@@ -430,3 +430,22 @@ def test_kept_tables_are_not_reused_under_another_stream(fq, monkeypatch, cut):
     torch.cuda.synchronize()
     assert waiting and ptr not in [t.data_ptr() for t in new]
     fq.check_device_status()
+
+
+@pytest.mark.parametrize("T,Hk,Hv", [(64 * 40 + 5, 2, 4), (70, 1, 1)])
+def test_state_only_scan_with_and_without_v_new(fq, T, Hk, Hv):
+    """A state-only scan may be asked for h alone: the same states as together with v_new."""
+    from flashqla_b200 import _cabi
+    from flashqla_b200.chunk import _launch_fwd
+    c = _cuda(orc.make_prefill_inputs(1, T, Hk, Hv, seed=73, with_h0=True))
+    g_cs, A, *_, w = fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], output_w=True)
+    got = []
+    for with_v_new in (True, False):
+        h = torch.full(((T + 63) // 64, Hv, 128, 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        fs = torch.empty(1, Hv, 128, 128, device="cuda")
+        _launch_fwd(None, c["k"], c["v"], None, c["beta"], c["h0"], None, g_cs, A, None, h,
+                    torch.empty_like(c["v"]) if with_v_new else None, fs, 1.0,
+                    flags=_cabi.CHUNK_STATE_ONLY | _cabi.CHUNK_SKIP_PREPARE, w=w)
+        got.append((h, fs))
+    fq.check_device_status()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
