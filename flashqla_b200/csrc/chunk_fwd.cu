@@ -702,16 +702,18 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::fence_proxy_async_smem();
         warp_arrive(&bars[kONormed], lane);
       }
-      if (valid == kChunk) {
-        if (warp == 12) {  // only the issuing warp waits for the tile to be complete
+      if (valid == kChunk || valid == 0) {
+        // Only the issuing warp waits for the tile to be complete, in a warm-up chunk too: the wait is also what keeps it
+        // from arriving on kOFree twice while another output warp has still to look at the first arrival.
+        if (warp == 12) {
           if (!wait(kTileDone, j & 1)) break;
-          if (lane == 0) {
+          if (lane == 0 && valid > 0) {
             ptx::tma_store_4d(&tm_o, so, 0, hv, t0, 0);
             ptx::tma_store_commit();
           }
           __syncwarp();
         }
-      } else if (valid > 0) {
+      } else {
         if (!wait(kTileDone, j & 1)) break;
         // ragged tail (always the last chunk of a sequence): row-masked 16-byte stores, 16 threads per row
         T* ob = static_cast<T*>(p.o);

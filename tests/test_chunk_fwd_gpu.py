@@ -449,3 +449,19 @@ def test_state_only_scan_with_and_without_v_new(fq, T, Hk, Hv):
         got.append((h, fs))
     fq.check_device_status()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("out", ["o", "h", "norm"])
+def test_warmup_chunks_repeat_bitwise(fq, out):
+    """Segments with several warm-up chunks each (decay of about -2 per chunk), 300 runs: bit-identical, no wait given up."""
+    T = 2048 + 70
+    c = _cuda(orc.make_prefill_inputs(1, T, 1, 2, seed=74, with_h0=True, gate_div=25.0))
+    kw = {"o": {}, "h": dict(output_h=True),
+          "norm": dict(out_norm_gate=torch.randn_like(c["v"]), out_norm_weight=torch.ones(128, device="cuda"))}[out]
+    bad, first = torch.zeros((), dtype=torch.int32, device="cuda"), None
+    for _ in range(300):
+        _, _, o, h, fs = fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], initial_state=c["h0"], **kw)
+        first = first or (o, fs)
+        bad += (o != first[0]).any().int() + (fs != first[1]).any().int()
+    fq.check_device_status()
+    assert int(bad) == 0
