@@ -178,6 +178,8 @@ extern "C" QLA_API int qla_layer_bwd(const QlaLayerBwdArgs* args, void* stream_)
     const int rc = a.qkv_dtype == QLA_DT_BF16 ? launch_rows<__nv_bfloat16>(a, stream) : launch_rows<__half>(a, stream);
     if (rc != QLA_OK) return rc;
   }
+  if (a.tokens == 0 && a.dsums != nullptr && a.num_v_heads > 0)  // the sums over no tokens
+    QLA_CHECK_CUDA(cudaMemsetAsync(a.dsums, 0, 2 * sizeof(float) * a.num_v_heads, stream));
   if (a.tokens == 0 || (a.da == nullptr && a.db_raw == nullptr)) return QLA_OK;
   QLA_CHECK_ARG(a.num_v_heads > 0, "num_v_heads must be positive");
   QLA_CHECK_ARG(a.da == nullptr || (a.a && a.A_log && a.dt_bias && a.dg && a.dsums && a.workspace), "NULL gate tensor");
