@@ -36,16 +36,21 @@ extern "C" QLA_API int qla_abi_version(void) { return QLA_ABI_VERSION; }
 
 namespace qla {
 namespace {
-// One warp waits, with the bounded wait every kernel of the library uses, for a barrier phase that nothing
-// will ever complete: the wait gives up after `limit_ns`, records barrier / parity / warp in the status word
-// and the kernel returns normally.
+// One warp waits, in both forms that the kernels of the library use, for a barrier phase that nothing will ever
+// complete: each wait gives up after `limit_ns` and its failure is recorded (that of the form that issues MMAs in a word
+// of its own; the status word gets barrier / parity / warp only when both were), and the kernel returns normally.
 __global__ void bounded_wait_selftest_kernel(int* status, unsigned long long limit_ns) {
   __shared__ uint64_t bar;
+  __shared__ int issuer_word;
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bar, 1);
     ptx::fence_mbar_init();
+    issuer_word = 0;
   }
   __syncthreads();
+  ptx::report_issuer(&issuer_word, ptx::mbar_wait_nocall(ptx::smem_u32(&bar), 0, true, limit_ns), 254);
+  __syncthreads();
+  if ((issuer_word & 0xffff) != (kStatusBarrierTimeout | (254 << 8))) return;
   const bool ok = ptx::mbar_wait_polling(&bar, 0, status, kStatusBarrierTimeout | (255 << 8), limit_ns);
   if (ok && status != nullptr) atomicCAS(status, 0, kStatusBadIndex);  // cannot happen: nobody arrives
 }

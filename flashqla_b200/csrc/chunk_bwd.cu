@@ -484,6 +484,7 @@ bwd_chunk_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if ((w >> 16) != kNoBar) ptx::umma_commit(&bars[w >> 16]);
       }
     }
+    ptx::report_issuer(p.status, ok, 128 + kNumBars);
   } else if (warp == kReduceWarp) {
     // =========================================================== sums of a step
     // It releases the slot of a step (partial sums, description) as one of the arrivals that let the next step's early tiles

@@ -466,6 +466,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         if (i >= 0) trace(0, i, 8);
       }
+      ptx::report_issuer(p.status, ok, kNumBars);
     }
   } else if (warp >= 16) {
     // =========================================================== Pg = s * G .* P

@@ -180,14 +180,20 @@ __device__ __forceinline__ bool mbar_wait_addr(uint32_t addr, uint32_t parity) {
 }
 
 // The wait of a warp that issues MMAs: no call.  Uniform registers do not survive a call, so that with one anywhere in the
-// issuing loop every descriptor lives in ordinary registers and is moved over for each instruction (26 instructions and 100
-// cycles per MMA instead of 8 and the tensor pipe's own time).  Bounded like the others; `alive` false: one poll.
-__device__ __forceinline__ bool mbar_wait_nocall(uint32_t addr, uint32_t parity, bool alive) {
+// issuing loop every descriptor lives in ordinary registers and is moved over for each instruction.  Bounded like the others,
+// but it reports nothing itself: the issuing warp does so behind its loop (report_issuer), where it costs the loop nothing.
+// `alive` false: one poll.
+__device__ __forceinline__ bool mbar_wait_nocall(uint32_t addr, uint32_t parity, bool alive,
+                                                 unsigned long long limit_ns = kWaitLimitNs) {
   if (mbar_try_wait_addr(addr, parity)) return alive;
-  const unsigned long long until = global_timer_ns() + (alive ? kWaitLimitNs : 0ull);
+  const unsigned long long until = global_timer_ns() + (alive ? limit_ns : 0ull);
   while (!mbar_try_wait_addr(addr, parity))
     if (global_timer_ns() > until) return false;
   return alive;
+}
+// `num_bars` (one past the kernel's last barrier) stands for "one of the issuer's waits".
+__device__ __forceinline__ void report_issuer(int* status, bool alive, int num_bars) {
+  if (!alive) record_wait_failure(status, kStatusBarrierTimeout | (num_bars << 8), 0);
 }
 
 __device__ __forceinline__ float ex2(float x) {  // 2^x, approximate (the MUFU behind __expf)

@@ -153,8 +153,9 @@ def _cache_get(cache: Dict, key: Tuple, cu_seqlens: torch.Tensor):
 
 
 def selftest_bounded_wait(device=None, limit_ms: float = 20.0) -> None:
-    """Launch the library's self-test kernel whose only wait can never complete: after ``limit_ms`` the bounded
-    wait gives up and records the fault in the device status word, which ``check_device_status`` then raises."""
+    """Launch the library's self-test kernel, which waits in both forms of the bounded wait for what can never come: after
+    ``limit_ms`` each gives up and records the fault, in the end in the device status word, which ``check_device_status``
+    then raises."""
     from . import _cabi
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     st = device_status(dev)
