@@ -10,6 +10,7 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _cabi, cp
 from .utils import device_status, host_seqlens, packed_batch
@@ -375,6 +376,13 @@ class ChunkGatedDeltaRuleFusedFunction(torch.autograd.Function):
         return (dq, dk, dv, da, db_raw, dA_log, ddt, None, dh0, None, None, None, None, None, None)
 
 
+def _transformed() -> bool:
+    """Whether forward-mode differentiation, a torch.func transform or a trace is active: they have to see an autograd
+    function (which refuses what it cannot do, and is what a trace records), not a call past autograd."""
+    return (forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None
+            or torch._C._functorch.maybe_current_level() is not None)
+
+
 @torch.compiler.disable
 def chunk_gated_delta_rule(
     q: torch.Tensor,
@@ -423,7 +431,8 @@ def chunk_gated_delta_rule(
     needs_grad = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad
         for t in (q, k, v, g, beta, initial_state, A_log, dt_bias, output_norm_gate, output_norm_weight))
-    if not needs_grad:
+    plain = not fused and output_norm_gate is None
+    if not needs_grad and not (plain and _transformed()):
         # inference: normalisation, activations and the output norm are folded into the kernels (no extra passes)
         out = _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_state, False, True, False,
                        transpose_state_layout, use_qk_l2norm_in_kernel, A_log if use_gate_in_kernel else None,

@@ -465,3 +465,23 @@ def test_warmup_chunks_repeat_bitwise(fq, out):
         bad += (o != first[0]).any().int() + (fs != first[1]).any().int()
     fq.check_device_status()
     assert int(bad) == 0
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning", "ignore::DeprecationWarning")
+def test_function_transforms_and_traces_without_gradients(fq):
+    """Forward-mode tangents and torch.func transforms are refused, not dropped, and a trace of the plain op computes it."""
+    import torch.autograd.forward_ad as fwAD
+    c = _cuda(orc.make_prefill_inputs(1, 130, 1, 2, seed=75))
+    op = lambda q: fq.chunk_gated_delta_rule(q, c["k"], c["v"], c["g"], c["beta"])[0]
+    with fwAD.dual_level():
+        with pytest.raises(NotImplementedError, match="jvp"):
+            op(fwAD.make_dual(c["q"], torch.ones_like(c["q"])))
+        assert torch.equal(op(c["q"]), fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"])[2])
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.func.jvp(op, (c["q"],), (torch.ones_like(c["q"]),))
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.vmap(op)(torch.stack([c["q"], c["q"]]))
+    traced = torch.jit.trace(op, (c["q"],), check_trace=False)
+    other = c["q"].flip(1).contiguous()
+    assert torch.equal(traced(other), op(other))
+    fq.check_device_status()
