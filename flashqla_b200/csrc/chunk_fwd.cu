@@ -776,6 +776,8 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int h0_row = p.h0_map != nullptr ? p.h0_map[seq] : seq;
     const bool h0_16 = st16 && !p.h0_kv;
     const bool h0_vk = p.transpose_state && !p.h0_kv;  // rows of h0 are [V][K]
+    // [V][K] states move in 16-byte pieces where the caller's tensor starts on 16 bytes, one by one where it does not
+    const bool h0_vec = (reinterpret_cast<uintptr_t>(p.h0) & 15u) == 0, fs_vec = (reinterpret_cast<uintptr_t>(final_state) & 15u) == 0;
     const int64_t h0_off = (static_cast<int64_t>(h0_row) * p.num_v_heads + hv) * kHeadDim * kHeadDim;
     const bool has_h0 = !init_identity && p.h0 != nullptr && h0_row >= 0 && lead == 0;
     const float* h0p = (has_h0 && !h0_16) ? static_cast<const float*>(p.h0) + h0_off : nullptr;
@@ -783,19 +785,22 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // 16 values k0 .. k0 + 15 of state column v: [V][K] rows in 16-byte pieces, [K][V] one coalesced store per k
     auto store_final16 = [&](int k0, const uint32_t (&x)[16]) {
       if (!kState16 || fs_out != nullptr) {
-        if (p.transpose_state) {
+        if (p.transpose_state && fs_vec) {
           float4* dst = reinterpret_cast<float4*>(fs_out + v * kHeadDim + k0);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             dst[j] = make_float4(__uint_as_float(x[4 * j]), __uint_as_float(x[4 * j + 1]), __uint_as_float(x[4 * j + 2]),
                                  __uint_as_float(x[4 * j + 3]));
+        } else if (p.transpose_state) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) fs_out[v * kHeadDim + k0 + j] = __uint_as_float(x[j]);
         } else {
           float* dst = fs_out + k0 * kHeadDim + v;
 #pragma unroll
           for (int j = 0; j < 16; ++j) dst[j * kHeadDim] = __uint_as_float(x[j]);
         }
       } else if (fs_out16 != nullptr) {
-        if (p.transpose_state) {
+        if (p.transpose_state && fs_vec) {
           uint4* dst = reinterpret_cast<uint4*>(fs_out16 + v * kHeadDim + k0);
 #pragma unroll
           for (int j = 0; j < 2; ++j)
@@ -803,6 +808,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                                 pack2<__nv_bfloat16>(__uint_as_float(x[8 * j + 2]), __uint_as_float(x[8 * j + 3])),
                                 pack2<__nv_bfloat16>(__uint_as_float(x[8 * j + 4]), __uint_as_float(x[8 * j + 5])),
                                 pack2<__nv_bfloat16>(__uint_as_float(x[8 * j + 6]), __uint_as_float(x[8 * j + 7])));
+        } else if (p.transpose_state) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) fs_out16[v * kHeadDim + k0 + j] = __float2bfloat16_rn(__uint_as_float(x[j]));
         } else {
           __nv_bfloat16* dst = fs_out16 + k0 * kHeadDim + v;
 #pragma unroll
@@ -821,6 +829,10 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const float* src = h0p + col_half * kHeadDim + v;
 #pragma unroll
         for (int j = 0; j < 64; ++j) x[j] = src[j * kHeadDim];
+      } else if (h0p != nullptr && !h0_vec) {
+        const float* src = h0p + v * kHeadDim + col_half;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) x[j] = src[j];
       } else if (h0p != nullptr) {  // [V][K]: 16-byte pieces of row v
         const float4* src = reinterpret_cast<const float4*>(h0p + v * kHeadDim + col_half);
 #pragma unroll
@@ -832,6 +844,10 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const __nv_bfloat16* src = h0p16 + col_half * kHeadDim + v;
 #pragma unroll
         for (int j = 0; j < 64; ++j) x[j] = __bfloat162float(src[j * kHeadDim]);
+      } else if (kState16 && h0p16 != nullptr && !h0_vec) {
+        const __nv_bfloat16* src = h0p16 + v * kHeadDim + col_half;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) x[j] = __bfloat162float(src[j]);
       } else if (kState16 && h0p16 != nullptr) {
         const uint4* src = reinterpret_cast<const uint4*>(h0p16 + v * kHeadDim + col_half);
 #pragma unroll

@@ -485,3 +485,29 @@ def test_function_transforms_and_traces_without_gradients(fq):
     other = c["q"].flip(1).contiguous()
     assert torch.equal(traced(other), op(other))
     fq.check_device_status()
+
+
+@pytest.mark.parametrize("T", [130, 2048 + 70])  # uncut, and cut into segments
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_states_that_do_not_start_on_16_bytes(fq, T, dtype, transposed):
+    """Pools (in and out) at an offset of one element: bitwise what an aligned pool gives."""
+    c = _cuda(orc.make_prefill_inputs(1, T, 1, 2, seed=76, with_h0=True))
+    rows = torch.tensor([1], dtype=torch.int32, device="cuda")
+    got = []
+    for offset in (0, 1):
+        flat = torch.zeros(3 * 2 * 128 * 128 + 16, dtype=dtype, device="cuda")
+        pool = flat[offset:offset + 3 * 2 * 128 * 128].view(3, 2, 128, 128)
+        assert (pool.data_ptr() % 16 == 0) == (offset == 0) and pool.is_contiguous()
+        pool[1] = c["h0"][0]
+        out = fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], initial_state=pool,
+                                            initial_state_indices=rows, final_state_out=pool, final_state_indices=rows,
+                                            transpose_state_layout=transposed)
+        got.append((out[2], pool))
+        if dtype == torch.float32:  # the plain argument as well
+            plain = fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], initial_state=pool[1:2],
+                                                  transpose_state_layout=transposed)
+            got[-1] += (plain[2], plain[4])
+    fq.check_device_status()
+    assert not torch.equal(got[0][1][1], c["h0"][0].to(dtype))
+    assert all(torch.equal(x, y) for x, y in zip(*got))
