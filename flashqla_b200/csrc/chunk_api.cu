@@ -125,6 +125,8 @@ extern "C" QLA_API int qla_chunk_fwd(const QlaChunkFwdArgs* args, void* stream_)
   fp.zero_v = (a.flags & QLA_CHUNK_ZERO_V) ? 1 : 0;
   const bool out_norm = (a.flags & QLA_CHUNK_OUT_GATED_RMSNORM) != 0;
   QLA_CHECK_ARG(!out_norm || (a.norm_gate && a.norm_weight), "QLA_CHUNK_OUT_GATED_RMSNORM needs norm_gate and norm_weight");
+  QLA_CHECK_ARG(!out_norm || ((reinterpret_cast<uintptr_t>(a.norm_gate) | reinterpret_cast<uintptr_t>(a.norm_weight)) & 15u) == 0,
+                "norm_gate and norm_weight must start on 16 bytes");
   QLA_CHECK_SUPPORTED(!out_norm || (!state_only && a.h == nullptr && a.v_new == nullptr),
                       "the output norm is an inference epilogue: not with QLA_CHUNK_STATE_ONLY, h or v_new");
   QLA_CHECK_SUPPORTED(a.state_dtype != QLA_DT_BF16 || (!state_only && !out_norm && a.h == nullptr && a.v_new == nullptr),

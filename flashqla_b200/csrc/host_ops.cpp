@@ -61,6 +61,7 @@ T* ptr(const Tensor& t) {
   return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr;
 }
 Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+Tensor aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 ? t : t.clone(); }
 Tensor as(const Tensor& t, const at::Device& dev, at::ScalarType dtype) {
   if (t.scalar_type() == dtype && t.device() == dev) return contiguous(t);
   return t.to(dev, dtype).contiguous();
@@ -377,11 +378,11 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   }
   Tensor gate, weight;
   if (norm_gate.has_value()) {
-    if (!norm_weight.has_value() || norm_gate->sizes() != v.sizes() || norm_gate->scalar_type() != v.scalar_type())
+    if (!norm_weight.has_value() || norm_weight->numel() < 128 || norm_gate->sizes() != v.sizes() || norm_gate->scalar_type() != v.scalar_type())
       value_error("out_norm_gate must have v's shape and dtype and needs out_norm_weight [128]");
     if (output_h || output_v_new) value_error("the output norm is an inference epilogue: not with output_h / output_v_new");
-    gate = contiguous(*norm_gate);
-    weight = as(*norm_weight, dev, at::kFloat);
+    gate = aligned16(contiguous(*norm_gate));
+    weight = aligned16(as(*norm_weight, dev, at::kFloat));
   }
 
   c10::cuda::OptionalCUDAGuard guard(dev);

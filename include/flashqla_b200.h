@@ -223,8 +223,9 @@ typedef struct QlaChunkFwdArgs {
   const int32_t* chunk_limit_b; /* QLA_CHUNK_DUAL_TRANSITION: chunk limits [N,Hv] of the second pass  */
   const int32_t* seq_map_b;     /* QLA_CHUNK_DUAL_TRANSITION: output rows [N] of the second pass      */
   float* final_state_b;         /* QLA_CHUNK_DUAL_TRANSITION: fp32 [rows,Hv,128,128] out              */
-  const void* norm_gate;        /* QLA_CHUNK_OUT_GATED_RMSNORM: z [B,T,Hv,128] in the q/k/v dtype     */
-  const float* norm_weight;     /* QLA_CHUNK_OUT_GATED_RMSNORM: fp32 [128]                            */
+  const void* norm_gate;        /* QLA_CHUNK_OUT_GATED_RMSNORM: z [B,T,Hv,128] in the q/k/v dtype,
+                                   from a 16-byte boundary                                          */
+  const float* norm_weight;     /* QLA_CHUNK_OUT_GATED_RMSNORM: fp32 [128], the same                  */
   float norm_eps;
   int32_t reserved2;
   const int32_t* lead;          /* [num_seqs, Hv] or NULL: chunks in FRONT of an interval (tokens of the interval

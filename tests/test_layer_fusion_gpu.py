@@ -54,6 +54,20 @@ def test_output_gated_rmsnorm_epilogue(B, T, Hk, Hv, cu):
     assert torch.equal(o_pub, o_fused)
 
 
+def test_output_norm_gate_and_weight_at_odd_offsets():
+    """Gate and weight that do not start on 16 bytes (the kernel reads 16-byte pieces): the same result."""
+    import flashqla_b200 as fq
+    c = {n: t.cuda() for n, t in orc.make_prefill_inputs(1, 130, 1, 2, seed=62).items()}
+    z, weight = torch.randn(1, 130, 2, 128, device="cuda").bfloat16(), torch.rand(128, device="cuda")
+    shift = lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+    run = lambda z, w: fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], out_norm_gate=z, out_norm_weight=w)[2]
+    assert shift(z).data_ptr() % 16 == 2 and shift(weight).data_ptr() % 16 == 4
+    assert torch.equal(run(shift(z), shift(weight)), run(z, weight))
+    with pytest.raises(ValueError, match="out_norm_weight"):
+        run(z, weight[:64])
+    fq.check_device_status()
+
+
 def test_fused_prologue_under_autograd():
     import flashqla_b200 as fq
     B, T, Hk, Hv = 2, 330, 2, 4
