@@ -112,7 +112,7 @@ Tensor recurrent_update(const OptTensor& A_log_, const Tensor& a_, const OptTens
   const Tensor q = contiguous(q_), k = contiguous(k_), v = contiguous(v_), a = contiguous(a_);
   Tensor b = contiguous(b_);
   const int64_t NT = q.size(1), Hk = q.size(2), K = q.size(3), Hv = v.size(2), V = v.size(3);
-  if (Hv % Hk != 0) value_error("num_value_heads must be divisible by num_key_heads");
+  if (Hk == 0 || Hv % Hk != 0) value_error("num_value_heads must be divisible by num_key_heads");
   if (K != 128 || V != 128) value_error("FlashQLA recurrent GDN kernel currently specializes Qwen GDN K=V=128");
   if (a.sizes() != at::IntArrayRef({1, NT, Hv})) value_error("a shape " + shape_str(a) + " does not match [1, total_tokens, HV]");
   if (b.sizes() != at::IntArrayRef({1, NT, Hv})) value_error("b shape " + shape_str(b) + " does not match [1, total_tokens, HV]");
@@ -201,6 +201,7 @@ void state_commit(const Tensor& state, const Tensor& inter, const Tensor& num_ac
   if (inter.dim() != 5 || inter.size(3) != 128 || inter.size(4) != 128)
     value_error("intermediate_states_buffer must be [slots, steps, HV, 128, 128]");
   const int64_t Hv = inter.size(2), elems = Hv * 128 * 128;
+  if (Hv == 0) value_error("intermediate_states_buffer has no heads");
   if (!state.is_contiguous() || !inter.is_contiguous())
     value_error("the state pool and intermediate_states_buffer must be contiguous");
   if ((state.scalar_type() != at::kFloat && state.scalar_type() != at::kBFloat16) || state.numel() % elems != 0)
@@ -236,7 +237,7 @@ Sizes chunk_check(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   require(q.dim() == 4 && k.sizes() == q.sizes() && v.dim() == 4, "q,k [B,T,Hk,K]; v [B,T,Hv,V]");
   Sizes s{q.size(0), q.size(1), q.size(2), v.size(2), q.size(0)};
   require(q.size(3) == 128 && v.size(3) == 128, "K = V = 128 only");
-  require(s.Hv % s.Hk == 0, "the number of v heads must be a multiple of the number of q/k heads");
+  require(s.Hk > 0 && s.Hv % s.Hk == 0, "the number of v heads must be a multiple of the number of q/k heads");
   const std::array<int64_t, 3> gates{s.B, s.T, s.Hv};
   require(g.sizes() == at::IntArrayRef(gates) && beta.sizes() == at::IntArrayRef(gates), "g, beta must be [B,T,Hv]");
   if (cu_seqlens.has_value()) {
@@ -587,7 +588,7 @@ py::tuple layer_bwd(const OptTensor& q_, const OptTensor& k_, const OptTensor& d
   }
   const int64_t Hv = dg.size(2);
   a.num_v_heads = Hv;
-  a.tokens = dg.numel() / Hv;
+  a.tokens = dg.size(0) * dg.size(1);
   if (a_in_.has_value()) {
     a_in = contiguous(*a_in_);
     A_log = as(*A_log_, dev, at::kFloat);

@@ -91,3 +91,21 @@ def test_chunk_tables_workspace_layout():
     t = ws.view(torch.int32)
     assert t[:6].tolist() == [0, 2, 3, 6, 7, 9]
     assert t[ws.numel() // 8:ws.numel() // 8 + 6].tolist() == [0, 4, 5, 11, 12, 15]
+
+
+def _native_update(q, v, a):
+    from flashqla_b200 import _cabi
+    return _cabi.host().recurrent_update(None, a, None, q, q, v, a, torch.zeros(1, v.shape[2], 128, 128), None, None, 1.0, 20.0,
+                                         True, None, False, None, None, None, None, None, False, True, True)
+
+
+def test_native_checks_survive_tensors_without_heads():
+    """A head count of zero is an error like any other, not a division by zero in native code (which ends the process)."""
+    from flashqla_b200 import _cabi
+    t = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="divisible"):
+        _native_update(t(1, 2, 0, 128), t(1, 2, 4, 128), t(1, 2, 4))
+    with pytest.raises(AssertionError, match="multiple"):
+        _cabi.host().chunk_check(t(1, 2, 0, 128), t(1, 2, 0, 128), t(1, 2, 4, 128), t(1, 2, 4), t(1, 2, 4), None, None, False)
+    with pytest.raises(ValueError, match="no heads"):
+        _cabi.host().state_commit(torch.zeros(1, 4, 128, 128), torch.zeros(1, 2, 0, 128, 128), torch.zeros(1), None, None)
