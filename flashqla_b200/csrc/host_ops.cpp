@@ -109,6 +109,9 @@ Tensor recurrent_update(const OptTensor& A_log_, const Tensor& a_, const OptTens
                         const OptTensor& inter_indices, std::optional<int64_t> cache_steps, const OptTensor& parent_token,
                         std::optional<int64_t> block_dv, bool assume_regular, bool b_is_beta, bool a_is_log_decay) {
   py::gil_scoped_release nogil;
+  if (q_.dim() != 4 || k_.dim() != 4 || v_.dim() != 4) value_error("q, k and v must be [1, total_tokens, heads, 128]");
+  if (k_.size(1) < q_.size(1) || k_.size(2) != q_.size(2) || k_.size(3) != q_.size(3) || v_.size(1) < q_.size(1))
+    value_error("k must have the shape of q, and v as many tokens");
   const Tensor q = contiguous(q_), k = contiguous(k_), v = contiguous(v_), a = contiguous(a_);
   Tensor b = contiguous(b_);
   const int64_t NT = q.size(1), Hk = q.size(2), K = q.size(3), Hv = v.size(2), V = v.size(3);
@@ -236,6 +239,7 @@ Sizes chunk_check(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   require(q.scalar_type() != at::kFloat, "ChunkGatedDeltaRuleFunction does not support float32. Please use bfloat16.");
   require(q.dim() == 4 && k.sizes() == q.sizes() && v.dim() == 4, "q,k [B,T,Hk,K]; v [B,T,Hv,V]");
   Sizes s{q.size(0), q.size(1), q.size(2), v.size(2), q.size(0)};
+  require(v.size(0) == s.B && v.size(1) >= s.T, "q,k [B,T,Hk,K]; v [B,T,Hv,V]");
   require(q.size(3) == 128 && v.size(3) == 128, "K = V = 128 only");
   require(s.Hk > 0 && s.Hv % s.Hk == 0, "the number of v heads must be a multiple of the number of q/k heads");
   const std::array<int64_t, 3> gates{s.B, s.T, s.Hv};

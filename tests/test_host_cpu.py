@@ -109,3 +109,15 @@ def test_native_checks_survive_tensors_without_heads():
         _cabi.host().chunk_check(t(1, 2, 0, 128), t(1, 2, 0, 128), t(1, 2, 4, 128), t(1, 2, 4), t(1, 2, 4), None, None, False)
     with pytest.raises(ValueError, match="no heads"):
         _cabi.host().state_commit(torch.zeros(1, 4, 128, 128), torch.zeros(1, 2, 0, 128, 128), torch.zeros(1), None, None)
+
+
+def test_native_checks_look_at_ranks_and_token_counts():
+    """q, k, v of another rank, and k or v with fewer tokens than q, are refused (they would be read past their end)."""
+    from flashqla_b200 import _cabi
+    t = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    for q, v in ((t(1, 2, 2, 128, 2), t(1, 2, 4, 128)), (t(1, 2, 2, 128), t(1, 2, 4, 128, 1)), (t(1, 2, 128), t(1, 2, 4, 128)),
+                 (t(1, 2, 2, 128), t(1, 1, 4, 128))):
+        with pytest.raises(ValueError, match="q, k and v must be|k must have"):
+            _native_update(q, v, t(1, 2, 4))
+    with pytest.raises(AssertionError, match="v .B,T,Hv,V."):
+        _cabi.host().chunk_check(t(1, 2, 2, 128), t(1, 2, 2, 128), t(1, 1, 4, 128), t(1, 2, 4), t(1, 2, 4), None, None, False)
