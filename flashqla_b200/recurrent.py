@@ -54,6 +54,8 @@ def fused_sigmoid_gating_delta_rule_update(
         raise ValueError("q, k, and v must have the same dtype")
     if not q.is_cuda:
         raise ValueError("FlashQLA recurrent GDN kernel requires CUDA tensors")
+    if a_is_log_decay:  # not used, whatever they are
+        A_log = dt_bias = None
     return _cabi.host().recurrent_update(
         A_log, a, dt_bias, q, k, v, b, initial_state_source, initial_state_indices, scale, softplus_beta,
         softplus_threshold, use_qk_l2norm_in_kernel, cu_seqlens, disable_state_update, intermediate_states_buffer,

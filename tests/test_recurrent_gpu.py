@@ -458,3 +458,16 @@ def test_other_threads_run_while_a_launch_waits(fq):
     torch.cuda.synchronize()
     fq.check_device_status()
     assert waited > 0.4 and gap[0] < 0.25 * waited, (waited, gap)
+
+
+def test_gate_parameters_are_ignored_with_log_decays(fq):
+    """With ``a_is_log_decay`` A_log and dt_bias are not looked at, tensors or not."""
+    q, k, v = (torch.randn(1, 3, h, 128, device="cuda", dtype=torch.bfloat16) for h in (2, 2, 4))
+    gate = torch.rand(1, 3, 4, device="cuda")
+    outs = []
+    for unused in (None, 0.0, torch.zeros(7)):
+        pool = torch.zeros(3, 4, 128, 128, device="cuda")
+        outs.append((fq.fused_sigmoid_gating_delta_rule_update(unused, -gate, unused, q, k, v, gate, pool, a_is_log_decay=True,
+                                                               b_is_beta=True), pool))
+    assert all(torch.equal(x, y) for got in outs[1:] for x, y in zip(got, outs[0]))
+    fq.check_device_status()
