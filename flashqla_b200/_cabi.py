@@ -174,7 +174,7 @@ _host = None
 
 def host():
     """The native host path of the tensor entry points (``csrc/host_ops.cpp``), loaded once.  Raises ``QlaError`` when it
-    has not been built."""
+    has not been built, or was built for another torch or Python."""
     global _host
     if _host is None:
         lib()  # the C-ABI library it links against
@@ -184,10 +184,21 @@ def host():
         from importlib.machinery import ExtensionFileLoader
         from importlib.util import module_from_spec, spec_from_loader
         loader = ExtensionFileLoader("_fq_host", str(path))
-        mod = module_from_spec(spec_from_loader("_fq_host", loader))
-        loader.exec_module(mod)
+        try:
+            mod = module_from_spec(spec_from_loader("_fq_host", loader))
+            loader.exec_module(mod)
+        except ImportError as e:
+            raise QlaError(f"{path} does not load here, rebuild it with `python -m flashqla_b200.build`: {e}") from e
+        _check_built_for_this_torch(mod)
         _host = mod
     return _host
+
+
+def _check_built_for_this_torch(mod) -> None:
+    here = torch.__version__.split("+")[0]
+    if mod.torch_version.split("+")[0] != here:
+        raise QlaError(f"the native host path was built for torch {mod.torch_version} and this is {here}: rebuild it with "
+                       "`python -m flashqla_b200.build`")
 
 
 def check(code: int, what: str) -> None:

@@ -42,12 +42,20 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
 
+def _torch_dir() -> Path:
+    from importlib.util import find_spec
+    return Path(find_spec("torch").submodule_search_locations[0])
+
+
 def _digest() -> str:
     h = hashlib.sha256()
     for f in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) +
                     [PKG.parent / "include" / "flashqla_b200.h", Path(__file__)]):
         h.update(f.name.encode())
         h.update(f.read_bytes())
+    # the host module is compiled against torch's C++ tensors and this interpreter
+    h.update(sys.implementation.cache_tag.encode())
+    h.update((_torch_dir() / "version.py").read_bytes())
     return h.hexdigest()
 
 
@@ -58,12 +66,11 @@ def is_current() -> bool:
 def _host_command() -> list[str]:
     """g++ command for the host module: torch's C++ tensors on one side, the C-ABI library on the other."""
     import sysconfig
-    from importlib.util import find_spec
-    torch_dir = Path(find_spec("torch").submodule_search_locations[0])
+    torch_dir = _torch_dir()
     cuda = Path(_nvcc()).resolve().parents[1]
     inc = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda / "include"]
-    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-shared", "-w",
-            *[f"-I{d}" for d in inc], f"-I{sysconfig.get_path('include')}", str(CSRC / "host_ops.cpp"), "-o", str(HOST_PATH),
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-shared", "-Wall",
+            "-Wextra", *[x for d in inc for x in ("-isystem", str(d))], "-isystem", sysconfig.get_path("include"), str(CSRC / "host_ops.cpp"), "-o", str(HOST_PATH),
             f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
             f"-L{LIB_DIR}", f"-l:{LIB_PATH.name}", f"-L{cuda / 'lib64'}", "-lcudart", "-Wl,-rpath,$ORIGIN"]
 

@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/utils/pybind.h>
 #include <torch/types.h>
+#include <torch/version.h>
 
 #include <algorithm>
 #include <array>
@@ -619,6 +620,7 @@ py::tuple layer_bwd(const OptTensor& q_, const OptTensor& k_, const OptTensor& d
 }  // namespace
 
 PYBIND11_MODULE(_fq_host, m) {
+  m.attr("torch_version") = TORCH_VERSION;  // (flashqla_b200._cabi.host compares it with the torch that is running)
   py::class_<Plan>(m, "Plan")
       .def(py::init([](Tensor cu, Tensor seg_next, Tensor seg_raw, Tensor raw_first, Tensor identity, Tensor seg_start_of,
                        Tensor seg_prev, Tensor tables, double threshold) {

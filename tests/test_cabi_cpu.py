@@ -107,3 +107,20 @@ def test_manifest_lists_every_kernel_with_its_cubin(built_lib):
             assert lib.qla_kernel_launch_info(k["kernel_name"].encode(), ctypes.byref(block), ctypes.byref(smem)) == 0
             assert block.value == 32 * k["num_warps"] and smem.value == k["shared"], k["kernel_name"]
     assert lib.qla_kernel_launch_info(b"no_such_kernel", ctypes.byref(block), ctypes.byref(smem)) == -1
+
+
+def test_another_torch_means_another_build(built_lib, tmp_path, monkeypatch):
+    """The host module is compiled against torch and Python: a build for others is neither current nor accepted."""
+    from types import SimpleNamespace
+    from flashqla_b200 import _cabi, build
+    assert build.is_current()
+    (tmp_path / "version.py").write_text("__version__ = '0.0'\n")
+    monkeypatch.setattr(build, "_torch_dir", lambda: tmp_path)
+    assert not build.is_current()
+    monkeypatch.undo()
+    monkeypatch.setattr("sys.implementation.cache_tag", "cpython-00")
+    assert not build.is_current()
+    monkeypatch.undo()
+    _cabi._check_built_for_this_torch(_cabi.host())
+    with pytest.raises(_cabi.QlaError, match="rebuild"):
+        _cabi._check_built_for_this_torch(SimpleNamespace(torch_version="0.0.0"))
