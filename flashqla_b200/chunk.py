@@ -160,13 +160,6 @@ def make_scan_only(q, k, v, beta, g_cumsum, A, o, final_state, initial_state=Non
     return run
 
 
-def forward_scan_only(q, k, v, beta, g_cumsum, A, o, final_state, initial_state=None, cu_seqlens=None,
-                      scale=None):
-    """Launch the chunk scan once over whole sequences (no context parallelism)."""
-    make_scan_only(q, k, v, beta, g_cumsum, A, o, final_state, initial_state, cu_seqlens, scale,
-                   auto_cp=False)()
-
-
 def chunk_gated_delta_rule_fwd(
     q: torch.Tensor,
     k: torch.Tensor,

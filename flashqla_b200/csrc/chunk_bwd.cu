@@ -45,7 +45,7 @@
 // Rows beyond the end of a sequence hold the next sequence's tokens (TMA does not know about sequences);
 // they never contribute because du, beta, rho and the ds rows of such tokens are exactly zero.
 #include "chunk_params.cuh"
-#include "mma_sync.cuh"
+#include "warp_pieces.cuh"
 
 namespace qla {
 namespace {

@@ -10,7 +10,7 @@
 //           K x K transition matrix M of the segment is needed as well.
 //   chain : for fallback entries  h0[seg + 1] += M[seg] * h0[seg], in segment order.
 #include "chunk_params.cuh"
-#include "mma_sync.cuh"
+#include "warp_pieces.cuh"
 
 namespace qla {
 namespace {

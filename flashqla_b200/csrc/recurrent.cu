@@ -12,7 +12,7 @@
 // rows in registers for the whole call (R*16 floats); the K-reductions (S.k and S.q) are three
 // xor-shuffles over the eight lanes of a row.  A CTA of 128 threads covers 16*R rows.
 #include "common.cuh"
-#include "mma_sync.cuh"
+#include "warp_pieces.cuh"
 
 namespace qla {
 namespace {

@@ -1,4 +1,4 @@
-// Warp-level pieces: ldmatrix, mma.sync m16n8k16 (16-bit inputs, fp32 accumulate) and cp.async.
+// Warp-level pieces: ldmatrix and cp.async.
 #pragma once
 
 #include "common.cuh"
@@ -21,28 +21,6 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t saddr) 
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(saddr)
                : "memory");
-}
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) { ldsm_x4(r, smem_addr(p)); }
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) { ldsm_x4_trans(r, smem_addr(p)); }
-
-template <typename T>
-__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                                          uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-template <>
-__device__ __forceinline__ void mma_16816<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // ---- cp.async (16-byte, L2 only); src_bytes = 0 zero-fills the destination
