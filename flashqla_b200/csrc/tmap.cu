@@ -28,10 +28,21 @@ int encode(CUtensorMap* out, const void* base, int rank, const cuuint64_t* dims,
     return QLA_ERR_INVALID_ARG;
   }
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = enc(out, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank,
-                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto make = [&]() {
+    return enc(out, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(base),
+               dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = make();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A thread that has not used the runtime yet (autograd's, when its allocations came from the cache) has no current
+    // context, and this is a driver call: selecting the device it is on brings the primary context about.
+    int dev = 0;
+    QLA_CHECK_CUDA(cudaGetDevice(&dev));
+    QLA_CHECK_CUDA(cudaSetDevice(dev));
+    r = make();
+  }
   if (r != CUDA_SUCCESS) {
     set_last_error("cuTensorMapEncodeTiled failed with CUresult %d (extents %llu x %llu x %llu)", static_cast<int>(r),
                    static_cast<unsigned long long>(dims[0]), static_cast<unsigned long long>(dims[1]),

@@ -511,3 +511,22 @@ def test_states_that_do_not_start_on_16_bytes(fq, T, dtype, transposed):
     fq.check_device_status()
     assert not torch.equal(got[0][1][1], c["h0"][0].to(dtype))
     assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
+def test_a_new_thread_has_a_context(fq):
+    """A thread whose first CUDA work is a call served from cached memory (as autograd's is in a later step): building the
+    tensor maps needs a context current in that thread, which no earlier call of it has brought about."""
+    import threading
+    c = _cuda(orc.make_prefill_inputs(1, 130, 1, 2, seed=77, with_h0=True, with_grads=True))
+    out = fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"], output_h=True, output_v_new=True, output_w=True)
+    forward = lambda: fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"])[2:3]
+    backward = lambda: fq.chunk_gated_delta_rule_bwd(c["q"], c["k"], c["v"], out[0], c["beta"], out[1], c["do"], h=out[3],
+                                                     v_new=out[5], w=out[6])[:5]
+    for call in (forward, backward):
+        want, got = [x.clone() for x in call()], []
+        torch.cuda.synchronize()
+        other = threading.Thread(target=lambda: got.extend(call()))
+        other.start()
+        other.join()
+        assert len(got) == len(want) and all(torch.equal(x, y) for x, y in zip(got, want))
+    fq.check_device_status()
