@@ -585,10 +585,12 @@ int launch_bwd_scan(const BwdParams& p, const BwdScanMode& mode, int64_t total_t
     if ((rc = make_tmap_3d(&tm_du, p.du, rows, 1, kChunk, 128, 64, true, is_bf16)) != QLA_OK) return rc;
   }
   const unsigned grid = static_cast<unsigned>(p.num_seqs) * p.num_v_heads * (mode.dual ? 2 : 1);
-  // The scan that stores du and dh is launched plainly.  Launched as a dependent its CTAs take the SMs in the order in which
-  // the kernel before it leaves them, and with one CTA per (sequence, head) on most but not all SMs that placement lasts for
-  // the whole scan: 4 x 8192 tokens of 32 heads (128 CTAs), forward and backward, 1965 us against 1876 us like this, while
-  // an early start is worth a few us.  The short state-only passes keep it.
+  // The scan that stores du and dh is launched plainly.  Forward and backward as a dependent / plainly, us, by CTAs: 96
+  // 193 / 188, 128 (4 x 4096 tokens) 988 / 952, 148 603 / 588, 160 724 / 706, 256 1020 / 988, 512 950 / 930, 1024
+  // 950 / 926; with 8 to 64 CTAs of short sequences the two are equal (the host is the bound there), and so at 512 CTAs of
+  // five chunks (336 / 340).  With up to one CTA per SM the order in which the kernel before leaves the SMs would decide
+  // a placement that lasts for the whole scan; why larger grids gain as well was not looked into.  The short state-only
+  // passes keep the early start.
   const bool dependent = mode.state_only != 0;
   if (is_bf16) {
     if ((rc = ensure_dynamic_smem<bwd_scan_kernel<__nv_bfloat16>>(kSmemBytes)) != QLA_OK) return rc;

@@ -27,8 +27,8 @@
 // What bounds it: that chain (about 1500 cycles of tensor-pipe time and hand-offs per chunk), and the traffic of
 // shared memory beside it: 72 KB of TMA writes and 112 KB of operand reads per chunk at 128 bytes a cycle.  Operands
 // that a thread produces therefore go to tensor memory (Vd as a shared-memory tile cost 48 KB per chunk), and Q K^T is
-// not stacked on other rows to fill M = 128.  All roles together execute 30 KB of code per chunk: the SM's
-// instruction cache holds 32 KB, and beyond it every line costs some 40 cycles.
+// not stacked on other rows to fill M = 128.  All roles share the SM's instruction cache (32 KB; 94 % of its requests hit),
+// so that code which is not needed costs even where it is not executed often: see kState16.
 // Thread v of a chain warpgroup owns TMEM lane v = column v of the state: it reads Vd^T rows
 // with tcgen05.ld, applies the gates, and writes the bf16 operand of the next MMA back with
 // tcgen05.st.  The fp32 state never leaves tensor memory between chunks.
@@ -185,7 +185,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   grid_dep_wait();    // earlier kernels of the stream have completed (see launch_dependent)
   grid_dep_launch();  // the next one may be scheduled; it waits the same way
   // (the shuffle tells the compiler that the role is the same for the whole warp: addresses, descriptors and loop
-  // counters of the single-warp roles then live in uniform registers, 10 % of the kernel's code)
+  // counters of the single-warp roles then live in uniform registers)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // A "dual" launch carries two passes over the same sequences in one grid: the CTAs of the second half run
   // the transition-matrix pass of context parallelism (start from the identity, V treated as zero) with their

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
     if (p.status != nullptr && threadIdx.x == 0) atomicCAS(p.status, 0, kStatusBadIndex);
   };
   // Work item -> (sequence, v-head, row tile) and the sequence's pool slot, looked up once, when the item's tile is
-  // requested (32-bit arithmetic: 64-bit divisions here were a quarter of a draft step's instructions).
+  // requested (32-bit arithmetic: 64-bit divisions are long sequences of instructions).
   struct Item {
     int n, h, tile;
     int64_t slot;
