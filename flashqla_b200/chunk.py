@@ -256,7 +256,7 @@ def _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_st
     plan, order, chunks = _lengths(q, v, cu_seqlens, auto_cp)
     return host.chunk_fwd(q, k, v, g, beta, scale, initial_state, h0_indices, cu_seqlens, order, chunks, output_final_state,
                           output_h, output_v_new, transposed, l2norm, A_log, dt_bias, beta_is_logit,
-                          fs_out, fs_indices, norm_gate, norm_weight, norm_eps, plan, cp.INLINE_WARMUP)
+                          fs_out, fs_indices, norm_gate, norm_weight, norm_eps, plan, cp.INLINE_WARMUP, cp.WARMUP_THRESHOLD)
 
 
 def chunk_gated_delta_rule_bwd(
@@ -286,7 +286,7 @@ def chunk_gated_delta_rule_bwd(
     host.chunk_check(q, k, v, g, beta, initial_state, cu_seqlens, transpose_state_layout)
     plan, _, chunks = _lengths(q, v, cu_seqlens, auto_cp)
     return host.chunk_bwd(q, k, v, g, beta, A, do, dht, scale, initial_state, cu_seqlens, chunks, h, v_new,
-                          transpose_state_layout, w, plan, cp.INLINE_WARMUP)
+                          transpose_state_layout, w, plan, cp.INLINE_WARMUP, cp.WARMUP_THRESHOLD)
 
 
 class ChunkGatedDeltaRuleFunction(torch.autograd.Function):

@@ -112,7 +112,7 @@ def get_plan(lens: Sequence[int], num_v_heads: int, device: torch.device) -> CpP
             plan.tables = {"ws": plan.dev["tables"].view(torch.uint8)}
             d = plan.dev
             plan.native = _cabi.host().Plan(d["cu"], d["seg_next"], d["seg_raw"], d["raw_first"], d["identity"],
-                                            d["seg_start_of"], d["seg_prev"], d["tables"], WARMUP_THRESHOLD)
+                                            d["seg_start_of"], d["seg_prev"], d["tables"])
         # Plans are never evicted: captured CUDA graphs and in-flight launches keep using a plan's device
         # tensors.  Past 256 distinct shapes new plans are simply not cached.
         if len(_PLAN_CACHE) < 256:

@@ -228,7 +228,6 @@ void state_commit(const Tensor& state, const Tensor& inter, const Tensor& num_ac
 struct Plan {
   Tensor cu, seg_next, seg_raw, raw_first, identity, seg_start_of, seg_prev, tables;
   int64_t num_segments, num_raw;
-  double threshold;
 };
 
 struct Sizes {
@@ -293,10 +292,10 @@ SegmentScratch segment_scratch(const Plan& p, int64_t Hv, const at::Device& dev,
   s.M = new_tensor({p.num_segments, Hv, 128, 128}, at::kFloat, dev);
   return s;
 }
-void segment_plan(const Plan& p, const SegmentScratch& s, int64_t Hv, const float* g_cumsum, const OptTensor& h0,
+void segment_plan(const Plan& p, double threshold, const SegmentScratch& s, int64_t Hv, const float* g_cumsum, const OptTensor& h0,
                   const int32_t* h0_map, bool h0_transposed, bool reverse, void* stream) {
   QlaCpPlanArgs a{};
-  a.num_segments = p.num_segments; a.num_v_heads = Hv; a.threshold = p.threshold; a.g_cumsum = g_cumsum;
+  a.num_segments = p.num_segments; a.num_v_heads = Hv; a.threshold = threshold; a.g_cumsum = g_cumsum;
   a.cu_seqlens = ptr<int32_t>(p.cu); a.seg_next = ptr<int32_t>(reverse ? p.seg_prev : p.seg_next);
   a.warm_limit = s.warm_limit; a.m_limit = s.m_limit; a.cp_h0 = s.h0.data_ptr<float>();
   a.seg_start_of = ptr<int32_t>(reverse ? p.seg_raw : p.seg_start_of); a.h0 = ptr(h0); a.h0_map = h0_map;
@@ -334,7 +333,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
                     bool output_final_state, bool output_h, bool output_v_new, bool transposed, bool l2norm,
                     const OptTensor& A_log_, const OptTensor& dt_bias_, bool beta_is_logit, const OptTensor& final_state_out,
                     const OptTensor& final_state_indices, const OptTensor& norm_gate, const OptTensor& norm_weight,
-                    double norm_eps, const Plan* plan, bool inline_warmup) {
+                    double norm_eps, const Plan* plan, bool inline_warmup, double threshold) {
   py::gil_scoped_release nogil;
   const Sizes s = chunk_check(q_, k_, v_, g_, beta_, initial_state_indices.has_value() ? OptTensor() : initial_state, cu_seqlens,
                               transposed);
@@ -435,7 +434,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
       a.beta_dtype = QLA_DT_F32;
     }
     const SegmentScratch sc = segment_scratch(*plan, Hv, dev, inline_warmup);
-    segment_plan(*plan, sc, Hv, a.g_cumsum, h0, ptr<int32_t>(h0_map), transposed, false, stream);
+    segment_plan(*plan, threshold, sc, Hv, a.g_cumsum, h0, ptr<int32_t>(h0_map), transposed, false, stream);
     // One launch, two passes: segment-end states from the trailing `warm_limit` chunks, written straight into the
     // successor's row, and the transition matrices of the (segment, head) pairs that never decayed below the threshold.
     QlaChunkFwdArgs b = a;
@@ -474,7 +473,8 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
 py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, const Tensor& A_,
                     const Tensor& do_, const OptTensor& dht_, std::optional<double> scale_, const OptTensor& initial_state,
                     const OptTensor& cu_seqlens, int64_t n_chunks, const OptTensor& h_,
-                    const OptTensor& v_new_, bool transposed, const OptTensor& w_, const Plan* plan, bool inline_warmup) {
+                    const OptTensor& v_new_, bool transposed, const OptTensor& w_, const Plan* plan, bool inline_warmup,
+                    double threshold) {
   py::gil_scoped_release nogil;
   const Sizes s = chunk_check(q_, k_, v_, g_, beta_, initial_state, cu_seqlens, transposed);
   if (!q_.is_cuda()) value_error("flashqla_b200 requires CUDA tensors");
@@ -538,7 +538,7 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     // -> reverse chaining.
     used_here(plan->cu);
     sc = segment_scratch(*plan, Hv, dev, inline_warmup);
-    segment_plan(*plan, sc, Hv, a.g_cumsum, dht, nullptr, transposed, true, stream);
+    segment_plan(*plan, threshold, sc, Hv, a.g_cumsum, dht, nullptr, transposed, true, stream);
     QlaChunkBwdArgs b{};
     b.batch = 1; b.seq_len = B * T; b.num_seqs = plan->num_segments; b.num_k_heads = Hk; b.num_v_heads = Hv;
     b.qkv_dtype = a.qkv_dtype; b.beta_dtype = QLA_DT_F32; b.flags = QLA_CHUNK_STATE_ONLY | QLA_CHUNK_DUAL_TRANSITION;
@@ -623,9 +623,9 @@ PYBIND11_MODULE(_fq_host, m) {
   m.attr("torch_version") = TORCH_VERSION;  // (flashqla_b200._cabi.host compares it with the torch that is running)
   py::class_<Plan>(m, "Plan")
       .def(py::init([](Tensor cu, Tensor seg_next, Tensor seg_raw, Tensor raw_first, Tensor identity, Tensor seg_start_of,
-                       Tensor seg_prev, Tensor tables, double threshold) {
+                       Tensor seg_prev, Tensor tables) {
         const int64_t n_seg = seg_next.numel(), n_raw = raw_first.numel() - 1;
-        return Plan{cu, seg_next, seg_raw, raw_first, identity, seg_start_of, seg_prev, tables, n_seg, n_raw, threshold};
+        return Plan{cu, seg_next, seg_raw, raw_first, identity, seg_start_of, seg_prev, tables, n_seg, n_raw};
       }));
   m.def("recurrent_update", &recurrent_update);
   m.def("state_commit", &state_commit);

@@ -530,3 +530,16 @@ def test_a_new_thread_has_a_context(fq):
         other.join()
         assert len(got) == len(want) and all(torch.equal(x, y) for x, y in zip(got, want))
     fq.check_device_status()
+
+
+def test_warmup_threshold_is_the_one_at_the_call(fq, monkeypatch):
+    """A plan is kept per list of lengths; the threshold of the warm-up is not part of it."""
+    from flashqla_b200 import cp
+    c = _cuda(orc.make_prefill_inputs(1, 2048, 1, 2, seed=78, gate_div=100.0))
+    run = lambda: fq.chunk_gated_delta_rule_fwd(c["q"], c["k"], c["v"], c["g"], c["beta"])[2].float()
+    o = run()
+    monkeypatch.setattr(cp, "WARMUP_THRESHOLD", 1.0)  # reached by the first chunk: a tail of one chunk of weak gates is kept
+    assert (run() - o).norm() > 0.05 * o.norm()
+    monkeypatch.undo()
+    assert torch.equal(run(), o)
+    fq.check_device_status()
