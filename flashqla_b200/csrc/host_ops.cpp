@@ -62,7 +62,7 @@ T* ptr(const Tensor& t) {
   return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr;
 }
 Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
-Tensor aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 ? t : t.clone(); }
+Tensor aligned(const Tensor& t, unsigned bytes) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & (bytes - 1)) == 0 ? t : t.clone(); }
 Tensor as(const Tensor& t, const at::Device& dev, at::ScalarType dtype) {
   if (t.scalar_type() == dtype && t.device() == dev) return contiguous(t);
   return t.to(dev, dtype).contiguous();
@@ -113,7 +113,7 @@ Tensor recurrent_update(const OptTensor& A_log_, const Tensor& a_, const OptTens
   if (q_.dim() != 4 || k_.dim() != 4 || v_.dim() != 4) value_error("q, k and v must be [1, total_tokens, heads, 128]");
   if (k_.size(1) < q_.size(1) || k_.size(2) != q_.size(2) || k_.size(3) != q_.size(3) || v_.size(1) < q_.size(1))
     value_error("k must have the shape of q, and v as many tokens");
-  const Tensor q = contiguous(q_), k = contiguous(k_), v = contiguous(v_), a = contiguous(a_);
+  const Tensor q = aligned(contiguous(q_), 8), k = aligned(contiguous(k_), 8), v = contiguous(v_), a = contiguous(a_);
   Tensor b = contiguous(b_);
   const int64_t NT = q.size(1), Hk = q.size(2), K = q.size(3), Hv = v.size(2), V = v.size(3);
   if (Hk == 0 || Hv % Hk != 0) value_error("num_value_heads must be divisible by num_key_heads");
@@ -386,8 +386,8 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     if (!norm_weight.has_value() || norm_weight->numel() < 128 || norm_gate->sizes() != v.sizes() || norm_gate->scalar_type() != v.scalar_type())
       value_error("out_norm_gate must have v's shape and dtype and needs out_norm_weight [128]");
     if (output_h || output_v_new) value_error("the output norm is an inference epilogue: not with output_h / output_v_new");
-    gate = aligned16(contiguous(*norm_gate));
-    weight = aligned16(as(*norm_weight, dev, at::kFloat));
+    gate = aligned(contiguous(*norm_gate), 16);
+    weight = aligned(as(*norm_weight, dev, at::kFloat), 16);
   }
 
   c10::cuda::OptionalCUDAGuard guard(dev);

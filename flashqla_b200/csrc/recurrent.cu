@@ -514,6 +514,13 @@ void launch_info_recurrent_kernel(int* block_threads, size_t* dynamic_smem_bytes
 }
 }  // namespace qla
 
+namespace qla {
+namespace {
+bool starts_on(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+constexpr const char* kAlignment = "q and k must start on 8 bytes, states and cached states on 16 (bf16 in the update: 8)";
+}  // namespace
+}  // namespace qla
+
 extern "C" QLA_API int qla_state_commit(const QlaStateCommitArgs* args, void* stream) {
   using namespace qla;
   QLA_CHECK_ARG(args != nullptr, "args is NULL");
@@ -525,6 +532,7 @@ extern "C" QLA_API int qla_state_commit(const QlaStateCommitArgs* args, void* st
   QLA_CHECK_SUPPORTED(a.inter_dtype == QLA_DT_F32 || a.inter_dtype == QLA_DT_BF16,
                       "intermediate_states_buffer must be fp32 or bf16");
   QLA_CHECK_SUPPORTED(a.state_dtype == QLA_DT_F32 || a.state_dtype == QLA_DT_BF16, "the state pool must be fp32 or bf16");
+  QLA_CHECK_ARG(starts_on(a.inter, 16) && starts_on(a.state, a.state_dtype == QLA_DT_BF16 ? 8 : 16), kAlignment);
   dim3 grid(a.num_seqs, a.num_v_heads);
   if (a.inter_dtype == QLA_DT_F32) state_commit_kernel<float><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
   else state_commit_kernel<__nv_bfloat16><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
@@ -553,6 +561,9 @@ extern "C" QLA_API int qla_recurrent_update(const QlaRecurrentArgs* args, void* 
   QLA_CHECK_ARG(a.state_slots > 0, "state_slots must be positive");
   QLA_CHECK_SUPPORTED(a.state_dtype == QLA_DT_F32 || a.state_dtype == QLA_DT_BF16,
                       "initial_state_source must be fp32 or bf16");
+  // (the pieces in which the kernel moves them)
+  QLA_CHECK_ARG(starts_on(a.q, 8) && starts_on(a.k, 8) && starts_on(a.state, a.state_dtype == QLA_DT_BF16 ? 8 : 16) &&
+                    starts_on(a.inter, a.inter_dtype == QLA_DT_BF16 ? 8 : 16), kAlignment);
   QLA_CHECK_ARG(a.parents == nullptr || a.parents_steps > 0, "parents_steps (second extent of parents) must be positive");
   QLA_CHECK_ARG(a.parents == nullptr || a.tokens_per_seq <= a.parents_steps,
                 "retrieve_parent_token has fewer columns than tokens per sequence");

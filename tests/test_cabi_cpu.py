@@ -124,3 +124,20 @@ def test_another_torch_means_another_build(built_lib, tmp_path, monkeypatch):
     _cabi._check_built_for_this_torch(_cabi.host())
     with pytest.raises(_cabi.QlaError, match="rebuild"):
         _cabi._check_built_for_this_torch(SimpleNamespace(torch_version="0.0.0"))
+
+
+@pytest.mark.parametrize("field,offset", [("q", 2), ("k", 4), ("state", 4), ("inter", 8)])
+def test_pointers_the_recurrent_kernels_cannot_read_are_refused(built_lib, field, offset):
+    """Tensors move in pieces of 8 or 16 bytes: a pointer between two pieces is an error before any launch."""
+    from flashqla_b200 import _cabi
+    ptrs = dict(q=4096, k=4096, v=4096, a=4096, b=4096, o=4096, state=4096, inter=4096, status=4096)
+    ptrs[field] += offset
+    a = _cabi.QlaRecurrentArgs(num_seqs=1, total_tokens=1, tokens_per_seq=1, num_k_heads=2, num_v_heads=2, qkv_dtype=1,
+                               flags=_cabi.REC_A_IS_LOG_DECAY | _cabi.REC_B_IS_BETA, state_slots=1, inter_slots=1, inter_steps=1, **ptrs)
+    assert _cabi.lib().qla_recurrent_update(a, None) == -1
+    assert b"start on" in _cabi.lib().qla_last_error()
+    if field in ("state", "inter"):
+        c = _cabi.QlaStateCommitArgs(num_seqs=1, num_v_heads=1, inter_steps=1, inter_slots=1, state_slots=1, accepted=4096,
+                                     inter=ptrs["inter"], state=ptrs["state"])
+        assert _cabi.lib().qla_state_commit(c, None) == -1
+        assert b"start on" in _cabi.lib().qla_last_error()

@@ -471,3 +471,18 @@ def test_gate_parameters_are_ignored_with_log_decays(fq):
                                                                b_is_beta=True), pool))
     assert all(torch.equal(x, y) for got in outs[1:] for x, y in zip(got, outs[0]))
     fq.check_device_status()
+
+
+def test_rows_and_pools_at_odd_offsets(fq):
+    """q and k at an offset of one element give the same result; a pool (updated in place) there is refused."""
+    q, k, v = (torch.randn(1, 3, h, 128, device="cuda", dtype=torch.bfloat16) for h in (2, 2, 4))
+    gate, base = torch.rand(1, 3, 4, device="cuda"), torch.randn(3, 4, 128, 128, device="cuda")
+    shift = lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+
+    def run(q, k, pool):
+        return fq.fused_sigmoid_gating_delta_rule_update(None, -gate, None, q, k, v, gate, pool, a_is_log_decay=True,
+                                                         b_is_beta=True), pool
+    assert all(torch.equal(x, y) for x, y in zip(run(shift(q), shift(k), base.clone()), run(q, k, base.clone())))
+    with pytest.raises(ValueError, match="start on"):
+        run(q, k, shift(base))
+    fq.check_device_status()
