@@ -65,6 +65,7 @@ def plan_segments(lens: Sequence[int], num_v_heads: int, num_sms: int = 148) -> 
         cost = rounds * (longest + WARMUP_COST * min(WARMUP_CHUNKS, longest))
         if best is None or cost < best:
             best, seg = cost, cand
+    # rounds of the longest sequence: too much for several unequal ones, which start longest first
     uncut = -(-chains // num_sms) * max(chunks)
     if best is None or best >= uncut:
         return CpPlan(use_cp=False)

@@ -579,7 +579,8 @@ extern "C" QLA_API int qla_recurrent_update(const QlaRecurrentArgs* args, void* 
   int rows = a.rows_per_cta;
   if (rows == 0) {
     // 32 rows per CTA keeps two independent rows in flight per thread; fall back to 16 rows while
-    // the grid would otherwise leave SMs idle (148 SMs, several CTAs each).
+    // the grid would otherwise leave SMs idle (148 SMs, several CTAs each).  (The line is drawn at four tiles per SM, not
+    // at what is resident of either height: 6 sequences of 16 heads are 768 tiles of 16 rows on 592 resident CTAs.)
     rows = (static_cast<int64_t>(a.num_seqs) * a.num_v_heads * 4 >= 4 * 148) ? 32 : 16;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
