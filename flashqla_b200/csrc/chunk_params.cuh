@@ -22,6 +22,8 @@ struct KktParams {
   int* status;
   int num_seqs, seq_len, num_k_heads, num_v_heads;
   int gate_dtype, beta_dtype;
+  // chosen by the launcher: pairs of chunks (equal lengths only), and the v-heads of a k-head over head_splits work items
+  int num_pairs, head_splits, heads_per_cta;
 };
 
 struct FwdParams {

@@ -324,6 +324,12 @@ __device__ __forceinline__ void tmem_ld_frag4(uint32_t taddr, uint32_t (&r)[16])
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld_frag2(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // The inverse of tmem_ld_frag4: the warp writes the fragments (tmem_wait_st before they are announced).
 __device__ __forceinline__ void tmem_st_frag4(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -448,6 +454,26 @@ __device__ __forceinline__ void umma_ss_k64(uint32_t d_tmem, uint64_t a_desc, ui
                ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate)),
                  "n"(A_STEP), "n"(B_STEP), "r"(commit1), "r"(commit2)
                : "memory");
+}
+// The same, M = 128, writing only the accumulator's lanes 0..63 whose bit of `mask_low` is clear and 64..127 of `mask_high`
+// (either mask serves two quadrants of 32 lanes).
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_ss_k64_lanes(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                  uint32_t mask_low, uint32_t mask_high, bool accumulate, uint32_t commit = 0) {
+#define QLA_UMMA_LANES_STEP                                                                                               \
+  "add.u32 alo, alo, %4; add.u32 blo, blo, %5; mov.b64 da, {alo, ahi}; mov.b64 db, {blo, bhi};\n"                          \
+  "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, {%6, %6, %7, %7}, t;\n"
+  asm volatile(
+      "{\n.reg .pred p, t, e, c1;\n.reg .b32 alo, ahi, blo, bhi;\n.reg .b64 da, db;\n"
+      "elect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %9, 0;\nsetp.eq.b32 t, 0, 0;\nsetp.ne.b32 c1, %8, 0;\nand.pred c1, c1, e;\n"
+      "mov.b64 {alo, ahi}, %1;\nmov.b64 {blo, bhi}, %2;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%6, %6, %7, %7}, p;\n"
+      QLA_UMMA_LANES_STEP QLA_UMMA_LANES_STEP QLA_UMMA_LANES_STEP
+      "@c1 tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%8];\n}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(A_STEP), "n"(B_STEP), "r"(mask_low), "r"(mask_high), "r"(commit),
+        "r"(static_cast<uint32_t>(accumulate))
+      : "memory");
+#undef QLA_UMMA_LANES_STEP
 }
 // The same with everything known at run time only: low words of both descriptors and their steps; `hi` is the high word.
 __device__ __forceinline__ void umma_ss_k64_steps(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc,

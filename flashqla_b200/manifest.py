@@ -52,9 +52,10 @@ KERNEL_RULES = {
         tensor_maps="A: 3-D (64, heads, tokens), box 64 x 1 x 64; q, k, v, w, o: 4-D (64 columns, heads, tokens, 2 halves), "
                     "box 64 x 1 x 64 x 2; 16-bit elements, 128B swizzle"),
     "kkt_solve_kernel": dict(
-        block=256, dynamic_smem=68608, cluster=1, grid="(pairs of 64-token chunks, Hk)",
+        block=128, dynamic_smem=71680, cluster=1, grid="(pairs of 64-token chunks) * Hk * (CTAs that share the v-heads of a k-head: head_splits)",
         params=[_TMAP + " k", _TMAP + " q", _TMAP + " A", _TMAP + " w", "KktParams (by value)"],
-        tensor_maps="3-D (width, heads, tokens), box 64 x 1 x 128 with 128B swizzle"),
+        tensor_maps="k, q, w: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 128 (w: 64) x 2; A: 3-D (64, heads, tokens), "
+                    "box 64 x 1 x 64; 16-bit elements, 128B swizzle"),
     "bwd_scan_kernel": dict(
         block=416, dynamic_smem=214016, cluster=1, grid="num_seqs * Hv (twice that for a dual state-only launch)",
         params=[_TMAP + " q", _TMAP + " k", _TMAP + " dO", _TMAP + " w", _TMAP + " dh (store)", _TMAP + " du (store)",

@@ -1,0 +1,59 @@
+"""The preparation kernel's own outputs, ``A`` and ``w``, against a triangular solve in 64 bits, where its work items can go wrong:
+sequences that end inside the first or second chunk of a pair (also many in a row), v-head groups that are spread over several
+items, and the in-kernel norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def solve(k, g, beta):
+    """``A [T, Hv, 64]`` and ``w [T, Hv, 128]`` of one sequence in 64 bits."""
+    T, Hk, Hv = k.shape[0], k.shape[1], g.shape[1]
+    A = torch.zeros(T, Hv, 64, dtype=torch.float64, device=k.device)
+    w = torch.zeros(T, Hv, 128, dtype=torch.float64, device=k.device)
+    for t0 in range(0, T, 64):
+        kk = k[t0:t0 + 64].repeat_interleave(Hv // Hk, 1).permute(1, 0, 2)
+        gc, b = g[t0:t0 + 64].cumsum(0).t(), beta[t0:t0 + 64].t()
+        n = kk.shape[1]
+        decay = torch.exp((gc[:, :, None] - gc[:, None, :]).tril())
+        L = (b[:, :, None] * decay * (kk @ kk.transpose(1, 2))).tril(-1)
+        eye = torch.eye(n, dtype=torch.float64, device=k.device)
+        X = torch.linalg.solve_triangular(eye + L, eye.expand(Hv, n, n), upper=False, unitriangular=True)
+        A[t0:t0 + n, :, :n] = X.permute(1, 0, 2)
+        w[t0:t0 + n] = -(X @ ((b * torch.exp(gc))[:, :, None] * kk)).permute(1, 0, 2)
+    return A, w
+
+
+@pytest.mark.parametrize("lens, heads, norm", [
+    ([1, 64, 65, 127, 128, 129, 63, 200], (2, 4), False),
+    ([40] * 700 + [300], (2, 2), False),        # several items per CTA, none of them with a second chunk
+    ([130, 3] * 300, (2, 4), True),
+    ([64 * 17 + 5], (1, 6), False),             # a small grid: the six v-heads as items of their own
+    ([777], (4, 8), True),
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_a_and_w(lens, heads, norm, dtype):
+    import flashqla_b200 as fq
+    gen = torch.Generator(device="cuda").manual_seed(len(lens))
+    T, (Hk, Hv) = sum(lens), heads
+    q, k, v = (torch.randn(1, T, n, 128, generator=gen, device="cuda") for n in (Hk, Hk, Hv))
+    if not norm:
+        k = torch.nn.functional.normalize(k, dim=-1)
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    g = torch.nn.functional.logsigmoid(torch.randn(1, T, Hv, generator=gen, device="cuda")) / 4
+    beta = torch.sigmoid(torch.randn(1, T, Hv, generator=gen, device="cuda"))
+    cu = torch.tensor([0] + lens).cumsum(0).int().cuda()
+    out = fq.chunk_gated_delta_rule_fwd(q, k, v, g, beta, cu_seqlens=cu, use_qk_l2norm_in_kernel=norm, output_w=True)
+    fq.check_device_status()
+    kd = k[0].double()
+    if norm:
+        kd = kd * torch.rsqrt(kd.pow(2).sum(-1, keepdim=True) + 1e-6)
+    eps = torch.finfo(dtype).eps / 2  # largest relative error of one rounding to the 16-bit type
+    for i in range(0, len(lens), max(1, len(lens) // 40)):
+        a, b = int(cu[i]), int(cu[i + 1])
+        A, w = solve(kd[a:b], g[0, a:b].double(), beta[0, a:b].double())
+        # A is rounded once, its lower left 32 x 32 blocks come from TF32 factors (2^-11 each, three of them)
+        assert float((out[1][0, a:b].double() - A).abs().max()) <= float(A.abs().max()) * (eps + 3 * 2.0 ** -11)
+        # w: A diag(beta gamma) rounded, the product rounded, and A's own error
+        assert float((out[5][0, a:b].double() - w).norm() / w.norm()) <= 3 * eps + 3 * 2.0 ** -11
