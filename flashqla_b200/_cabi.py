@@ -20,6 +20,7 @@ REC_QK_L2NORM, REC_DISABLE_STATE_UPDATE, REC_A_IS_LOG_DECAY, REC_B_IS_BETA = 1, 
 CHUNK_TRANSPOSE_STATE, CHUNK_STATE_ONLY, CHUNK_QK_L2NORM, CHUNK_SKIP_PREPARE = 1, 2, 4, 8
 CHUNK_INIT_IDENTITY, CHUNK_ZERO_V, CHUNK_PREPARE_ONLY, CHUNK_A_GIVEN, CHUNK_TABLES_READY = 16, 32, 64, 128, 256
 CHUNK_GATE_ACT, CHUNK_BETA_LOGIT, CHUNK_H0_KV_F32, CHUNK_DUAL_TRANSITION, CHUNK_OUT_GATED_RMSNORM = 512, 1024, 2048, 4096, 8192
+CHUNK_W_IN_SCAN = 16384
 
 
 class QlaError(RuntimeError):

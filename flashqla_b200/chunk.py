@@ -248,15 +248,16 @@ def _lengths(q, v, cu_seqlens, auto_cp):
 
 def _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_state, output_h, auto_cp, output_v_new,
              transposed, l2norm, A_log, dt_bias, beta_is_logit, h0_indices, fs_out, fs_indices, norm_gate, norm_weight,
-             norm_eps):
+             norm_eps, keep=True):
     """``(g_cumsum, A, o, h, final_state, v_new, w, qk_rnorm, activated beta)`` of the raw forward (``None`` for what was
-    not asked for)."""
+    not asked for).  Without ``keep`` (inference: ``o`` and the states are all that is wanted) ``A`` and ``w`` do not exist
+    either: the scan forms ``w`` itself instead of reading 256 bytes per token and head that the preparation wrote."""
     host = _cabi.host()
     host.chunk_check(q, k, v, g, beta, None if h0_indices is not None else initial_state, cu_seqlens, transposed)
     plan, order, chunks = _lengths(q, v, cu_seqlens, auto_cp)
     return host.chunk_fwd(q, k, v, g, beta, scale, initial_state, h0_indices, cu_seqlens, order, chunks, output_final_state,
                           output_h, output_v_new, transposed, l2norm, A_log, dt_bias, beta_is_logit,
-                          fs_out, fs_indices, norm_gate, norm_weight, norm_eps, plan, cp.INLINE_WARMUP, cp.WARMUP_THRESHOLD)
+                          fs_out, fs_indices, norm_gate, norm_weight, norm_eps, plan, cp.INLINE_WARMUP, cp.WARMUP_THRESHOLD, keep)
 
 
 def chunk_gated_delta_rule_bwd(
@@ -430,7 +431,7 @@ def chunk_gated_delta_rule(
         out = _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_state, False, True, False,
                        transpose_state_layout, use_qk_l2norm_in_kernel, A_log if use_gate_in_kernel else None,
                        dt_bias if use_gate_in_kernel else None, use_beta_sigmoid_in_kernel, None, None, None,
-                       output_norm_gate, output_norm_weight, output_norm_eps)
+                       output_norm_gate, output_norm_weight, output_norm_eps, keep=False)
         return out[2], out[4]
     if fused:
         o, final_state = ChunkGatedDeltaRuleFusedFunction.apply(

@@ -64,6 +64,17 @@ constexpr uint32_t kOffVn = kOffO + 16384;           // kAux: the v_new tile in 
 constexpr uint32_t kOffH = kOffO + 2 * 16384;        // and 16 KiB for half of the h tile ([64 k][128 v] as two halves)
 constexpr uint32_t kSmemBytes = kOffO + 2 * 16384 + 1024, kSmemBytesAux = kSmemBytes + 16384;
 
+// kWIn (Wt formed by the kernel itself): {Q, V} in two stages, {K, A diag(beta)} in three, because Wt of a chunk is formed
+// one chunk ahead; one Wt tile and one operand tile for it.
+constexpr uint32_t kQvV = 16384, kQvBytes = 32768;            // Q tile, V tile
+constexpr uint32_t kOffKa = 2 * kQvBytes, kKaA = 16384, kKaBytes = 24576;  // K tile, A tile
+constexpr int kKaStages = 3;
+constexpr uint32_t kOffWt = kOffKa + kKaStages * kKaBytes;    // 16 KiB: Wt^T [128 k][64 tokens], SW128
+constexpr uint32_t kOffAw = kOffWt + 16384;                   // 8 KiB: -A diag(beta gamma) [64][64], SW128
+constexpr uint32_t kOffPgWIn = kOffAw + 8192;
+constexpr uint32_t kOffOWIn = kOffPgWIn + 2 * 8192;
+constexpr uint32_t kSmemBytesWIn = kOffOWIn + 2 * 16384 + 1024;
+
 struct alignas(16) Gates {
   // g * log2(e) in the two roles it plays for the aux warps, which form s exp(g_c - g_d) r_q[c] r_k[d] as
   // ex2(g2row[c] + log2 s - g2col[d]); r_q, r_k = 1 / |q_t|, 1 / |k_t| with in-kernel L2 norm, else 1
@@ -82,6 +93,9 @@ enum Bar {
   kFull0 = 0, kFull1, kEmpty0, kEmpty1,
   kPDone, kPgReady, kD2Done, kVdReady, kVdStored, kSDone, kSbfReady, kSScaled, kAbReady0, kAbReady1,
   kD4Done, kORead, kOFree, kOReady, kONormed, kVnRead, kVnReady, kHRead, kHReady, kHFree, kGate0, kGate1, kGate2, kGate3,
+  // kWIn: {K, A} stages (kFull*, kEmpty* are those of {Q, V}), operand of Wt written, Wt in tensor memory, read from there,
+  // written to its tile, Q K^T read from the columns that Wt uses next
+  kKaFull0, kKaFull1, kKaFull2, kKaEmpty0, kKaEmpty1, kKaEmpty2, kAwReady, kWDone, kWRead, kWReady, kD0Read,
   kNumBars
 };
 
@@ -175,7 +189,10 @@ static __device__ __noinline__ bool norm_rows(uint32_t so, const T* z, int strid
 // kState16: h0 / final_state are bf16 (state pools); its own instantiation, like kNorm: the code of the plain
 // forward must stay small (it is the instruction cache, not the work, that a few extra branches in the
 // unrolled state loops cost: +20 % on the whole scan when they were part of the plain kernel).
-template <typename T, bool kStateOnly, bool kAux, bool kTrace, bool kNorm = false, bool kState16 = false>
+// kWIn: A holds A diag(beta) and there is no w: Wt = (-A diag(beta gamma)) K is one more product here, formed one chunk ahead
+// of its use.  It saves the write and the read of 256 bytes per token and head: 32768 tokens of 16 / 32 heads 135 + 233 -> 94 + 212 us
+// (preparation + scan), 540 k packed tokens of 8 / 8 heads 557 + 1205 -> 398 + 976; 16 chains alone pay 0.1 us per chunk.
+template <typename T, bool kStateOnly, bool kAux, bool kTrace, bool kNorm = false, bool kState16 = false, bool kWIn = false>
 __global__ void __launch_bounds__(kThreads, 1)
 chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_a,
@@ -236,14 +253,16 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // reuse needs no barrier of its own: chunk i + 2 is only written after MMA3 of chunk i has finished, which needs
   // both warpgroups to have left chunk i - 1 and MMA4 of chunk i - 2 (the last use of its Pg) to have been issued.
   __shared__ Gates gate_ring[kGateRing];
+  __shared__ float w_factor[kWIn ? 4 : 1][64];  // kWIn: -exp(g) / |k|, ring by chunk: A diag(beta) times this is the operand of Wt
+  constexpr uint32_t kPgTiles = kWIn ? kOffPgWIn : kOffPg, kOTiles = kWIn ? kOffOWIn : kOffO;
 
   if (tid == 0) {
 #pragma unroll 1
     for (int b = 0; b < kNumBars; ++b) {
-      int count = 1;  // kFull*, kEmpty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kOFree: one commit / one thread
-      if (b == kAbReady0 || b == kAbReady1) count = 2;
+      int count = 1;  // kFull*, kEmpty*, kKaEmpty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
+      if (b == kAbReady0 || b == kAbReady1 || b == kAwReady || (b >= kKaFull0 && b <= kKaFull2)) count = 2;
       else if (b == kPgReady || b == kORead || b == kOReady || b == kVnRead || b == kVnReady || b == kHRead ||
-               b == kHReady)
+               b == kHReady || b == kWRead || b == kWReady || b == kD0Read)
         count = 4;
       else if (b == kVdReady || b == kVdStored || b == kSbfReady || b == kSScaled || b == kONormed) count = 8;
       ptx::mbar_init(&bars[b], count);
@@ -253,8 +272,12 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
   if (!kStateOnly && warp >= 12) {  // the block of Pg above the diagonal (rows 0..31, columns 32..63) of both tiles
     for (int x = tid - 384; x < 2 * 32 * 4; x += 128)
-      *reinterpret_cast<uint4*>(smem + kOffPg + (x >> 7) * 8192 + ptx::sw128_offset((x >> 2) & 31, 4 + (x & 3))) =
+      *reinterpret_cast<uint4*>(smem + kPgTiles + (x >> 7) * 8192 + ptx::sw128_offset((x >> 2) & 31, 4 + (x & 3))) =
           make_uint4(0, 0, 0, 0);
+    ptx::fence_proxy_async_smem();
+  }
+  if (kWIn && warp < 4) {  // and the same block of the operand of Wt
+    *reinterpret_cast<uint4*>(smem + kOffAw + ptx::sw128_offset(tid >> 2, 4 + (tid & 3))) = make_uint4(0, 0, 0, 0);
     ptx::fence_proxy_async_smem();
   }
   if (warp == 8) {
@@ -302,6 +325,106 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // before the wait for the stage: their global-memory latency overlaps it.
     constexpr int kPrefetchAhead = 4;
     const float log2e = 1.4426950408889634f;
+    if constexpr (kWIn) {
+      // {K, A} and the factors of Wt run one chunk ahead of {Q, V} and the gate vectors: chunk i + 1 of the former is loaded when
+      // MMA3 of chunk i - 2 is through, chunk i of the latter when MMAq of chunk i - 2 is.
+      float g[2], gl = 0.f;
+      float2 rn[2];
+      auto fetch = [&](int i) {
+        const int t0 = seq_start + (first_chunk + i) * kChunk;
+        const int valid = min(kChunk, seq_end - t0);
+        const int64_t row = static_cast<int64_t>(t0) * p.num_v_heads + hv;
+        gl = p.g_cumsum[row + (valid - 1) * p.num_v_heads];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int c = min(lane + 32 * r, valid - 1);  // rows past the end repeat the last gate
+          g[r] = p.g_cumsum[row + c * p.num_v_heads];
+          rn[r] = make_float2(1.f, 1.f);
+          if (p.rnorm != nullptr)
+            rn[r] = *reinterpret_cast<const float2*>(p.rnorm + ((static_cast<int64_t>(t0) + c) * p.num_k_heads + hk) * 2);
+        }
+      };
+      auto load_ka = [&](int c, int slot) {
+        if (lane == 0) {
+          uint8_t* st = smem + kOffKa + slot * kKaBytes;
+          uint64_t* full = &bars[kKaFull0 + slot];
+          const int t0 = seq_start + (first_chunk + c) * kChunk;
+          ptx::mbar_expect_tx(full, kKaBytes);
+          ptx::tma_load_4d(st, &tm_k, full, 0, hk, t0, 0);
+          ptx::tma_load_3d(st + kKaA, &tm_a, full, 0, hv, t0);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 2; ++r) w_factor[c & 3][lane + 32 * r] = -ptx::ex2(g[r] * log2e) * rn[r].y;
+        warp_arrive(&bars[kKaFull0 + slot], lane);
+      };
+      if (nproc > 0) {
+        fetch(0);
+        load_ka(0, 0);
+      }
+      int slot = 1, ka_phase = 1;  // of chunk i + 1: ring slot, and parity of its last release (none before chunk 3)
+#pragma unroll 1
+      for (int i = 0; i < nproc; ++i) {
+        const int s = i & 1;
+        const int t0 = seq_start + (first_chunk + i) * kChunk;
+        const int valid = min(kChunk, seq_end - t0);
+        const float gi[2] = {g[0], g[1]}, gli = gl;
+        const float2 rni[2] = {rn[0], rn[1]};
+        if (i + 1 < nproc) fetch(i + 1);  // (requested before the wait for the stage)
+        if (i >= 2 && !wait(kEmpty0 + s, ((i >> 1) - 1) & 1)) break;
+        if (lane == 0) {
+          uint8_t* st = smem + s * kQvBytes;
+          uint64_t* full = &bars[kFull0 + s];
+          ptx::mbar_expect_tx(full, (kStateOnly ? 0 : 16384) + (zero_v ? 0 : 16384));
+          if (!zero_v) ptx::tma_load_4d(st + kQvV, &tm_v, full, 0, hv, t0, 0);
+          if (!kStateOnly) ptx::tma_load_4d(st, &tm_q, full, 0, hk, t0, 0);
+        }
+        __syncwarp();
+        Gates* gs = gates_of(i);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int c = lane + 32 * r;
+          const float g2 = gi[r] * log2e;
+          gs->g2row[c] = g2 + ptx::lg2(rni[r].x);
+          gs->g2col[c] = g2 - ptx::lg2(rni[r].y);
+          gs->sgamma[c] = p.scale * ptx::ex2(g2) * rni[r].x;
+          gs->rho[c] = c < valid ? ptx::ex2((gli - gi[r]) * log2e) * rni[r].y : 0.f;
+        }
+        gs->egl = ptx::ex2(gli * log2e);
+        gs->valid = valid;
+        warp_arrive(&bars[kGate0 + (i & 3)], lane);
+        if (i + 1 < nproc) {
+          if (i >= 2 && !wait(kKaEmpty0 + slot, ka_phase)) break;
+          load_ka(i + 1, slot);
+          if (++slot == kKaStages) {
+            slot = 0;
+            ka_phase ^= 1;
+          }
+        }
+        if (lane == 0) {
+          // the first demand loads go out before any prefetch; the prefetches of chunks 2.. follow chunk 1
+#pragma unroll 1
+          for (int c = (i == 1) ? 2 : i + kPrefetchAhead; i >= 1 && c <= i + kPrefetchAhead && c < nproc; ++c) {
+            const int pt0 = seq_start + (first_chunk + c) * kChunk;
+            ptx::tma_prefetch_l2_4d(&tm_k, 0, hk, pt0, 0);
+            ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
+            if (!zero_v) ptx::tma_prefetch_l2_4d(&tm_v, 0, hv, pt0, 0);
+            if (!kStateOnly) ptx::tma_prefetch_l2_4d(&tm_q, 0, hk, pt0, 0);
+          }
+        }
+        // the gate scalars of the chunk that many ahead as well
+        if (i + kPrefetchAhead < nproc) {
+          const int64_t ahead = static_cast<int64_t>(t0) + kPrefetchAhead * kChunk;
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int64_t tk = min(ahead + lane + 32 * r, static_cast<int64_t>(seq_end) - 1);
+            ptx::prefetch_l2(p.g_cumsum + tk * p.num_v_heads + hv);
+            if (p.rnorm != nullptr) ptx::prefetch_l2(p.rnorm + (tk * p.num_k_heads + hk) * 2);
+          }
+        }
+        __syncwarp();
+      }
+    } else
 #pragma unroll 1
     for (int i = 0; i < nproc; ++i) {
       const int s = i & 1;
@@ -399,7 +522,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const uint64_t d_kmn = ptx::smem_desc_sw128(ptx::smem_u32(smem + kStageK), 8192, 1024);  // K tile, MN-major
       const uint64_t d_a = ptx::smem_desc_sw128(ptx::smem_u32(smem + kStageA), 16, 1024);
       const uint64_t d_v = ptx::smem_desc_sw128(ptx::smem_u32(smem + kStageV), 8192, 1024);    // V tile, MN-major
-      const uint64_t d_pg = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffPg), 16, 1024);
+      const uint64_t d_pg = ptx::smem_desc_sw128(ptx::smem_u32(smem + kPgTiles), 16, 1024);
       const uint32_t id_p = ptx::mma_idesc(64, 64, fmt, ptx::kMajorK, ptx::kMajorK);
       constexpr int kHalf = (8192 >> 4) - 3 * 2;  // from k-step 3 to k-step 4 of a 128-wide tile
       // The CTA owns all 512 columns, so the allocation starts at column 0 of lane 0: tensor-memory
@@ -410,6 +533,74 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       auto bar_addr = [&](int b) { return bar0 + 8u * static_cast<uint32_t>(b); };
       bool ok = tmem == tmem0;
       if (!ok) ptx::record_wait_failure(p.status, kStatusBadTmemBase, 0);
+      if constexpr (kWIn) {
+        // The same order with MMAw(i + 1) in gap 1: D0 = K^T (-A diag(beta gamma))^T, which the Pg warps turn into the Wt tile while
+        // MMA3, MMA4 and MMAu run.  D0 is Q K^T of a chunk and Wt of the next one by turns.
+        const uint64_t q_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem), 16, 1024);
+        const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kQvV), 8192, 1024);
+        const uint64_t k_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa), 16, 1024);
+        const uint64_t kmn_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa), 8192, 1024);
+        const uint64_t a_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa + kKaA), 16, 1024);
+        const uint64_t w_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffWt), 8192, 1024);  // MN-major
+        const uint64_t aw_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffAw), 16, 1024);
+        const uint32_t id_w = ptx::mma_idesc(128, 64, fmt, ptx::kMajorK, ptx::kMajorMN);
+        int slot = 0, phase = 0, slot_i = 0;  // of chunk i + 1 in the {K, A} ring; slot of chunk i
+#pragma unroll 1
+        for (int i = -1; ok && i < nproc; ++i) {
+          const int ph = i & 1, j = i + 1;
+          const uint64_t ka_i = static_cast<uint64_t>(slot_i * (kKaBytes >> 4)), ka_j = static_cast<uint64_t>(slot * (kKaBytes >> 4));
+          if (i >= 0) {
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSbfReady), ph, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kWReady), ph, true))) break;
+            ptx::tc_fence_after_sync();
+            ptx::umma_ts_k128_rolled<128, 128>(tmem0 + kColD2, tmem0 + kColSbf, w_desc, id_w, kStateOnly ? !zero_v : true,
+                                               bar_addr(kD2Done));
+            if (!kStateOnly)
+              ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf,
+                                                 q_desc + static_cast<uint64_t>(ph * (kQvBytes >> 4)), id_n64, false,
+                                                 bar_addr(kEmpty0 + ph));
+          }
+          if (j < nproc) {
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kKaFull0 + slot), phase, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kAwReady), j & 1, true))) break;
+            if (!kStateOnly && i >= 0 && !(ok = ptx::mbar_wait_nocall(bar_addr(kD0Read), ph, true))) break;
+            ptx::tc_fence_after_sync();
+            ptx::umma_ss_k64<128, 2>(tmem0 + kColD0, kmn_desc + ka_j, aw_desc, id_u, false, bar_addr(kWDone));
+          }
+          if (i >= 0) {
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdReady), ph, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSScaled), ph, true))) break;
+            ptx::tc_fence_after_sync();
+            ptx::umma_ts_k64_halves<128>(tmem0 + kColS, tmem0 + kColD2, kmn_desc + ka_i, id_mn128, true, bar_addr(kSDone),
+                                         bar_addr(kKaEmpty0 + slot_i));
+            if (kStateOnly) ptx::umma_commit(&bars[kEmpty0 + ph]);
+            if (!kStateOnly) {
+              if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdStored), ph, true))) break;
+              if (!(ok = ptx::mbar_wait_nocall(bar_addr(kPgReady), ph, true))) break;
+              if (i > 0 && !(ok = ptx::mbar_wait_nocall(bar_addr(kORead), ph ^ 1, true))) break;
+              ptx::tc_fence_after_sync();
+              ptx::umma_ts_k64_halves<2>(tmem0 + kColD4, tmem0 + kColD2 + 16, d_pg + static_cast<uint64_t>(ph * (8192 >> 4)),
+                                         id_n64, false, bar_addr(kD4Done));
+            }
+          }
+          if (j < nproc) {
+            const uint64_t qv = static_cast<uint64_t>((j & 1) * (kQvBytes >> 4));
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + (j & 1)), (j >> 1) & 1, true))) break;
+            ptx::tc_fence_after_sync();
+            if (!zero_v) ptx::umma_ss_k64<128, 2>(tmem0 + kColD2, v_desc + qv, a_desc + ka_j, id_u, false);
+            if (!kStateOnly) {
+              if (!(ok = ptx::mbar_wait_nocall(bar_addr(kWRead), j & 1, true))) break;
+              ptx::tc_fence_after_sync();
+              ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, q_desc + qv, k_desc + ka_j, id_p, false, bar_addr(kPDone));
+            }
+          }
+          slot_i = slot;
+          if (++slot == kKaStages) {
+            slot = 0;
+            phase ^= 1;
+          }
+        }
+      } else
 #pragma unroll 1
       for (int i = -1; ok && i < nproc; ++i) {
         const int ph = i & 1;
@@ -476,19 +667,49 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t tm = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
     const float log2_scale = __log2f(p.scale);
     const int p_row = (warp & 3) * 16 + (lane >> 2), p_cols = warp < 18 ? 32 : 64;
+    // kWIn: Wt of chunk j, from the accumulator (lane = column k) to its tile [k][token]
+    auto form_w = [&](int j) {
+      if (!wait(kWDone, j & 1)) return false;
+      ptx::tc_fence_after_sync();
+      uint32_t y[2][16];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t x[32];
+        ptx::tmem_ld32(tm + kColD0 + 32 * h, x);
+        ptx::tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) y[h][e] = pack2<T>(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1]));
+      }
+      if (!kStateOnly) {
+        ptx::tc_fence_before_sync();
+        warp_arrive(&bars[kWRead], lane);
+      }
+      // (MMA2 of chunk j - 1, which read the tile, precedes this chunk's product in the pipe)
+      const uint32_t at = ptx::sw128_offset((warp & 3) * 32 + lane, 0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          *reinterpret_cast<uint4*>(smem + kOffWt + (at ^ ((4 * h + e) << 4))) =
+              make_uint4(y[h][4 * e], y[h][4 * e + 1], y[h][4 * e + 2], y[h][4 * e + 3]);
+      ptx::fence_proxy_async_smem();
+      warp_arrive(&bars[kWReady], lane);
+      return true;
+    };
     // kNorm: these warps have time to spare behind their tile and take half of the rows of the output tile's norm
     auto norm_half = [&](int j) {
       const int t0 = seq_start + (first_chunk + j) * kChunk;
       const int valid = j < lead ? 0 : min(kChunk, seq_end - t0);
       const T* z = static_cast<const T*>(p.norm_gate) + (static_cast<int64_t>(t0) * p.num_v_heads + hv) * kHeadDim;
-      const bool fine = norm_rows<T>(ptx::smem_u32(smem + kOffO + (j & 1) * 16384), z, p.num_v_heads * kHeadDim, p.norm_weight,
+      const bool fine = norm_rows<T>(ptx::smem_u32(smem + kOTiles + (j & 1) * 16384), z, p.num_v_heads * kHeadDim, p.norm_weight,
                                      p.norm_eps, valid, 8, bar0 + 8u * kOReady, j & 1);
       ptx::fence_proxy_async_smem();
       warp_arrive(&bars[kONormed], lane);
       return fine;
     };
+    const bool begun = !kWIn || nproc == 0 || form_w(0);
 #pragma unroll 1
-    for (int i = 0; (!kStateOnly || (kAux && p.h != nullptr)) && i < nproc; ++i) {
+    for (int i = 0; begun && (!kStateOnly || kWIn || (kAux && p.h != nullptr)) && i < nproc; ++i) {
       const int ph = i & 1;
       if (!kStateOnly) {
         if (warp == 16) trace(2, i, 8);
@@ -502,7 +723,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::tc_fence_after_sync();
         if (warp == 16) trace(2, i, 9);
         // (tile i & 1 was last read by MMA4 of chunk i - 2: see the wait at the end)
-        const uint32_t pg = ptx::smem_u32(smem + kOffPg) + ph * 8192;
+        const uint32_t pg = ptx::smem_u32(smem + kPgTiles) + ph * 8192;
 #pragma unroll 1
         for (int db = 0; db < p_cols; db += 32) {
           uint32_t pr[16], m[8];
@@ -526,14 +747,17 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         ptx::fence_proxy_async_smem();
         ptx::tc_fence_before_sync();
+        if (kWIn) warp_arrive(&bars[kD0Read], lane);
         // Before announcing this tile, make sure MMA4 of the previous chunk has finished: the next iteration overwrites the
         // tile it read.  Waiting HERE (MMA4 of this chunk cannot be issued before the arrival below) keeps this warp at
         // most one phase behind the D4Done barrier; behind the arrival it could fall two behind and wait forever.
         if (i > 0 && !wait(kD4Done, (i - 1) & 1)) break;
         warp_arrive(&bars[kPgReady], lane);
+        if (kWIn && i + 1 < nproc && !form_w(i + 1)) break;
         if (kNorm && i > 0 && !norm_half(i - 1)) break;
         if (kNorm && i == nproc - 1 && !norm_half(i)) break;
       }
+      if (kWIn && kStateOnly && i + 1 < nproc && !form_w(i + 1)) break;
       if (warp == 16) trace(2, i, 10);
       if (kAux && p.h != nullptr) {
         // h of this chunk = the 16-bit copy of the state that enters it, transposed to [K][V] through a shared-memory
@@ -601,7 +825,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int valid = j < lead ? 0 : min(kChunk, seq_end - t0);  // nothing of a warm-up chunk is stored
       // two output tiles: the store of chunk j - 2 must have read this one.  kAux: one, and one for v_new: both stores of
       // chunk j - 1 must have read theirs
-      uint8_t* so = smem + kOffO + (kAux ? 0 : (j & 1) * 16384);
+      uint8_t* so = smem + kOTiles + (kAux ? 0 : (j & 1) * 16384);
       if (j > (kAux ? 0 : 1)) {
         if (tl == 0) {
           if (kAux) ptx::tma_store_wait_read();
@@ -731,6 +955,38 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // (B operand of MMAu).  A is lower triangular: row r ends in 16-byte piece r / 8, what lies behind is zero (or
     // belongs to tokens past the end, whose rows nothing reads).  Six pieces per lane: warp 11 rows 32..63 pieces
     // 2..7, warp 10 the first two of those rows and the four of rows 0..31.
+    if constexpr (kWIn) {
+      // The same pieces of A diag(beta), which is B operand of MMAu as it is, times -exp(g) / |k|: B operand of MMAw
+      int slot = 0, phase = 0;
+#pragma unroll 1
+      for (int j = 0; j < nproc; ++j) {
+        if (!wait(kKaFull0 + slot, phase)) break;
+        if (j > 0 && !wait(kWDone, (j - 1) & 1)) break;  // the operand of chunk j - 1 has been read
+        const float* f = w_factor[j & 3];
+        const uint8_t* at = smem + kOffKa + slot * kKaBytes + kKaA;
+#pragma unroll 2
+        for (int x = 0; x < 6; ++x) {
+          const bool low = warp == 10 && x < 4;
+          const int c16 = (warp == 11) ? x + 2 : (low ? x : x - 4);
+          const uint32_t off = ptx::sw128_offset(low ? lane : 32 + lane, c16);
+          const uint4 raw = *reinterpret_cast<const uint4*>(at + off);
+          const float4 b0 = *reinterpret_cast<const float4*>(&f[c16 * 8]);
+          const float4 b1 = *reinterpret_cast<const float4*>(&f[c16 * 8 + 4]);
+          const T* e = reinterpret_cast<const T*>(&raw);
+          *reinterpret_cast<uint4*>(smem + kOffAw + off) =
+              make_uint4(pack2<T>(Cvt<T>::to_f32(e[0]) * b0.x, Cvt<T>::to_f32(e[1]) * b0.y),
+                         pack2<T>(Cvt<T>::to_f32(e[2]) * b0.z, Cvt<T>::to_f32(e[3]) * b0.w),
+                         pack2<T>(Cvt<T>::to_f32(e[4]) * b1.x, Cvt<T>::to_f32(e[5]) * b1.y),
+                         pack2<T>(Cvt<T>::to_f32(e[6]) * b1.z, Cvt<T>::to_f32(e[7]) * b1.w));
+        }
+        ptx::fence_proxy_async_smem();
+        warp_arrive(&bars[kAwReady], lane);
+        if (++slot == kKaStages) {
+          slot = 0;
+          phase ^= 1;
+        }
+      }
+    } else
 #pragma unroll 1
     for (int j = 0; j < nproc; ++j) {
       const int sj = j & 1;
@@ -995,7 +1251,9 @@ int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const voi
   if ((rc = make_tmap_halves(&tm_q, state_only ? k : q, total_tokens, p.num_k_heads, 64, is_bf16)) != QLA_OK) return rc;
   if ((rc = make_tmap_halves(&tm_v, v, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
   if ((rc = make_tmap_3d(&tm_a, A, total_tokens, p.num_v_heads, 64, 64, 64, true, is_bf16)) != QLA_OK) return rc;
-  if ((rc = make_tmap_halves(&tm_w, w, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
+  const bool w_in = w == nullptr;  // A holds A diag(beta), the kernel forms Wt itself
+  tm_w = tm_k;
+  if (!w_in && (rc = make_tmap_halves(&tm_w, w, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
   if ((rc = make_tmap_halves(&tm_o, state_only ? v : p.o, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
   tm_vn = tm_h = tm_o;
   if (p.v_new != nullptr && (rc = make_tmap_halves(&tm_vn, p.v_new, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
@@ -1003,30 +1261,26 @@ int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const voi
   const uint64_t h_rows = (static_cast<uint64_t>(total_tokens) / kChunk + p.num_seqs) * p.num_v_heads * kHeadDim;
   if (p.h != nullptr && (rc = make_tmap_halves(&tm_h, p.h, h_rows, 1, 64, is_bf16)) != QLA_OK) return rc;
   const unsigned grid = static_cast<unsigned>(p.num_seqs) * p.num_v_heads * (p.dual ? 2 : 1);
-#define QLA_LAUNCH_FWD(T, SO, AUX, TR)                                                                          \
-  do {                                                                                                          \
-    { const int rc_ = ensure_dynamic_smem<chunk_fwd_kernel<T, SO, AUX, TR>>(AUX ? kSmemBytesAux : kSmemBytes); if (rc_ != QLA_OK) return rc_; }  \
-    QLA_CHECK_CUDA(launch_dependent(chunk_fwd_kernel<T, SO, AUX, TR>, dim3(grid), dim3(kThreads), AUX ? kSmemBytesAux : kSmemBytes, stream, tm_q, tm_k, tm_v, tm_a, tm_w, tm_o, tm_vn, tm_h, p)); \
+#define QLA_LAUNCH_FWD(BYTES, ...)                                                                                             \
+  do {                                                                                                                         \
+    const int rc_ = ensure_dynamic_smem<chunk_fwd_kernel<__VA_ARGS__>>(BYTES);                                                 \
+    if (rc_ != QLA_OK) return rc_;                                                                                             \
+    QLA_CHECK_CUDA(launch_dependent(chunk_fwd_kernel<__VA_ARGS__>, dim3(grid), dim3(kThreads), BYTES, stream, tm_q, tm_k, tm_v, \
+                                    tm_a, tm_w, tm_o, tm_vn, tm_h, p));                                                        \
   } while (0)
-#define QLA_LAUNCH_FWD_NORM(T)                                                                                   \
-  do {                                                                                                          \
-    { const int rc_ = ensure_dynamic_smem<chunk_fwd_kernel<T, false, false, false, true>>(kSmemBytes); if (rc_ != QLA_OK) return rc_; }  \
-    QLA_CHECK_CUDA(launch_dependent(chunk_fwd_kernel<T, false, false, false, true>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_q, tm_k, tm_v, tm_a, tm_w, tm_o, tm_vn, tm_h, p)); \
-  } while (0)
-#define QLA_LAUNCH_FWD_ST16(T)                                                                                   \
-  do {                                                                                                          \
-    { const int rc_ = ensure_dynamic_smem<chunk_fwd_kernel<T, false, false, false, false, true>>(kSmemBytes); if (rc_ != QLA_OK) return rc_; }  \
-    QLA_CHECK_CUDA(launch_dependent(chunk_fwd_kernel<T, false, false, false, false, true>, dim3(grid), dim3(kThreads), kSmemBytes, stream, tm_q, tm_k, tm_v, tm_a, tm_w, tm_o, tm_vn, tm_h, p)); \
-  } while (0)
-#define QLA_DISPATCH_FWD(T)                                                                  \
-  do {                                                                                       \
-    if (p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD_ST16(T);                                \
-    else if (p.norm_gate != nullptr) QLA_LAUNCH_FWD_NORM(T);                                 \
-    else if (traced) QLA_LAUNCH_FWD(T, false, false, true);                                  \
-    else if (state_only && aux) QLA_LAUNCH_FWD(T, true, true, false);                        \
-    else if (state_only) QLA_LAUNCH_FWD(T, true, false, false);                              \
-    else if (aux) QLA_LAUNCH_FWD(T, false, true, false);                                     \
-    else QLA_LAUNCH_FWD(T, false, false, false);                                             \
+#define QLA_DISPATCH_FWD(T)                                                                                   \
+  do {                                                                                                        \
+    if (w_in && p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, true, true); \
+    else if (w_in && p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, true, false, true);  \
+    else if (w_in && state_only) QLA_LAUNCH_FWD(kSmemBytesWIn, T, true, false, false, false, false, true);    \
+    else if (w_in) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, false, true);                 \
+    else if (p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false, false, true);   \
+    else if (p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false, true);                \
+    else if (traced) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, true);                                       \
+    else if (state_only && aux) QLA_LAUNCH_FWD(kSmemBytesAux, T, true, true, false);                          \
+    else if (state_only) QLA_LAUNCH_FWD(kSmemBytes, T, true, false, false);                                   \
+    else if (aux) QLA_LAUNCH_FWD(kSmemBytesAux, T, false, true, false);                                       \
+    else QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false);                                                  \
   } while (0)
   // the traced variant (plain full forward only) is a separate instantiation so that normal launches
   // carry no tracing code
@@ -1034,8 +1288,6 @@ int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const voi
   if (is_bf16) QLA_DISPATCH_FWD(__nv_bfloat16);
   else QLA_DISPATCH_FWD(__half);
 #undef QLA_DISPATCH_FWD
-#undef QLA_LAUNCH_FWD_NORM
-#undef QLA_LAUNCH_FWD_ST16
 #undef QLA_LAUNCH_FWD
   QLA_CHECK_CUDA(cudaGetLastError());
   return QLA_OK;

@@ -326,14 +326,15 @@ Tensor table_workspace(QlaChunkFwdArgs& a, const at::Device& dev) {
 }
 
 // The raw forward (chunk.chunk_gated_delta_rule_fwd says what the arguments mean).  `order` is the order in which the
-// sequences of cu_seqlens are started, `plan` the context-parallel plan or None.
+// sequences of cu_seqlens are started, `plan` the context-parallel plan or None.  Without `keep` (and h, v_new) A and w are not
+// wanted either.
 py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_,
                     std::optional<double> scale, const OptTensor& initial_state, const OptTensor& initial_state_indices,
                     const OptTensor& cu_seqlens, const OptTensor& order, int64_t n_chunks,
                     bool output_final_state, bool output_h, bool output_v_new, bool transposed, bool l2norm,
                     const OptTensor& A_log_, const OptTensor& dt_bias_, bool beta_is_logit, const OptTensor& final_state_out,
                     const OptTensor& final_state_indices, const OptTensor& norm_gate, const OptTensor& norm_weight,
-                    double norm_eps, const Plan* plan, bool inline_warmup, double threshold) {
+                    double norm_eps, const Plan* plan, bool inline_warmup, double threshold, bool keep) {
   py::gil_scoped_release nogil;
   const Sizes s = chunk_check(q_, k_, v_, g_, beta_, initial_state_indices.has_value() ? OptTensor() : initial_state, cu_seqlens,
                               transposed);
@@ -394,7 +395,12 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   void* stream = current_stream(dev);
   const Tensor cu = as_i32(cu_seqlens, dev);
   const Tensor g_cumsum = new_tensor({B, T, Hv}, at::kFloat, dev), A = new_tensor({B, T, Hv, 64}, dtype, dev);
-  const Tensor w = new_tensor({B, T, Hv, 128}, dtype, dev), o = at::empty_like(v);
+  // A call that keeps neither A nor w: the scan forms w itself, and A is scratch in its own form.  From 65536 tokens x heads on:
+  // preparation + scan, us, with w / without: 16 chains of 32 chunks 62 / 64, 32 of 32 69 / 69, 64 of 32 83 / 77, 128 of 32 111 / 92,
+  // 512 of 32 (8 / 8 heads) 456 / 357, 512 of 4 89 / 81; with fewer the one more hand-off at the start of a scan costs what the
+  // preparation gains.
+  const bool w_in_scan = !keep && !output_h && !output_v_new && B * T * Hv >= 65536;
+  const Tensor w = w_in_scan ? Tensor() : new_tensor({B, T, Hv, 128}, dtype, dev), o = at::empty_like(v);
   Tensor h, v_new, rnorm, beta_act, final_state, A_log, dt_bias;
   if (output_h)
     h = cu.defined() ? new_h(n_chunks, T, N, Hv, dtype, dev).unsqueeze(0) : new_tensor({B, chunks_of(T), Hv, 128, 128}, dtype, dev);
@@ -417,7 +423,7 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   a.g_cumsum = ptr<float>(g_cumsum); a.A = ptr(A); a.w = ptr(w); a.qk_rnorm = ptr<float>(rnorm);
   a.A_log = ptr<float>(A_log); a.dt_bias = ptr<float>(dt_bias); a.beta_out = ptr<float>(beta_act);
   a.status = status_word(dev); a.cu_seqlens = ptr<int32_t>(cu);
-  const int norm_flag = l2norm ? QLA_CHUNK_QK_L2NORM : 0;
+  const int norm_flag = (l2norm ? QLA_CHUNK_QK_L2NORM : 0) | (w_in_scan ? QLA_CHUNK_W_IN_SCAN : 0);
   const int act_flags = (A_log.defined() ? QLA_CHUNK_GATE_ACT : 0) | (beta_is_logit ? QLA_CHUNK_BETA_LOGIT : 0);
   const int out_flag = gate.defined() ? QLA_CHUNK_OUT_GATED_RMSNORM : 0, layout = transposed ? QLA_CHUNK_TRANSPOSE_STATE : 0;
   if (final_state.defined() || h0.has_value()) a.state_dtype = dtype_code(final_state.defined() ? final_state : *h0);
@@ -466,7 +472,8 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   }
   py::gil_scoped_acquire gil;
   auto opt = [](const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); };
-  return py::make_tuple(g_cumsum, A, o, opt(h), opt(final_state), opt(v_new), w, opt(rnorm), opt(beta_act));
+  return py::make_tuple(g_cumsum, w_in_scan ? py::none() : py::cast(A), o, opt(h), opt(final_state), opt(v_new), opt(w), opt(rnorm),
+                        opt(beta_act));
 }
 
 // The raw backward (chunk.chunk_gated_delta_rule_bwd): `g_` is the cumulative gate of the forward.

@@ -297,9 +297,11 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
     ptx::mbar_expect_tx(&bar_k, 32768);
     ptx::tma_load_4d(sK, &tm_k, &bar_k, 0, x.hk, x.tok0, 0);
   };
-  auto load_q = [&](const Item& x) {  // (only for its row norms)
+  // Q is only wanted for its row norms.  Its tile visits the memory of the K tile when that has been multiplied, and (kW) with a
+  // CTA's first item both chunks' areas, which nothing uses yet: one short prompt does not wait for a second copy.
+  auto load_q = [&](const Item& x, uint8_t* to) {
     ptx::mbar_expect_tx(&bar_q, 32768);
-    ptx::tma_load_4d(sK, &tm_q, &bar_q, 0, x.hk, x.tok0, 0);
+    ptx::tma_load_4d(to, &tm_q, &bar_q, 0, x.hk, x.tok0, 0);
   };
   if (tid == 0) {
     ptx::mbar_init(&bar_k, 1);
@@ -373,7 +375,10 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
     const Item first = locate();
     if (lane == 0) {
       s_item[0][ci] = first;
-      if (ci == 0) load_k(first);
+      if (ci == 0) {
+        load_k(first);
+        if (kW && norm && first.split == 0) load_q(first, smem + 32768);
+      }
     }
     fetch_gates(first, first.hv0);
     activate(first, first.hv0);
@@ -423,23 +428,23 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
   };
   // One thread per chunk says when the chunk is through with K (after its last product); the second one to do so loads the next
   // item's.  With the norms the Q tile visits the same memory in between, and each chunk says so a second time.
-  const bool q_norms = norm && cur.split == 0;
+  const bool q_first = kW && norm && cur.split == 0 && item == blockIdx.x, q_norms = norm && cur.split == 0 && !q_first;
   auto release_k = [&]() {
     unsigned before;
     asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(ptx::smem_u32(&k_released)) : "memory");
-    if (before == 1 && q_norms) load_q(cur);
+    if (before == 1 && q_norms) load_q(cur, sK);
     if (before == (q_norms ? 3 : 1)) {
       k_released = 0;
       if (more) load_k(nxt);
     }
   };
-  auto row_norm = [&]() {  // |row|^2 of the row tid of the tile: half rows, then their sum
+  auto row_norm = [&](const uint8_t* tile) {  // 1 / |row tid|: half rows, then their sum
     float sum[2] = {0.f, 0.f};
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
 #pragma unroll 2
       for (int c16 = 0; c16 < 8; ++c16) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(sK + half * 16384 + ptx::sw128_offset(tid, c16));
+        const uint4 raw = *reinterpret_cast<const uint4*>(tile + half * 16384 + ptx::sw128_offset(tid, c16));
         const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
         for (int x = 0; x < 8; ++x) sum[half] += Cvt<T>::to_f32(e[x]) * Cvt<T>::to_f32(e[x]);
@@ -448,12 +453,16 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
     return rsqrtf(sum[0] + sum[1] + p.norm_eps);
   };
   // 1 / |q| of this item's rows, once Q has come to where K was; then the next item's K may come
-  auto finish_q = [&]() {
+  auto finish_q = [&](const uint8_t* tile) {
     if (ptx::mbar_wait_addr(a_q, q_turn)) {
-      const float rq = row_norm();
+      const float rq = row_norm(tile);
       if ((tid & 63) < cur.valid) p.rnorm[((static_cast<int64_t>(cur.tok0) + tid) * p.num_k_heads + cur.hk) * 2] = rq;
     }
     q_turn ^= 1;
+    if (q_first) {
+      __syncthreads();  // (the tile lies in both chunks' areas)
+      return;
+    }
     chunk_sync(ci);
     if (part == 0 && lane == 0) release_k();
   };
@@ -479,7 +488,7 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
         if (!norm) publish(s_gates[ci][buf % kGateBuffers]);
       }
     }
-    if (q_norms) finish_q();
+    if (q_norms || q_first) finish_q(q_first ? smem + 32768 : sK);
     chunk_sync(ci);
   } else {
   // K K^T of this chunk (an M = 128 product with the rows of both chunks, of which only this chunk's lanes are written), read
@@ -504,11 +513,12 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
   if (norm) {
     Gates& gt = s_gates[ci][buf % kGateBuffers];
     if (ptx::mbar_wait_addr(a_k, turn)) {
-      const float rk = row_norm();
+      const float rk = row_norm(sK);
       gt.row[tid & 63] = ptx::lg2(rk);  // (for the warp that forms the gates)
       if ((tid & 63) < valid && cur.split == 0) p.rnorm[((static_cast<int64_t>(cur.tok0) + tid) * p.num_k_heads + cur.hk) * 2 + 1] = rk;
     }
-    chunk_sync(ci);
+    if (q_first) finish_q(smem + 32768);
+    else chunk_sync(ci);
     if (part == 0) {
       lrk[0] = gt.row[lane];
       lrk[1] = gt.row[lane + 32];
@@ -644,7 +654,7 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
         }
         __syncwarp();
       }
-      if (!kW && q_norms && hv == hv0) finish_q();  // (Q has been under way since K K^T)
+      if (!kW && q_norms && hv == hv0) finish_q(sK);  // (Q has been under way since K K^T)
       // ---- 2: X[R + 1][R] = X[R + 1][R + 1] N[R + 1][R] X[R][R]; the diagonal blocks leave beside it
       {
         const float* bg = &gt.bg[32 * part];
@@ -795,7 +805,7 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
     }
   }
   }  // valid
-  if (kW && valid > 0 && q_norms) finish_q();
+  if (kW && valid > 0 && q_norms) finish_q(sK);
   }  // items
 
   if (part == 0 && lane == 0) ptx::tma_store_wait_read();  // shared memory stays allocated until the last stores have read it

@@ -16,7 +16,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from .chunk import chunk_gated_delta_rule_fwd
+from .chunk import _forward
 
 
 def prefill_into_state_pool(
@@ -48,9 +48,15 @@ def prefill_into_state_pool(
         raise ValueError(f"state_indices must have one entry per sequence ({N}), got {state_indices.numel()}")
     # The kernels index the pool themselves: a sequence reads its slot when it starts and writes it when it ends
     # (slots of different sequences must differ), so nothing is gathered or scattered around the call.
-    out = chunk_gated_delta_rule_fwd(
-        q, k, v, g, beta, scale=scale, cu_seqlens=cu_seqlens, output_final_state=True, transpose_state_layout=True,
-        initial_state=state_pool if continue_from_pool else None,
-        initial_state_indices=state_indices if continue_from_pool else None,
-        final_state_out=state_pool, final_state_indices=state_indices, **forward_kwargs)
-    return out[2], state_pool
+    o = _output(q, k, v, g, beta, scale, cu_seqlens, state_pool if continue_from_pool else None,
+                state_indices if continue_from_pool else None, state_pool, state_indices, **forward_kwargs)
+    return o, state_pool
+
+
+def _output(q, k, v, g, beta, scale, cu_seqlens, initial_state, initial_state_indices, final_state_out, final_state_indices, *,
+            output_h=False, auto_cp=True, output_v_new=False, use_qk_l2norm_in_kernel=False, A_log=None, dt_bias=None,
+            beta_is_logit=False, output_w=False, out_norm_gate=None, out_norm_weight=None, out_norm_eps=1e-6):
+    """``o`` of ``chunk_gated_delta_rule_fwd`` with these arguments, [V][K] states; nothing else of its result is kept."""
+    return _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, True, output_h, auto_cp, output_v_new, True,
+                    use_qk_l2norm_in_kernel, A_log, dt_bias, beta_is_logit, initial_state_indices, final_state_out,
+                    final_state_indices, out_norm_gate, out_norm_weight, out_norm_eps, keep=False)[2]

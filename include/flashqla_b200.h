@@ -152,11 +152,15 @@ enum { /* flags of QlaChunkFwdArgs / QlaChunkBwdArgs */
   QLA_CHUNK_OUT_GATED_RMSNORM = 8192, /* o leaves through the gated RMS norm that follows the op in a GDN
                                     layer: o * rsqrt(mean_v(o^2) + norm_eps) * norm_weight[v] *
                                     silu(norm_gate[t,h,v]); inference epilogue (no h / v_new)    */
-  QLA_CHUNK_DUAL_TRANSITION = 4096 /* with QLA_CHUNK_STATE_ONLY: the same launch also runs the
+  QLA_CHUNK_DUAL_TRANSITION = 4096, /* with QLA_CHUNK_STATE_ONLY: the same launch also runs the
                                     INIT_IDENTITY | ZERO_V pass of every (sequence, head) with
                                     chunk_limit_b, writing its K x K result to row seq_map_b[n]
                                     of final_state_b (fp32): warm-up and transition pass of
                                     context parallelism as one grid                           */
+  QLA_CHUNK_W_IN_SCAN = 16384    /* the scan forms w itself: no w (may be NULL), and A is
+                                    A diag(beta), out of the preparation step and in with
+                                    QLA_CHUNK_SKIP_PREPARE.  For calls that keep neither: not
+                                    with QLA_CHUNK_A_GIVEN, h or v_new                        */
 };
 
 /*

@@ -1,0 +1,73 @@
+"""Calls that keep neither ``A`` nor ``w`` (inference from 65536 tokens x heads on): the scan forms ``w`` itself.  Compared with the
+raw forward, which the other files hold to the oracle, over the forms such a call can take."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(lens, Hk, Hv, dtype, weak, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    T = sum(lens)
+    q, k, v = (torch.randn(1, T, n, 128, generator=gen, device="cuda") for n in (Hk, Hk, Hv))
+    q, k = (torch.nn.functional.normalize(x, dim=-1) for x in (q, k))
+    g = torch.nn.functional.logsigmoid(torch.randn(1, T, Hv, generator=gen, device="cuda"))
+    if weak:  # heads that hardly ever forget: transition matrices of the segments
+        g = g / 64
+        g[..., 0] = 0
+    beta = torch.sigmoid(torch.randn(1, T, Hv, generator=gen, device="cuda"))
+    h0 = 0.1 * torch.randn(len(lens) + 3, Hv, 128, 128, generator=gen, device="cuda")
+    cu = torch.tensor([0] + list(lens)).cumsum(0).int().cuda()
+    return q.to(dtype), k.to(dtype), v.to(dtype), g, beta, h0, cu
+
+
+def close(a, b, dtype):
+    """Either is within 3.6e-3 (bf16; 4.5e-4 fp16) of exact arithmetic, so they are within twice that of each other."""
+    rel = float((a.double() - b.double()).norm() / b.double().norm())
+    return rel <= (7.2e-3 if dtype == torch.bfloat16 else 9e-4)
+
+
+CASES = [  # lengths, heads, weak gates
+    ([65536 // 8 + 1], (4, 8), False),                     # segments, warm-up inside the scan
+    ([65536 // 4 + 37], (2, 4), True),                     # segments, state-only passes and transition matrices
+    ([1, 63, 64, 65, 127, 128, 129, 192, 193, 2048, 777], (16, 32), False),
+    ([3] * 500 + [641], (8, 32), True),                    # one chunk each: the rings turn over with every sequence
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lens, heads, weak", CASES)
+def test_op(lens, heads, weak, dtype):
+    import flashqla_b200 as fq
+    q, k, v, g, beta, h0, cu = inputs(lens, *heads, dtype, weak, 3)
+    assert q.shape[1] * heads[1] >= 65536
+    h0 = h0[:len(lens)]
+    raw = fq.chunk_gated_delta_rule_fwd(q, k, v, g, beta, initial_state=h0, cu_seqlens=cu)
+    with torch.no_grad():
+        o, final = fq.chunk_gated_delta_rule(q, k, v, g, beta, initial_state=h0, output_final_state=True, cu_seqlens=cu)
+    fq.check_device_status()
+    assert close(o, raw[2], dtype) and close(final, raw[4], dtype)
+    with torch.no_grad():
+        again = fq.chunk_gated_delta_rule(q, k, v, g, beta, initial_state=h0, output_final_state=True, cu_seqlens=cu)
+    assert torch.equal(o, again[0]) and torch.equal(final, again[1])
+
+
+@pytest.mark.parametrize("pool_dtype, norm", [(torch.float32, True), (torch.bfloat16, False)])
+@pytest.mark.parametrize("lens, heads, weak", CASES)
+def test_pool(lens, heads, weak, pool_dtype, norm):
+    import flashqla_b200 as fq
+    q, k, v, g, beta, h0, cu = inputs(lens, *heads, torch.bfloat16, weak, 4)
+    slots = torch.randperm(len(h0), device="cuda")[:len(lens)].int()
+    slots[0] = -1  # no slot: from zero, nothing written
+    gate = dict(out_norm_gate=torch.randn_like(v), out_norm_weight=torch.rand(128, device="cuda") + 0.5) if norm else {}
+    pools = [h0.to(pool_dtype).clone() for _ in range(2)]
+    raw = fq.chunk_gated_delta_rule_fwd(
+        3 * q, 2 * k, v, g, beta, initial_state=pools[0], initial_state_indices=slots, final_state_out=pools[0],
+        final_state_indices=slots, cu_seqlens=cu, transpose_state_layout=True, use_qk_l2norm_in_kernel=True, **gate)
+    o, _ = fq.prefill_into_state_pool(3 * q, 2 * k, v, g, beta, pools[1], slots, cu_seqlens=cu, continue_from_pool=True,
+                                      use_qk_l2norm_in_kernel=True, **gate)
+    fq.check_device_status()
+    assert close(o, raw[2], torch.bfloat16) and close(pools[1], pools[0], torch.bfloat16)
+    rest = torch.ones(len(h0), dtype=torch.bool, device="cuda")
+    rest[slots[1:].long()] = False
+    assert torch.equal(pools[1][rest], h0.to(pool_dtype)[rest])
