@@ -256,19 +256,17 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __shared__ float w_factor[kWIn ? 4 : 1][64];  // kWIn: -exp(g) / |k|, ring by chunk: A diag(beta) times this is the operand of Wt
   constexpr uint32_t kPgTiles = kWIn ? kOffPgWIn : kOffPg, kOTiles = kWIn ? kOffOWIn : kOffO;
 
-  if (tid == 0) {
-#pragma unroll 1
-    for (int b = 0; b < kNumBars; ++b) {
-      int count = 1;  // kFull*, kEmpty*, kKaEmpty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
-      if (b == kAbReady0 || b == kAbReady1 || b == kAwReady || (b >= kKaFull0 && b <= kKaFull2)) count = 2;
-      else if (b == kPgReady || b == kORead || b == kOReady || b == kVnRead || b == kVnReady || b == kHRead ||
-               b == kHReady || b == kWRead || b == kWReady || b == kD0Read)
-        count = 4;
-      else if (b == kVdReady || b == kVdStored || b == kSbfReady || b == kSScaled || b == kONormed) count = 8;
-      ptx::mbar_init(&bars[b], count);
-    }
+  if (tid < (kWIn ? kNumBars : kKaFull0)) {  // (a thread each: one after the other they were 0.5 us of a CTA's start)
+    const int b = tid;
+    int count = 1;  // kFull*, kEmpty*, kKaEmpty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
+    if (b == kAbReady0 || b == kAbReady1 || b == kAwReady || (b >= kKaFull0 && b <= kKaFull2)) count = 2;
+    else if (b == kPgReady || b == kORead || b == kOReady || b == kVnRead || b == kVnReady || b == kHRead ||
+             b == kHReady || b == kWRead || b == kWReady || b == kD0Read)
+      count = 4;
+    else if (b == kVdReady || b == kVdStored || b == kSbfReady || b == kSScaled || b == kONormed) count = 8;
+    ptx::mbar_init(&bars[b], count);
     ptx::fence_mbar_init();
-    ptx::mbar_wait_setup(p.status, bars, 0);
+    if (tid == 0) ptx::mbar_wait_setup(p.status, bars, 0);
   }
   if (!kStateOnly && warp >= 12) {  // the block of Pg above the diagonal (rows 0..31, columns 32..63) of both tiles
     for (int x = tid - 384; x < 2 * 32 * 4; x += 128)
