@@ -19,6 +19,7 @@ device-to-host copy.
 """
 from __future__ import annotations
 
+import heapq
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -50,6 +51,16 @@ class CpPlan:
 _PLAN_CACHE: Dict[Tuple, CpPlan] = {}
 
 
+def _uncut_makespan(chunks: Sequence[int], num_v_heads: int, num_sms: int) -> int:
+    """Chunks until the last SM is through when every sequence and head is one chain, longest sequences first, each on the SM
+    that is free first (which is how the scan starts them)."""
+    busy = [0] * num_sms
+    for c in sorted(chunks, reverse=True):
+        for _ in range(num_v_heads):
+            heapq.heapreplace(busy, busy[0] + c)
+    return max(busy)
+
+
 def plan_segments(lens: Sequence[int], num_v_heads: int, num_sms: int = 148) -> CpPlan:
     """Decide whether to cut sequences and where.  Pure function of lengths, head count, SM count."""
     chunks = [(n + CHUNK - 1) // CHUNK for n in lens]
@@ -65,9 +76,7 @@ def plan_segments(lens: Sequence[int], num_v_heads: int, num_sms: int = 148) -> 
         cost = rounds * (longest + WARMUP_COST * min(WARMUP_CHUNKS, longest))
         if best is None or cost < best:
             best, seg = cost, cand
-    # rounds of the longest sequence: too much for several unequal ones, which start longest first
-    uncut = -(-chains // num_sms) * max(chunks)
-    if best is None or best >= uncut:
+    if best is None or best >= _uncut_makespan(chunks, num_v_heads, num_sms):
         return CpPlan(use_cp=False)
     cu, seg_next, seg_raw, raw_first = [0], [], [], [0]
     start = 0
