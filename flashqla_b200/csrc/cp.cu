@@ -10,7 +10,6 @@
 //           K x K transition matrix M of the segment is needed as well.
 //   chain : for fallback entries  h0[seg + 1] += M[seg] * h0[seg], in segment order.
 #include "chunk_params.cuh"
-#include "warp_pieces.cuh"
 
 namespace qla {
 namespace {
@@ -149,39 +148,73 @@ __global__ void __launch_bounds__(kPlanThreads) cp_plan_lead_kernel(const QlaCpP
 }
 
 // The chain  h[next] += M[seg] h[seg]  over the segments of one sequence and head, in order.  A link is a dependent
-// 128 x 128 by 128 x 8 product: the columns are split over CTAs (8 each), the matrices of the next links are already on
-// their way into shared memory while one is multiplied (they are read once per CTA, from L2), and the carried columns
-// stay in shared memory.  32 segments of one sequence: 36 us; with 32-column slabs, rows read from global memory in
-// front of every product, the same chain took 950 us.
+// 128 x 128 by 128 x 8 product: the columns are split over CTAs (8 each), warp w of a CTA has rows 16 w .. 16 w + 15.  The
+// product runs on mma.sync with both operands split into two TF32 values (hi hi + hi lo + lo hi: 2^-22 of a product, beside
+// fp32 sums of 128 terms).  A warp's rows of M come straight from global memory (L2) as fragments, those of the next
+// link while this one is multiplied; the carried columns pass through shared memory, split by the thread that
+// formed them, in two buffers: one barrier per link.  What bounds it: 64 KB of M per link and CTA, L2 to SM (40 bytes per ns
+// and SM).  36 links of 4 heads take 59 us; with fp32 products from shared memory and seven barriers per link they took 96.
 constexpr int kChainCols = 8;
-constexpr int kChainStride = kHeadDim + 4;  // floats per row of M: 16-byte rows, conflict-free float4 reads
+constexpr int kChainStride = 144;  // floats from column to column of the carried state: conflict-free float4 fragments
 constexpr int kChainThreads = 256;
 constexpr int kChainFlags = 256;
-constexpr size_t kChainSmem = (2 * kHeadDim * kChainStride + 3 * kHeadDim * kChainCols) * sizeof(float);
 
-__global__ void __launch_bounds__(kChainThreads) cp_chain_kernel(float* __restrict__ h0, const float* __restrict__ M,
-                                                                 const int32_t* __restrict__ m_limit,
-                                                                 const int32_t* __restrict__ raw_first_seg, int num_heads,
-                                                                 int reverse) {
+// x = hi + lo, both TF32 (Veltkamp's splitting; lo loses what lies below 2^-22 of x)
+__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
+  const float c = __fmul_rn(x, 8193.f);
+  hi = __fsub_rn(c, __fsub_rn(c, x));
+  lo = __uint_as_float(__float_as_uint(__fsub_rn(x, hi)) & 0xffffe000u);
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const float (&a)[4], float b0, float b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+        "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+
+__global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __restrict__ h0, const float* __restrict__ M,
+                                                                    const int32_t* __restrict__ m_limit,
+                                                                    const int32_t* __restrict__ raw_first_seg, int num_heads,
+                                                                    int reverse) {
   grid_dep_wait();
   grid_dep_launch();
   const int c0 = blockIdx.x * kChainCols, h = blockIdx.y, r = blockIdx.z, tid = threadIdx.x;
   const int s0 = raw_first_seg[r], links = raw_first_seg[r + 1] - s0 - 1;
-  extern __shared__ __align__(16) float chain_smem[];
-  float* sM[2] = {chain_smem, chain_smem + kHeadDim * kChainStride};
-  float* sH = chain_smem + 2 * kHeadDim * kChainStride;  // the carried columns [128][8]
-  float* sP = sH + kHeadDim * kChainCols;                // partial sums [2][128][8]
+  __shared__ __align__(16) float s_h[2][2][kChainCols * kChainStride];  // [buffer][hi | lo][column][row]
   __shared__ int flags[kChainFlags];
   // link i leads from segment seg_of(i) to seg_of(i + 1)
   auto seg_of = [&](int i) { return reverse ? s0 + links - i : s0 + i; };
-  auto state_of = [&](int i) { return h0 + (static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim * kHeadDim + c0; };
-  auto load_m = [&](int i, int buf) {
-    const float* m = M + (static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim * kHeadDim;
-    for (int e = tid; e < kHeadDim * 32; e += kChainThreads)
-      mm::cp_async16(sM[buf] + (e >> 5) * kChainStride + (e & 31) * 4, m + e * 4, true);
+  const int warp = tid >> 5, g = (tid & 31) >> 2, c = tid & 3;
+  // this thread's values of a state: rows row and row + 8, columns c0 + 2 c, + 1 (fragment of the product's accumulator)
+  const int row = 16 * warp + g;
+  auto state_of = [&](int i) {
+    return h0 + (static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim * kHeadDim + row * kHeadDim + c0 + 2 * c;
   };
-  // thread: rows row, row + 32, row + 64, row + 96, columns cq .. cq + 3, a quarter of the inner dimension
-  const int row = tid & 31, cq = ((tid >> 5) & 1) * 4, jq = tid >> 6;
+  auto load_state = [&](int i, float (&x)[4]) {
+    const float* s = state_of(i);
+    const float2 lo = *reinterpret_cast<const float2*>(s), hi = *reinterpret_cast<const float2*>(s + 8 * kHeadDim);
+    x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
+  };
+  auto carry = [&](int buf, const float (&x)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float hi, lo;
+      split_tf32(x[e], hi, lo);
+      const int at = (2 * c + (e & 1)) * kChainStride + row + 8 * (e >> 1);
+      s_h[buf][0][at] = hi;
+      s_h[buf][1][at] = lo;
+    }
+  };
+  // Rows row and row + 8 of M, columns 16 t + 4 c .. + 3: values 0, 1 are slots c, c + 4 of k-step 2 t, values 2, 3 of 2 t + 1.
+  float4 raw[8][2];
+  auto load_m = [&](int i) {
+    const float* m = M + ((static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim + row) * kHeadDim + 4 * c;
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) raw[t][x] = *reinterpret_cast<const float4*>(m + 8 * x * kHeadDim + 16 * t);
+  };
+  int buf = 0;
   for (int b0 = 0; b0 < links; b0 += kChainFlags) {
     const int nb = min(kChainFlags, links - b0);
     int mine = 0;
@@ -189,77 +222,63 @@ __global__ void __launch_bounds__(kChainThreads) cp_chain_kernel(float* __restri
     for (int i = tid; i < nb; i += kChainThreads) mine |= (flags[i] = m_limit[seg_of(b0 + i) * num_heads + h]);
     // the usual case (every segment decays below the threshold) has nothing to chain
     if (__syncthreads_or(mine) == 0) continue;
-    int buf = 0;
     bool have_h = false;
-    if (flags[0] != 0) load_m(b0, 0);
-    mm::cp_async_commit();
-    for (int i = 0; i < nb; ++i, buf ^= 1) {
-      if (i + 1 < nb && flags[i + 1] != 0) load_m(b0 + i + 1, buf ^ 1);
-      mm::cp_async_commit();
+    float add[4] = {0.f, 0.f, 0.f, 0.f};  // the next state as it is: what the product is added to
+    if (flags[0] != 0) {
+      load_m(b0);
+      load_state(b0 + 1, add);
+    }
+    for (int i = 0; i < nb; ++i) {
+      const bool next = i + 1 < nb && flags[i + 1] != 0;
       if (flags[i] == 0) {  // (uniform)
         have_h = false;
+        if (next) {
+          load_m(b0 + i + 1);
+          load_state(b0 + i + 2, add);
+        }
         continue;
       }
-      const int e4 = tid * 4, er = e4 / kChainCols, ec = e4 & (kChainCols - 1);  // this thread's 4 of the 1024 values
-      float4 add = *reinterpret_cast<const float4*>(state_of(b0 + i + 1) + er * kHeadDim + ec);
-      if (!have_h) *reinterpret_cast<float4*>(sH + e4) = *reinterpret_cast<const float4*>(state_of(b0 + i) + er * kHeadDim + ec);
+      if (!have_h) {
+        float x[4];
+        load_state(b0 + i, x);
+        carry(buf, x);
+      }
       have_h = true;
-      mm::cp_async_wait<1>();
-      __syncthreads();
-      float acc[4][4] = {};
-#pragma unroll 2
-      for (int j = jq * 32; j < jq * 32 + 32; j += 4) {
-        float4 m[4], x[4];
+      float mh[16][4], ml[16][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          m[q] = *reinterpret_cast<const float4*>(sM[buf] + (row + 32 * q) * kChainStride + j);
-          x[q] = *reinterpret_cast<const float4*>(sH + (j + q) * kChainCols + cq);
-        }
+      for (int t = 0; t < 8; ++t) {
+        const float a[8] = {raw[t][0].x, raw[t][1].x, raw[t][0].y, raw[t][1].y, raw[t][0].z, raw[t][1].z, raw[t][0].w, raw[t][1].w};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float mv[4] = {m[q].x, m[q].y, m[q].z, m[q].w};
-#pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            acc[q][0] = fmaf(mv[y], x[y].x, acc[q][0]);
-            acc[q][1] = fmaf(mv[y], x[y].y, acc[q][1]);
-            acc[q][2] = fmaf(mv[y], x[y].z, acc[q][2]);
-            acc[q][3] = fmaf(mv[y], x[y].w, acc[q][3]);
-          }
-        }
+        for (int e = 0; e < 8; ++e) split_tf32(a[e], mh[2 * t + (e >> 2)][e & 3], ml[2 * t + (e >> 2)][e & 3]);
       }
-      // the four quarters of the inner dimension: 2, 3 hand over to 0, 1, then 1 to 0 (fixed order)
-#pragma unroll
-      for (int half = 2; half > 0; half >>= 1) {
-        __syncthreads();
-        if (jq >= half && jq < 2 * half) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            *reinterpret_cast<float4*>(sP + ((jq - half) * kHeadDim + row + 32 * q) * kChainCols + cq) =
-                make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
-        }
-        __syncthreads();
-        if (jq < half) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 p = *reinterpret_cast<const float4*>(sP + (jq * kHeadDim + row + 32 * q) * kChainCols + cq);
-            acc[q][0] += p.x; acc[q][1] += p.y; acc[q][2] += p.z; acc[q][3] += p.w;
-          }
-        }
+      float out[4] = {add[0], add[1], add[2], add[3]};
+      if (next) {
+        load_m(b0 + i + 1);
+        load_state(b0 + i + 2, add);
       }
-      if (jq == 0) {
+      __syncthreads();  // the carried columns are complete
+      float acc[2][3][4] = {};
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<float4*>(sP + (kHeadDim + row + 32 * q) * kChainCols + cq) =
-              make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+      for (int t = 0; t < 8; ++t) {
+        const float4 xh = *reinterpret_cast<const float4*>(&s_h[buf][0][g * kChainStride + 16 * t + 4 * c]);
+        const float4 xl = *reinterpret_cast<const float4*>(&s_h[buf][1][g * kChainStride + 16 * t + 4 * c]);
+        mma_tf32(acc[0][0], ml[2 * t], xh.x, xh.y);
+        mma_tf32(acc[0][1], mh[2 * t], xl.x, xl.y);
+        mma_tf32(acc[0][2], mh[2 * t], xh.x, xh.y);
+        mma_tf32(acc[1][0], ml[2 * t + 1], xh.z, xh.w);
+        mma_tf32(acc[1][1], mh[2 * t + 1], xl.z, xl.w);
+        mma_tf32(acc[1][2], mh[2 * t + 1], xh.z, xh.w);
       }
-      __syncthreads();
-      const float4 p = *reinterpret_cast<const float4*>(sP + kHeadDim * kChainCols + e4);
-      add.x += p.x; add.y += p.y; add.z += p.z; add.w += p.w;
-      *reinterpret_cast<float4*>(sH + e4) = add;
-      *reinterpret_cast<float4*>(state_of(b0 + i + 1) + er * kHeadDim + ec) = add;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        out[e] += ((acc[0][0][e] + acc[1][0][e]) + (acc[0][1][e] + acc[1][1][e])) + (acc[0][2][e] + acc[1][2][e]);
+      buf ^= 1;
+      carry(buf, out);
+      float* dst = state_of(b0 + i + 1);
+      *reinterpret_cast<float2*>(dst) = make_float2(out[0], out[1]);
+      *reinterpret_cast<float2*>(dst + 8 * kHeadDim) = make_float2(out[2], out[3]);
     }
-    mm::cp_async_wait<0>();
-    __threadfence_block();  // a link behind this batch reads the state written last (by the same thread)
+    // (a link behind this batch reads the state written last, each value by the thread that wrote it)
   }
 }
 
@@ -291,8 +310,7 @@ extern "C" QLA_API int qla_cp_chain(const QlaCpChainArgs* a, void* stream) {
   QLA_CHECK_ARG(a != nullptr && a->h0 && a->M && a->m_limit && a->raw_first_seg, "NULL pointer in QlaCpChainArgs");
   QLA_CHECK_ARG(a->num_raw_seqs > 0 && a->num_v_heads > 0, "bad sizes");
   dim3 grid(kHeadDim / kChainCols, a->num_v_heads, a->num_raw_seqs);
-  { const int rc = ensure_dynamic_smem<cp_chain_kernel>(kChainSmem); if (rc != QLA_OK) return rc; }
-  QLA_CHECK_CUDA(launch_dependent(cp_chain_kernel, grid, dim3(kChainThreads), kChainSmem, static_cast<cudaStream_t>(stream), a->h0, a->M,
+  QLA_CHECK_CUDA(launch_dependent(cp_chain_kernel, grid, dim3(kChainThreads), 0, static_cast<cudaStream_t>(stream), a->h0, a->M,
                                   a->m_limit, a->raw_first_seg, a->num_v_heads, a->reverse));
   return QLA_OK;
 }

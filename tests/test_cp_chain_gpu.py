@@ -1,0 +1,38 @@
+"""The chain of segment states h[s + 1] += M[s] h[s] (``qla_cp_chain``) by itself, against 64 bits: one link, links that are left out,
+either direction, several sequences, and more links than the kernel looks at in one batch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("segments, skip, reverse", [
+    ([2], [], False),
+    ([5, 1, 3], [], False),
+    ([5, 1, 3], [1], True),
+    ([38], [0, 7, 8, 20], False),
+    ([300], [255, 256], False),   # the kernel takes 256 flags at a time
+    ([300], [40, 43], True),
+])
+def test_chain(segments, skip, reverse):
+    from flashqla_b200 import _cabi
+    Hv, n = 2, sum(segments)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    h = torch.randn(n, Hv, 128, 128, generator=gen, device="cuda")
+    M = torch.randn(n, Hv, 128, 128, generator=gen, device="cuda") * (0.9 / 128 ** 0.5)
+    limit = torch.ones(n, Hv, dtype=torch.int32, device="cuda")
+    limit[skip, 0] = 0  # (of one head only)
+    first = torch.tensor([0] + segments).cumsum(0).int().cuda()
+    ref = h.double()
+    for a, b in zip(first.tolist()[:-1], first.tolist()[1:]):
+        order = list(range(a, b))
+        order = order[::-1] if reverse else order
+        for s, t in zip(order[:-1], order[1:]):
+            for hd in range(Hv):
+                if limit[s, hd]:
+                    ref[t, hd] += M[s, hd].double() @ ref[s, hd]
+    args = _cabi.QlaCpChainArgs(num_raw_seqs=len(segments), num_v_heads=Hv, h0=h.data_ptr(), M=M.data_ptr(),
+                                m_limit=limit.data_ptr(), raw_first_seg=first.data_ptr(), reverse=int(reverse))
+    _cabi.check(_cabi.lib().qla_cp_chain(args, _cabi.current_stream(h.device)), "qla_cp_chain")
+    # a product loses up to 2^-21 of itself to the splitting, sums of 128 in fp32; |M| |h| is up to ten times |M h| here
+    assert float((h.double() - ref).norm() / ref.norm()) <= 1e-5
