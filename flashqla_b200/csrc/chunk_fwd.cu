@@ -24,8 +24,9 @@
 // Between two state updates only  MMA2 -> (V' = rho .* Vd) -> MMA3 -> (16-bit copy of the state)  are
 // serial; the other products are issued into the two gaps and complete in their shadow.
 //
-// What bounds it: that chain (about 1500 cycles of tensor-pipe time and hand-offs per chunk), and the traffic of
-// shared memory beside it: 72 KB of TMA writes and 112 KB of operand reads per chunk at 128 bytes a cycle.  Operands
+// What bounds it: that chain (1.6 us per chunk with the SM to itself: 1700 cycles of products in order, and hand-offs between
+// 20 warps that share its issue slots), and with every SM busy the memory behind it (36 - 38 bytes per ns and SM).
+// Shared memory moves 72 KB of TMA writes and 112 KB of operand reads per chunk at 128 bytes a cycle.  Operands
 // that a thread produces therefore go to tensor memory (Vd as a shared-memory tile cost 48 KB per chunk), and Q K^T is
 // not stacked on other rows to fill M = 128.  All roles share the SM's instruction cache (32 KB; 94 % of its requests hit),
 // so that code which is not needed costs even where it is not executed often: see kState16.
@@ -35,8 +36,10 @@
 //
 // Warp roles (640 threads): warps 0-7 the chain (two warpgroups: tokens 0..31 | 32..63 of Vd, columns 0..63 | 64..127
 // of the state conversion), warp 8 TMA producer + gate vectors, warp 9 MMA issuer, warps 10, 11 A diag(beta) of the
-// next chunk, warps 12-15 the output, warps 16-19 Pg.  Two smem stages of {Wt,Q,K,V,A}, a four-deep ring of gate vectors; all
-// waits are bounded mbarrier waits that raise a status word instead of hanging.
+// next chunk, warps 12-15 the output, warps 16-19 Pg.  Two smem stages of {Wt,Q}, {K} and {V,A}, each reloaded as soon as its last
+// product has read it (with the whole stage waiting for MMA3, and Q K^T behind MMA4: 512 chains of 32 chunks, 8 / 8 heads,
+// 306 us, now 287; with the output norm 379 -> 366), a four-deep ring of gate vectors; all waits are bounded mbarrier
+// waits that raise a status word instead of hanging.
 #include "chunk_params.cuh"
 
 namespace qla {
@@ -96,6 +99,8 @@ enum Bar {
   // kWIn: {K, A} stages (kFull*, kEmpty* are those of {Q, V}), operand of Wt written, Wt in tensor memory, read from there,
   // written to its tile, Q K^T read from the columns that Wt uses next
   kKaFull0, kKaFull1, kKaFull2, kKaEmpty0, kKaEmpty1, kKaEmpty2, kAwReady, kWDone, kWRead, kWReady, kD0Read,
+  // otherwise: {V, A} and K of a stage (kFull*, kEmpty* are those of {Wt, Q})
+  kVaFull0, kVaFull1, kVaEmpty0, kVaEmpty1, kKFull0, kKFull1, kKEmpty0, kKEmpty1,
   kNumBars
 };
 
@@ -256,9 +261,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __shared__ float w_factor[kWIn ? 4 : 1][64];  // kWIn: -exp(g) / |k|, ring by chunk: A diag(beta) times this is the operand of Wt
   constexpr uint32_t kPgTiles = kWIn ? kOffPgWIn : kOffPg, kOTiles = kWIn ? kOffOWIn : kOffO;
 
-  if (tid < (kWIn ? kNumBars : kKaFull0)) {  // (a thread each: one after the other they were 0.5 us of a CTA's start)
+  if (tid < kNumBars) {  // (a thread each: one after the other they were 0.5 us of a CTA's start)
     const int b = tid;
-    int count = 1;  // kFull*, kEmpty*, kKaEmpty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
+    int count = 1;  // k*Full*, k*Empty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
     if (b == kAbReady0 || b == kAbReady1 || b == kAwReady || (b >= kKaFull0 && b <= kKaFull2)) count = 2;
     else if (b == kPgReady || b == kORead || b == kOReady || b == kVnRead || b == kVnReady || b == kHRead ||
              b == kHReady || b == kWRead || b == kWReady || b == kD0Read)
@@ -319,181 +324,144 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // =========================================================== TMA producer, gate vectors
     // L2 prefetch runs kPrefetchAhead chunks ahead of the demand loads: with every SM streaming its own
     // sequence the DRAM latency of a tile exceeds one chunk period, and only two stages fit in shared
-    // memory, so the tiles are pulled into L2 early and the demand TMA then hits L2.  The gate scalars are requested
-    // before the wait for the stage: their global-memory latency overlaps it.
+    // memory, so the tiles are pulled into L2 early and the demand TMA then hits L2.
+    // Tiles are reloaded as their last product has read them.  kWIn: {Q, V} of chunk i behind MMAq of chunk i - 2, {K, A} of chunk i + 1
+    // behind MMA3 of chunk i - 2.  Otherwise {Wt, Q} of chunk i behind MMAq and K behind MMA3 of chunk i - 2, {V, A} of chunk i + 1
+    // behind MMAu of chunk i - 1.  Gate vectors of chunk i follow when MMA3 of chunk i - 2 is through: the last readers of their ring
+    // slot (the output of chunk i - 4, which MMA4 of chunk i - 3 waited for) have left it.  Their scalars are requested a chunk before.
     constexpr int kPrefetchAhead = 4;
     const float log2e = 1.4426950408889634f;
-    if constexpr (kWIn) {
-      // {K, A} and the factors of Wt run one chunk ahead of {Q, V} and the gate vectors: chunk i + 1 of the former is loaded when
-      // MMA3 of chunk i - 2 is through, chunk i of the latter when MMAq of chunk i - 2 is.
-      float g[2], gl = 0.f;
-      float2 rn[2];
-      auto fetch = [&](int i) {
-        const int t0 = seq_start + (first_chunk + i) * kChunk;
-        const int valid = min(kChunk, seq_end - t0);
-        const int64_t row = static_cast<int64_t>(t0) * p.num_v_heads + hv;
-        gl = p.g_cumsum[row + (valid - 1) * p.num_v_heads];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const int c = min(lane + 32 * r, valid - 1);  // rows past the end repeat the last gate
-          g[r] = p.g_cumsum[row + c * p.num_v_heads];
-          rn[r] = make_float2(1.f, 1.f);
-          if (p.rnorm != nullptr)
-            rn[r] = *reinterpret_cast<const float2*>(p.rnorm + ((static_cast<int64_t>(t0) + c) * p.num_k_heads + hk) * 2);
-        }
-      };
-      auto load_ka = [&](int c, int slot) {
-        if (lane == 0) {
-          uint8_t* st = smem + kOffKa + slot * kKaBytes;
-          uint64_t* full = &bars[kKaFull0 + slot];
-          const int t0 = seq_start + (first_chunk + c) * kChunk;
-          ptx::mbar_expect_tx(full, kKaBytes);
-          ptx::tma_load_4d(st, &tm_k, full, 0, hk, t0, 0);
-          ptx::tma_load_3d(st + kKaA, &tm_a, full, 0, hv, t0);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < 2; ++r) w_factor[c & 3][lane + 32 * r] = -ptx::ex2(g[r] * log2e) * rn[r].y;
-        warp_arrive(&bars[kKaFull0 + slot], lane);
-      };
-      if (nproc > 0) {
-        fetch(0);
-        load_ka(0, 0);
-      }
-      int slot = 1, ka_phase = 1;  // of chunk i + 1: ring slot, and parity of its last release (none before chunk 3)
-#pragma unroll 1
-      for (int i = 0; i < nproc; ++i) {
-        const int s = i & 1;
-        const int t0 = seq_start + (first_chunk + i) * kChunk;
-        const int valid = min(kChunk, seq_end - t0);
-        const float gi[2] = {g[0], g[1]}, gli = gl;
-        const float2 rni[2] = {rn[0], rn[1]};
-        if (i + 1 < nproc) fetch(i + 1);  // (requested before the wait for the stage)
-        if (i >= 2 && !wait(kEmpty0 + s, ((i >> 1) - 1) & 1)) break;
-        if (lane == 0) {
-          uint8_t* st = smem + s * kQvBytes;
-          uint64_t* full = &bars[kFull0 + s];
-          ptx::mbar_expect_tx(full, (kStateOnly ? 0 : 16384) + (zero_v ? 0 : 16384));
-          if (!zero_v) ptx::tma_load_4d(st + kQvV, &tm_v, full, 0, hv, t0, 0);
-          if (!kStateOnly) ptx::tma_load_4d(st, &tm_q, full, 0, hk, t0, 0);
-        }
-        __syncwarp();
-        Gates* gs = gates_of(i);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const int c = lane + 32 * r;
-          const float g2 = gi[r] * log2e;
-          gs->g2row[c] = g2 + ptx::lg2(rni[r].x);
-          gs->g2col[c] = g2 - ptx::lg2(rni[r].y);
-          gs->sgamma[c] = p.scale * ptx::ex2(g2) * rni[r].x;
-          gs->rho[c] = c < valid ? ptx::ex2((gli - gi[r]) * log2e) * rni[r].y : 0.f;
-        }
-        gs->egl = ptx::ex2(gli * log2e);
-        gs->valid = valid;
-        warp_arrive(&bars[kGate0 + (i & 3)], lane);
-        if (i + 1 < nproc) {
-          if (i >= 2 && !wait(kKaEmpty0 + slot, ka_phase)) break;
-          load_ka(i + 1, slot);
-          if (++slot == kKaStages) {
-            slot = 0;
-            ka_phase ^= 1;
-          }
-        }
-        if (lane == 0) {
-          // the first demand loads go out before any prefetch; the prefetches of chunks 2.. follow chunk 1
-#pragma unroll 1
-          for (int c = (i == 1) ? 2 : i + kPrefetchAhead; i >= 1 && c <= i + kPrefetchAhead && c < nproc; ++c) {
-            const int pt0 = seq_start + (first_chunk + c) * kChunk;
-            ptx::tma_prefetch_l2_4d(&tm_k, 0, hk, pt0, 0);
-            ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
-            if (!zero_v) ptx::tma_prefetch_l2_4d(&tm_v, 0, hv, pt0, 0);
-            if (!kStateOnly) ptx::tma_prefetch_l2_4d(&tm_q, 0, hk, pt0, 0);
-          }
-        }
-        // the gate scalars of the chunk that many ahead as well
-        if (i + kPrefetchAhead < nproc) {
-          const int64_t ahead = static_cast<int64_t>(t0) + kPrefetchAhead * kChunk;
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const int64_t tk = min(ahead + lane + 32 * r, static_cast<int64_t>(seq_end) - 1);
-            ptx::prefetch_l2(p.g_cumsum + tk * p.num_v_heads + hv);
-            if (p.rnorm != nullptr) ptx::prefetch_l2(p.rnorm + (tk * p.num_k_heads + hk) * 2);
-          }
-        }
-        __syncwarp();
-      }
-    } else
-#pragma unroll 1
-    for (int i = 0; i < nproc; ++i) {
-      const int s = i & 1;
+    struct Scalars {
+      float g[2], b[2], gl;
+      float2 rn[2];  // (1 / |q|, 1 / |k|)
+    };
+    auto fetch = [&](int i, Scalars& x) {
       const int t0 = seq_start + (first_chunk + i) * kChunk;
       const int valid = min(kChunk, seq_end - t0);
       const int64_t row = static_cast<int64_t>(t0) * p.num_v_heads + hv;
-      float g[2], b[2];
-      float2 rn[2];  // (1 / |q|, 1 / |k|)
-      const float gl = p.g_cumsum[row + (valid - 1) * p.num_v_heads];
+      x.gl = p.g_cumsum[row + (valid - 1) * p.num_v_heads];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int c = min(lane + 32 * r, valid - 1);  // rows past the end repeat the last gate
         const int64_t at = row + c * p.num_v_heads;
-        g[r] = p.g_cumsum[at];
-        b[r] = load_scalar(p.beta, p.beta_dtype, at);
-        rn[r] = make_float2(1.f, 1.f);
+        x.g[r] = p.g_cumsum[at];
+        if (!kWIn) x.b[r] = load_scalar(p.beta, p.beta_dtype, at);
+        x.rn[r] = make_float2(1.f, 1.f);
         if (p.rnorm != nullptr)
-          rn[r] = *reinterpret_cast<const float2*>(p.rnorm + ((static_cast<int64_t>(t0) + c) * p.num_k_heads + hk) * 2);
+          x.rn[r] = *reinterpret_cast<const float2*>(p.rnorm + ((static_cast<int64_t>(t0) + c) * p.num_k_heads + hk) * 2);
       }
-      trace(0, i, 9);
-      if (i >= 2 && !wait(kEmpty0 + s, ((i >> 1) - 1) & 1)) break;
-      trace(0, i, 10);
-      if (lane == 0) {
-        uint8_t* st = stage_ptr(s);
-        uint32_t bytes = 16384 + 8192 + 16384;  // K + A + Wt
-        if (!kStateOnly) bytes += 16384;  // Q
-        if (!zero_v) bytes += 16384;    // V
-        uint64_t* full = &bars[kFull0 + s];
-        ptx::mbar_expect_tx(full, bytes);
-        ptx::tma_load_3d(st + kStageA, &tm_a, full, 0, hv, t0);
-        if (!zero_v) ptx::tma_load_4d(st + kStageV, &tm_v, full, 0, hv, t0, 0);
-        ptx::tma_load_4d(st + kStageWQ, &tm_w, full, 0, hv, t0, 0);
-        if (!kStateOnly) ptx::tma_load_4d(st + kStageWQ + 16384, &tm_q, full, 0, hk, t0, 0);
-        ptx::tma_load_4d(st + kStageK, &tm_k, full, 0, hk, t0, 0);
+    };
+    auto put_w_factor = [&](int c, int slot, const Scalars& x) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) w_factor[c & 3][lane + 32 * r] = -ptx::ex2(x.g[r] * log2e) * x.rn[r].y;
+      warp_arrive(&bars[kKaFull0 + slot], lane);
+    };
+    auto token_of = [&](int c) { return seq_start + (first_chunk + c) * kChunk; };
+    auto load_early = [&](int c, int slot) {  // what a chunk needs first
+      if (lane == 0 && kWIn) {
+        uint8_t* st = smem + kOffKa + slot * kKaBytes;
+        uint64_t* full = &bars[kKaFull0 + slot];
+        ptx::mbar_expect_tx(full, kKaBytes);
+        ptx::tma_load_4d(st, &tm_k, full, 0, hk, token_of(c), 0);
+        ptx::tma_load_3d(st + kKaA, &tm_a, full, 0, hv, token_of(c));
+      } else if (lane == 0 && !zero_v) {
+        uint8_t* st = stage_ptr(slot);
+        uint64_t* full = &bars[kVaFull0 + slot];
+        ptx::mbar_expect_tx(full, 8192 + 16384);
+        ptx::tma_load_3d(st + kStageA, &tm_a, full, 0, hv, token_of(c));
+        ptx::tma_load_4d(st + kStageV, &tm_v, full, 0, hv, token_of(c), 0);
       }
       __syncwarp();
+    };
+    Scalars cur = {}, nxt = {};
+    if (nproc > 0) {
+      load_early(0, 0);
+      fetch(0, cur);
+    }
+    int slot = 1, phase = 1;  // of chunk i + 1's early tiles: ring slot, and parity of its last release
+#pragma unroll 1
+    for (int i = 0; i < nproc; ++i) {
+      const int s = i & 1;
+      trace(0, i, 9);
+      if (i + 1 < nproc) fetch(i + 1, nxt);
+      if (i >= 2 && !wait(kEmpty0 + s, ((i >> 1) - 1) & 1)) break;
+      if (lane == 0) {
+        uint64_t* full = &bars[kFull0 + s];
+        if (kWIn) {
+          uint8_t* st = smem + s * kQvBytes;
+          ptx::mbar_expect_tx(full, (kStateOnly ? 0 : 16384) + (zero_v ? 0 : 16384));
+          if (!zero_v) ptx::tma_load_4d(st + kQvV, &tm_v, full, 0, hv, token_of(i), 0);
+          if (!kStateOnly) ptx::tma_load_4d(st, &tm_q, full, 0, hk, token_of(i), 0);
+        } else {
+          uint8_t* st = stage_ptr(s) + kStageWQ;
+          ptx::mbar_expect_tx(full, kStateOnly ? 16384 : 32768);
+          if (!kStateOnly) ptx::tma_load_4d(st + 16384, &tm_q, full, 0, hk, token_of(i), 0);
+          ptx::tma_load_4d(st, &tm_w, full, 0, hv, token_of(i), 0);
+        }
+      }
+      __syncwarp();
+      if (!kWIn) {
+        if (i >= 2 && !wait(kKEmpty0 + s, ((i >> 1) - 1) & 1)) break;
+        if (lane == 0) {
+          uint64_t* full = &bars[kKFull0 + s];
+          ptx::mbar_expect_tx(full, 16384);
+          ptx::tma_load_4d(stage_ptr(s) + kStageK, &tm_k, full, 0, hk, token_of(i), 0);
+        }
+        __syncwarp();
+      }
+      trace(0, i, 10);
+      if (i + 1 < nproc) {
+        if (kWIn) {
+          if (i >= kKaStages - 1 && !wait(kKaEmpty0 + slot, phase)) break;
+        } else if (i >= 1 && !zero_v && !wait(kVaEmpty0 + slot, phase)) {
+          break;
+        }
+        load_early(i + 1, slot);
+      }
+      if (kWIn && i == 0) put_w_factor(0, 0, cur);
+      const int valid = min(kChunk, seq_end - token_of(i));
       Gates* gs = gates_of(i);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int c = lane + 32 * r;
         const bool ok = c < valid;
-        const float g2 = g[r] * log2e;
-        gs->g2row[c] = g2 + ptx::lg2(rn[r].x);
-        gs->g2col[c] = g2 - ptx::lg2(rn[r].y);
-        gs->sgamma[c] = p.scale * ptx::ex2(g2) * rn[r].x;
-        gs->rho[c] = ok ? ptx::ex2((gl - g[r]) * log2e) * rn[r].y : 0.f;
-        gs->beta[c] = ok ? b[r] : 0.f;
+        const float g2 = cur.g[r] * log2e;
+        gs->g2row[c] = g2 + ptx::lg2(cur.rn[r].x);
+        gs->g2col[c] = g2 - ptx::lg2(cur.rn[r].y);
+        gs->sgamma[c] = p.scale * ptx::ex2(g2) * cur.rn[r].x;
+        gs->rho[c] = ok ? ptx::ex2((cur.gl - cur.g[r]) * log2e) * cur.rn[r].y : 0.f;
+        if (!kWIn) gs->beta[c] = ok ? cur.b[r] : 0.f;
       }
-      gs->egl = ptx::ex2(gl * log2e);
+      gs->egl = ptx::ex2(cur.gl * log2e);
       gs->valid = valid;
       warp_arrive(&bars[kGate0 + (i & 3)], lane);
+      if (i + 1 < nproc) {
+        if (kWIn) put_w_factor(i + 1, slot, nxt);
+        if (++slot == (kWIn ? kKaStages : 2)) {
+          slot = 0;
+          phase ^= 1;
+        }
+        cur = nxt;
+      }
       if (lane == 0) {
         // the first demand loads go out before any prefetch; the prefetches of chunks 2.. follow chunk 1
 #pragma unroll 1
         for (int c = (i == 1) ? 2 : i + kPrefetchAhead; i >= 1 && c <= i + kPrefetchAhead && c < nproc; ++c) {
-          const int pt0 = seq_start + (first_chunk + c) * kChunk;
-          ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
+          const int pt0 = token_of(c);
+          if (kWIn || !zero_v) ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
           if (!zero_v) ptx::tma_prefetch_l2_4d(&tm_v, 0, hv, pt0, 0);
-          ptx::tma_prefetch_l2_4d(&tm_w, 0, hv, pt0, 0);
+          if (!kWIn) ptx::tma_prefetch_l2_4d(&tm_w, 0, hv, pt0, 0);
           if (!kStateOnly) ptx::tma_prefetch_l2_4d(&tm_q, 0, hk, pt0, 0);
           ptx::tma_prefetch_l2_4d(&tm_k, 0, hk, pt0, 0);
         }
       }
-      // the gate scalars of the chunk that many ahead as well: their latency is on the way to A diag(beta)
-      if (i + kPrefetchAhead < nproc) {
-        const int64_t ahead = static_cast<int64_t>(t0) + kPrefetchAhead * kChunk;
+      if (i + kPrefetchAhead < nproc) {  // and the scalars
+        const int64_t ahead = token_of(i + kPrefetchAhead);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const int64_t tk = min(ahead + lane + 32 * r, static_cast<int64_t>(seq_end) - 1);
           ptx::prefetch_l2(p.g_cumsum + tk * p.num_v_heads + hv);
-          ptx::prefetch_l2(static_cast<const uint8_t*>(p.beta) + (tk * p.num_v_heads + hv) * (p.beta_dtype == QLA_DT_F32 ? 4 : 2));
+          if (!kWIn) ptx::prefetch_l2(static_cast<const uint8_t*>(p.beta) + (tk * p.num_v_heads + hv) * (p.beta_dtype == QLA_DT_F32 ? 4 : 2));
           if (p.rnorm != nullptr) ptx::prefetch_l2(p.rnorm + (tk * p.num_k_heads + hk) * 2);
         }
       }
@@ -611,21 +579,32 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           ptx::tc_fence_after_sync();
           ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColD2, tmem0 + kColSbf, d_w + so, id_n64,
                                              kStateOnly ? !zero_v : true, bar_addr(kD2Done));
+          if (kStateOnly) ptx::umma_commit(&bars[kEmpty0 + ph]);
           trace(0, i, 3);
           // gap 1 (the chain computes V'): MMAq: Dq[i & 1] = S0^T_bf16 Q^T; the output of chunk i - 2, which read that
           // buffer, was waited for in front of MMA4(i - 1)
           if (!kStateOnly)
             ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf, d_w + so + (16384 >> 4), id_n64,
-                                               false);
+                                               false, bar_addr(kEmpty0 + ph));
+          // MMA0(i + 1): D0 = Q K^T, once Pg of chunk i has been formed from it.  (In gap 2 its 384 cycles stood between two MMA2.)
+          if (!kStateOnly && i + 1 < nproc) {
+            const int sj = (i + 1) & 1;
+            const uint64_t sn = static_cast<uint64_t>(sj * (kStageBytes >> 4));
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kPgReady), ph, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + sj), ((i + 1) >> 1) & 1, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kKFull0 + sj), ((i + 1) >> 1) & 1, true))) break;
+            ptx::tc_fence_after_sync();
+            ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, d_w + sn + (16384 >> 4), d_k + sn, id_p, false,
+                                                         bar_addr(kPDone));
+          }
           trace(0, i, 4);
           // MMA3: S^T += V'^T K   (B = K tile read MN-major: 64-column halves are 8 KiB apart)
           if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdReady), ph, true))) break;
           if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSScaled), ph, true))) break;
           trace(0, i, 6);
           ptx::tc_fence_after_sync();
-          // (second commit: every MMA that reads this stage has been issued and tracked)
           ptx::umma_ts_k64_halves<128>(tmem0 + kColS, tmem0 + kColD2, d_kmn + so, id_mn128, true, bar_addr(kSDone),
-                                       bar_addr(kEmpty0 + (i & 1)));
+                                       bar_addr(kKEmpty0 + ph));
           trace(0, i, 7);
           // gap 2 (both warpgroups convert the state).  MMA4: D4 = Vd^T Pg^T, once the output of chunk i - 1 has read D4
           if (!kStateOnly) {
@@ -645,11 +624,18 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (i + 1 < nproc) {
           const int j = i + 1, sj = j & 1;
           const uint64_t sn = static_cast<uint64_t>(sj * (kStageBytes >> 4));
-          if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + sj), (j >> 1) & 1, true))) break;
-          if (!(ok = ptx::mbar_wait_nocall(bar_addr(kAbReady0 + sj), (j >> 1) & 1, true))) break;
-          ptx::tc_fence_after_sync();
-          if (!zero_v) ptx::umma_ss_k64<128, 2>(tmem0 + kColD2, d_v + sn, d_a + sn, id_u, false);
-          if (!kStateOnly)
+          if (!zero_v) {
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVaFull0 + sj), (j >> 1) & 1, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kAbReady0 + sj), (j >> 1) & 1, true))) break;
+            ptx::tc_fence_after_sync();
+            ptx::umma_ss_k64<128, 2>(tmem0 + kColD2, d_v + sn, d_a + sn, id_u, false, bar_addr(kVaEmpty0 + sj));
+          }
+          if (kStateOnly || i < 0) {
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + sj), (j >> 1) & 1, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kKFull0 + sj), (j >> 1) & 1, true))) break;
+            ptx::tc_fence_after_sync();
+          }
+          if (!kStateOnly && i < 0)
             ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, d_w + sn + (16384 >> 4), d_k + sn, id_p, false,
                                                          bar_addr(kPDone));
         }
@@ -962,7 +948,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (j > 0 && !wait(kWDone, (j - 1) & 1)) break;  // the operand of chunk j - 1 has been read
         const float* f = w_factor[j & 3];
         const uint8_t* at = smem + kOffKa + slot * kKaBytes + kKaA;
-#pragma unroll 2
+#pragma unroll 3
         for (int x = 0; x < 6; ++x) {
           const bool low = warp == 10 && x < 4;
           const int c16 = (warp == 11) ? x + 2 : (low ? x : x - 4);
@@ -986,13 +972,13 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     } else
 #pragma unroll 1
-    for (int j = 0; j < nproc; ++j) {
+    for (int j = 0; !zero_v && j < nproc; ++j) {
       const int sj = j & 1;
       if (!wait(kGate0 + (j & 3), (j >> 2) & 1)) break;
-      if (!wait(kFull0 + sj, (j >> 1) & 1)) break;
+      if (!wait(kVaFull0 + sj, (j >> 1) & 1)) break;
       const float* beta = gates_of(j)->beta;
       uint8_t* at = stage_ptr(sj) + kStageA;
-#pragma unroll 2
+#pragma unroll 3
       for (int x = 0; x < 6; ++x) {
         const bool low = warp == 10 && x < 4;
         const int c16 = (warp == 11) ? x + 2 : (low ? x : x - 4);
@@ -1009,7 +995,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       ptx::fence_proxy_async_smem();
       // one barrier per stage: these warps run one chunk ahead, and a waiter must never fall two phases behind
-      // (MMA3's commit releases the stage: it comes after MMAu, which waited for this)
+      // (MMAu's commit releases the tile)
       warp_arrive(&bars[kAbReady0 + sj], lane);
     }
   } else {
