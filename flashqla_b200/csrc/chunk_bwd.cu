@@ -313,20 +313,18 @@ bwd_chunk_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   };
   __shared__ StepInfo info[2];
 
-  if (tid == 0) {
-#pragma unroll 1
-    for (int b = 0; b < kNumBars; ++b) {
-      int count = 1;  // tcgen05.commit, the producer's expect_tx arrival, or one thread
-      if (b == kEarlyFull) count = 33;
-      else if (b == kEarlyFree) count = 2 * kGroupWarps + 2;
-      else if (b == kLateFree) count = 2 * kGroupWarps + 1;
-      else if (b == kL1Ready) count = 2 * kGroupWarps;
-      else if (b == kRedReady) count = 3 * kGroupWarps;
-      else if (b == kDaReady || b == kM1Ready || b == kDlReady || (b >= kQ0Ready && b <= kDkReady)) count = kGroupWarps;
-      ptx::mbar_init(&bars[b], count);
-    }
+  if (tid < kNumBars) {  // (a thread each)
+    const int b = tid;
+    int count = 1;  // tcgen05.commit, the producer's expect_tx arrival, or one thread
+    if (b == kEarlyFull) count = 33;
+    else if (b == kEarlyFree) count = 2 * kGroupWarps + 2;
+    else if (b == kLateFree) count = 2 * kGroupWarps + 1;
+    else if (b == kL1Ready) count = 2 * kGroupWarps;
+    else if (b == kRedReady) count = 3 * kGroupWarps;
+    else if (b == kDaReady || b == kM1Ready || b == kDlReady || (b >= kQ0Ready && b <= kDkReady)) count = kGroupWarps;
+    ptx::mbar_init(&bars[b], count);
     ptx::fence_mbar_init();
-    ptx::mbar_wait_setup(p.status, bars, 128);  // (+ 128 in the recorded barrier index: this kernel)
+    if (tid == 0) ptx::mbar_wait_setup(p.status, bars, 128);  // (+ 128 in the recorded barrier index: this kernel)
   }
   if (warp == kProducerWarp) {
     ptx::tmem_alloc(&tmem_base_s, 512);

@@ -138,16 +138,14 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __shared__ __align__(16) float aux_g[2 * 2 * 64];  // [aux warp][chunk parity][64] cumulative gates (log2 domain)
   __shared__ Gates gate_ring[kGateRing];
 
-  if (tid == 0) {
-#pragma unroll 1
-    for (int b = 0; b < kNumBars; ++b) {
-      int count = 1;  // commits: kPDone*, kD2Done, kDu0Done, kSDone
-      if (b == kFull0 || b == kFull1) count = 33;
-      else if (b == kEmpty0 || b == kEmpty1) count = 3;
-      else if (b == kPgReady || b == kQsReady) count = 2;
-      else if (b == kDuReady || b == kSbfReady || b == kSScaled || b == kTileReady) count = 8;
-      ptx::mbar_init(&bars[b], count);
-    }
+  if (tid < kNumBars) {  // (a thread each)
+    const int b = tid;
+    int count = 1;  // commits: kPDone*, kD2Done, kDu0Done, kSDone
+    if (b == kFull0 || b == kFull1) count = 33;
+    else if (b == kEmpty0 || b == kEmpty1) count = 3;
+    else if (b == kPgReady || b == kQsReady) count = 2;
+    else if (b == kDuReady || b == kSbfReady || b == kSScaled || b == kTileReady) count = 8;
+    ptx::mbar_init(&bars[b], count);
     ptx::fence_mbar_init();
   }
   if (warp == 8) {
