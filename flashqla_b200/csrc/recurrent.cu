@@ -427,14 +427,19 @@ int resident_ctas(size_t smem, int* out) {
 }
 
 template <typename T, typename InterT, typename StateT, int R, bool kTree>
+int resident_tiles(int* out) {
+  constexpr size_t smem = kRecStages * R * 4 * 128 * sizeof(typename StatePiece<StateT>::Raw);
+  const int rc = ensure_dynamic_smem<recurrent_kernel<T, InterT, StateT, R, kTree>>(smem);
+  return rc != QLA_OK ? rc : resident_ctas<recurrent_kernel<T, InterT, StateT, R, kTree>>(smem, out);
+}
+
+template <typename T, typename InterT, typename StateT, int R, bool kTree>
 int launch_recurrent_rows(const QlaRecurrentArgs& a, cudaStream_t stream) {
   const int64_t items = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / (16 * R));
   QLA_CHECK_SUPPORTED(items < (int64_t(1) << 31), "too many (sequence, head) pairs");
   constexpr size_t smem = kRecStages * R * 4 * 128 * sizeof(typename StatePiece<StateT>::Raw);
   int resident = 0;
-  int rc = ensure_dynamic_smem<recurrent_kernel<T, InterT, StateT, R, kTree>>(smem);
-  if (rc != QLA_OK) return rc;
-  rc = resident_ctas<recurrent_kernel<T, InterT, StateT, R, kTree>>(smem, &resident);
+  const int rc = resident_tiles<T, InterT, StateT, R, kTree>(&resident);
   if (rc != QLA_OK) return rc;
   // one CTA per item while they all fit at once; otherwise as many CTAs as are resident, each walking the
   // items with stride gridDim.x
@@ -445,13 +450,27 @@ int launch_recurrent_rows(const QlaRecurrentArgs& a, cudaStream_t stream) {
   return QLA_OK;
 }
 
+template <typename T, typename InterT, typename StateT, bool kTree>
+int launch_recurrent_tree(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
+  // Tiles of 16 rows while they are all resident at once, which spreads a small batch over the most SMs; a second round of
+  // them costs the latency of every step again.  With the line at four tiles of 32 rows per SM: 96 heads of 7 tree steps 17.5 us, now
+  // 13.2; 112 heads of 4 steps 11.4 -> 9.7; 144 heads of one step 7.0 -> 5.3, with a bf16 pool 6.8 -> 4.8.
+  if (rows == 0) {
+    const int64_t tiles = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / 16);
+    int resident = 2 * 148;  // (at least: the smallest calls, which are host-bound, do not look it up)
+    if (tiles > resident) {
+      const int rc = resident_tiles<T, InterT, StateT, 1, kTree>(&resident);
+      if (rc != QLA_OK) return rc;
+    }
+    rows = tiles <= resident ? 16 : 32;
+  }
+  return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, kTree>(a, stream)
+                    : launch_recurrent_rows<T, InterT, StateT, 2, kTree>(a, stream);
+}
 template <typename T, typename InterT, typename StateT>
 int launch_recurrent_state(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
-  if (a.parents != nullptr)
-    return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, true>(a, stream)
-                      : launch_recurrent_rows<T, InterT, StateT, 2, true>(a, stream);
-  return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, false>(a, stream)
-                    : launch_recurrent_rows<T, InterT, StateT, 2, false>(a, stream);
+  return a.parents != nullptr ? launch_recurrent_tree<T, InterT, StateT, true>(a, rows, stream)
+                              : launch_recurrent_tree<T, InterT, StateT, false>(a, rows, stream);
 }
 template <typename T, typename InterT>
 int launch_recurrent(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
@@ -576,13 +595,7 @@ extern "C" QLA_API int qla_recurrent_update(const QlaRecurrentArgs* args, void* 
                 "retrieve_parent_token needs intermediate_states_buffer");
   QLA_CHECK_ARG(a.rows_per_cta == 0 || a.rows_per_cta == 16 || a.rows_per_cta == 32,
                 "rows_per_cta must be 0, 16 or 32");
-  int rows = a.rows_per_cta;
-  if (rows == 0) {
-    // 32 rows per CTA keeps two independent rows in flight per thread; fall back to 16 rows while
-    // the grid would otherwise leave SMs idle (148 SMs, several CTAs each).  (The line is drawn at four tiles per SM, not
-    // at what is resident of either height: 6 sequences of 16 heads are 768 tiles of 16 rows on 592 resident CTAs.)
-    rows = (static_cast<int64_t>(a.num_seqs) * a.num_v_heads * 4 >= 4 * 148) ? 32 : 16;
-  }
+  const int rows = a.rows_per_cta;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool inter_bf16 = a.inter != nullptr && a.inter_dtype == QLA_DT_BF16;
   if (a.qkv_dtype == QLA_DT_BF16) {
