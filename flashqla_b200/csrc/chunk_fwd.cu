@@ -948,7 +948,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (j > 0 && !wait(kWDone, (j - 1) & 1)) break;  // the operand of chunk j - 1 has been read
         const float* f = w_factor[j & 3];
         const uint8_t* at = smem + kOffKa + slot * kKaBytes + kKaA;
-#pragma unroll 3
+#pragma unroll 2
         for (int x = 0; x < 6; ++x) {
           const bool low = warp == 10 && x < 4;
           const int c16 = (warp == 11) ? x + 2 : (low ? x : x - 4);
