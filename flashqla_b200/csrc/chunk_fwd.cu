@@ -664,10 +664,8 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int e = 0; e < 16; ++e) y[h][e] = pack2<T>(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1]));
       }
-      if (!kStateOnly) {
-        ptx::tc_fence_before_sync();
-        warp_arrive(&bars[kWRead], lane);
-      }
+      ptx::tc_fence_before_sync();  // (kStateOnly: kWReady below is what the product that overwrites the columns waits for)
+      if (!kStateOnly) warp_arrive(&bars[kWRead], lane);
       // (MMA2 of chunk j - 1, which read the tile, precedes this chunk's product in the pipe)
       const uint32_t at = ptx::sw128_offset((warp & 3) * 32 + lane, 0);
 #pragma unroll
