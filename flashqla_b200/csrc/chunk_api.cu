@@ -50,7 +50,7 @@ extern "C" QLA_API int qla_chunk_fwd(const QlaChunkFwdArgs* args, void* stream_)
   const bool state_only = (a.flags & QLA_CHUNK_STATE_ONLY) != 0;
   const bool skip_prepare = (a.flags & QLA_CHUNK_SKIP_PREPARE) != 0;
   const bool w_in_scan = (a.flags & QLA_CHUNK_W_IN_SCAN) != 0;
-  QLA_CHECK_ARG(a.k && a.beta && a.g_cumsum && a.A && (a.w || w_in_scan) && a.status,
+  QLA_CHECK_ARG(a.k && a.beta && a.g_cumsum && a.A && a.w && a.status,
                 "k, beta, g_cumsum, A, w, status are required");
   QLA_CHECK_SUPPORTED(!w_in_scan || (!(a.flags & QLA_CHUNK_A_GIVEN) && a.h == nullptr && a.v_new == nullptr),
                       "QLA_CHUNK_W_IN_SCAN keeps neither A nor w: not with QLA_CHUNK_A_GIVEN, h or v_new");
@@ -99,7 +99,7 @@ extern "C" QLA_API int qla_chunk_fwd(const QlaChunkFwdArgs* args, void* stream_)
   if (!skip_prepare) {
     KktParams kp{};
     kp.g = a_given ? static_cast<const void*>(a.g_cumsum) : a.g; kp.beta = a.beta; kp.g_cumsum = a.g_cumsum;
-    kp.A = a.A; kp.A_in = a_given ? a.A : nullptr; kp.w = w_in_scan ? nullptr : a.w;
+    kp.A = a.A; kp.A_in = a_given ? a.A : nullptr; kp.w = a.w; kp.aw = w_in_scan ? a.w : nullptr;
     kp.rnorm = l2norm ? a.qk_rnorm : nullptr; kp.norm_eps = 1e-6f;
     kp.A_log = gate_act ? a.A_log : nullptr; kp.dt_bias = gate_act ? a.dt_bias : nullptr;
     kp.beta_out = beta_logit ? a.beta_out : nullptr;
@@ -145,7 +145,7 @@ extern "C" QLA_API int qla_chunk_fwd(const QlaChunkFwdArgs* args, void* stream_)
   fp.trace = current_trace_buffer();
   fp.trace_count = current_trace_count();
   const void* v = a.v ? a.v : a.k;  // never dereferenced with QLA_CHUNK_ZERO_V, only used for the tensor map
-  return launch_chunk_fwd(fp, a.q, a.k, v, a.A, w_in_scan ? nullptr : a.w, total_tokens, is_bf16, state_only, stream);
+  return launch_chunk_fwd(fp, a.q, a.k, v, a.A, a.w, w_in_scan, total_tokens, is_bf16, state_only, stream);
 }
 
 namespace qla {

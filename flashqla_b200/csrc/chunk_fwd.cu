@@ -67,14 +67,13 @@ constexpr uint32_t kOffVn = kOffO + 16384;           // kAux: the v_new tile in 
 constexpr uint32_t kOffH = kOffO + 2 * 16384;        // and 16 KiB for half of the h tile ([64 k][128 v] as two halves)
 constexpr uint32_t kSmemBytes = kOffO + 2 * 16384 + 1024, kSmemBytesAux = kSmemBytes + 16384;
 
-// kWIn (Wt formed by the kernel itself): {Q, V} in two stages, {K, A diag(beta)} in three, because Wt of a chunk is formed
-// one chunk ahead; one Wt tile and one operand tile for it.
-constexpr uint32_t kQvV = 16384, kQvBytes = 32768;            // Q tile, V tile
-constexpr uint32_t kOffKa = 2 * kQvBytes, kKaA = 16384, kKaBytes = 24576;  // K tile, A tile
+// kWIn (Wt formed by the kernel itself): {Q, V, A} in two stages, {K, -A diag(beta gamma)} in three, because Wt of a chunk is
+// formed one chunk ahead; one Wt tile.
+constexpr uint32_t kQvV = 16384, kQvA = 32768, kQvBytes = 40960;  // Q tile, V tile, A tile
+constexpr uint32_t kOffKa = 2 * kQvBytes, kKaAw = 16384, kKaBytes = 24576;  // K tile, operand tile of Wt
 constexpr int kKaStages = 3;
 constexpr uint32_t kOffWt = kOffKa + kKaStages * kKaBytes;    // 16 KiB: Wt^T [128 k][64 tokens], SW128
-constexpr uint32_t kOffAw = kOffWt + 16384;                   // 8 KiB: -A diag(beta gamma) [64][64], SW128
-constexpr uint32_t kOffPgWIn = kOffAw + 8192;
+constexpr uint32_t kOffPgWIn = kOffWt + 16384;
 constexpr uint32_t kOffOWIn = kOffPgWIn + 2 * 8192;
 constexpr uint32_t kSmemBytesWIn = kOffOWIn + 2 * 16384 + 1024;
 
@@ -96,9 +95,9 @@ enum Bar {
   kFull0 = 0, kFull1, kEmpty0, kEmpty1,
   kPDone, kPgReady, kD2Done, kVdReady, kVdStored, kSDone, kSbfReady, kSScaled, kAbReady0, kAbReady1,
   kD4Done, kORead, kOFree, kOReady, kONormed, kVnRead, kVnReady, kHRead, kHReady, kHFree, kGate0, kGate1, kGate2, kGate3,
-  // kWIn: {K, A} stages (kFull*, kEmpty* are those of {Q, V}), operand of Wt written, Wt in tensor memory, read from there,
-  // written to its tile, Q K^T read from the columns that Wt uses next
-  kKaFull0, kKaFull1, kKaFull2, kKaEmpty0, kKaEmpty1, kKaEmpty2, kAwReady, kWDone, kWRead, kWReady, kD0Read,
+  // kWIn: {K, operand of Wt} stages (kFull*, kEmpty* are those of {Q, V, A}), Wt in tensor memory, read from there, written to its
+  // tile, Q K^T read from the columns that Wt uses next
+  kKaFull0, kKaFull1, kKaFull2, kKaEmpty0, kKaEmpty1, kKaEmpty2, kWDone, kWRead, kWReady, kD0Read,
   // otherwise: {V, A} and K of a stage (kFull*, kEmpty* are those of {Wt, Q})
   kVaFull0, kVaFull1, kVaEmpty0, kVaEmpty1, kKFull0, kKFull1, kKEmpty0, kKEmpty1,
   kNumBars
@@ -194,9 +193,11 @@ static __device__ __noinline__ bool norm_rows(uint32_t so, const T* z, int strid
 // kState16: h0 / final_state are bf16 (state pools); its own instantiation, like kNorm: the code of the plain
 // forward must stay small (it is the instruction cache, not the work, that a few extra branches in the
 // unrolled state loops cost: +20 % on the whole scan when they were part of the plain kernel).
-// kWIn: A holds A diag(beta) and there is no w: Wt = (-A diag(beta gamma)) K is one more product here, formed one chunk ahead
-// of its use.  It saves the write and the read of 256 bytes per token and head: 32768 tokens of 16 / 32 heads 135 + 233 -> 94 + 212 us
-// (preparation + scan), 540 k packed tokens of 8 / 8 heads 557 + 1205 -> 398 + 976; 16 chains alone pay 0.1 us per chunk.
+// kWIn: in place of A and w come A diag(beta) (rounded as this kernel rounds it otherwise) and -A diag(beta gamma) (as the preparation
+// kernel does for w): Wt, the product of the latter with K, is formed here, one chunk ahead of its use.  Operands and
+// orders are the same, so that results are the same bits.  It saves the write and the read of 128 bytes per token and head: 32768
+// tokens of 16 / 32 heads 138 + 227 -> 108 + 225 us (preparation + scan), 540 k packed tokens of 8 / 8 heads 588 + 1137 -> 467 + 1002.
+// (With A diag(beta) scaled here from A instead: 103 + 244 and 439 + 1090.)
 template <typename T, bool kStateOnly, bool kAux, bool kTrace, bool kNorm = false, bool kState16 = false, bool kWIn = false>
 __global__ void __launch_bounds__(kThreads, 1)
 chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -258,13 +259,12 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // reuse needs no barrier of its own: chunk i + 2 is only written after MMA3 of chunk i has finished, which needs
   // both warpgroups to have left chunk i - 1 and MMA4 of chunk i - 2 (the last use of its Pg) to have been issued.
   __shared__ Gates gate_ring[kGateRing];
-  __shared__ float w_factor[kWIn ? 4 : 1][64];  // kWIn: -exp(g) / |k|, ring by chunk: A diag(beta) times this is the operand of Wt
   constexpr uint32_t kPgTiles = kWIn ? kOffPgWIn : kOffPg, kOTiles = kWIn ? kOffOWIn : kOffO;
 
   if (tid < kNumBars) {  // (a thread each: one after the other they were 0.5 us of a CTA's start)
     const int b = tid;
     int count = 1;  // k*Full*, k*Empty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
-    if (b == kAbReady0 || b == kAbReady1 || b == kAwReady || (b >= kKaFull0 && b <= kKaFull2)) count = 2;
+    if (b == kAbReady0 || b == kAbReady1) count = 2;
     else if (b == kPgReady || b == kORead || b == kOReady || b == kVnRead || b == kVnReady || b == kHRead ||
              b == kHReady || b == kWRead || b == kWReady || b == kD0Read)
       count = 4;
@@ -277,10 +277,6 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     for (int x = tid - 384; x < 2 * 32 * 4; x += 128)
       *reinterpret_cast<uint4*>(smem + kPgTiles + (x >> 7) * 8192 + ptx::sw128_offset((x >> 2) & 31, 4 + (x & 3))) =
           make_uint4(0, 0, 0, 0);
-    ptx::fence_proxy_async_smem();
-  }
-  if (kWIn && warp < 4) {  // and the same block of the operand of Wt
-    *reinterpret_cast<uint4*>(smem + kOffAw + ptx::sw128_offset(tid >> 2, 4 + (tid & 3))) = make_uint4(0, 0, 0, 0);
     ptx::fence_proxy_async_smem();
   }
   if (warp == 8) {
@@ -325,8 +321,8 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // L2 prefetch runs kPrefetchAhead chunks ahead of the demand loads: with every SM streaming its own
     // sequence the DRAM latency of a tile exceeds one chunk period, and only two stages fit in shared
     // memory, so the tiles are pulled into L2 early and the demand TMA then hits L2.
-    // Tiles are reloaded as their last product has read them.  kWIn: {Q, V} of chunk i behind MMAq of chunk i - 2, {K, A} of chunk i + 1
-    // behind MMA3 of chunk i - 2.  Otherwise {Wt, Q} of chunk i behind MMAq and K behind MMA3 of chunk i - 2, {V, A} of chunk i + 1
+    // Tiles are reloaded as their last product has read them.  kWIn: {Q, V, A} of chunk i behind MMAq of chunk i - 2, {K, operand of Wt}
+    // of chunk i + 1 behind MMA3 of chunk i - 2.  Otherwise {Wt, Q} of chunk i behind MMAq and K behind MMA3 of chunk i - 2, {V, A} of chunk i + 1
     // behind MMAu of chunk i - 1.  Gate vectors of chunk i follow when MMA3 of chunk i - 2 is through: the last readers of their ring
     // slot (the output of chunk i - 4, which MMA4 of chunk i - 3 waited for) have left it.  Their scalars are requested a chunk before.
     constexpr int kPrefetchAhead = 4;
@@ -351,11 +347,6 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           x.rn[r] = *reinterpret_cast<const float2*>(p.rnorm + ((static_cast<int64_t>(t0) + c) * p.num_k_heads + hk) * 2);
       }
     };
-    auto put_w_factor = [&](int c, int slot, const Scalars& x) {
-#pragma unroll
-      for (int r = 0; r < 2; ++r) w_factor[c & 3][lane + 32 * r] = -ptx::ex2(x.g[r] * log2e) * x.rn[r].y;
-      warp_arrive(&bars[kKaFull0 + slot], lane);
-    };
     auto token_of = [&](int c) { return seq_start + (first_chunk + c) * kChunk; };
     auto load_early = [&](int c, int slot) {  // what a chunk needs first
       if (lane == 0 && kWIn) {
@@ -363,7 +354,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         uint64_t* full = &bars[kKaFull0 + slot];
         ptx::mbar_expect_tx(full, kKaBytes);
         ptx::tma_load_4d(st, &tm_k, full, 0, hk, token_of(c), 0);
-        ptx::tma_load_3d(st + kKaA, &tm_a, full, 0, hv, token_of(c));
+        ptx::tma_load_3d(st + kKaAw, &tm_w, full, 0, hv, token_of(c));
       } else if (lane == 0 && !zero_v) {
         uint8_t* st = stage_ptr(slot);
         uint64_t* full = &bars[kVaFull0 + slot];
@@ -389,8 +380,11 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         uint64_t* full = &bars[kFull0 + s];
         if (kWIn) {
           uint8_t* st = smem + s * kQvBytes;
-          ptx::mbar_expect_tx(full, (kStateOnly ? 0 : 16384) + (zero_v ? 0 : 16384));
-          if (!zero_v) ptx::tma_load_4d(st + kQvV, &tm_v, full, 0, hv, token_of(i), 0);
+          ptx::mbar_expect_tx(full, (kStateOnly ? 0 : 16384) + (zero_v ? 0 : 16384 + 8192));
+          if (!zero_v) {
+            ptx::tma_load_3d(st + kQvA, &tm_a, full, 0, hv, token_of(i));
+            ptx::tma_load_4d(st + kQvV, &tm_v, full, 0, hv, token_of(i), 0);
+          }
           if (!kStateOnly) ptx::tma_load_4d(st, &tm_q, full, 0, hk, token_of(i), 0);
         } else {
           uint8_t* st = stage_ptr(s) + kStageWQ;
@@ -418,7 +412,6 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         load_early(i + 1, slot);
       }
-      if (kWIn && i == 0) put_w_factor(0, 0, cur);
       const int valid = min(kChunk, seq_end - token_of(i));
       Gates* gs = gates_of(i);
 #pragma unroll
@@ -436,7 +429,6 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       gs->valid = valid;
       warp_arrive(&bars[kGate0 + (i & 3)], lane);
       if (i + 1 < nproc) {
-        if (kWIn) put_w_factor(i + 1, slot, nxt);
         if (++slot == (kWIn ? kKaStages : 2)) {
           slot = 0;
           phase ^= 1;
@@ -448,9 +440,10 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll 1
         for (int c = (i == 1) ? 2 : i + kPrefetchAhead; i >= 1 && c <= i + kPrefetchAhead && c < nproc; ++c) {
           const int pt0 = token_of(c);
-          if (kWIn || !zero_v) ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
+          if (!zero_v) ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
           if (!zero_v) ptx::tma_prefetch_l2_4d(&tm_v, 0, hv, pt0, 0);
-          if (!kWIn) ptx::tma_prefetch_l2_4d(&tm_w, 0, hv, pt0, 0);
+          if (kWIn) ptx::tma_prefetch_l2_3d(&tm_w, 0, hv, pt0);
+          else ptx::tma_prefetch_l2_4d(&tm_w, 0, hv, pt0, 0);
           if (!kStateOnly) ptx::tma_prefetch_l2_4d(&tm_q, 0, hk, pt0, 0);
           ptx::tma_prefetch_l2_4d(&tm_k, 0, hk, pt0, 0);
         }
@@ -506,11 +499,11 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kQvV), 8192, 1024);
         const uint64_t k_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa), 16, 1024);
         const uint64_t kmn_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa), 8192, 1024);
-        const uint64_t a_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa + kKaA), 16, 1024);
+        const uint64_t a_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kQvA), 16, 1024);
         const uint64_t w_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffWt), 8192, 1024);  // MN-major
-        const uint64_t aw_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffAw), 16, 1024);
+        const uint64_t aw_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffKa + kKaAw), 16, 1024);
         const uint32_t id_w = ptx::mma_idesc(128, 64, fmt, ptx::kMajorK, ptx::kMajorMN);
-        int slot = 0, phase = 0, slot_i = 0;  // of chunk i + 1 in the {K, A} ring; slot of chunk i
+        int slot = 0, phase = 0, slot_i = 0;  // of chunk i + 1 in the {K, operand of Wt} ring; slot of chunk i
 #pragma unroll 1
         for (int i = -1; ok && i < nproc; ++i) {
           const int ph = i & 1, j = i + 1;
@@ -528,10 +521,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
           if (j < nproc) {
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kKaFull0 + slot), phase, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kAwReady), j & 1, true))) break;
             if (!kStateOnly && i >= 0 && !(ok = ptx::mbar_wait_nocall(bar_addr(kD0Read), ph, true))) break;
             ptx::tc_fence_after_sync();
-            ptx::umma_ss_k64<128, 2>(tmem0 + kColD0, kmn_desc + ka_j, aw_desc, id_u, false, bar_addr(kWDone));
+            ptx::umma_ss_k64<128, 2>(tmem0 + kColD0, kmn_desc + ka_j, aw_desc + ka_j, id_u, false, bar_addr(kWDone));
           }
           if (i >= 0) {
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdReady), ph, true))) break;
@@ -553,7 +545,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const uint64_t qv = static_cast<uint64_t>((j & 1) * (kQvBytes >> 4));
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + (j & 1)), (j >> 1) & 1, true))) break;
             ptx::tc_fence_after_sync();
-            if (!zero_v) ptx::umma_ss_k64<128, 2>(tmem0 + kColD2, v_desc + qv, a_desc + ka_j, id_u, false);
+            if (!zero_v) ptx::umma_ss_k64<128, 2>(tmem0 + kColD2, v_desc + qv, a_desc + qv, id_u, false);
             if (!kStateOnly) {
               if (!(ok = ptx::mbar_wait_nocall(bar_addr(kWRead), j & 1, true))) break;
               ptx::tc_fence_after_sync();
@@ -937,40 +929,8 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // (B operand of MMAu).  A is lower triangular: row r ends in 16-byte piece r / 8, what lies behind is zero (or
     // belongs to tokens past the end, whose rows nothing reads).  Six pieces per lane: warp 11 rows 32..63 pieces
     // 2..7, warp 10 the first two of those rows and the four of rows 0..31.
-    if constexpr (kWIn) {
-      // The same pieces of A diag(beta), which is B operand of MMAu as it is, times -exp(g) / |k|: B operand of MMAw
-      int slot = 0, phase = 0;
 #pragma unroll 1
-      for (int j = 0; j < nproc; ++j) {
-        if (!wait(kKaFull0 + slot, phase)) break;
-        if (j > 0 && !wait(kWDone, (j - 1) & 1)) break;  // the operand of chunk j - 1 has been read
-        const float* f = w_factor[j & 3];
-        const uint8_t* at = smem + kOffKa + slot * kKaBytes + kKaA;
-#pragma unroll 2
-        for (int x = 0; x < 6; ++x) {
-          const bool low = warp == 10 && x < 4;
-          const int c16 = (warp == 11) ? x + 2 : (low ? x : x - 4);
-          const uint32_t off = ptx::sw128_offset(low ? lane : 32 + lane, c16);
-          const uint4 raw = *reinterpret_cast<const uint4*>(at + off);
-          const float4 b0 = *reinterpret_cast<const float4*>(&f[c16 * 8]);
-          const float4 b1 = *reinterpret_cast<const float4*>(&f[c16 * 8 + 4]);
-          const T* e = reinterpret_cast<const T*>(&raw);
-          *reinterpret_cast<uint4*>(smem + kOffAw + off) =
-              make_uint4(pack2<T>(Cvt<T>::to_f32(e[0]) * b0.x, Cvt<T>::to_f32(e[1]) * b0.y),
-                         pack2<T>(Cvt<T>::to_f32(e[2]) * b0.z, Cvt<T>::to_f32(e[3]) * b0.w),
-                         pack2<T>(Cvt<T>::to_f32(e[4]) * b1.x, Cvt<T>::to_f32(e[5]) * b1.y),
-                         pack2<T>(Cvt<T>::to_f32(e[6]) * b1.z, Cvt<T>::to_f32(e[7]) * b1.w));
-        }
-        ptx::fence_proxy_async_smem();
-        warp_arrive(&bars[kAwReady], lane);
-        if (++slot == kKaStages) {
-          slot = 0;
-          phase ^= 1;
-        }
-      }
-    } else
-#pragma unroll 1
-    for (int j = 0; !zero_v && j < nproc; ++j) {
+    for (int j = 0; !kWIn && !zero_v && j < nproc; ++j) {
       const int sj = j & 1;
       if (!wait(kGate0 + (j & 3), (j >> 2) & 1)) break;
       if (!wait(kVaFull0 + sj, (j >> 1) & 1)) break;
@@ -1225,7 +1185,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }  // namespace
 
 int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const void* v, const void* A,
-                     const void* w, int64_t total_tokens, bool is_bf16, bool state_only, cudaStream_t stream) {
+                     const void* w, bool w_in_scan, int64_t total_tokens, bool is_bf16, bool state_only, cudaStream_t stream) {
   CUtensorMap tm_q, tm_k, tm_v, tm_a, tm_w, tm_o, tm_vn, tm_h;
   int rc;
   const bool aux = p.h != nullptr || p.v_new != nullptr;
@@ -1233,9 +1193,9 @@ int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const voi
   if ((rc = make_tmap_halves(&tm_q, state_only ? k : q, total_tokens, p.num_k_heads, 64, is_bf16)) != QLA_OK) return rc;
   if ((rc = make_tmap_halves(&tm_v, v, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
   if ((rc = make_tmap_3d(&tm_a, A, total_tokens, p.num_v_heads, 64, 64, 64, true, is_bf16)) != QLA_OK) return rc;
-  const bool w_in = w == nullptr;  // A holds A diag(beta), the kernel forms Wt itself
-  tm_w = tm_k;
-  if (!w_in && (rc = make_tmap_halves(&tm_w, w, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
+  rc = w_in_scan ? make_tmap_3d(&tm_w, w, total_tokens, p.num_v_heads, 64, 64, 64, true, is_bf16)
+                 : make_tmap_halves(&tm_w, w, total_tokens, p.num_v_heads, 64, is_bf16);
+  if (rc != QLA_OK) return rc;
   if ((rc = make_tmap_halves(&tm_o, state_only ? v : p.o, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
   tm_vn = tm_h = tm_o;
   if (p.v_new != nullptr && (rc = make_tmap_halves(&tm_vn, p.v_new, total_tokens, p.num_v_heads, 64, is_bf16)) != QLA_OK) return rc;
@@ -1252,10 +1212,10 @@ int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const voi
   } while (0)
 #define QLA_DISPATCH_FWD(T)                                                                                   \
   do {                                                                                                        \
-    if (w_in && p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, true, true); \
-    else if (w_in && p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, true, false, true);  \
-    else if (w_in && state_only) QLA_LAUNCH_FWD(kSmemBytesWIn, T, true, false, false, false, false, true);    \
-    else if (w_in) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, false, true);                 \
+    if (w_in_scan && p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, true, true); \
+    else if (w_in_scan && p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, true, false, true);  \
+    else if (w_in_scan && state_only) QLA_LAUNCH_FWD(kSmemBytesWIn, T, true, false, false, false, false, true);    \
+    else if (w_in_scan) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, false, true);                 \
     else if (p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false, false, true);   \
     else if (p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false, true);                \
     else if (traced) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, true);                                       \

@@ -11,7 +11,9 @@ struct KktParams {
   float* g_cumsum;              // out; in when A_in is given
   void* A;                      // out (unused when A_in is given)
   const void* A_in;             // optional: A from an earlier call -> only w is produced
-  void* w;                      // out: -(A diag(beta gamma) K), [NT, Hv, 128]; NULL: A receives A diag(beta), the scan forms w
+  void* w;                      // out: -(A diag(beta gamma) K), [NT, Hv, 128]
+  void* aw;                     // out or NULL: -A diag(beta gamma), [NT, Hv, 64], instead of w, which the scan forms from it; A is then
+                                // A diag(beta)
   float* rnorm;                 // out or NULL: [NT, Hk, 2] = 1/|q_t|, 1/|k_t| (in-kernel q/k L2 norm)
   float norm_eps;               // added to the squared norm
   const float* A_log;           // [Hv] or NULL: g = -exp(A_log[h]) * softplus(raw gate + dt_bias[h])
@@ -122,8 +124,8 @@ int launch_chunk_tables(const int32_t* cu, int n, int32_t* pair_offsets, int32_t
                         cudaStream_t stream);
 int launch_kkt_solve(const KktParams& p, const void* k, const void* q, int64_t total_tokens, int pairs_upper,
                      bool is_bf16, cudaStream_t stream);
-// `w` NULL: A holds A diag(beta) and the scan forms w itself.
+// `w`: the prepared w, or with `w_in_scan` -A diag(beta gamma), [NT, Hv, 64], from which the scan forms it (`A` is A diag(beta)).
 int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const void* v, const void* A,
-                     const void* w, int64_t total_tokens, bool is_bf16, bool state_only, cudaStream_t stream);
+                     const void* w, bool w_in_scan, int64_t total_tokens, bool is_bf16, bool state_only, cudaStream_t stream);
 
 }  // namespace qla

@@ -395,12 +395,12 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   void* stream = current_stream(dev);
   const Tensor cu = as_i32(cu_seqlens, dev);
   const Tensor g_cumsum = new_tensor({B, T, Hv}, at::kFloat, dev), A = new_tensor({B, T, Hv, 64}, dtype, dev);
-  // A call that keeps neither A nor w: the scan forms w itself, and A is scratch in its own form.  From 65536 tokens x heads on:
-  // preparation + scan, us, with w / without: 16 chains of 32 chunks 62 / 64, 32 of 32 69 / 69, 64 of 32 83 / 77, 128 of 32 111 / 92,
-  // 512 of 32 (8 / 8 heads) 456 / 357, 512 of 4 89 / 81; with fewer the one more hand-off at the start of a scan costs what the
-  // preparation gains.
-  const bool w_in_scan = !keep && !output_h && !output_v_new && B * T * Hv >= 65536;
-  const Tensor w = w_in_scan ? Tensor() : new_tensor({B, T, Hv, 128}, dtype, dev), o = at::empty_like(v);
+  // A call that keeps neither A nor w: the scan forms w itself, and A is scratch in its own form.  The results are the same bits, and
+  // no size was found where it is slower (whole calls, us, with w / without: 1 x 64 tokens of 16 / 32 heads 14.6 / 12.8, 1 x 777 34.0 /
+  // 33.7, 8 x 500 of 8 / 8 heads 28.0 / 27.0; preparation + scan: 64 chains of 32 chunks 68 / 59, 512 of 32 431 / 382, 512 of 4 85 / 74,
+  // 8000 of 1 498 / 480).
+  const bool w_in_scan = !keep && !output_h && !output_v_new;
+  const Tensor w = new_tensor({B, T, Hv, w_in_scan ? 64 : 128}, dtype, dev), o = at::empty_like(v);
   Tensor h, v_new, rnorm, beta_act, final_state, A_log, dt_bias;
   if (output_h)
     h = cu.defined() ? new_h(n_chunks, T, N, Hv, dtype, dev).unsqueeze(0) : new_tensor({B, chunks_of(T), Hv, 128, 128}, dtype, dev);
@@ -472,8 +472,8 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
   }
   py::gil_scoped_acquire gil;
   auto opt = [](const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); };
-  return py::make_tuple(g_cumsum, w_in_scan ? py::none() : py::cast(A), o, opt(h), opt(final_state), opt(v_new), opt(w), opt(rnorm),
-                        opt(beta_act));
+  return py::make_tuple(g_cumsum, w_in_scan ? py::none() : py::cast(A), o, opt(h), opt(final_state), opt(v_new),
+                        w_in_scan ? py::none() : py::cast(w), opt(rnorm), opt(beta_act));
 }
 
 // The raw backward (chunk.chunk_gated_delta_rule_bwd): `g_` is the cumulative gate of the forward.

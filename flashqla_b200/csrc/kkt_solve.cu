@@ -84,18 +84,16 @@ __device__ __forceinline__ constexpr int swz(int r) { return ((r & 2) << 2) | (r
 
 // ---- shared memory (offsets from a 1024-byte aligned base): the K tile of both chunks, 32 KiB, as two [128][64] halves (columns
 // 0..63 | 64..127), SW128; then per chunk
-template <bool kW>
 struct Area {
-  static constexpr uint32_t kAw = 0;             // kW, 8 KiB: -A diag(beta gamma), 16 bit, [64][64] SW128; later columns 0..63 of Wt
-  static constexpr uint32_t kX = kW ? 8192 : 0;  // 6 fp32 blocks X00, X11, X10, X22, X33, X32; later (8 KiB) A, 16 bit, [64][64] SW128;
-                                                 // later columns 64..127 of Wt
+  static constexpr uint32_t kAw = 0;    // 8 KiB: -A diag(beta gamma), 16 bit, [64][64] SW128; kW: later columns 0..63 of Wt
+  static constexpr uint32_t kX = 8192;  // 6 fp32 blocks X00, X11, X10, X22, X33, X32; later (8 KiB) A, 16 bit, [64][64] SW128;
+                                        // kW: later columns 64..127 of Wt
   static constexpr uint32_t kN = kX + 6 * kBlock * 4;  // 4 blocks N20, N21, N30, N31 as fragments [s][lane] float4, TF32
   static constexpr uint32_t kBytes = kX + 11264;
   static constexpr size_t kSmem = 32768 + 2 * kBytes;
   static_assert(kN + 4096 <= kBytes && kBytes % 1024 == 0, "shared-memory map");
-  static constexpr int kCtasPerSm = kW ? 3 : 4;
-  static constexpr int kTmemColumns = kW ? 128 : 64;  // K K^T, and Wt over it
 };
+constexpr int kCtasPerSm = 3;
 constexpr int kKktThreads = 128;
 
 // Fragments of a block, one array for all uses: value e of the pair [s][h] of lane 4 g + c is element (g + 8 h, 8 s + 2 c + e), which
@@ -195,10 +193,11 @@ __device__ __forceinline__ void product_3xtf32(Frag& out, const Frag& a, const F
 #pragma unroll
     for (int h = 0; h < 2; ++h) out[s][h] = add2(out[s][h], small[s][h]);
 }
-// A finished block, as 16-bit registers for the A tile.  kW: A, and -A diag(beta gamma) goes to its tile (`aw_at` is this lane's
-// stmatrix address there, bg the factors of the block's columns); otherwise A diag(beta), bg = beta.
-template <typename T, bool kW>
-__device__ __forceinline__ void emit(uint32_t (&av)[4], uint32_t aw_at, const Frag& f, const float* bg, int lane) {
+// A finished block, as 16-bit registers for the A tile: A, or with `beta` A diag(beta), the product of the rounded A rounded once
+// more, as a scan that reads A forms it.  -A diag(beta gamma) goes to its tile (`aw_at` is this lane's stmatrix address there).
+// bg, beta: factors of the block's columns.
+template <typename T, bool kBeta>
+__device__ __forceinline__ void emit(uint32_t (&av)[4], uint32_t aw_at, const Frag& f, const float* bg, const float* beta, int lane) {
   uint32_t aw[4];
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
@@ -209,18 +208,23 @@ __device__ __forceinline__ void emit(uint32_t (&av)[4], uint32_t aw_at, const Fr
       unpack(mul2(f[s][h], b), lo, hi);
       aw[2 * s + h] = pack2<T>(lo, hi);
       unpack(f[s][h], lo, hi);
-      av[2 * s + h] = kW ? pack2<T>(lo, hi) : aw[2 * s + h];
+      av[2 * s + h] = pack2<T>(lo, hi);
+      if (kBeta) {
+        const T* a = reinterpret_cast<const T*>(&av[2 * s + h]);
+        const float2 b2 = *reinterpret_cast<const float2*>(beta + 8 * s + 2 * (lane & 3));
+        av[2 * s + h] = pack2<T>(Cvt<T>::to_f32(a[0]) * b2.x, Cvt<T>::to_f32(a[1]) * b2.y);
+      }
     }
   }
-  if (kW) ptx::stmatrix_x4(aw_at, aw[0], aw[1], aw[2], aw[3]);
+  ptx::stmatrix_x4(aw_at, aw[0], aw[1], aw[2], aw[3]);
 }
 __device__ __forceinline__ void chunk_sync(int ci) {  // the two warps that own one chunk
   asm volatile("bar.sync %0, 64;" ::"r"(ci + 1) : "memory");
 }
 
-// kW: A and w are written.  Otherwise A diag(beta) alone, for a scan that forms Wt itself.
+// kW: A and w are written.  Otherwise A diag(beta) and -A diag(beta gamma), for a scan that forms Wt from it.
 template <typename T, bool kW>
-__global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_kernel(const __grid_constant__ CUtensorMap tm_k,
+__global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(const __grid_constant__ CUtensorMap tm_k,
                                                                                    const __grid_constant__ CUtensorMap tm_q,
                                                                                    const __grid_constant__ CUtensorMap tm_a,
                                                                                    const __grid_constant__ CUtensorMap tm_w,
@@ -276,7 +280,8 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
   if (blockIdx.x >= total_items) return;
 
   extern __shared__ __align__(1024) uint8_t smem[];  // (the compiler pads what is in front of it to that alignment)
-  using M = Area<kW>;
+  using M = Area;
+  constexpr int kTmemColumns = kW ? 128 : 64;  // K K^T, and Wt over it
   uint8_t *sK = smem, *area = smem + 32768 + ci * M::kBytes;
   float* sX = reinterpret_cast<float*>(area + M::kX);
   float* sN = reinterpret_cast<float*>(area + M::kN);
@@ -284,7 +289,8 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
   struct alignas(16) Gates {
     float row[64];  // g log2(e) + log2(|beta| / |k_c|)
     float col[64];  // -(g log2(e)) - log2 |k_d|     (|k| = 1 without in-kernel norm)
-    float bg[64];   // kW: -beta * gamma, otherwise beta
+    float bg[64];   // -beta * gamma
+    float beta[kW ? 4 : 64];  // (kW: not used)
   };
   constexpr int kGateBuffers = kW ? 2 : 1;
   __shared__ Gates s_gates[2][kGateBuffers];  // of the two chunks; kW: the head's and the next one's
@@ -368,7 +374,8 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
       const float er = gc2[r] + (ptx::lg2(fabsf(bv[r])) + lrk[r]);  // (beta = 0: -inf, every power below is 0)
       gt.row[t] = er;
       gt.col[t] = lrk[r] - gc2[r];
-      gt.bg[t] = kW ? copysignf(ptx::ex2(er), -bv[r]) : bv[r];
+      gt.bg[t] = copysignf(ptx::ex2(er), -bv[r]);
+      if (!kW) gt.beta[t] = bv[r];
     }
   };
   if (part == 0) {
@@ -385,7 +392,7 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
     if (!norm) publish(s_gates[ci][0]);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(&tmem_base_s, M::kTmemColumns);
+    ptx::tmem_alloc(&tmem_base_s, kTmemColumns);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
@@ -571,7 +578,7 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int r = 32 * part + 16 * rb + 8 * h + g;
-            const float e = gt.row[r], sign = copysignf(1.f, kW ? gt.bg[r] : -gt.bg[r]);  // -sign(beta)
+            const float e = gt.row[r], sign = copysignf(1.f, gt.bg[r]);  // -sign(beta)
             er[rb][h] = f2(e, e);
             sg[rb][h] = f2(sign, sign);
           }
@@ -657,25 +664,25 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
       if (!kW && q_norms && hv == hv0) finish_q(sK);  // (Q has been under way since K K^T)
       // ---- 2: X[R + 1][R] = X[R + 1][R + 1] N[R + 1][R] X[R][R]; the diagonal blocks leave beside it
       {
-        const float* bg = &gt.bg[32 * part];
+        const float *bg = &gt.bg[32 * part], *beta = &gt.beta[kW ? 0 : 32 * part];
         const int R = 2 * part;
         Frag d0t, d0, d1, t, y;
         load_t(d0t, own, lm);
         load_n(d1, own + kBlock, lm);
         load_n(d0, own, lm);
         product_3xtf32(t, d0t, off);  // T^T = X[R][R]^T N^T
-        emit<T, kW>(av[0], aw_tile + lm.tile(R, R), d0, bg, lane);
-        emit<T, kW>(av[1], aw_tile + lm.tile(R + 1, R + 1), d1, bg + 16, lane);
+        emit<T, !kW>(av[0], aw_tile + lm.tile(R, R), d0, bg, beta, lane);
+        emit<T, !kW>(av[1], aw_tile + lm.tile(R + 1, R + 1), d1, bg + 16, beta + 16, lane);
         product_3xtf32(y, d1, t);
         store_n(own + 2 * kBlock, y, lm);
-        emit<T, kW>(av[2], aw_tile + lm.tile(R + 1, R), y, bg, lane);
-        if (kW) zero_above(area + M::kAw);
+        emit<T, !kW>(av[2], aw_tile + lm.tile(R + 1, R), y, bg, beta, lane);
+        zero_above(area + M::kAw);
         if (kW) next_gates();
       }
       chunk_sync(ci);
       // ---- 3: column block m = part of the lower left quarter, X[2:4][m] = X[2:4][2:4] (N[2:4][0:2] X[0:2][m])
       {
-        const float* bg = &gt.bg[16 * part];
+        const float *bg = &gt.bg[16 * part], *beta = &gt.beta[kW ? 0 : 16 * part];
         Frag a, b2, b3, x22, x32, x33, t2, t3, y2, y3;
         load_t(a, sX + (part ? 1 : 2) * kBlock, lm);  // X11^T | X10^T
         load_f(b2, sN + 256, lane);
@@ -706,8 +713,8 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
         product_tf32(y2, x22, t2);
         product_tf32(y3, x32, t2);
         product_tf32(y3, x33, t3);
-        emit<T, kW>(av[3], aw_tile + lm.tile(2, part), y2, bg, lane);
-        emit<T, kW>(av[4], aw_tile + lm.tile(3, part), y3, bg, lane);
+        emit<T, !kW>(av[3], aw_tile + lm.tile(2, part), y2, bg, beta, lane);
+        emit<T, !kW>(av[4], aw_tile + lm.tile(3, part), y3, bg, beta, lane);
       }
     } else {
       // A comes from an earlier call: a row per thread (what lies in its upper right quarter is not looked at)
@@ -740,7 +747,14 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
       const uint64_t db = ptx::smem_desc_sw128(ptx::smem_u32(sK) + ci * 8192u, 16384, 1024);
       ptx::umma_ss_k64_lanes<2, 128>(tmem, da, db, idesc, low_off, high_off, false, a_w);
     }
-    if (!kW) next_gates();
+    if (!kW) {
+      if (full && part == 0 && lane == 0) {
+        ptx::tma_store_3d(&tm_w, area + M::kAw, 0, hv, t0);
+        ptx::tma_store_commit();
+      }
+      __syncwarp();
+      next_gates();
+    }
     if (!kW || p.A_in == nullptr) {
       const int R = 2 * part;
       auto put = [&](int r, int col, const uint32_t (&x)[4]) { ptx::stmatrix_x4(a_tile + lm.tile(r, col), x[0], x[1], x[2], x[3]); };
@@ -758,10 +772,13 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
           ptx::tma_store_commit();
         }
       } else {  // ragged tail: the next sequence owns the rows behind it
-        T* arow = static_cast<T*>(p.A) + (static_cast<int64_t>(t0) * p.num_v_heads + hv) * 64;
-        for (int x = 32 * part + lane; x < valid * 8; x += 64)
-          *reinterpret_cast<uint4*>(arow + static_cast<int64_t>(x >> 3) * p.num_v_heads * 64 + (x & 7) * 8) =
-              *reinterpret_cast<const uint4*>(area + M::kX + ptx::sw128_offset(x >> 3, x & 7));
+        const int64_t first = (static_cast<int64_t>(t0) * p.num_v_heads + hv) * 64;
+        for (int x = 32 * part + lane; x < valid * 8; x += 64) {
+          const int64_t to = first + static_cast<int64_t>(x >> 3) * p.num_v_heads * 64 + (x & 7) * 8;
+          const uint32_t from = ptx::sw128_offset(x >> 3, x & 7);
+          *reinterpret_cast<uint4*>(static_cast<T*>(p.A) + to) = *reinterpret_cast<const uint4*>(area + M::kX + from);
+          if (!kW) *reinterpret_cast<uint4*>(static_cast<T*>(p.aw) + to) = *reinterpret_cast<const uint4*>(area + M::kAw + from);
+        }
         chunk_sync(ci);  // (the tile is overwritten)
       }
     }
@@ -811,7 +828,7 @@ __global__ void __launch_bounds__(kKktThreads, Area<kW>::kCtasPerSm) kkt_solve_k
   if (part == 0 && lane == 0) ptx::tma_store_wait_read();  // shared memory stays allocated until the last stores have read it
   ptx::tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) ptx::tmem_dealloc(tmem, M::kTmemColumns);
+  if (warp == 1) ptx::tmem_dealloc(tmem, kTmemColumns);
 }
 
 // pair_offsets[n] = sum_{m<n} ceil(len_m / 128), chunk_offsets[n] = sum_{m<n} ceil(len_m / 64): one warp, 32
@@ -855,7 +872,7 @@ int launch_chunk_tables(const int32_t* cu, int n, int32_t* pair_offsets, int32_t
 template <typename T, bool kW>
 static int launch_kkt(const KktParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_q, const CUtensorMap& tm_a, const CUtensorMap& tm_w, unsigned grid,
                       cudaStream_t stream) {
-  constexpr size_t smem = Area<kW>::kSmem;
+  constexpr size_t smem = Area::kSmem;
   const int rc = ensure_dynamic_smem<kkt_solve_kernel<T, kW>>(smem);
   if (rc != QLA_OK) return rc;
   QLA_CHECK_CUDA(launch_dependent(kkt_solve_kernel<T, kW>, dim3(grid), dim3(kKktThreads), smem, stream, tm_k, tm_q, tm_a, tm_w, p));
@@ -865,7 +882,7 @@ static int launch_kkt(const KktParams& p, const CUtensorMap& tm_k, const CUtenso
 
 int launch_kkt_solve(const KktParams& params, const void* k, const void* q, int64_t total_tokens, int pairs_upper, bool is_bf16, cudaStream_t stream) {
   KktParams p = params;
-  const bool with_w = p.w != nullptr;
+  const bool with_w = p.aw == nullptr;
   CUtensorMap tm_k, tm_q, tm_a, tm_w;
   int rc = make_tmap_halves(&tm_k, k, total_tokens, p.num_k_heads, 128, is_bf16);
   if (rc != QLA_OK) return rc;
@@ -875,13 +892,14 @@ int launch_kkt_solve(const KktParams& params, const void* k, const void* q, int6
   // A leaves through a [64 tokens][64] tile; in rebuild mode (A given) the map is made but unused
   rc = make_tmap_3d(&tm_a, p.A, total_tokens, p.num_v_heads, 64, kChunk, 64, true, is_bf16);
   if (rc != QLA_OK) return rc;
-  tm_w = tm_k;
-  if (with_w && (rc = make_tmap_halves(&tm_w, p.w, total_tokens, p.num_v_heads, kChunk, is_bf16)) != QLA_OK) return rc;
+  rc = with_w ? make_tmap_halves(&tm_w, p.w, total_tokens, p.num_v_heads, kChunk, is_bf16)
+              : make_tmap_3d(&tm_w, p.aw, total_tokens, p.num_v_heads, 64, kChunk, 64, true, is_bf16);
+  if (rc != QLA_OK) return rc;
   const int group = p.num_v_heads / p.num_k_heads;
   int slots = 0, dev = 0;
   QLA_CHECK_CUDA(cudaGetDevice(&dev));
   QLA_CHECK_CUDA(cudaDeviceGetAttribute(&slots, cudaDevAttrMultiProcessorCount, dev));
-  slots *= with_w ? Area<true>::kCtasPerSm : Area<false>::kCtasPerSm;
+  slots *= kCtasPerSm;
   // Work items: the v-heads of a k-head stay together, which reads K once, unless the rounds of resident CTAs come out shorter
   // with fewer heads per item.  Getting an item under way costs about as much as 0.6 heads.
   double best = 0;
@@ -905,7 +923,7 @@ int launch_kkt_solve(const KktParams& params, const void* k, const void* q, int6
 
 void launch_info_kkt_solve_kernel(int* block_threads, size_t* dynamic_smem_bytes) {
   *block_threads = kKktThreads;
-  *dynamic_smem_bytes = Area<true>::kSmem;
+  *dynamic_smem_bytes = Area::kSmem;
 }
 
 }  // namespace qla

@@ -157,10 +157,11 @@ enum { /* flags of QlaChunkFwdArgs / QlaChunkBwdArgs */
                                     chunk_limit_b, writing its K x K result to row seq_map_b[n]
                                     of final_state_b (fp32): warm-up and transition pass of
                                     context parallelism as one grid                           */
-  QLA_CHUNK_W_IN_SCAN = 16384    /* the scan forms w itself: no w (may be NULL), and A is
-                                    A diag(beta), out of the preparation step and in with
-                                    QLA_CHUNK_SKIP_PREPARE.  For calls that keep neither: not
-                                    with QLA_CHUNK_A_GIVEN, h or v_new                        */
+  QLA_CHUNK_W_IN_SCAN = 16384    /* the scan forms w itself: the buffer A holds A diag(beta) and the
+                                    buffer w, [B, T, Hv, 64], -A diag(beta e^g), both out of the
+                                    preparation step and in with QLA_CHUNK_SKIP_PREPARE.  Results
+                                    are the same.  For calls that keep neither: not with
+                                    QLA_CHUNK_A_GIVEN, h or v_new                                 */
 };
 
 /*

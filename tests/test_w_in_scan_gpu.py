@@ -1,5 +1,5 @@
-"""Calls that keep neither ``A`` nor ``w`` (inference from 65536 tokens x heads on): the scan forms ``w`` itself.  Compared with the
-raw forward, which the other files hold to the oracle, over the forms such a call can take."""
+"""Calls that keep no ``w`` (inference): the scan forms ``w`` itself, of the same operands in the same
+order, so that the results are those of the raw forward, which the other files hold to the oracle, bit by bit."""
 import pytest
 import torch
 
@@ -21,13 +21,9 @@ def inputs(lens, Hk, Hv, dtype, weak, seed):
     return q.to(dtype), k.to(dtype), v.to(dtype), g, beta, h0, cu
 
 
-def close(a, b, dtype):
-    """Either is within 3.6e-3 (bf16; 4.5e-4 fp16) of exact arithmetic, so they are within twice that of each other."""
-    rel = float((a.double() - b.double()).norm() / b.double().norm())
-    return rel <= (7.2e-3 if dtype == torch.bfloat16 else 9e-4)
-
-
 CASES = [  # lengths, heads, weak gates
+    ([1], (1, 1), False),
+    ([130, 64], (2, 4), True),
     ([65536 // 8 + 1], (4, 8), False),                     # segments, warm-up inside the scan
     ([65536 // 4 + 37], (2, 4), True),                     # segments, state-only passes and transition matrices
     ([1, 63, 64, 65, 127, 128, 129, 192, 193, 2048, 777], (16, 32), False),
@@ -40,13 +36,12 @@ CASES = [  # lengths, heads, weak gates
 def test_op(lens, heads, weak, dtype):
     import flashqla_b200 as fq
     q, k, v, g, beta, h0, cu = inputs(lens, *heads, dtype, weak, 3)
-    assert q.shape[1] * heads[1] >= 65536
     h0 = h0[:len(lens)]
     raw = fq.chunk_gated_delta_rule_fwd(q, k, v, g, beta, initial_state=h0, cu_seqlens=cu)
     with torch.no_grad():
         o, final = fq.chunk_gated_delta_rule(q, k, v, g, beta, initial_state=h0, output_final_state=True, cu_seqlens=cu)
     fq.check_device_status()
-    assert close(o, raw[2], dtype) and close(final, raw[4], dtype)
+    assert torch.equal(o, raw[2]) and torch.equal(final, raw[4])
     with torch.no_grad():
         again = fq.chunk_gated_delta_rule(q, k, v, g, beta, initial_state=h0, output_final_state=True, cu_seqlens=cu)
     assert torch.equal(o, again[0]) and torch.equal(final, again[1])
@@ -67,7 +62,7 @@ def test_pool(lens, heads, weak, pool_dtype, norm):
     o, _ = fq.prefill_into_state_pool(3 * q, 2 * k, v, g, beta, pools[1], slots, cu_seqlens=cu, continue_from_pool=True,
                                       use_qk_l2norm_in_kernel=True, **gate)
     fq.check_device_status()
-    assert close(o, raw[2], torch.bfloat16) and close(pools[1], pools[0], torch.bfloat16)
+    assert torch.equal(o, raw[2]) and torch.equal(pools[1], pools[0])
     rest = torch.ones(len(h0), dtype=torch.bool, device="cuda")
     rest[slots[1:].long()] = False
     assert torch.equal(pools[1][rest], h0.to(pool_dtype)[rest])
