@@ -148,28 +148,20 @@ __global__ void __launch_bounds__(kPlanThreads) cp_plan_lead_kernel(const QlaCpP
 }
 
 // The chain  h[next] += M[seg] h[seg]  over the segments of one sequence and head, in order.  A link is a dependent
-// 128 x 128 by 128 x 8 product: the columns are split over CTAs (8 each), warp w of a CTA has rows 16 w .. 16 w + 15.  The
-// product runs on mma.sync with both operands split into two TF32 values (hi hi + hi lo + lo hi: 2^-22 of a product, beside
-// fp32 sums of 128 terms).  A warp's rows of M come straight from global memory (L2) as fragments, those of the next
-// link while this one is multiplied; the carried columns pass through shared memory, split by the thread that
-// formed them, in two buffers: one barrier per link.  What bounds it: 64 KB of M per link and CTA, L2 to SM (40 bytes per ns
-// and SM).  36 links of 4 heads take 59 us; with fp32 products from shared memory and seven barriers per link they took 96.
+// 128 x 128 by 128 x 8 product in fp32: the columns are split over CTAs (8 each), warp w of a CTA has rows 16 w .. 16 w + 15, and a
+// lane every fourth row and 16 of the inner index of each: 4 x 8 sums, two columns per instruction, which the eight lanes
+// of a row then add up in a tree.  A thread's part of M comes straight from global memory (L2), that of the next link
+// while this one is multiplied; the carried columns pass through shared memory in two buffers: one barrier per link.  What
+// bounds it: 64 KB of M per link and CTA, L2 to SM (40 bytes per ns and SM).  36 links of 4 heads take 58 us (59 with split TF32
+// factors on mma.sync, whose error against 64 bits was 2 to 7 times that of fp32; 97 with M through shared memory).
 constexpr int kChainCols = 8;
-constexpr int kChainStride = 144;  // floats from column to column of the carried state: conflict-free float4 fragments
+constexpr int kChainGroup = 4 * kChainCols + 4;  // floats from four rows of the carried columns to the next four: conflict-free float4
 constexpr int kChainThreads = 256;
 constexpr int kChainFlags = 256;
 
-// x = hi + lo, both TF32 (Veltkamp's splitting; lo loses what lies below 2^-22 of x)
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-  const float c = __fmul_rn(x, 8193.f);
-  hi = __fsub_rn(c, __fsub_rn(c, x));
-  lo = __uint_as_float(__float_as_uint(__fsub_rn(x, hi)) & 0xffffe000u);
-}
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const float (&a)[4], float b0, float b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
-        "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {  // two fp32 values per instruction
+  unsigned long long& r = reinterpret_cast<unsigned long long&>(acc);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
 }
 
 __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __restrict__ h0, const float* __restrict__ M,
@@ -180,40 +172,63 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
   grid_dep_launch();
   const int c0 = blockIdx.x * kChainCols, h = blockIdx.y, r = blockIdx.z, tid = threadIdx.x;
   const int s0 = raw_first_seg[r], links = raw_first_seg[r + 1] - s0 - 1;
-  __shared__ __align__(16) float s_h[2][2][kChainCols * kChainStride];  // [buffer][hi | lo][column][row]
+  __shared__ __align__(16) float s_h[2][kHeadDim / 4 * kChainGroup];  // [buffer][row / 4][row % 4][column]
   __shared__ int flags[kChainFlags];
   // link i leads from segment seg_of(i) to seg_of(i + 1)
   auto seg_of = [&](int i) { return reverse ? s0 + links - i : s0 + i; };
-  const int warp = tid >> 5, g = (tid & 31) >> 2, c = tid & 3;
-  // this thread's values of a state: rows row and row + 8, columns c0 + 2 c, + 1 (fragment of the product's accumulator)
-  const int row = 16 * warp + g;
+  // rows 16 warp + rg + 4 i (i = 0..3), inner indices 32 t + 4 sl .. + 3 (t = 0..3)
+  const int warp = tid >> 5, rg = (tid >> 3) & 3, sl = tid & 7;
+  // after the sums this thread has row `row`, columns col .. col + 3
+  const int row = 16 * warp + rg + 4 * (sl >> 1), col = 4 * (sl & 1);
   auto state_of = [&](int i) {
-    return h0 + (static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim * kHeadDim + row * kHeadDim + c0 + 2 * c;
+    return reinterpret_cast<float4*>(h0 + ((static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim + row) * kHeadDim + c0 + col);
   };
-  auto load_state = [&](int i, float (&x)[4]) {
-    const float* s = state_of(i);
-    const float2 lo = *reinterpret_cast<const float2*>(s), hi = *reinterpret_cast<const float2*>(s + 8 * kHeadDim);
-    x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
+  auto carry = [&](int buf, float4 x) {
+    *reinterpret_cast<float4*>(&s_h[buf][(row >> 2) * kChainGroup + (row & 3) * kChainCols + col]) = x;
   };
-  auto carry = [&](int buf, const float (&x)[4]) {
+  using Part = float4[4][4];  // [i][t]
+  auto load_m = [&](int i, Part& part) {
+    const float* m = M + ((static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim + 16 * warp + rg) * kHeadDim + 4 * sl;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float hi, lo;
-      split_tf32(x[e], hi, lo);
-      const int at = (2 * c + (e & 1)) * kChainStride + row + 8 * (e >> 1);
-      s_h[buf][0][at] = hi;
-      s_h[buf][1][at] = lo;
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) part[x][t] = *reinterpret_cast<const float4*>(m + 4 * x * kHeadDim + 32 * t);
+  };
+  // this thread's four values of the product of `m` and the carried columns in `buf`
+  auto product = [&](const Part& m, int buf) {
+    float2 acc[4][4] = {};  // [i][pair of columns]
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float* x = &s_h[buf][(8 * t + sl) * kChainGroup];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 lo = *reinterpret_cast<const float4*>(x + e * kChainCols), hi = *reinterpret_cast<const float4*>(x + e * kChainCols + 4);
+        const float2 xs[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float mv = e == 0 ? m[i][t].x : e == 1 ? m[i][t].y : e == 2 ? m[i][t].z : m[i][t].w;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) fma2(acc[i][c], make_float2(mv, mv), xs[c]);
+        }
+      }
     }
-  };
-  // Rows row and row + 8 of M, columns 16 t + 4 c .. + 3: values 0, 1 are slots c, c + 4 of k-step 2 t, values 2, 3 of 2 t + 1.
-  float4 raw[8][2];
-  auto load_m = [&](int i) {
-    const float* m = M + ((static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim + row) * kHeadDim + 4 * c;
+    // the eight lanes of a row: a lane passes on the half it does not keep, three times
+    auto add = [&](float2 keep, float2 send, int lanes) {
+      return make_float2(keep.x + __shfl_xor_sync(0xffffffffu, send.x, lanes), keep.y + __shfl_xor_sync(0xffffffffu, send.y, lanes));
+    };
+    const bool b2 = sl & 4, b1 = sl & 2, b0 = sl & 1;
+    float2 y[2][4], z[4], out[2];
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int x = 0; x < 2; ++x) raw[t][x] = *reinterpret_cast<const float4*>(m + 8 * x * kHeadDim + 16 * t);
+      for (int c = 0; c < 4; ++c) y[i][c] = add(b2 ? acc[2 + i][c] : acc[i][c], b2 ? acc[i][c] : acc[2 + i][c], 4);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) z[c] = add(b1 ? y[1][c] : y[0][c], b1 ? y[0][c] : y[1][c], 2);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) out[c] = add(b0 ? z[2 + c] : z[c], b0 ? z[c] : z[2 + c], 1);
+    return make_float4(out[0].x, out[0].y, out[1].x, out[1].y);
   };
+  Part parts[2];  // of this link and the next, by turns
   int buf = 0;
   for (int b0 = 0; b0 < links; b0 += kChainFlags) {
     const int nb = min(kChainFlags, links - b0);
@@ -223,60 +238,39 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
     // the usual case (every segment decays below the threshold) has nothing to chain
     if (__syncthreads_or(mine) == 0) continue;
     bool have_h = false;
-    float add[4] = {0.f, 0.f, 0.f, 0.f};  // the next state as it is: what the product is added to
+    float4 add = make_float4(0.f, 0.f, 0.f, 0.f);  // the next state as it is: what the product is added to
     if (flags[0] != 0) {
-      load_m(b0);
-      load_state(b0 + 1, add);
+      load_m(b0, parts[0]);
+      add = *state_of(b0 + 1);
     }
-    for (int i = 0; i < nb; ++i) {
+    // link i with its matrix in `m`; the next link's is on its way to `m_next` when it returns
+    auto link = [&](int i, Part& m, Part& m_next) {
       const bool next = i + 1 < nb && flags[i + 1] != 0;
       if (flags[i] == 0) {  // (uniform)
         have_h = false;
         if (next) {
-          load_m(b0 + i + 1);
-          load_state(b0 + i + 2, add);
+          load_m(b0 + i + 1, m_next);
+          add = *state_of(b0 + i + 2);
         }
-        continue;
+        return;
       }
-      if (!have_h) {
-        float x[4];
-        load_state(b0 + i, x);
-        carry(buf, x);
-      }
+      if (!have_h) carry(buf, *state_of(b0 + i));
       have_h = true;
-      float mh[16][4], ml[16][4];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float a[8] = {raw[t][0].x, raw[t][1].x, raw[t][0].y, raw[t][1].y, raw[t][0].z, raw[t][1].z, raw[t][0].w, raw[t][1].w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) split_tf32(a[e], mh[2 * t + (e >> 2)][e & 3], ml[2 * t + (e >> 2)][e & 3]);
-      }
-      float out[4] = {add[0], add[1], add[2], add[3]};
+      float4 out = add;
       if (next) {
-        load_m(b0 + i + 1);
-        load_state(b0 + i + 2, add);
+        load_m(b0 + i + 1, m_next);
+        add = *state_of(b0 + i + 2);
       }
       __syncthreads();  // the carried columns are complete
-      float acc[2][3][4] = {};
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float4 xh = *reinterpret_cast<const float4*>(&s_h[buf][0][g * kChainStride + 16 * t + 4 * c]);
-        const float4 xl = *reinterpret_cast<const float4*>(&s_h[buf][1][g * kChainStride + 16 * t + 4 * c]);
-        mma_tf32(acc[0][0], ml[2 * t], xh.x, xh.y);
-        mma_tf32(acc[0][1], mh[2 * t], xl.x, xl.y);
-        mma_tf32(acc[0][2], mh[2 * t], xh.x, xh.y);
-        mma_tf32(acc[1][0], ml[2 * t + 1], xh.z, xh.w);
-        mma_tf32(acc[1][1], mh[2 * t + 1], xl.z, xl.w);
-        mma_tf32(acc[1][2], mh[2 * t + 1], xh.z, xh.w);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        out[e] += ((acc[0][0][e] + acc[1][0][e]) + (acc[0][1][e] + acc[1][1][e])) + (acc[0][2][e] + acc[1][2][e]);
+      const float4 x = product(m, buf);
+      out.x += x.x; out.y += x.y; out.z += x.z; out.w += x.w;
       buf ^= 1;
       carry(buf, out);
-      float* dst = state_of(b0 + i + 1);
-      *reinterpret_cast<float2*>(dst) = make_float2(out[0], out[1]);
-      *reinterpret_cast<float2*>(dst + 8 * kHeadDim) = make_float2(out[2], out[3]);
+      *state_of(b0 + i + 1) = out;
+    };
+    for (int i = 0; i < nb; i += 2) {
+      link(i, parts[0], parts[1]);
+      if (i + 1 < nb) link(i + 1, parts[1], parts[0]);
     }
     // (a link behind this batch reads the state written last, each value by the thread that wrote it)
   }

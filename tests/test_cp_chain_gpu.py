@@ -36,3 +36,48 @@ def test_chain(segments, skip, reverse):
     _cabi.check(_cabi.lib().qla_cp_chain(args, _cabi.current_stream(h.device)), "qla_cp_chain")
     # a product loses up to 2^-21 of itself to the splitting, sums of 128 in fp32; |M| |h| is up to ten times |M h| here
     assert float((h.double() - ref).norm() / ref.norm()) <= 1e-5
+
+
+def chain(h, M):
+    """``h`` after the links of one sequence, by the kernel."""
+    from flashqla_b200 import _cabi
+    n, Hv = h.shape[:2]
+    out, limit = h.clone(), torch.ones(n, Hv, dtype=torch.int32, device="cuda")
+    first = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    args = _cabi.QlaCpChainArgs(num_raw_seqs=1, num_v_heads=Hv, h0=out.data_ptr(), M=M.data_ptr(), m_limit=limit.data_ptr(),
+                                raw_first_seg=first.data_ptr(), reverse=0)
+    _cabi.check(_cabi.lib().qla_cp_chain(args, _cabi.current_stream(h.device)), "qla_cp_chain")
+    return out
+
+
+def plain(h, M):
+    """The same in the type of ``h``, sums of 128 products one after the other."""
+    out = h.clone()
+    for s in range(len(h) - 1):
+        acc = torch.zeros_like(out[0])
+        for j in range(128):
+            acc += M[s][:, :, j, None] * out[s][:, None, j]
+        out[s + 1] += acc
+    return out
+
+
+@pytest.mark.parametrize("segments, norm", [(2, 0.9), (38, 0.9), (38, 1.0)])
+def test_chain_is_as_exact_as_fp32(segments, norm):
+    gen = torch.Generator(device="cuda").manual_seed(segments)
+    h = torch.randn(segments, 2, 128, 128, generator=gen, device="cuda")
+    M = torch.randn(segments, 2, 128, 128, generator=gen, device="cuda") * (norm / 128 ** 0.5)
+    ref = plain(h.double(), M.double())
+    error = lambda x: float((x.double() - ref).norm() / ref.norm())
+    assert error(chain(h, M)) <= error(plain(h, M))  # (16 terms one after the other, then a tree: 16 + 3 roundings instead of 128)
+
+
+def test_chain_beyond_the_range_of_a_splitting():
+    """Values up to the end of the fp32 range, and infinities that stay in their column."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    h = 1e37 * torch.randn(3, 1, 128, 128, generator=gen, device="cuda")
+    M = torch.randn(3, 1, 128, 128, generator=gen, device="cuda") * (0.5 / 128 ** 0.5)
+    h[0, 0, 5, 7] = float("inf")
+    out, ref = chain(h, M), plain(h, M)
+    assert torch.equal(torch.isfinite(out), torch.isfinite(ref)) and torch.equal(torch.isnan(out), torch.isnan(ref))
+    fine = torch.isfinite(ref)
+    assert float((out[fine].double() - ref[fine].double()).norm() / ref[fine].double().norm()) <= 1e-5
