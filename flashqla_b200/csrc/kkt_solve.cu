@@ -146,15 +146,15 @@ __device__ __forceinline__ void load_f(Frag& f, const float* frag, int lane) {
 __device__ __forceinline__ void clear(Frag& f) { f[0][0] = f[0][1] = f[1][0] = f[1][1] = 0; }
 // Rounded to TF32 (11 significant bits), to nearest: the upper part of Veltkamp's splitting, two values per instruction.
 // (cvt.rna.tf32.f32 takes 22 cycles and the time of four instructions; beyond 4e34 the splitting overflows.)
+__device__ __forceinline__ F2 nearest_tf32(F2 x) {
+  const F2 minus = f2(-1.f, -1.f), y = mul2(x, f2(8193.f, 8193.f));
+  return fma2(fma2(x, minus, y), minus, y);
+}
 __device__ __forceinline__ void round_tf32(Frag& f) {
-  const F2 k = f2(8193.f, 8193.f), minus = f2(-1.f, -1.f);
 #pragma unroll
   for (int s = 0; s < 2; ++s)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const F2 x = mul2(f[s][h], k);
-      f[s][h] = fma2(fma2(f[s][h], minus, x), minus, x);
-    }
+    for (int h = 0; h < 2; ++h) f[s][h] = nearest_tf32(f[s][h]);
 }
 // acc += A B^T for fragments of A and B that hold TF32 values.
 __device__ __forceinline__ void product_tf32(Frag& acc, const Frag& a, const Frag& b) {
@@ -168,21 +168,23 @@ __device__ __forceinline__ void product_tf32(Frag& acc, const Frag& a, const Fra
           "mov.b64 %0, {c0, c1};\nmov.b64 %1, {c2, c3};\n}\n"
           : "+l"(acc[t][0]), "+l"(acc[t][1]) : "l"(a[s][0]), "l"(a[s][1]), "l"(b[s][t]));
 }
-// A B^T of fp32 operands, nearly to fp32 precision: each as a sum of two TF32 values (cut, not rounded: 21 bits), the product
-// of the small parts left out.
+// A B^T of fp32 operands, to fp32 precision: each as a sum of two TF32 values (the upper one rounded to nearest, so that the
+// lower one, which has 12 bits, is cut by one: 2^-23 of the operand), the product of the small parts left out (2^-24).
 __device__ __forceinline__ F2 cut_tf32(F2 x) { return x & 0xffffe000ffffe000ull; }
-__device__ __forceinline__ void product_3xtf32(Frag& out, const Frag& a, const Frag& b) {
+__device__ __forceinline__ void split_tf32(const Frag& x, Frag& hi, Frag& lo) {
   const F2 minus = f2(-1.f, -1.f);
-  Frag ah, al, bh, bl, small;
 #pragma unroll
   for (int s = 0; s < 2; ++s)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      ah[s][h] = cut_tf32(a[s][h]);
-      al[s][h] = cut_tf32(fma2(ah[s][h], minus, a[s][h]));
-      bh[s][h] = cut_tf32(b[s][h]);
-      bl[s][h] = cut_tf32(fma2(bh[s][h], minus, b[s][h]));
+      hi[s][h] = nearest_tf32(x[s][h]);
+      lo[s][h] = cut_tf32(fma2(hi[s][h], minus, x[s][h]));
     }
+}
+__device__ __forceinline__ void product_3xtf32(Frag& out, const Frag& a, const Frag& b) {
+  Frag ah, al, bh, bl, small;
+  split_tf32(a, ah, al);
+  split_tf32(b, bh, bl);
   clear(out);
   clear(small);
   product_tf32(out, ah, bh);
