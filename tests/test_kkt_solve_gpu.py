@@ -75,3 +75,22 @@ def test_off_diagonal_blocks_are_as_exact_as_fp32():
     A, ref = out[1][0].view(-1, 64, Hv, 64), solve(k.double(), g.double(), beta.double())[0].half().view(-1, 64, Hv, 64)
     wrong = [(A[:, d + 16:d + 32, :, d:d + 16] != ref[:, d + 16:d + 32, :, d:d + 16]).double().mean() for d in (0, 32)]
     assert float(sum(wrong)) / 2 <= 0.06
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16])
+def test_values_up_to_the_end_of_the_range(dtype):
+    """Gates that grow: entries of A up to 1e36 (a splitting by 8193 x would overflow from 4e34 on)."""
+    import flashqla_b200 as fq
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    T, H = 64, 2
+    k = torch.nn.functional.normalize(torch.randn(T, H, 128, generator=gen, device="cuda"), dim=-1).to(dtype)
+    g, beta = torch.full((T, H), 1.39, device="cuda"), torch.rand(T, H, generator=gen, device="cuda")
+    v = torch.randn(1, T, H, 128, generator=gen, device="cuda").to(dtype)
+    A = fq.chunk_gated_delta_rule_fwd(v, k[None], v, g[None], beta[None])[1][0]
+    fq.check_device_status()
+    ref = solve(k.double(), g.double(), beta.double())[0]
+    assert float(ref.abs().max()) > 1e35
+    # relative to what the decay makes of an entry: one rounding to 16 bits, three TF32 factors
+    gc = g.double().cumsum(0)
+    scale = torch.exp(gc[:, None, :] - gc[None, :, :]).transpose(1, 2)
+    assert float(((A.double() - ref) / scale).abs().max()) <= float((ref / scale).abs().max()) * (torch.finfo(dtype).eps / 2 + 3 * 2.0 ** -11)
