@@ -285,8 +285,8 @@ def chunk_gated_delta_rule_bwd(
     oracle's convention, tests/ref_gdr.py:378)."""
     host = _cabi.host()
     host.chunk_check(q, k, v, g, beta, initial_state, cu_seqlens, transpose_state_layout)
-    plan, _, chunks = _lengths(q, v, cu_seqlens, auto_cp)
-    return host.chunk_bwd(q, k, v, g, beta, A, do, dht, scale, initial_state, cu_seqlens, chunks, h, v_new,
+    plan, order, chunks = _lengths(q, v, cu_seqlens, auto_cp)
+    return host.chunk_bwd(q, k, v, g, beta, A, do, dht, scale, initial_state, cu_seqlens, order, chunks, h, v_new,
                           transpose_state_layout, w, plan, cp.INLINE_WARMUP, cp.WARMUP_THRESHOLD)
 
 

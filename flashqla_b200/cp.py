@@ -53,7 +53,7 @@ _PLAN_CACHE: Dict[Tuple, CpPlan] = {}
 
 def _uncut_makespan(chunks: Sequence[int], num_v_heads: int, num_sms: int) -> int:
     """Chunks until the last SM is through when every sequence and head is one chain, longest sequences first, each on the SM
-    that is free first (which is how the scan starts them)."""
+    that is free first (which is how both scans start them)."""
     busy = [0] * num_sms
     for c in sorted(chunks, reverse=True):
         for _ in range(num_v_heads):

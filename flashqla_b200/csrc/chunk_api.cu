@@ -255,6 +255,8 @@ extern "C" QLA_API int qla_chunk_bwd(const QlaChunkBwdArgs* args, void* stream_)
     sp.dht = a.seg_dht; sp.dht_kv = 1;
     mode.out_map = a.seg_dh0_map;
     mode.lead = a.seg_lead;
+  } else {
+    mode.seq_order = a.seq_order;
   }
   int rc = launch_bwd_scan(sp, mode, total_tokens, is_bf16, stream);
   if (rc != QLA_OK) return rc;

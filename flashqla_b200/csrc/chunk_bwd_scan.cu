@@ -106,7 +106,8 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int32_t* out_map = pass_b ? mode.out_map_b : mode.out_map;
   float* out_states = pass_b ? mode.out_b : p.dh0;
   const int hv = cta % p.num_v_heads;
-  const int seq = cta / p.num_v_heads;
+  const int slot = cta / p.num_v_heads;
+  const int seq = mode.seq_order ? mode.seq_order[slot] : slot;  // CTAs start in grid order: the caller's order of sequences
   const int hk = hv / (p.num_v_heads / p.num_k_heads);
   int seq_start, seq_end;
   if (p.cu_seqlens != nullptr) {

@@ -101,6 +101,7 @@ struct BwdParams {
 struct BwdScanMode {
   const int32_t* chunk_limit;   // [num_seqs, Hv] or NULL: only the FIRST chunk_limit chunks of an interval (<= 0: none)
   const int32_t* out_map;       // [num_seqs] row of dh0 an interval writes (< 0: none) or NULL (identity)
+  const int32_t* seq_order;     // [num_seqs] interval that a slot of the grid takes, or NULL (grid order)
   const int32_t* lead;          // [num_seqs, Hv] or NULL: chunks BEHIND an interval (same sequence) that are scanned first
                                 // from a zero gradient, nothing of them stored: the warm-up of a segment inside its own scan
   int chunks_upper;             // rows of the dh / du workspace in chunks (extent of the store maps); unused when state_only

@@ -476,10 +476,11 @@ py::tuple chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
                         w_in_scan ? py::none() : py::cast(w), opt(rnorm), opt(beta_act));
 }
 
-// The raw backward (chunk.chunk_gated_delta_rule_bwd): `g_` is the cumulative gate of the forward.
+// The raw backward (chunk.chunk_gated_delta_rule_bwd): `g_` is the cumulative gate of the forward, `order` the order in which the
+// sequences of cu_seqlens are started.
 py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, const Tensor& A_,
                     const Tensor& do_, const OptTensor& dht_, std::optional<double> scale_, const OptTensor& initial_state,
-                    const OptTensor& cu_seqlens, int64_t n_chunks, const OptTensor& h_,
+                    const OptTensor& cu_seqlens, const OptTensor& order, int64_t n_chunks, const OptTensor& h_,
                     const OptTensor& v_new_, bool transposed, const OptTensor& w_, const Plan* plan, bool inline_warmup,
                     double threshold) {
   py::gil_scoped_release nogil;
@@ -557,6 +558,9 @@ py::tuple chunk_bwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const 
     segment_chain(*plan, sc, Hv, true, stream);
     a.num_segments = plan->num_segments; a.seg_cu = ptr<int32_t>(plan->cu); a.seg_dht = ptr<float>(sc.h0);
     a.seg_dh0_map = ptr<int32_t>(plan->seg_start_of); a.seg_lead = sc.lead; a.seg_tables = ptr<int32_t>(plan->tables);
+  } else if (order.has_value()) {
+    used_here(*order);
+    a.seq_order = ptr<int32_t>(order);
   }
   const size_t bytes = qla_chunk_bwd_workspace_bytes(&a);
   const Tensor ws = new_tensor({static_cast<int64_t>(bytes)}, at::kByte, dev);

@@ -326,6 +326,8 @@ typedef struct QlaChunkBwdArgs {
   const int32_t* tables;     /* ready chunk tables of cu_seqlens (the workspace content of QLA_CHUNK_TABLES_READY) or NULL:
                                 computed by a launch                                                               */
   const int32_t* seg_tables; /* the same for seg_cu                                                                */
+  const int32_t* seq_order;  /* device int32 [N] or NULL: the order in which the reverse scan starts the sequences (as in
+                                QlaChunkFwdArgs); not with num_segments                                            */
 } QlaChunkBwdArgs;
 
 QLA_API size_t qla_chunk_bwd_workspace_bytes(const QlaChunkBwdArgs* args);
