@@ -509,11 +509,14 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           const int ph = i & 1, j = i + 1;
           const uint64_t ka_i = static_cast<uint64_t>(slot_i * (kKaBytes >> 4)), ka_j = static_cast<uint64_t>(slot * (kKaBytes >> 4));
           if (i >= 0) {
+            trace(0, i, 0);
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSbfReady), ph, true))) break;
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kWReady), ph, true))) break;
+            trace(0, i, 2);
             ptx::tc_fence_after_sync();
             ptx::umma_ts_k128_rolled<128, 128>(tmem0 + kColD2, tmem0 + kColSbf, w_desc, id_w, kStateOnly ? !zero_v : true,
                                                bar_addr(kD2Done));
+            trace(0, i, 3);
             if (!kStateOnly)
               ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf,
                                                  q_desc + static_cast<uint64_t>(ph * (kQvBytes >> 4)), id_n64, false,
@@ -526,11 +529,14 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             ptx::umma_ss_k64<128, 2>(tmem0 + kColD0, kmn_desc + ka_j, aw_desc + ka_j, id_u, false, bar_addr(kWDone));
           }
           if (i >= 0) {
+            trace(0, i, 4);
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdReady), ph, true))) break;
             if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSScaled), ph, true))) break;
+            trace(0, i, 6);
             ptx::tc_fence_after_sync();
             ptx::umma_ts_k64_halves<128>(tmem0 + kColS, tmem0 + kColD2, kmn_desc + ka_i, id_mn128, true, bar_addr(kSDone),
                                          bar_addr(kKaEmpty0 + slot_i));
+            trace(0, i, 7);
             if (kStateOnly) ptx::umma_commit(&bars[kEmpty0 + ph]);
             if (!kStateOnly) {
               if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdStored), ph, true))) break;
@@ -552,6 +558,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
               ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, q_desc + qv, k_desc + ka_j, id_p, false, bar_addr(kPDone));
             }
           }
+          if (i >= 0) trace(0, i, 8);
           slot_i = slot;
           if (++slot == kKaStages) {
             slot = 0;
@@ -1215,6 +1222,7 @@ int launch_chunk_fwd(const FwdParams& p, const void* q, const void* k, const voi
     if (w_in_scan && p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, true, true); \
     else if (w_in_scan && p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, true, false, true);  \
     else if (w_in_scan && state_only) QLA_LAUNCH_FWD(kSmemBytesWIn, T, true, false, false, false, false, true);    \
+    else if (w_in_scan && traced) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, true, false, false, true);   \
     else if (w_in_scan) QLA_LAUNCH_FWD(kSmemBytesWIn, T, false, false, false, false, false, true);                 \
     else if (p.state_dtype == QLA_DT_BF16) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false, false, true);   \
     else if (p.norm_gate != nullptr) QLA_LAUNCH_FWD(kSmemBytes, T, false, false, false, true);                \

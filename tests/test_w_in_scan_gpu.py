@@ -66,3 +66,24 @@ def test_pool(lens, heads, weak, pool_dtype, norm):
     rest = torch.ones(len(h0), dtype=torch.bool, device="cuda")
     rest[slots[1:].long()] = False
     assert torch.equal(pools[1][rest], h0.to(pool_dtype)[rest])
+
+
+def test_trace_is_filled():
+    """A trace buffer that is set records calls that keep nothing, too, and changes no result."""
+    import flashqla_b200 as fq
+    from flashqla_b200 import _cabi
+    q, k, v, g, beta, _, cu = inputs([64 * 12], 1, 2, torch.bfloat16, False, 6)
+    with torch.no_grad():
+        plain = fq.chunk_gated_delta_rule(q, k, v, g, beta, output_final_state=True, cu_seqlens=cu)
+        buf = torch.zeros(3 * 4 * 16 + 3 * 2, dtype=torch.int64, device="cuda")  # roles x chunks x events, then the two CTAs
+        _cabi.check(_cabi.lib().qla_set_trace_buffer(buf.data_ptr(), buf.numel()), "qla_set_trace_buffer")
+        try:
+            traced = fq.chunk_gated_delta_rule(q, k, v, g, beta, output_final_state=True, cu_seqlens=cu)
+            torch.cuda.synchronize()
+        finally:
+            _cabi.check(_cabi.lib().qla_set_trace_buffer(None, 0), "qla_set_trace_buffer")
+    fq.check_device_status()
+    assert torch.equal(plain[0], traced[0]) and torch.equal(plain[1], traced[1])
+    phases, ctas = buf[:192].view(3, 4, 16), buf[192:].view(2, 3)
+    assert (phases[0, :, [0, 2, 3, 4, 6, 7, 8, 9, 10, 11]] > 0).all() and (phases[1, :, 2:6] > 0).all() and (phases[2, :, [6, 8, 9, 10, 12]] > 0).all()
+    assert (ctas[:, 0] > 0).all() and (ctas[:, 1] > ctas[:, 0]).all()
