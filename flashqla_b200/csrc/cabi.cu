@@ -67,7 +67,7 @@ extern "C" QLA_API int qla_selftest_bounded_wait(int32_t* status, uint64_t limit
 }
 
 namespace qla {
-void launch_info_chunk_fwd_kernel(int*, size_t*);
+void launch_info_chunk_fwd_kernel(bool aux, bool w_in_scan, int*, size_t*);
 void launch_info_bwd_scan_kernel(int*, size_t*);
 void launch_info_bwd_chunk_kernel(int*, size_t*);
 void launch_info_kkt_solve_kernel(int*, size_t*);
@@ -80,7 +80,9 @@ extern "C" QLA_API int qla_kernel_launch_info(const char* kernel, int32_t* block
   int block = 0;
   size_t smem = 0;
   const std::string name(kernel);
-  if (name == "chunk_fwd_kernel") launch_info_chunk_fwd_kernel(&block, &smem);
+  if (name == "chunk_fwd_kernel") launch_info_chunk_fwd_kernel(false, false, &block, &smem);
+  else if (name == "chunk_fwd_kernel:aux") launch_info_chunk_fwd_kernel(true, false, &block, &smem);
+  else if (name == "chunk_fwd_kernel:w_in_scan") launch_info_chunk_fwd_kernel(false, true, &block, &smem);
   else if (name == "bwd_scan_kernel") launch_info_bwd_scan_kernel(&block, &smem);
   else if (name == "bwd_chunk_kernel") launch_info_bwd_chunk_kernel(&block, &smem);
   else if (name == "kkt_solve_kernel") launch_info_kkt_solve_kernel(&block, &smem);

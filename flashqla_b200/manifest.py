@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+import re
 import sys
 from pathlib import Path
 
@@ -45,17 +46,26 @@ def _type_name(t) -> str:
 # Launch rules of the main kernels: what a launcher has to know besides the cubin.  Block size and dynamic shared
 # memory are checked against the library itself (qla_kernel_launch_info) by the tests.
 _TMAP = "CUtensorMap (128 B, __grid_constant__)"
+# chunk_fwd_kernel has three forms with different shared memory, by its template arguments (_chunk_fwd_form): plain, :aux (stores h
+# and / or v_new) and :w_in_scan (QLA_CHUNK_W_IN_SCAN).
+_CHUNK_FWD = dict(
+    block=640, cluster=1, grid="num_seqs * Hv (x 2 with QLA_CHUNK_DUAL_TRANSITION)",
+    params=[_TMAP + " " + n for n in ("q", "k", "v", "A", "w", "o", "v_new", "h")] + ["FwdParams (by value)"],
+    tensor_maps="A (:w_in_scan: also w): 3-D (64, heads, tokens), box 64 x 1 x 64; q, k, v, w, o, v_new: 4-D (64 columns, heads, tokens, "
+                "2 halves), box 64 x 1 x 64 x 2; h: the same over rows of [chunks * Hv * 128, 128]; 16-bit elements, 128B swizzle; any "
+                "map for what a launch does not use")
 KERNEL_RULES = {
-    "chunk_fwd_kernel": dict(
-        block=640, dynamic_smem=197632, cluster=1, grid="num_seqs * Hv (x 2 with QLA_CHUNK_DUAL_TRANSITION)",
-        params=[_TMAP + " q", _TMAP + " k", _TMAP + " v", _TMAP + " A", _TMAP + " w", _TMAP + " o", "FwdParams (by value)"],
-        tensor_maps="A: 3-D (64, heads, tokens), box 64 x 1 x 64; q, k, v, w, o: 4-D (64 columns, heads, tokens, 2 halves), "
-                    "box 64 x 1 x 64 x 2; 16-bit elements, 128B swizzle"),
+    "chunk_fwd_kernel": dict(_CHUNK_FWD, dynamic_smem=197632),
+    "chunk_fwd_kernel:aux": dict(_CHUNK_FWD, dynamic_smem=214016),
+    "chunk_fwd_kernel:w_in_scan": dict(_CHUNK_FWD, dynamic_smem=222208),
     "kkt_solve_kernel": dict(
-        block=128, dynamic_smem=71680, cluster=1, grid="(pairs of 64-token chunks) * Hk * (CTAs that share the v-heads of a k-head: head_splits)",
-        params=[_TMAP + " k", _TMAP + " q", _TMAP + " A", _TMAP + " w", "KktParams (by value)"],
-        tensor_maps="k, q, w: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 128 (w: 64) x 2; A: 3-D (64, heads, tokens), "
-                    "box 64 x 1 x 64; 16-bit elements, 128B swizzle"),
+        block=128, dynamic_smem=71680, cluster=1,
+        grid="min(items, 3 * SMs), persistent; items = (pairs of 64-token chunks) * Hk * head_splits",
+        params=[_TMAP + " k", _TMAP + " q", _TMAP + " A", _TMAP + " w",
+                "KktParams (by value; the launcher sets num_pairs (equal lengths), heads_per_cta and head_splits = "
+                "ceil(Hv / Hk / heads_per_cta))"],
+        tensor_maps="k, q, w: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 128 (w: 64) x 2; A, and w of the form with "
+                    "kW = 0: 3-D (64, heads, tokens), box 64 x 1 x 64; 16-bit elements, 128B swizzle"),
     "bwd_scan_kernel": dict(
         block=416, dynamic_smem=214016, cluster=1, grid="num_seqs * Hv (twice that for a dual state-only launch)",
         params=[_TMAP + " q", _TMAP + " k", _TMAP + " dO", _TMAP + " w", _TMAP + " dh (store)", _TMAP + " du (store)",
@@ -74,6 +84,12 @@ KERNEL_RULES = {
 }
 
 
+def _chunk_fwd_form(mangled: str) -> str:
+    """Suffix of the rule of an instantiation: chunk_fwd_kernel<T, kStateOnly, kAux, kTrace, kNorm, kState16, kWIn>."""
+    flags = re.search(r"chunk_fwd_kernelI\w+?((?:Lb[01]E){6})", mangled).group(1)[2::4]
+    return ":aux" if flags[1] == "1" else ":w_in_scan" if flags[5] == "1" else ""
+
+
 def _kernel_entries(directory: Path) -> list:
     """Per-kernel entries from what the build recorded (``kernels.ptxas.json``: the compiler's own report)."""
     rec = Path(directory) / "kernels.ptxas.json"
@@ -83,6 +99,8 @@ def _kernel_entries(directory: Path) -> list:
     for src, kernels in json.loads(rec.read_text()).items():
         for k in kernels:
             base = next((n for n in KERNEL_RULES if n in k["mangled"]), None)
+            if base == "chunk_fwd_kernel":
+                base += _chunk_fwd_form(k["mangled"])
             rule = KERNEL_RULES.get(base, {})
             entries.append({
                 "export_name": k["mangled"], "kernel_name": base or k["mangled"], "source": src,

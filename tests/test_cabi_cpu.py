@@ -109,6 +109,26 @@ def test_manifest_lists_every_kernel_with_its_cubin(built_lib):
     assert lib.qla_kernel_launch_info(b"no_such_kernel", ctypes.byref(block), ctypes.byref(smem)) == -1
 
 
+def test_manifest_gives_every_form_of_the_scan_its_shared_memory(built_lib):
+    """chunk_fwd_kernel<T, kStateOnly, kAux, kTrace, kNorm, kState16, kWIn>: the forms with kAux and kWIn use more than the plain one."""
+    import json
+    from flashqla_b200 import _cabi, manifest
+    m = json.loads((built_lib.parent / manifest.MANIFEST_NAME).read_text())
+    lib, seen, shared = _cabi.lib(), set(), {}
+    for k in m["kernels"]:
+        form = re.search(r"chunk_fwd_kernelI\w+?Lb[01]ELb([01])ELb[01]ELb[01]ELb[01]ELb([01])E", k["export_name"])
+        if form is None:
+            continue
+        name = "chunk_fwd_kernel" + {("0", "0"): "", ("1", "0"): ":aux", ("0", "1"): ":w_in_scan"}[form.groups()]
+        block, smem = ctypes.c_int32(), ctypes.c_size_t()
+        assert lib.qla_kernel_launch_info(name.encode(), ctypes.byref(block), ctypes.byref(smem)) == 0
+        assert k["kernel_name"] == name and k["shared"] == smem.value and len(k["param_names"]) == 9
+        assert k["shared"] + k["static_shared"] <= 227 * 1024
+        seen.add(name)
+        shared[name] = smem.value
+    assert len(seen) == 3 and shared["chunk_fwd_kernel"] < min(shared["chunk_fwd_kernel:aux"], shared["chunk_fwd_kernel:w_in_scan"])
+
+
 def test_another_torch_means_another_build(built_lib, tmp_path, monkeypatch):
     """The host module is compiled against torch and Python: a build for others is neither current nor accepted."""
     from types import SimpleNamespace
