@@ -463,6 +463,17 @@ int launch_recurrent_tree(const QlaRecurrentArgs& a, int rows, cudaStream_t stre
       if (rc != QLA_OK) return rc;
     }
     rows = tiles <= resident ? 16 : 32;
+    // A tree's tiles of 32 rows with fp32 scratch are resident three per SM, not four: a second round of them that is more than a
+    // quarter full takes longer than two rounds of 16 rows.  128 / 136 / 144 / 147 heads of 8 steps, us: 16 rows 22.5 / 23.3 / 23.3 /
+    // 23.9, 32 rows 21.3 / 23.5 / 24.9 / 26.0; of 3 steps 11.4 / 11.4 / 11.4 / 11.5 and 11.3 / 11.6 / 12.3 / 12.5.
+    if constexpr (kTree && std::is_same<InterT, float>::value) {
+      int resident32 = 0;
+      if (rows == 32 && tiles <= 2 * static_cast<int64_t>(resident)) {
+        const int rc = resident_tiles<T, InterT, StateT, 2, kTree>(&resident32);
+        if (rc != QLA_OK) return rc;
+        if (4 * (tiles / 2) > 5 * static_cast<int64_t>(resident32)) rows = 16;
+      }
+    }
   }
   return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, kTree>(a, stream)
                     : launch_recurrent_rows<T, InterT, StateT, 2, kTree>(a, stream);

@@ -25,3 +25,34 @@ def test_decode_around_the_line(n, pool_dtype):
     # fp32 arithmetic, one rounding of o (2^-9 of values up to 1) and of a bf16 state
     assert orc.max_abs(o.float().cpu(), ref) <= 3e-3
     assert orc.max_abs(pool.float().cpu(), ref_state) <= (1e-4 if pool_dtype == torch.float32 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("n, rows", [(74, 16), (75, 32), (111, 32), (138, 32), (139, 16), (148, 16), (149, 32)])
+def test_trees_with_fp32_scratch(n, rows):
+    """32-row tiles of a tree are resident three per SM: with 139 to 148 heads two rounds of 16 rows take less time.  Either height
+    gives the same bits."""
+    import flashqla_b200 as fq
+    from torch.profiler import ProfilerActivity, profile
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line depends on the number of SMs")
+    gen = torch.Generator().manual_seed(n)
+    q, k, v = (torch.randn(1, 3 * n, 1, 128, generator=gen).bfloat16().cuda() for _ in range(3))
+    a, b = (torch.randn(1, 3 * n, 1, generator=gen).cuda() for _ in range(2))
+    pool = (0.1 * torch.randn(n, 1, 128, 128, generator=gen)).cuda()
+    parents = torch.tensor([[-1, 0, 0]] * n, dtype=torch.int32, device="cuda")
+
+    def step(block_dv):
+        scratch = torch.zeros(n, 3, 1, 128, 128, device="cuda")
+        o = fq.fused_sigmoid_gating_delta_rule_update(
+            torch.zeros(1, device="cuda"), a, torch.zeros(1, device="cuda"), q, k, v, b, pool, torch.arange(n, dtype=torch.int32, device="cuda"),
+            use_qk_l2norm_in_kernel=True, disable_state_update=True, intermediate_states_buffer=scratch,
+            intermediate_state_indices=torch.arange(n, dtype=torch.int32, device="cuda"), retrieve_parent_token=parents, block_dv=block_dv)
+        return o, scratch
+
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        got = step(None)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "recurrent_kernel" in e.name]
+    assert names and all(f", {rows // 16}, true>" in name for name in names), names
+    for other in (step(16), step(32)):
+        assert torch.equal(got[0], other[0]) and torch.equal(got[1], other[1])
