@@ -36,8 +36,8 @@ def prefill_into_state_pool(
     (``[slots, Hv, V, K]`` fp32, contiguous, updated in place).  With ``continue_from_pool`` the sequences
     start from the states already in their slots (chunked prefill of a long prompt, prefix reuse), else from
     zero.  A slot index of ``-1`` starts from zero and writes nothing.  The pool may be fp32 or bf16.  Returns
-    ``(o, state_pool)``.  ``forward_kwargs`` go to ``chunk_gated_delta_rule_fwd``
-    (``use_qk_l2norm_in_kernel``, ``A_log`` ...)."""
+    ``(o, state_pool)``.  ``forward_kwargs`` are those of ``chunk_gated_delta_rule_fwd`` that are not
+    determined here (``use_qk_l2norm_in_kernel``, ``A_log`` ...); what they ask for beside ``o`` is not returned."""
     if state_pool.dim() != 4 or state_pool.dtype not in (torch.float32, torch.bfloat16) or not state_pool.is_contiguous():
         raise ValueError("state_pool must be a contiguous float32 or bfloat16 tensor [slots, Hv, V, K]")
     Hv = v.shape[2]

@@ -121,3 +121,15 @@ def test_native_checks_look_at_ranks_and_token_counts():
             _native_update(q, v, t(1, 2, 4))
     with pytest.raises(AssertionError, match="v .B,T,Hv,V."):
         _cabi.host().chunk_check(t(1, 2, 2, 128), t(1, 2, 2, 128), t(1, 1, 4, 128), t(1, 2, 4), t(1, 2, 4), None, None, False)
+
+
+def test_prefill_into_state_pool_takes_the_raw_forwards_keywords():
+    """What ``prefill_into_state_pool`` passes on has the names and defaults of ``chunk_gated_delta_rule_fwd``."""
+    import inspect
+    from flashqla_b200 import chunk, handoff
+    raw = inspect.signature(chunk.chunk_gated_delta_rule_fwd).parameters
+    passed = {n: p.default for n, p in inspect.signature(handoff._output).parameters.items() if p.kind is p.KEYWORD_ONLY}
+    assert passed == {n: raw[n].default for n in passed}
+    fixed = {"q", "k", "v", "g", "beta", "scale", "initial_state", "cu_seqlens", "output_final_state", "transpose_state_layout",
+             "initial_state_indices", "final_state_out", "final_state_indices"}
+    assert set(raw) == set(passed) | fixed
