@@ -31,7 +31,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 K = V = 128
-MEASURED_SCAN_DRAM_BYTES_PER_TOKEN_HK16_HV32 = 38918.0
+MEASURED_SCAN_DRAM_BYTES_PER_TOKEN_HK16_HV32 = 35499.0
 CHUNK = 64
 
 
@@ -164,7 +164,7 @@ def measure(fn, steps, warmup, world, device, flush_l2=False, min_seconds=None):
 # ------------------------------------------------------------------------------------ workloads
 def SCAN_DRAM_BYTES_PER_TOKEN_HEADS(Hk, Hv):
     """DRAM bytes per token moved by one launch of the chunk scan: dram__bytes_read + dram__bytes_write of an
-    ncu capture of this kernel on a smaller case (8192 tokens, 16 k-heads / 32 v-heads: 318.8 MB = 38.9 KB
+    ncu capture of this kernel on a smaller case (8192 tokens, 16 k-heads / 32 v-heads: 290.8 MB = 35.5 KB
     per token), scaled by the head counts of this rank."""
     # the scan reads q, k per k-head (512 B) and v, w, A, gates per v-head and writes o (904 B)
     return MEASURED_SCAN_DRAM_BYTES_PER_TOKEN_HK16_HV32 * (Hk * 512 + Hv * 904) / (16 * 512 + 32 * 904)

@@ -251,7 +251,7 @@ def _forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, output_final_st
              norm_eps, keep=True):
     """``(g_cumsum, A, o, h, final_state, v_new, w, qk_rnorm, activated beta)`` of the raw forward (``None`` for what was
     not asked for).  Without ``keep`` (inference: ``o`` and the states are all that is wanted) ``A`` and ``w`` do not exist
-    either: the scan forms ``w`` itself instead of reading 256 bytes per token and head that the preparation wrote."""
+    either: the scan forms ``w`` itself, from an operand of half its size.  ``o`` and the states are the same bits."""
     host = _cabi.host()
     host.chunk_check(q, k, v, g, beta, None if h0_indices is not None else initial_state, cu_seqlens, transposed)
     plan, order, chunks = _lengths(q, v, cu_seqlens, auto_cp)

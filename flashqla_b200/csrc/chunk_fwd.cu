@@ -38,8 +38,8 @@
 // of the state conversion), warp 8 TMA producer + gate vectors, warp 9 MMA issuer, warps 10, 11 A diag(beta) of the
 // next chunk, warps 12-15 the output, warps 16-19 Pg.  Two smem stages of {Wt,Q}, {K} and {V,A}, each reloaded as soon as its last
 // product has read it (with the whole stage waiting for MMA3, and Q K^T behind MMA4: 512 chains of 32 chunks, 8 / 8 heads,
-// 306 us, now 287; with the output norm 379 -> 366), a four-deep ring of gate vectors; all waits are bounded mbarrier
-// waits that raise a status word instead of hanging.
+// 306 us, now 287; with the output norm 379 -> 366; kWIn has stages of its own, see its map), a four-deep ring of gate
+// vectors; all waits are bounded mbarrier waits that raise a status word instead of hanging.
 #include "chunk_params.cuh"
 
 namespace qla {
@@ -196,8 +196,8 @@ static __device__ __noinline__ bool norm_rows(uint32_t so, const T* z, int strid
 // kWIn: in place of A and w come A diag(beta) (rounded as this kernel rounds it otherwise) and -A diag(beta gamma) (as the preparation
 // kernel does for w): Wt, the product of the latter with K, is formed here, one chunk ahead of its use.  Operands and
 // orders are the same, so that results are the same bits.  It saves the write and the read of 128 bytes per token and head: 32768
-// tokens of 16 / 32 heads 138 + 227 -> 108 + 225 us (preparation + scan), 540 k packed tokens of 8 / 8 heads 588 + 1137 -> 467 + 1002.
-// (With A diag(beta) scaled here from A instead: 103 + 244 and 439 + 1090.)
+// tokens of 16 / 32 heads 140 + 226 -> 114 + 225 us (preparation + scan), 540 k packed tokens of 8 / 8 heads 584 + 1141 -> 501 + 1015.
+// (With A diag(beta) scaled here from A the preparation took 6 % less and the scan 9 % more.)
 template <typename T, bool kStateOnly, bool kAux, bool kTrace, bool kNorm = false, bool kState16 = false, bool kWIn = false>
 __global__ void __launch_bounds__(kThreads, 1)
 chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -261,7 +261,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __shared__ Gates gate_ring[kGateRing];
   constexpr uint32_t kPgTiles = kWIn ? kOffPgWIn : kOffPg, kOTiles = kWIn ? kOffOWIn : kOffO;
 
-  if (tid < kNumBars) {  // (a thread each: one after the other they were 0.5 us of a CTA's start)
+  if (tid < kNumBars) {  // (a thread each: one after the other they were 3 us of a CTA's start: scan of 64 tokens 9.8 -> 6.9 us)
     const int b = tid;
     int count = 1;  // k*Full*, k*Empty*, kGate*, kPDone, kD2Done, kSDone, kD4Done, kWDone, kOFree: one commit / one thread
     if (b == kAbReady0 || b == kAbReady1) count = 2;
@@ -466,9 +466,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // Every lane runs this loop and all waits; the tcgen05.mma / commit instructions are issued by one
     // elected lane inside the ptx::umma_* blocks.  Keeping the warp converged keeps descriptors and
     // addresses on the uniform datapath, which is what makes a product cost no more than its time on
-    // the tensor pipe.  The loop is software pipelined over i = -1 .. nproc - 1 so that every product is
-    // issued from exactly one place in the code:
-    //   [MMA2(i)] [MMAq(i)] [MMA3(i)] [MMA4(i), MMAu(i+1), MMA0(i+1)]
+    // the tensor pipe.  The loop is software pipelined over i = -1 .. nproc - 1:
+    //   [MMA2(i)] [MMAq(i), MMA0(i+1)] [MMA3(i)] [MMA4(i), MMAu(i+1)]           (MMA0 of the first chunk behind its MMAu)
+    //   [MMA2(i)] [MMAq(i), MMAw(i+1)] [MMA3(i)] [MMA4(i), MMAu(i+1), MMA0(i+1)]  kWIn
     // Between two state updates only MMA2 -> (chain: V') -> MMA3 -> (both warpgroups: 16-bit state copy)
     // are serial; the other products sit in the two gaps and complete in their shadow.
     {
@@ -619,7 +619,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (kAux && i >= 0 && p.v_new != nullptr && !(ok = ptx::mbar_wait_nocall(bar_addr(kVnRead), ph, true))) break;
         // the state-independent products of the next chunk.  MMAu(i + 1): D2 = V^T (A diag(beta))^T; A operand = V tile
         // read MN-major, B operand = the A tile scaled in place (D2: MMA3 and MMA4 precede in the pipe).
-        // MMA0(i + 1): D0 = Q K^T (Pg of chunk i, formed from D0, was waited for above).
+        // The first chunk's MMA0 too: there is no gap 1 in front of it.
         if (i + 1 < nproc) {
           const int j = i + 1, sj = j & 1;
           const uint64_t sn = static_cast<uint64_t>(sj * (kStageBytes >> 4));

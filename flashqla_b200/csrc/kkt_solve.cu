@@ -13,19 +13,20 @@
 // Per head, in 16 x 16 blocks of N = -L and X = (I + L)^-1, kept as fragments of mma.sync:
 //   1  N from K K^T and the gates; the two diagonal blocks of a warp are inverted by fp32 forward substitution, one per
 //      half-warp, lane = column
-//   2  X10 = X11 N10 X00 and X32 = X33 N32 X22: split TF32 products, 21 bits per factor
+//   2  X10 = X11 N10 X00 and X32 = X33 N32 X22: split TF32 products, to fp32 precision
 //   3  X[2:4][0:2] = X[2:4][2:4] N[2:4][0:2] X[0:2][0:2]: TF32 products, one block column per warp
-//   4  Wt = (-A diag(beta gamma)) K: a tcgen05 product, read back and stored through a swizzled tile (TMA)
+//   4  Wt = (-A diag(beta gamma)) K: a tcgen05 product, read back and stored through a swizzled tile (TMA); for a scan that forms
+//      Wt itself its operand is stored instead, and A diag(beta) in place of A
 // A product of three factors stays in registers: with T^T as the accumulator of the first product, its fragments ARE the B
 // fragments of the second, because k may be numbered as one likes (slot c stands for k = 2c, slot c + 4 for 2c + 1).  Every
 // block leaves as soon as its warp has it, in both 16-bit forms, by stmatrix.  Beside the chain the part 0 warp forms the
 // next head's gates, and the next item's K is in L2 when it starts and in shared memory when this one has been multiplied.
 //
 // What bounds it: the writes (402 of 536 MB for 32768 tokens, 32 v-heads; without any arithmetic they take 102 us) and, beside them,
-// a chain of dependent phases of some 1500 instructions per warp and head, 7 cycles each with three CTAs per SM.  Two warps per chunk
+// a chain of dependent phases of some 1700 instructions per warp and head, 7 cycles each with three CTAs per SM.  Two warps per chunk
 // instead of four, 16 x 16 blocks whose substitution does not waste half of its lanes, products in registers instead of through
-// shared memory and items in a loop: 10.1 k -> 6.4 k warp instructions per 128 tokens and head, 32768 tokens of 16 / 32 heads
-// 184 -> 132 us, 540 k packed tokens of 8 / 8 heads 836 -> 550, 32768 of 32 / 32 heads 197 -> 148.  Four warps per chunk (the emission of
+// shared memory and items in a loop: 10.1 k -> 7.0 k warp instructions per 128 tokens and head, 32768 tokens of 16 / 32 heads
+// 184 -> 140 us, 540 k packed tokens of 8 / 8 heads 836 -> 584, 32768 of 32 / 32 heads 197 -> 154.  Four warps per chunk (the emission of
 // blocks and the gates on the other two): 161 us, with 9.0 k instructions.
 #include <algorithm>
 #include <cmath>
