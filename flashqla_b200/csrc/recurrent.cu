@@ -454,7 +454,8 @@ template <typename T, typename InterT, typename StateT, bool kTree>
 int launch_recurrent_tree(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
   // Tiles of 16 rows while they are all resident at once, which spreads a small batch over the most SMs; a second round of
   // them costs the latency of every step again.  With the line at four tiles of 32 rows per SM: 96 heads of 7 tree steps 17.5 us, now
-  // 13.2; 112 heads of 4 steps 11.4 -> 9.7; 144 heads of one step 7.0 -> 5.3, with a bf16 pool 6.8 -> 4.8.
+  // 13.2; 112 heads of 4 steps 11.4 -> 9.7; 144 heads of one step 7.0 -> 5.3, with a bf16 pool 6.8 -> 4.8.  (Just above the line it is
+  // rough: 80 heads of 8 steps with fp32 scratch 14.3 with 16 rows, 14.7 with 32; of 4 steps 9.7 and 9.2; 92 of 8 15.5 and 14.8.)
   if (rows == 0) {
     const int64_t tiles = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / 16);
     int resident = 2 * 148;  // (at least: the smallest calls, which are host-bound, do not look it up)
