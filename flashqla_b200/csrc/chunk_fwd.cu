@@ -25,7 +25,7 @@
 // serial; the other products are issued into the two gaps and complete in their shadow.
 //
 // What bounds it: that chain (1.6 us per chunk with the SM to itself: 1700 cycles of products in order, and hand-offs between
-// 20 warps that share its issue slots), and with every SM busy the memory behind it (36 - 38 bytes per ns and SM).
+// 20 warps that share its issue slots), and with every SM busy the memory behind it (42 - 48 bytes per ns and SM; bulk copies alone 46 - 53).
 // Shared memory moves 72 KB of TMA writes and 112 KB of operand reads per chunk at 128 bytes a cycle.  Operands
 // that a thread produces therefore go to tensor memory (Vd as a shared-memory tile cost 48 KB per chunk), and Q K^T is
 // not stacked on other rows to fill M = 128.  All roles share the SM's instruction cache (32 KB; 94 % of its requests hit),
@@ -318,9 +318,10 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   if (warp == 8) {
     // =========================================================== TMA producer, gate vectors
-    // L2 prefetch runs kPrefetchAhead chunks ahead of the demand loads: with every SM streaming its own
-    // sequence the DRAM latency of a tile exceeds one chunk period, and only two stages fit in shared
-    // memory, so the tiles are pulled into L2 early and the demand TMA then hits L2.
+    // Tiles are not prefetched into L2.  A tensor prefetch costs the SM's copy engine and the fabric what a load costs: tiles of 128 CTAs
+    // by bulk copies, four loaded and three stored per chunk, take 292 us without prefetches and 378 with the tiles requested four chunks
+    // ahead.  Here, without and with: 4 x 8192 tokens of 32 heads with h and v_new 362 and 470 us, 540 k packed tokens of 8 / 8
+    // heads 957 and 1020, 32768 tokens of 16 / 32 heads 215 and 226, few chains (one prompt of 777 tokens) equal.
     // Tiles are reloaded as their last product has read them.  kWIn: {Q, V, A} of chunk i behind MMAq of chunk i - 2, {K, operand of Wt}
     // of chunk i + 1 behind MMA3 of chunk i - 2.  Otherwise {Wt, Q} of chunk i behind MMAq and K behind MMA3 of chunk i - 2, {V, A} of chunk i + 1
     // behind MMAu of chunk i - 1.  Gate vectors of chunk i follow when MMA3 of chunk i - 2 is through: the last readers of their ring
@@ -435,20 +436,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         cur = nxt;
       }
-      if (lane == 0) {
-        // the first demand loads go out before any prefetch; the prefetches of chunks 2.. follow chunk 1
-#pragma unroll 1
-        for (int c = (i == 1) ? 2 : i + kPrefetchAhead; i >= 1 && c <= i + kPrefetchAhead && c < nproc; ++c) {
-          const int pt0 = token_of(c);
-          if (!zero_v) ptx::tma_prefetch_l2_3d(&tm_a, 0, hv, pt0);
-          if (!zero_v) ptx::tma_prefetch_l2_4d(&tm_v, 0, hv, pt0, 0);
-          if (kWIn) ptx::tma_prefetch_l2_3d(&tm_w, 0, hv, pt0);
-          else ptx::tma_prefetch_l2_4d(&tm_w, 0, hv, pt0, 0);
-          if (!kStateOnly) ptx::tma_prefetch_l2_4d(&tm_q, 0, hk, pt0, 0);
-          ptx::tma_prefetch_l2_4d(&tm_k, 0, hk, pt0, 0);
-        }
-      }
-      if (i + kPrefetchAhead < nproc) {  // and the scalars
+      if (i + kPrefetchAhead < nproc) {  // the scalars of a chunk to come
         const int64_t ahead = token_of(i + kPrefetchAhead);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
