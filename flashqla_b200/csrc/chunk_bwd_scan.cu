@@ -13,19 +13,23 @@
 //
 // The kernel mirrors the forward scan (chunk_fwd.cu): everything is computed TRANSPOSED so that each
 // tcgen05.mma has M = 128 (the V dimension on the 128 TMEM lanes) and dependent operands stay in tensor memory:
-//   MMA0  D0[128,64]  = [K;Q] K^T            (SS)  rows 64..127 are P = Q K^T; state independent
+//   MMA0  D0[64,64]   = Q K^T                (SS, M = 64)  state independent
 //   MMAu  Du0[128,64] = dO^T Pg              (SS)  A = dO tile read MN-major, B = Pg tile read MN-major
 //   MMA2  D2[128,64]  = dS1^T_bf16 K^T       (TS)  chain
 //   MMAq  dS^T[128,128] += dO^T (s gamma .* Q)              (SS, both operands MN-major)  off the chain
 //   MMA3  dS^T[128,128] += du^T_bf16 w                     (TS, B = w tile read MN-major)  chain
 // Thread v of a compute warpgroup owns TMEM lane v (column v of dS): it forms du = Du0 + rho .* D2, writes
 // the 16-bit operand of the next product back with tcgen05.st and its 128 bytes of du^T to the workspace.
-// Warp roles (416 threads): warps 0-7 compute (both warpgroups take half of the token columns of every
+// Warp roles (512 threads): warps 0-7 compute (both warpgroups take half of the token columns of every
 // chain phase and half of the state columns of the state conversion), warp 8 TMA producer + gate vectors,
-// warp 9 MMA issuer, warps 10-11 operand tiles (Pg, s gamma .* Q in place), warp 12 sends du^T and dh^T of every
-// chunk to the workspace with TMA stores from swizzled staging tiles (a thread owns a whole row of either: stored
-// straight from registers, every 16-byte piece of a warp's store instruction would fall into a different
-// 128-byte line).
+// warp 9 MMA issuer, warp 10 sends du^T and dh^T of every chunk to the workspace with TMA stores from swizzled staging
+// tiles (a thread owns a whole row of either: stored straight from registers, every 16-byte piece of a warp's store
+// instruction would fall into a different 128-byte line), warps 12-15 operand tiles (Pg, s gamma .* Q in place).
+// {K, Q, dO} of a stage are reloaded as soon as MMAq has read them, w as soon as MMA3 has.
+// What bounds it: with every SM busy the memory (4 x 8192 tokens of 32 heads 293 us; bulk copies of as many bytes by 128 CTAs 292), else
+// the chain.  With two warps for the operand tiles (a row of Pg per thread: longer than the rest of a chunk), Q K^T as rows of an M = 128
+// product, the stage released as a whole behind MMA3 and the copy of the state read twice: 368 us; 9 packed documents of
+// 16 / 32 heads 124, now 96.
 // Every wait is a bounded mbarrier wait that raises the status word instead of hanging.
 #include "chunk_params.cuh"
 
@@ -38,7 +42,7 @@ constexpr uint32_t kColSbf = 128;   // 16-bit copy of dS^T (A operand of MMA2), 
 constexpr uint32_t kColD2 = 192;    // (K dS1)^T
 constexpr uint32_t kColDu0 = 256;   // (Pg^T dO)^T
 constexpr uint32_t kColDu16 = 320;  // 16-bit du^T (A operand of MMA3), 32 columns
-constexpr uint32_t kColD0 = 384;    // [K;Q] K^T, two buffers of 64 columns (chunk parity)
+constexpr uint32_t kColD0 = 384;    // Q K^T (M = 64: 16 lanes of every quadrant), two buffers of 64 columns (chunk parity)
 
 // ---- shared-memory map (offsets from a 1024-byte aligned base)
 constexpr uint32_t kStageKQ = 0;         // 32 KiB: half h (columns 64h..) = [K rows 8 KiB | Q rows 8 KiB]; SW128
@@ -61,13 +65,15 @@ struct alignas(16) Gates {
 constexpr int kGateRing = 4;
 
 enum Bar {
-  kFull0 = 0, kFull1, kEmpty0, kEmpty1, kPDone0, kPDone1,
+  kFull0 = 0, kFull1, kEmpty0, kEmpty1,      // {K, Q, dO} of a stage, and the gate vectors
+  kWFull0, kWFull1, kWEmpty0, kWEmpty1,      // w
+  kPDone0, kPDone1,
   kPgReady, kQsReady, kD2Done, kDu0Done, kDuReady, kSDone, kSbfReady, kSScaled,
   kTileReady,  // the compute warps have written this chunk's staging tiles (8 arrivals)
   kTileFree,   // the store warp's TMA stores of this chunk have read them (1 arrival)
   kNumBars
 };
-constexpr int kThreads = 416;
+constexpr int kThreads = 512;
 
 __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
   __syncwarp();
@@ -96,7 +102,7 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? ptx::kFmtBF16 : ptx::kFmtF16;
   grid_dep_wait();    // earlier kernels of the stream have completed (see launch_dependent)
   grid_dep_launch();  // the next one may be scheduled; it waits the same way
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // (the same for the whole warp: see chunk_fwd.cu)
   // context-parallel passes: the second half of a "dual" grid computes the K x K transition matrix of the reverse
   // recurrence over an interval's first chunks (identity start, dO treated as zero)
   const bool pass_b = mode.dual && blockIdx.x >= static_cast<unsigned>(p.num_seqs) * p.num_v_heads;
@@ -136,18 +142,23 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
   __shared__ uint64_t bars[kNumBars];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(16) float aux_g[2 * 2 * 64];  // [aux warp][chunk parity][64] cumulative gates (log2 domain)
   __shared__ Gates gate_ring[kGateRing];
 
   if (tid < kNumBars) {  // (a thread each)
     const int b = tid;
-    int count = 1;  // commits: kPDone*, kD2Done, kDu0Done, kSDone
+    int count = 1;  // commits: k*Empty*, kPDone*, kD2Done, kDu0Done, kSDone; kWFull*; kTileFree
     if (b == kFull0 || b == kFull1) count = 33;
-    else if (b == kEmpty0 || b == kEmpty1) count = 3;
-    else if (b == kPgReady || b == kQsReady) count = 2;
+    else if (b == kPgReady || b == kQsReady) count = 4;
     else if (b == kDuReady || b == kSbfReady || b == kSScaled || b == kTileReady) count = 8;
     ptx::mbar_init(&bars[b], count);
     ptx::fence_mbar_init();
+    if (tid == 0) ptx::mbar_wait_setup(p.status, bars, 64);  // + 64: the backward scan
+  }
+  if (warp >= 12) {  // the block of Pg above the diagonal (rows 0..31, columns 32..63) of both tiles
+    for (int x = tid - 384; x < 2 * 32 * 4; x += 128)
+      *reinterpret_cast<uint4*>(smem + kOffPg + (x >> 7) * 8192 + ptx::sw128_offset((x >> 2) & 31, 4 + (x & 3))) =
+          make_uint4(0, 0, 0, 0);
+    ptx::fence_proxy_async_smem();
   }
   if (warp == 8) {
     ptx::tmem_alloc(&tmem_base_s, 512);
@@ -157,18 +168,24 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem = tmem_base_s;
-  int* status = p.status;
-  auto wait = [&](int b, uint32_t parity) {
-    return ptx::mbar_wait_warp_call(&bars[b], parity, status, kStatusBarrierTimeout | ((b + 64) << 8));  // + 64: the backward scan
-  };
+  const uint32_t bar0 = ptx::smem_u32(&bars[0]);
+  auto wait = [&](int b, uint32_t parity) { return ptx::mbar_wait_addr(bar0 + 8u * static_cast<uint32_t>(b), parity); };
   auto stage_ptr = [&](int s) { return smem + s * kStageBytes; };
   auto gates_of = [&](int i) { return &gate_ring[i & (kGateRing - 1)]; };
   auto chunk_of = [&](int i) { return nproc - 1 - i; };
 
   if (warp == 8) {
     // =========================================================== producer: TMA + gate vectors
-    // (no prefetches into L2: see chunk_fwd.cu; 4 x 8192 tokens of 32 heads 368 us without and 415 with them)
+    // (no prefetches of tiles into L2: see chunk_fwd.cu; 4 x 8192 tokens of 32 heads 368 us without and 415 with them)
+    constexpr int kGatesAhead = 4;
     for (int i = 0; i < nproc; ++i) {
+      if (i + kGatesAhead < nproc) {  // the gates of a chunk to come
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int64_t tk = min(seq_start + chunk_of(i + kGatesAhead) * kChunk + lane + 32 * r, tok_end - 1);
+          ptx::prefetch_l2(p.g_cumsum + tk * p.num_v_heads + hv);
+        }
+      }
       const int s = i & 1, use = i >> 1;
       const int t0 = seq_start + chunk_of(i) * kChunk;
       const int valid = min(kChunk, (chunk_of(i) >= own_chunks ? tok_end : seq_end) - t0);
@@ -185,15 +202,15 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       uint8_t* st = stage_ptr(s);
       if (lane == 0) {
         uint64_t* full = &bars[kFull0 + s];
-        ptx::mbar_expect_tx(full, kStageBytes);
+        ptx::mbar_expect_tx(full, kStageBytes - 16384);
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           ptx::tma_load_3d(st + kStageKQ + h * 16384, &tm_k, full, h * 64, hk, t0);
           ptx::tma_load_3d(st + kStageKQ + h * 16384 + 8192, &tm_q, full, h * 64, hk, t0);
           ptx::tma_load_3d(st + kStageDO + h * 8192, &tm_do, full, h * 64, hv, t0);
-          ptx::tma_load_3d(st + kStageW + h * 8192, &tm_w, full, h * 64, hv, t0);
         }
       }
+      __syncwarp();
       Gates* gs = gates_of(i);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -210,6 +227,14 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         gs->valid = valid;
       }
       ptx::mbar_arrive(&bars[kFull0 + s]);
+      if (use > 0 && !wait(kWEmpty0 + s, (use - 1) & 1)) break;
+      if (lane == 0) {
+        uint64_t* full = &bars[kWFull0 + s];
+        ptx::mbar_expect_tx(full, 16384);
+        ptx::tma_load_3d(st + kStageW, &tm_w, full, 0, hv, t0);
+        ptx::tma_load_3d(st + kStageW + 8192, &tm_w, full, 64, hv, t0);
+      }
+      __syncwarp();
     }
   } else if (warp == 9) {
     // =========================================================== MMA issuer (whole warp, converged)
@@ -225,66 +250,67 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint64_t d_wmn = ptx::smem_desc_sw128(ptx::smem_u32(smem + kStageW), 8192, 1024);         // w tile, MN-major
     const uint64_t d_pg = ptx::smem_desc_sw128(ptx::smem_u32(smem + kOffPg), 8192, 1024);           // Pg, MN-major
     constexpr int kHalf = (16384 >> 4) - 3 * 2;  // from k-step 3 to k-step 4: the second 64-column half
+    const uint64_t d_q = d_kq + (8192 >> 4);                                                        // Q rows, K-major
+    const uint32_t id_p = ptx::mma_idesc(64, 64, fmt, ptx::kMajorK, ptx::kMajorK);                  // MMA0
     constexpr uint32_t tmem0 = 0;
-    const uint32_t bar0 = ptx::smem_u32(&bars[0]);
     auto bar_addr = [&](int b) { return bar0 + 8u * static_cast<uint32_t>(b); };
     bool ok = tmem == tmem0;
-    if (!ok) ptx::record_wait_failure(status, kStatusBadTmemBase, 0);
-    auto issue_mma0 = [&](int j) {  // D0[j & 1] = [K;Q] K^T of chunk j
+    if (!ok) ptx::record_wait_failure(p.status, kStatusBadTmemBase, 0);
+    auto ready = [&](int b, uint32_t parity) { return __all_sync(0xffffffffu, ptx::mbar_test_wait(&bars[b], parity)) != 0; };
+    auto issue_mma0 = [&](int j) {  // D0[j & 1] = Q K^T of chunk j
       const uint64_t sn = static_cast<uint64_t>((j & 1) * (kStageBytes >> 4));
       ptx::tc_fence_after_sync();
-      ptx::umma_ss_k128<2, kHalf, 2, kHalf>(tmem0 + kColD0 + (j & 1) * 64, d_kq + sn, d_kq + sn, id_n64, false,
-                                            bar_addr(kPDone0 + (j & 1)));
+      ptx::umma_ss_k128<2, kHalf, 2, kHalf>(tmem0 + kColD0 + (j & 1) * 64, d_q + sn, d_kq + sn, id_p, false, bar_addr(kPDone0 + (j & 1)));
     };
-    bool p0_issued = false;  // MMA0 of the next chunk already issued in gap 1
+    auto issue_mmau = [&](int j) {  // Du0 = dO^T Pg (the compute warps read Du0 of the chunk before in front of its MMA3)
+      ptx::tc_fence_after_sync();
+      if (!zero_do)
+        ptx::umma_ss_k64<128, 128>(tmem0 + kColDu0, d_do + static_cast<uint64_t>((j & 1) * (kStageBytes >> 4)),
+                                   d_pg + static_cast<uint64_t>((j & 1) * (8192 >> 4)), id_u, false, bar_addr(kDu0Done));
+    };
+    // [MMA2(i)] [MMAq(i), MMA0(i + 1)] [MMA3(i)] [MMAu(i + 1)] with MMA0 behind MMA3 where its tiles land late, and MMAu behind
+    // MMA2(i + 1) where Pg comes late
+    bool p_issued = false, u_issued = false;
 #pragma unroll 1
     for (int i = -1; ok && i < nproc; ++i) {
-      const int ph = i & 1;
-      const uint64_t so = static_cast<uint64_t>((i & 1) * (kStageBytes >> 4));
+      const int ph = i & 1, j = i + 1;
+      const uint64_t so = static_cast<uint64_t>(ph * (kStageBytes >> 4));
+      p_issued = false;
       if (i >= 0) {
         // MMA2: D2 = dS1^T_bf16 K^T
-        if (!(ok = wait(kSbfReady, ph))) break;
+        if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSbfReady), ph, true))) break;
         ptx::tc_fence_after_sync();
         ptx::umma_ts_k128<2, kHalf>(tmem0 + kColD2, tmem0 + kColSbf, d_kq + so, id_n64, false, bar_addr(kD2Done));
-        // gap 1 (the compute warps form du): MMAq, off the chain, and - when its tiles have landed - MMA0 of
-        // the next chunk, so that Pg of that chunk is ready long before its MMAu
-        if (!(ok = wait(kQsReady, ph))) break;
-        if (!(ok = wait(kSScaled, ph))) break;
-        ptx::tc_fence_after_sync();
-        if (!zero_do) ptx::umma_ss_k64<128, 128>(tmem0 + kColS, d_do + so, d_qmn + so, id_q, true);
-        p0_issued = false;
-        if (i + 1 < nproc) {
-          const int j = i + 1;
-          const bool landed =
-              __all_sync(0xffffffffu, ptx::mbar_test_wait(&bars[kFull0 + (j & 1)], (j >> 1) & 1)) != 0;
-          if (landed) {
-            issue_mma0(j);
-            p0_issued = true;
-          }
+        if (!u_issued) {
+          if (!(ok = ptx::mbar_wait_nocall(bar_addr(kPgReady), ph, true))) break;
+          issue_mmau(i);
         }
-        // MMA3: dS^T += du^T_bf16 w; its completion also releases the stage
-        if (!(ok = wait(kDuReady, ph))) break;
+        // gap 1 (the compute warps form du): MMAq, off the chain, and MMA0 of the next chunk
+        if (!(ok = ptx::mbar_wait_nocall2(bar_addr(kQsReady), ph, bar_addr(kSScaled), ph))) break;
         ptx::tc_fence_after_sync();
-        ptx::umma_ts_k64<128>(tmem0 + kColS, tmem0 + kColDu16, d_wmn + so, id_s, true, bar_addr(kSDone),
-                              bar_addr(kEmpty0 + ph));
+        if (!zero_do) ptx::umma_ss_k64<128, 128>(tmem0 + kColS, d_do + so, d_qmn + so, id_q, true, bar_addr(kEmpty0 + ph));
+        else ptx::umma_commit(&bars[kEmpty0 + ph]);
+        if (j < nproc && ready(kFull0 + (j & 1), (j >> 1) & 1)) {
+          issue_mma0(j);
+          p_issued = true;
+        }
+        // MMA3: dS^T += du^T_bf16 w
+        if (!(ok = ptx::mbar_wait_nocall2(bar_addr(kDuReady), ph, bar_addr(kWFull0 + ph), (i >> 1) & 1))) break;
+        ptx::tc_fence_after_sync();
+        ptx::umma_ts_k64<128>(tmem0 + kColS, tmem0 + kColDu16, d_wmn + so, id_s, true, bar_addr(kSDone), bar_addr(kWEmpty0 + ph));
       }
-      // gap 2 (the compute warps convert the state): the state-independent products of the next chunk
-      if (i + 1 < nproc) {
-        const int j = i + 1;
-        const uint64_t sn = static_cast<uint64_t>((j & 1) * (kStageBytes >> 4));
-        if (!p0_issued) {
-          if (!(ok = wait(kFull0 + (j & 1), (j >> 1) & 1))) break;
+      // gap 2 (the compute warps convert the state)
+      if (j < nproc) {
+        if (!p_issued) {
+          if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + (j & 1)), (j >> 1) & 1, true))) break;
           issue_mma0(j);
         }
-        // MMAu: Du0 = dO^T Pg (the compute warps read Du0 of this chunk before DuReady, MMA3 precedes in the pipe)
-        if (!(ok = wait(kPgReady, j & 1))) break;
-        ptx::tc_fence_after_sync();
-        if (!zero_do)
-          ptx::umma_ss_k64<128, 128>(tmem0 + kColDu0, d_do + sn, d_pg + static_cast<uint64_t>((j & 1) * (8192 >> 4)),
-                                     id_u, false, bar_addr(kDu0Done));
+        u_issued = ready(kPgReady, j & 1);
+        if (u_issued) issue_mmau(j);
       }
     }
-  } else if (warp == 12) {
+    ptx::report_issuer(p.status, ok, kNumBars + 64);
+  } else if (warp == 10) {
     // =========================================================== store warp: du^T and dh^T tiles -> workspace
     if (!state_only) {
       bool ok = true;
@@ -310,75 +336,73 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (lane == 0) ptx::tma_store_wait_all();
     }
-  } else if (warp >= 10) {
-    // =========================================================== aux warps 10, 11: operand tiles
-    const int r = tid - 320;  // 0..63: row of the A / Pg / Q tiles
+  } else if (warp >= 12) {
+    // =========================================================== operand tiles
+    // Pg: rows 16 q .. 16 q + 15 per warp (q = TMEM quadrant: the rows of an M = 64 accumulator), in the fragment layout of 8 x 8
+    // matrices, which stmatrix writes to the swizzled tile.  Warps 12, 13 have no causal entry in columns 32..63; that part of
+    // their rows is zeroed once at start-up.
     const uint32_t tm = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    float* my_g = aux_g + (warp - 10) * 128;
     const float log2_scale = __log2f(p.scale);
-    bool ok = true;
+    const int p_row = (warp & 3) * 16 + (lane >> 2), p_cols = warp < 14 ? 32 : 64;
+    const int q_row = tid & 63, q_half = (tid >> 6) & 1;
 #pragma unroll 1
-    for (int j = 0; ok && j < nproc; ++j) {
+    for (int j = 0; j < nproc; ++j) {
       const int sj = j & 1;
-      if (!(ok = wait(kFull0 + sj, (j >> 1) & 1))) break;
+      if (!wait(kFull0 + sj, (j >> 1) & 1)) break;
       const Gates* gs = gates_of(j);
-      my_g[sj * 64 + lane] = gs->g2[lane];
-      my_g[sj * 64 + 32 + lane] = gs->g2[32 + lane];
       const int valid = gs->valid;
-      // (a) Pg = s G .* P from D0 rows 64..127 (TMEM quadrants 2, 3), rows beyond the sequence end zeroed.
+      // s exp(g_c - g_d) = 2^((g2_c + log2 s) - g2_d); above the diagonal the exponent may overflow, the select below discards
+      // those entries, and rows beyond the sequence end
+      const float gr0 = gs->g2[p_row] + log2_scale, gr1 = gs->g2[p_row + 8] + log2_scale;
+      const float* gcol = gs->g2 + 2 * (lane & 3);
+      const int last0 = p_row < valid ? p_row : -1, last1 = p_row + 8 < valid ? p_row + 8 : -1;  // last column that counts
       // The Pg tile of this parity was last read by MMAu two chunks ago, which precedes this chunk's MMA0 in
       // the tensor pipe and therefore has completed when PDone fires.
-      if (!(ok = wait(kPDone0 + sj, (j >> 1) & 1))) break;
+      if (!wait(kPDone0 + sj, (j >> 1) & 1)) break;
       ptx::tc_fence_after_sync();
-      const float* gsg = my_g + sj * 64;
-      const int c = r;
-      const float gc = gsg[c] + log2_scale;
-      uint8_t* pg = smem + kOffPg + sj * 8192;
+      const uint32_t pg = ptx::smem_u32(smem + kOffPg) + sj * 8192;
 #pragma unroll 1
-      for (int db = 0; db < 64; db += 16) {
-        uint32_t pr[16];
-        ptx::tmem_ld16(tm + kColD0 + sj * 64 + db, pr);
+      for (int db = 0; db < p_cols; db += 32) {
+        uint32_t pr[16], m[8];
+        ptx::tmem_ld_frag4(tm + kColD0 + sj * 64 + db, pr);
         ptx::tmem_wait_ld();
 #pragma unroll
-        for (int j8 = 0; j8 < 16; j8 += 8) {
-          const float4 ga = *reinterpret_cast<const float4*>(&gsg[db + j8]);
-          const float4 gb = *reinterpret_cast<const float4*>(&gsg[db + j8 + 4]);
-          const float gd[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
-          float x[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float val = ptx::ex2(gc - gd[e]) * __uint_as_float(pr[j8 + e]);
-            x[e] = (db + j8 + e <= c && c < valid) ? val : 0.f;
-          }
-          *reinterpret_cast<uint4*>(pg + ptx::sw128_offset(c, (db + j8) >> 3)) =
-              make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
+        for (int x = 0; x < 4; ++x) {
+          const float2 gc = *reinterpret_cast<const float2*>(gcol + db + 8 * x);
+          const int d = db + 8 * x + 2 * (lane & 3);
+          const float x0 = ptx::ex2(gr0 - gc.x) * __uint_as_float(pr[4 * x]);
+          const float x1 = ptx::ex2(gr0 - gc.y) * __uint_as_float(pr[4 * x + 1]);
+          const float y0 = ptx::ex2(gr1 - gc.x) * __uint_as_float(pr[4 * x + 2]);
+          const float y1 = ptx::ex2(gr1 - gc.y) * __uint_as_float(pr[4 * x + 3]);
+          m[2 * x] = pack2<T>(d <= last0 ? x0 : 0.f, d + 1 <= last0 ? x1 : 0.f);
+          m[2 * x + 1] = pack2<T>(d <= last1 ? y0 : 0.f, d + 1 <= last1 ? y1 : 0.f);
         }
+        // matrices (columns 8 j, rows 0..7), (8 j, rows 8..15), (8 (j + 1), ..), ..: lane -> row of matrix lane / 8
+        const int r = (warp & 3) * 16 + (lane & 15), c16 = (db >> 3) + (lane >> 4);
+        ptx::stmatrix_x4(pg + ptx::sw128_offset(r, c16), m[0], m[1], m[2], m[3]);
+        ptx::stmatrix_x4(pg + ptx::sw128_offset(r, c16 + 2), m[4], m[5], m[6], m[7]);
       }
       ptx::fence_proxy_async_smem();
       ptx::tc_fence_before_sync();
       warp_arrive(&bars[kPgReady], lane);
-      // (b) Q rows times s gamma (0 beyond the sequence end), in place: MMA0 has read the raw tile
-      const float f = gs->sgam[r];
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        uint8_t* qt = stage_ptr(sj) + kStageKQ + h * 16384 + 8192;
+      // Q rows times s gamma (0 beyond the sequence end), in place: MMA0 has read the raw tile
+      const float f = gs->sgam[q_row];
+      uint8_t* qt = stage_ptr(sj) + kStageKQ + q_half * 16384 + 8192;
 #pragma unroll 2
-        for (int c16 = 0; c16 < 8; ++c16) {
-          uint4* ptr = reinterpret_cast<uint4*>(qt + ptx::sw128_offset(r, c16));
-          uint4 raw = *ptr;
-          const T* e = reinterpret_cast<const T*>(&raw);
-          raw = make_uint4(pack2<T>(Cvt<T>::to_f32(e[0]) * f, Cvt<T>::to_f32(e[1]) * f),
-                           pack2<T>(Cvt<T>::to_f32(e[2]) * f, Cvt<T>::to_f32(e[3]) * f),
-                           pack2<T>(Cvt<T>::to_f32(e[4]) * f, Cvt<T>::to_f32(e[5]) * f),
-                           pack2<T>(Cvt<T>::to_f32(e[6]) * f, Cvt<T>::to_f32(e[7]) * f));
-          *ptr = raw;
-        }
+      for (int c16 = 0; c16 < 8; ++c16) {
+        uint4* ptr = reinterpret_cast<uint4*>(qt + ptx::sw128_offset(q_row, c16));
+        uint4 raw = *ptr;
+        const T* e = reinterpret_cast<const T*>(&raw);
+        raw = make_uint4(pack2<T>(Cvt<T>::to_f32(e[0]) * f, Cvt<T>::to_f32(e[1]) * f),
+                         pack2<T>(Cvt<T>::to_f32(e[2]) * f, Cvt<T>::to_f32(e[3]) * f),
+                         pack2<T>(Cvt<T>::to_f32(e[4]) * f, Cvt<T>::to_f32(e[5]) * f),
+                         pack2<T>(Cvt<T>::to_f32(e[6]) * f, Cvt<T>::to_f32(e[7]) * f));
+        *ptr = raw;
       }
       ptx::fence_proxy_async_smem();
       warp_arrive(&bars[kQsReady], lane);
-      warp_arrive(&bars[kEmpty0 + sj], lane);  // aux no longer touches stage sj
     }
-  } else {
+  } else if (warp < 8) {
     // =========================================================== compute warpgroups
     const int wg = warp >> 2;   // token columns [32 wg, 32 wg + 32) of the chain phases, state columns [64 wg, ..)
     const int v = tid & 127;    // TMEM lane = column v of dS
@@ -502,48 +526,42 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           warp_arrive(&bars[kTileReady], lane);  // only du^T this time
         }
       } else {
-        // the dh^T staging tile is single: the stores of the previous chunk (issued a chunk period ago) must
-        // have read it
-        if (!state_only && i > 0 && !(alive = wait(kTileFree, (i - 1) & 1))) break;
         // (a) critical: 16-bit copy of the new state -> MMA2 of the next chunk may start; the same values are dh
-        uint8_t* ht = smem + kOffDhT + wg * 16384 + v * 128;  // this warpgroup's 64 columns = half wg of the tile
-#pragma unroll 1
+        uint32_t sf[64], sb[2][16];
+        ptx::tmem_ld32(tm + kColS + col_half, reinterpret_cast<uint32_t(&)[32]>(sf[0]));
+        ptx::tmem_ld32(tm + kColS + col_half + 32, reinterpret_cast<uint32_t(&)[32]>(sf[32]));
+        ptx::tmem_wait_ld();
+#pragma unroll
         for (int h = 0; h < 2; ++h) {
-          uint32_t sf[32], sb[16];
-          ptx::tmem_ld32(tm + kColS + col_half + 32 * h, sf);
-          ptx::tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) sb[j >> 1] = pack2<T>(__uint_as_float(sf[j]), __uint_as_float(sf[j + 1]));
-          ptx::tmem_st16(tm + kColSbf + col_half / 2 + 16 * h, sb);
-          if (!state_only) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              *reinterpret_cast<uint4*>(ht + (((4 * h + j) ^ (v & 7)) << 4)) =
-                  make_uint4(sb[4 * j], sb[4 * j + 1], sb[4 * j + 2], sb[4 * j + 3]);
-          }
+          for (int j = 0; j < 32; j += 2)
+            sb[h][j >> 1] = pack2<T>(__uint_as_float(sf[32 * h + j]), __uint_as_float(sf[32 * h + j + 1]));
+          ptx::tmem_st16(tm + kColSbf + col_half / 2 + 16 * h, sb[h]);
         }
         ptx::tmem_wait_st();
         ptx::tc_fence_before_sync();
         warp_arrive(&bars[kSbfReady], lane);
-        if (!state_only) {
-          ptx::fence_proxy_async_smem();
-          warp_arrive(&bars[kTileReady], lane);
-        }
         // (b) off the critical path: decay of the fp32 state for the next chunk (needed by MMAq / MMA3 only)
         if (!(alive = wait(kFull0 + ((i + 1) & 1), ((i + 1) >> 1) & 1))) break;
         const float egl_next = gates_of(i + 1)->egl;
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          uint32_t sf[32];
-          ptx::tmem_ld32(tm + kColS + col_half + 32 * h, sf);
-          ptx::tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) sf[j] = __float_as_uint(__uint_as_float(sf[j]) * egl_next);
-          ptx::tmem_st32(tm + kColS + col_half + 32 * h, sf);
-        }
+        for (int j = 0; j < 64; ++j) sf[j] = __float_as_uint(__uint_as_float(sf[j]) * egl_next);
+        ptx::tmem_st32(tm + kColS + col_half, reinterpret_cast<const uint32_t(&)[32]>(sf[0]));
+        ptx::tmem_st32(tm + kColS + col_half + 32, reinterpret_cast<const uint32_t(&)[32]>(sf[32]));
         ptx::tmem_wait_st();
         ptx::tc_fence_before_sync();
         warp_arrive(&bars[kSScaled], lane);
+        // (c) dh: the staging tile is single, the stores of the previous chunk (issued a chunk period ago) must have read it
+        if (!state_only) {
+          if (i > 0 && !(alive = wait(kTileFree, (i - 1) & 1))) break;
+          uint8_t* ht = smem + kOffDhT + wg * 16384 + v * 128;  // this warpgroup's 64 columns = half wg of the tile
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(ht + ((j ^ (v & 7)) << 4)) =
+                make_uint4(sb[j >> 2][4 * (j & 3)], sb[j >> 2][4 * (j & 3) + 1], sb[j >> 2][4 * (j & 3) + 2], sb[j >> 2][4 * (j & 3) + 3]);
+          ptx::fence_proxy_async_smem();
+          warp_arrive(&bars[kTileReady], lane);
+        }
       }
     }
   }

@@ -175,6 +175,19 @@ __device__ __forceinline__ bool mbar_wait_nocall(uint32_t addr, uint32_t parity,
     if (global_timer_ns() > until) return false;
   return alive;
 }
+// Several barriers at once: one look at all of them, whose latencies overlap (a wait that is over already takes some 70 cycles, and an
+// issuer has ten of them per chunk), then one after the other.
+__device__ __forceinline__ bool mbar_wait_nocall2(uint32_t a, uint32_t pa, uint32_t b, uint32_t pb) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred P, Q;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 Q, [%3], %4;\n"
+      "and.pred P, P, Q;\nselp.b32 %0, 1, 0, P;\n}\n"
+      : "=r"(ok) : "r"(a), "r"(pa), "r"(b), "r"(pb) : "memory");
+  if (ok != 0) return true;
+  return mbar_wait_nocall(a, pa, true) && mbar_wait_nocall(b, pb, true);
+}
 // `num_bars` (one past the kernel's last barrier) stands for "one of the issuer's waits".
 __device__ __forceinline__ void report_issuer(int* status, bool alive, int num_bars) {
   if (!alive) record_wait_failure(status, kStatusBarrierTimeout | (num_bars << 8), 0);

@@ -67,7 +67,7 @@ KERNEL_RULES = {
         tensor_maps="k, q, w: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 128 (w: 64) x 2; A, and w of the form with "
                     "kW = 0: 3-D (64, heads, tokens), box 64 x 1 x 64; 16-bit elements, 128B swizzle"),
     "bwd_scan_kernel": dict(
-        block=416, dynamic_smem=214016, cluster=1, grid="num_seqs * Hv (twice that for a dual state-only launch)",
+        block=512, dynamic_smem=214016, cluster=1, grid="num_seqs * Hv (twice that for a dual state-only launch)",
         params=[_TMAP + " q", _TMAP + " k", _TMAP + " dO", _TMAP + " w", _TMAP + " dh (store)", _TMAP + " du (store)",
                 "BwdParams (by value)", "BwdScanMode (by value)"],
         tensor_maps="loads: 3-D (width, heads, tokens), box 64 x 1 x 64 with 128B swizzle; stores: workspace rows "
