@@ -24,7 +24,7 @@
 // Between two state updates only  MMA2 -> (V' = rho .* Vd) -> MMA3 -> (16-bit copy of the state)  are
 // serial; the other products are issued into the two gaps and complete in their shadow.
 //
-// What bounds it: that chain (1.6 us per chunk with the SM to itself: 1700 cycles of products in order, and hand-offs between
+// What bounds it: that chain (1.4 us per chunk with the SM to itself: 1700 cycles of products in order, and hand-offs between
 // 20 warps that share its issue slots), and with every SM busy the memory behind it (42 - 48 bytes per ns and SM; bulk copies alone 46 - 53).
 // Shared memory moves 72 KB of TMA writes and 112 KB of operand reads per chunk at 128 bytes a cycle.  Operands
 // that a thread produces therefore go to tensor memory (Vd as a shared-memory tile cost 48 KB per chunk), and Q K^T is
@@ -95,9 +95,9 @@ enum Bar {
   kFull0 = 0, kFull1, kEmpty0, kEmpty1,
   kPDone, kPgReady, kD2Done, kVdReady, kVdStored, kSDone, kSbfReady, kSScaled, kAbReady0, kAbReady1,
   kD4Done, kORead, kOFree, kOReady, kONormed, kVnRead, kVnReady, kHRead, kHReady, kHFree, kGate0, kGate1, kGate2, kGate3,
-  // kWIn: {K, operand of Wt} stages (kFull*, kEmpty* are those of {Q, V, A}), Wt in tensor memory, read from there, written to its
-  // tile, Q K^T read from the columns that Wt uses next
-  kKaFull0, kKaFull1, kKaFull2, kKaEmpty0, kKaEmpty1, kKaEmpty2, kWDone, kWRead, kWReady, kD0Read,
+  kD0Read,  // Q K^T has been read from its columns, which the next chunk's (kWIn: Wt of the next chunk) takes
+  // kWIn: {K, operand of Wt} stages (kFull*, kEmpty* are those of {Q, V, A}), Wt in tensor memory, read from there, written to its tile
+  kKaFull0, kKaFull1, kKaFull2, kKaEmpty0, kKaEmpty1, kKaEmpty2, kWDone, kWRead, kWReady,
   // otherwise: {V, A} and K of a stage (kFull*, kEmpty* are those of {Wt, Q})
   kVaFull0, kVaFull1, kVaEmpty0, kVaEmpty1, kKFull0, kKFull1, kKEmpty0, kKEmpty1,
   kNumBars
@@ -365,7 +365,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       __syncwarp();
     };
-    Scalars cur = {}, nxt = {};
+    Scalars cur = {};
     if (nproc > 0) {
       load_early(0, 0);
       fetch(0, cur);
@@ -375,7 +375,6 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     for (int i = 0; i < nproc; ++i) {
       const int s = i & 1;
       trace(0, i, 9);
-      if (i + 1 < nproc) fetch(i + 1, nxt);
       if (i >= 2 && !wait(kEmpty0 + s, ((i >> 1) - 1) & 1)) break;
       if (lane == 0) {
         uint64_t* full = &bars[kFull0 + s];
@@ -434,7 +433,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           slot = 0;
           phase ^= 1;
         }
-        cur = nxt;
+        fetch(i + 1, cur);  // (used behind the next chunk's copies)
       }
       if (i + kPrefetchAhead < nproc) {  // the scalars of a chunk to come
         const int64_t ahead = token_of(i + kPrefetchAhead);
@@ -459,6 +458,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     //   [MMA2(i)] [MMAq(i), MMAw(i+1)] [MMA3(i)] [MMA4(i), MMAu(i+1), MMA0(i+1)]  kWIn
     // Between two state updates only MMA2 -> (chain: V') -> MMA3 -> (both warpgroups: 16-bit state copy)
     // are serial; the other products sit in the two gaps and complete in their shadow.
+    // The warp's own time counts: with an election per product, one wait after the other and D0 released behind the arithmetic of Pg
+    // a chunk took it 2900 cycles.  Products in one block each, waits of one place together, D0 read first: one prompt of 777 tokens
+    // 43.1 -> 41.8 us, 32768 tokens of 16 / 32 heads 215 -> 205, 540 k packed tokens of 8 / 8 heads 957 -> 936.
     {
       const uint32_t id_n64 = ptx::mma_idesc(128, 64, fmt, ptx::kMajorK, ptx::kMajorK);
       const uint32_t id_mn128 = ptx::mma_idesc(128, 128, fmt, ptx::kMajorK, ptx::kMajorMN);
@@ -498,28 +500,27 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           const uint64_t ka_i = static_cast<uint64_t>(slot_i * (kKaBytes >> 4)), ka_j = static_cast<uint64_t>(slot * (kKaBytes >> 4));
           if (i >= 0) {
             trace(0, i, 0);
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSbfReady), ph, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kWReady), ph, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall2(bar_addr(kSbfReady), ph, bar_addr(kWReady), ph))) break;
             trace(0, i, 2);
             ptx::tc_fence_after_sync();
-            ptx::umma_ts_k128_rolled<128, 128>(tmem0 + kColD2, tmem0 + kColSbf, w_desc, id_w, kStateOnly ? !zero_v : true,
+            ptx::umma_ts_k128<128, 128>(tmem0 + kColD2, tmem0 + kColSbf, w_desc, id_w, kStateOnly ? !zero_v : true,
                                                bar_addr(kD2Done));
             trace(0, i, 3);
             if (!kStateOnly)
-              ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf,
+              ptx::umma_ts_k128<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf,
                                                  q_desc + static_cast<uint64_t>(ph * (kQvBytes >> 4)), id_n64, false,
                                                  bar_addr(kEmpty0 + ph));
           }
           if (j < nproc) {
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kKaFull0 + slot), phase, true))) break;
-            if (!kStateOnly && i >= 0 && !(ok = ptx::mbar_wait_nocall(bar_addr(kD0Read), ph, true))) break;
+            if (kStateOnly || i < 0 ? !(ok = ptx::mbar_wait_nocall(bar_addr(kKaFull0 + slot), phase, true))
+                                    : !(ok = ptx::mbar_wait_nocall2(bar_addr(kKaFull0 + slot), phase, bar_addr(kD0Read), ph)))
+              break;
             ptx::tc_fence_after_sync();
             ptx::umma_ss_k64<128, 2>(tmem0 + kColD0, kmn_desc + ka_j, aw_desc + ka_j, id_u, false, bar_addr(kWDone));
           }
           if (i >= 0) {
             trace(0, i, 4);
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdReady), ph, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSScaled), ph, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall2(bar_addr(kVdReady), ph, bar_addr(kSScaled), ph))) break;
             trace(0, i, 6);
             ptx::tc_fence_after_sync();
             ptx::umma_ts_k64_halves<128>(tmem0 + kColS, tmem0 + kColD2, kmn_desc + ka_i, id_mn128, true, bar_addr(kSDone),
@@ -527,9 +528,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             trace(0, i, 7);
             if (kStateOnly) ptx::umma_commit(&bars[kEmpty0 + ph]);
             if (!kStateOnly) {
-              if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdStored), ph, true))) break;
-              if (!(ok = ptx::mbar_wait_nocall(bar_addr(kPgReady), ph, true))) break;
-              if (i > 0 && !(ok = ptx::mbar_wait_nocall(bar_addr(kORead), ph ^ 1, true))) break;
+              if (!(ok = ptx::mbar_wait_nocall3(bar_addr(kVdStored), ph, bar_addr(kPgReady), ph, bar_addr(i > 0 ? kORead : kVdStored),
+                                                i > 0 ? ph ^ 1 : ph)))
+                break;
               ptx::tc_fence_after_sync();
               ptx::umma_ts_k64_halves<2>(tmem0 + kColD4, tmem0 + kColD2 + 16, d_pg + static_cast<uint64_t>(ph * (8192 >> 4)),
                                          id_n64, false, bar_addr(kD4Done));
@@ -543,7 +544,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (!kStateOnly) {
               if (!(ok = ptx::mbar_wait_nocall(bar_addr(kWRead), j & 1, true))) break;
               ptx::tc_fence_after_sync();
-              ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, q_desc + qv, k_desc + ka_j, id_p, false, bar_addr(kPDone));
+              ptx::umma_ss_k128<2, kHalf, 2, kHalf>(tmem0 + kColD0, q_desc + qv, k_desc + ka_j, id_p, false, bar_addr(kPDone));
             }
           }
           if (i >= 0) trace(0, i, 8);
@@ -564,30 +565,29 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSbfReady), ph, true))) break;
           trace(0, i, 2);
           ptx::tc_fence_after_sync();
-          ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColD2, tmem0 + kColSbf, d_w + so, id_n64,
+          ptx::umma_ts_k128<2, kHalf>(tmem0 + kColD2, tmem0 + kColSbf, d_w + so, id_n64,
                                              kStateOnly ? !zero_v : true, bar_addr(kD2Done));
           if (kStateOnly) ptx::umma_commit(&bars[kEmpty0 + ph]);
           trace(0, i, 3);
           // gap 1 (the chain computes V'): MMAq: Dq[i & 1] = S0^T_bf16 Q^T; the output of chunk i - 2, which read that
           // buffer, was waited for in front of MMA4(i - 1)
           if (!kStateOnly)
-            ptx::umma_ts_k128_rolled<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf, d_w + so + (16384 >> 4), id_n64,
+            ptx::umma_ts_k128<2, kHalf>(tmem0 + kColDq + ph * 64, tmem0 + kColSbf, d_w + so + (16384 >> 4), id_n64,
                                                false, bar_addr(kEmpty0 + ph));
-          // MMA0(i + 1): D0 = Q K^T, once Pg of chunk i has been formed from it.  (In gap 2 its 384 cycles stood between two MMA2.)
+          // MMA0(i + 1): D0 = Q K^T, once the Pg warps have read that of chunk i.  (In gap 2 its 384 cycles stood between two MMA2.)
           if (!kStateOnly && i + 1 < nproc) {
             const int sj = (i + 1) & 1;
             const uint64_t sn = static_cast<uint64_t>(sj * (kStageBytes >> 4));
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kPgReady), ph, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kFull0 + sj), ((i + 1) >> 1) & 1, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kKFull0 + sj), ((i + 1) >> 1) & 1, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall3(bar_addr(kD0Read), ph, bar_addr(kFull0 + sj), ((i + 1) >> 1) & 1, bar_addr(kKFull0 + sj),
+                                              ((i + 1) >> 1) & 1)))
+              break;
             ptx::tc_fence_after_sync();
-            ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, d_w + sn + (16384 >> 4), d_k + sn, id_p, false,
+            ptx::umma_ss_k128<2, kHalf, 2, kHalf>(tmem0 + kColD0, d_w + sn + (16384 >> 4), d_k + sn, id_p, false,
                                                          bar_addr(kPDone));
           }
           trace(0, i, 4);
           // MMA3: S^T += V'^T K   (B = K tile read MN-major: 64-column halves are 8 KiB apart)
-          if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdReady), ph, true))) break;
-          if (!(ok = ptx::mbar_wait_nocall(bar_addr(kSScaled), ph, true))) break;
+          if (!(ok = ptx::mbar_wait_nocall2(bar_addr(kVdReady), ph, bar_addr(kSScaled), ph))) break;
           trace(0, i, 6);
           ptx::tc_fence_after_sync();
           ptx::umma_ts_k64_halves<128>(tmem0 + kColS, tmem0 + kColD2, d_kmn + so, id_mn128, true, bar_addr(kSDone),
@@ -595,9 +595,9 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           trace(0, i, 7);
           // gap 2 (both warpgroups convert the state).  MMA4: D4 = Vd^T Pg^T, once the output of chunk i - 1 has read D4
           if (!kStateOnly) {
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVdStored), ph, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kPgReady), ph, true))) break;
-            if (i > 0 && !(ok = ptx::mbar_wait_nocall(bar_addr(kORead), ph ^ 1, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall3(bar_addr(kVdStored), ph, bar_addr(kPgReady), ph, bar_addr(i > 0 ? kORead : kVdStored),
+                                              i > 0 ? ph ^ 1 : ph)))
+              break;
             ptx::tc_fence_after_sync();
             ptx::umma_ts_k64_halves<2>(tmem0 + kColD4, tmem0 + kColD2 + 16, d_pg + static_cast<uint64_t>(ph * (8192 >> 4)),
                                        id_n64, false, bar_addr(kD4Done));
@@ -612,8 +612,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           const int j = i + 1, sj = j & 1;
           const uint64_t sn = static_cast<uint64_t>(sj * (kStageBytes >> 4));
           if (!zero_v) {
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kVaFull0 + sj), (j >> 1) & 1, true))) break;
-            if (!(ok = ptx::mbar_wait_nocall(bar_addr(kAbReady0 + sj), (j >> 1) & 1, true))) break;
+            if (!(ok = ptx::mbar_wait_nocall2(bar_addr(kVaFull0 + sj), (j >> 1) & 1, bar_addr(kAbReady0 + sj), (j >> 1) & 1))) break;
             ptx::tc_fence_after_sync();
             ptx::umma_ss_k64<128, 2>(tmem0 + kColD2, d_v + sn, d_a + sn, id_u, false, bar_addr(kVaEmpty0 + sj));
           }
@@ -623,7 +622,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             ptx::tc_fence_after_sync();
           }
           if (!kStateOnly && i < 0)
-            ptx::umma_ss_k128_rolled<2, kHalf, 2, kHalf>(tmem0 + kColD0, d_w + sn + (16384 >> 4), d_k + sn, id_p, false,
+            ptx::umma_ss_k128<2, kHalf, 2, kHalf>(tmem0 + kColD0, d_w + sn + (16384 >> 4), d_k + sn, id_p, false,
                                                          bar_addr(kPDone));
         }
         if (i >= 0) trace(0, i, 8);
@@ -642,15 +641,10 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     auto form_w = [&](int j) {
       if (!wait(kWDone, j & 1)) return false;
       ptx::tc_fence_after_sync();
-      uint32_t y[2][16];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t x[32];
-        ptx::tmem_ld32(tm + kColD0 + 32 * h, x);
-        ptx::tmem_wait_ld();
-#pragma unroll
-        for (int e = 0; e < 16; ++e) y[h][e] = pack2<T>(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1]));
-      }
+      uint32_t x[2][32];
+      ptx::tmem_ld32(tm + kColD0, x[0]);
+      ptx::tmem_ld32(tm + kColD0 + 32, x[1]);
+      ptx::tmem_wait_ld();
       ptx::tc_fence_before_sync();  // (kStateOnly: kWReady below is what the product that overwrites the columns waits for)
       if (!kStateOnly) warp_arrive(&bars[kWRead], lane);
       // (MMA2 of chunk j - 1, which read the tile, precedes this chunk's product in the pipe)
@@ -659,8 +653,12 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          *reinterpret_cast<uint4*>(smem + kOffWt + (at ^ ((4 * h + e) << 4))) =
-              make_uint4(y[h][4 * e], y[h][4 * e + 1], y[h][4 * e + 2], y[h][4 * e + 3]);
+        {
+          uint32_t y[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) y[c] = pack2<T>(__uint_as_float(x[h][8 * e + 2 * c]), __uint_as_float(x[h][8 * e + 2 * c + 1]));
+          *reinterpret_cast<uint4*>(smem + kOffWt + (at ^ ((4 * h + e) << 4))) = make_uint4(y[0], y[1], y[2], y[3]);
+        }
       ptx::fence_proxy_async_smem();
       warp_arrive(&bars[kWReady], lane);
       return true;
@@ -693,11 +691,16 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (warp == 16) trace(2, i, 9);
         // (tile i & 1 was last read by MMA4 of chunk i - 2: see the wait at the end)
         const uint32_t pg = ptx::smem_u32(smem + kPgTiles) + ph * 8192;
+        // all of D0 first: the product that takes its columns next (kWIn: Wt of the next chunk) does not wait for the arithmetic
+        uint32_t pr[16], pr1[16];
+        ptx::tmem_ld_frag4(tm + kColD0, pr);
+        ptx::tmem_ld_frag4(tm + kColD0 + 32, pr1);
+        ptx::tmem_wait_ld();
+        ptx::tc_fence_before_sync();
+        warp_arrive(&bars[kD0Read], lane);
 #pragma unroll 1
         for (int db = 0; db < p_cols; db += 32) {
-          uint32_t pr[16], m[8];
-          ptx::tmem_ld_frag4(tm + kColD0 + db, pr);
-          ptx::tmem_wait_ld();
+          uint32_t m[8];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float2 gc = *reinterpret_cast<const float2*>(gcol + db + 8 * j);
@@ -713,10 +716,10 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           const int r = (warp & 3) * 16 + (lane & 15), c16 = (db >> 3) + (lane >> 4);
           ptx::stmatrix_x4(pg + ptx::sw128_offset(r, c16), m[0], m[1], m[2], m[3]);
           ptx::stmatrix_x4(pg + ptx::sw128_offset(r, c16 + 2), m[4], m[5], m[6], m[7]);
+#pragma unroll
+          for (int x = 0; x < 16; ++x) pr[x] = pr1[x];
         }
         ptx::fence_proxy_async_smem();
-        ptx::tc_fence_before_sync();
-        if (kWIn) warp_arrive(&bars[kD0Read], lane);
         // Before announcing this tile, make sure MMA4 of the previous chunk has finished: the next iteration overwrites the
         // tile it read.  Waiting HERE (MMA4 of this chunk cannot be issued before the arrival below) keeps this warp at
         // most one phase behind the D4Done barrier; behind the arrival it could fall two behind and wait forever.

@@ -188,6 +188,18 @@ __device__ __forceinline__ bool mbar_wait_nocall2(uint32_t a, uint32_t pa, uint3
   if (ok != 0) return true;
   return mbar_wait_nocall(a, pa, true) && mbar_wait_nocall(b, pb, true);
 }
+__device__ __forceinline__ bool mbar_wait_nocall3(uint32_t a, uint32_t pa, uint32_t b, uint32_t pb, uint32_t c, uint32_t pc) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred P, Q, R;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 Q, [%3], %4;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 R, [%5], %6;\n"
+      "and.pred P, P, Q;\nand.pred P, P, R;\nselp.b32 %0, 1, 0, P;\n}\n"
+      : "=r"(ok) : "r"(a), "r"(pa), "r"(b), "r"(pb), "r"(c), "r"(pc) : "memory");
+  if (ok != 0) return true;
+  return mbar_wait_nocall(a, pa, true) && mbar_wait_nocall(b, pb, true) && mbar_wait_nocall(c, pc, true);
+}
 // `num_bars` (one past the kernel's last barrier) stands for "one of the issuer's waits".
 __device__ __forceinline__ void report_issuer(int* status, bool alive, int num_bars) {
   if (!alive) record_wait_failure(status, kStatusBarrierTimeout | (num_bars << 8), 0);
@@ -440,7 +452,8 @@ __host__ __device__ constexpr uint32_t mma_idesc(uint32_t m, uint32_t n, uint32_
 // lives in per-thread registers and has to be moved to uniform registers one by one: measured ~55-68
 // cycles of issue per instruction, more than the tensor pipe needs for N <= 128.  Issued from a
 // converged warp with the leader picked by elect.sync INSIDE the asm block, the operand arithmetic stays
-// on the uniform datapath and the cost drops to the pipe's own (34 cycles at N = 64, 68 at N = 128).
+// on the uniform datapath and the cost drops to 22 cycles, below the pipe's own (34 at N = 64, 68 at N = 128).  (As a loop with an
+// election per instruction it was 50: the issuer of a scan, with 40 products and a dozen waits per chunk, was what a chunk took.)
 // Descriptor steps are 32-bit adds on the low word (the 14-bit address field never carries).
 // All steps are in units of 16 bytes.  `JUMP` replaces `STEP` between k-steps 3 and 4 (the second
 // 64-element half of a 128-wide operand).  Every block ends with up to two tcgen05.commit on the
@@ -564,40 +577,6 @@ __device__ __forceinline__ void umma_ts_k128(uint32_t d_tmem, uint32_t a_tmem, u
 #undef QLA_UMMA_TS_STEP
 #undef QLA_UMMA_TS_HEAD
 #undef QLA_UMMA_COMMITS
-// The K = 128 products as a loop of two instructions per turn, for kernels whose code has to fit the instruction
-// cache (see mbar_wait_addr); with warp-uniform operands a turn takes less than the tensor pipe needs for it.
-template <int B_STEP, int B_JUMP>
-__device__ __forceinline__ void umma_ts_k128_rolled(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                    bool accumulate, uint32_t commit1 = 0) {
-#pragma unroll 2
-  for (int k = 0; k < 8; ++k) {
-    asm volatile(
-        "{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate || k > 0)) : "memory");
-    a_tmem += 8;
-    b_desc += (k == 3) ? B_JUMP : B_STEP;
-  }
-  if (commit1 != 0)
-    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n"
-                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(commit1) : "memory");
-}
-template <int A_STEP, int A_JUMP, int B_STEP, int B_JUMP>
-__device__ __forceinline__ void umma_ss_k128_rolled(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                    bool accumulate, uint32_t commit1 = 0) {
-#pragma unroll 2
-  for (int k = 0; k < 8; ++k) {
-    asm volatile(
-        "{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate || k > 0)) : "memory");
-    a_desc += (k == 3) ? A_JUMP : A_STEP;
-    b_desc += (k == 3) ? B_JUMP : B_STEP;
-  }
-  if (commit1 != 0)
-    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n"
-                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(commit1) : "memory");
-}
 // tcgen05.commit from a converged warp (same elected lane as the umma_* helpers).
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile(
