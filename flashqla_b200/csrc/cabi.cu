@@ -86,7 +86,7 @@ extern "C" QLA_API int qla_kernel_launch_info(const char* kernel, int32_t* block
   else if (name == "bwd_scan_kernel") launch_info_bwd_scan_kernel(&block, &smem);
   else if (name == "bwd_chunk_kernel") launch_info_bwd_chunk_kernel(&block, &smem);
   else if (name == "kkt_solve_kernel") launch_info_kkt_solve_kernel(&block, &smem);
-  else if (name == "recurrent_kernel") launch_info_recurrent_kernel(&block, &smem);
+  else if (name == "recurrent_kernel" || name == "recurrent_chain_kernel" || name == "recurrent_step_kernel") launch_info_recurrent_kernel(&block, &smem);
   else {
     set_last_error("unknown kernel '%s'", kernel);
     return QLA_ERR_INVALID_ARG;

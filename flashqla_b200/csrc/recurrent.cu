@@ -3,7 +3,8 @@
 // and ragged sequences (cu_seqlens).  One kernel covers what the reference spreads over 29
 // generated kernels (flash_qla/ops/gated_delta_rule/recurrent_fused.py:290-6249); the per-token
 // math follows the canonical body at :346-487 and the reload rule of the warp kernels at
-// :5803-5836 (a parent equal to the previous step is not reloaded).
+// :5803-5836 (a parent equal to the previous step is not reloaded).  Two forms of it, for one step and for chains that are
+// bound by instructions, give the same bits (launch_recurrent_state says which call takes which).
 //
 // The op is HBM-bound: every (sequence, v-head) streams a 64 KiB fp32 state in and out.
 // Mapping: the state of one head is [V=128 rows][K=128 floats]; a row is 512 B.  Eight lanes share
@@ -101,8 +102,9 @@ struct StatePiece<__nv_bfloat16> {
 
 // kTree: a step may restart from the cached state of an earlier one (parents given).  That state is requested one step
 // ahead, before the arithmetic of the step in between, into registers of its own.
-template <typename T, typename InterT, typename StateT, int R, bool kTree>
-__global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p, const uint32_t total_items) {
+// kOne: one token per sequence; nothing of the loop over steps is left.
+template <typename T, typename InterT, typename StateT, int R, bool kTree, bool kOne>
+__device__ __forceinline__ void recurrent_items(const QlaRecurrentArgs& p, const uint32_t total_items) {
   constexpr int D = kHeadDim;
   constexpr int BV = 16 * R;
   constexpr int kTiles = D / BV;
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
     // With one step per state HBM is the bound, the rows come in the shadow of the state, and the extra requests cost
     // 8 us of 168, so decode does without.
     const int step = static_cast<int>(threadIdx.x / 8u), what = static_cast<int>(threadIdx.x & 7u);
-    if (p.tokens_per_seq > 1 && step < p.tokens_per_seq) {
+    if (!kOne && p.tokens_per_seq > 1 && step < p.tokens_per_seq) {
       const int64_t t = static_cast<int64_t>(next.n) * p.tokens_per_seq + step;
       const int64_t qk = (t * p.num_k_heads + next.h / (p.num_v_heads / p.num_k_heads)) * D + (what & 1) * 64;
       const int64_t vg = t * p.num_v_heads + next.h;
@@ -197,7 +199,10 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
   const int hk = h / (p.num_v_heads / p.num_k_heads);
 
   int t0, len;
-  if (p.tokens_per_seq > 0) {
+  if (kOne) {
+    t0 = n;
+    len = 1;
+  } else if (p.tokens_per_seq > 0) {
     t0 = n * p.tokens_per_seq;
     len = p.tokens_per_seq;
   } else {
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
   const bool tree = kTree && cidx >= 0;
   if (tree) par_next = parent_of(1);
 
-  for (int step = 0; step < len; ++step) {
+  for (int step = 0; kOne ? step < 1 : step < len; ++step) {
     const int64_t t = t0 + step;
 
     if (kTree && restart) {
@@ -326,7 +331,7 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
     float vrow[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) vrow[r] = Cvt<T>::to_f32(v_raw[r]);
-    if (step + 1 < len) fetch_inputs(t + 1);
+    if (!kOne && step + 1 < len) fetch_inputs(t + 1);
 
     // q and k stay as loaded: the factors scale / |q| and 1 / |k| are folded into the scalars that use them.  With the
     // state S before the step (decayed: e^g S) the output is q . (e^g S + delta k) = e^g (q . S) + delta (q . k): both
@@ -350,7 +355,7 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
       ks = rsqrtf(group8_sum(sum2(kk2)) + 1e-6f);
     }
 
-    if (step > 0 && (step & 31) == 0) fetch_gates(step);
+    if (!kOne && step > 0 && (step & 31) == 0) fetch_gates(step);
     const float decay = __shfl_sync(0xffffffffu, decay_l, step & 31), beta = __shfl_sync(0xffffffffu, beta_l, step & 31);
 
     float dot[R], out[R];  // k . S, q . S
@@ -389,7 +394,7 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
         ob[(t * p.num_v_heads + h) * D + row0 + 16 * r] = Cvt<T>::from_f32(out[r]);
     }
 
-    if (cidx >= 0 && step < p.inter_steps) {
+    if (cidx >= 0 && (kOne || step < p.inter_steps)) {
       InterT* dst = ib + (((cidx * p.inter_steps + step) * p.num_v_heads + h) * D + row0) * D + col0;
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -397,6 +402,284 @@ __global__ void __launch_bounds__(128) recurrent_kernel(const QlaRecurrentArgs p
         for (int j = 0; j < 4; ++j) store4(dst + (r * 16) * D + j * 32, S[r][j]);
     }
   }
+
+  if (!(p.flags & QLA_REC_DISABLE_STATE_UPDATE) && sidx >= 0) {
+    StateT* sp = static_cast<StateT*>(p.state) + ((sidx * p.num_v_heads + h) * D + row0) * D + col0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) store4(sp + (r * 16) * D + j * 32, S[r][j]);
+  }
+  }  // items
+}
+
+template <typename T, typename InterT, typename StateT, int R, bool kTree>
+__global__ void __launch_bounds__(128) recurrent_kernel(const __grid_constant__ QlaRecurrentArgs p, const uint32_t total_items) {
+  recurrent_items<T, InterT, StateT, R, kTree, false>(p, total_items);
+}
+template <typename T, typename InterT, typename StateT, int R>
+__global__ void __launch_bounds__(128, R == 2 ? 5 : 7) recurrent_step_kernel(const __grid_constant__ QlaRecurrentArgs p, const uint32_t total_items) {
+  recurrent_items<T, InterT, StateT, R, false, true>(p, total_items);
+}
+
+constexpr int kBlockSteps = 4;  // draft tokens prepared at a time, one per warp
+
+// What a block of steps needs beside the state, fp32: q and k as loaded, v of the tile's rows, and per step the scalars (ks = 1 / |k|,
+// qs = scale / |q|).
+template <int R>
+struct alignas(16) StepInputs {
+  float q[kBlockSteps][kHeadDim], k[kBlockSteps][kHeadDim], v[kBlockSteps][16 * R];
+  struct alignas(16) Scalars {
+    float decay, beta, ks, qs, qk, pad[3];
+  } s[kBlockSteps];
+};
+
+// Several steps per sequence, all sequences of one length, no tree.  q, k, v and gates of a block of steps are unpacked, multiplied and
+// activated once per CTA and read from shared memory by its rows; in recurrent_kernel every warp does that for itself, which is most
+// of its instructions.
+template <typename T, typename InterT, typename StateT, int R>
+__global__ void __launch_bounds__(128, R == 2 ? 5 : 8) recurrent_chain_kernel(const QlaRecurrentArgs p, const uint32_t total_items) {
+  constexpr int D = kHeadDim;
+  constexpr int BV = 16 * R;
+  constexpr int kTiles = D / BV;
+  // [kRecStages][R * 4 pieces][128 threads] float4: every thread stages exactly the 16-byte pieces it owns, so
+  // no barrier is needed between the copy and its use
+  using Piece = StatePiece<StateT>;
+  extern __shared__ __align__(16) uint8_t s_stage_raw[];
+  typename Piece::Raw* s_stage = reinterpret_cast<typename Piece::Raw*>(s_stage_raw);
+  __shared__ StepInputs<R> s_inputs[2];
+  grid_dep_wait();    // earlier kernels of the stream have completed (see launch_dependent)
+  grid_dep_launch();  // the next one may be scheduled; it waits the same way
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int sub = lane & 7, grp = lane >> 3;
+  const int col0 = sub * 4;  // first owned column of j = 0; j-th is col0 + 32 j
+  const int len = p.tokens_per_seq;
+
+  // A slot outside the pool is never touched: the sequence runs from a zero state without write-back, and
+  // the status word says that an index was bad.
+  auto bad_index = [&]() {
+    if (p.status != nullptr && threadIdx.x == 0) atomicCAS(p.status, 0, kStatusBadIndex);
+  };
+  // Work item -> (sequence, v-head, row tile) and the sequence's pool slot, looked up once, when the item's tile is
+  // requested (32-bit arithmetic: 64-bit divisions are long sequences of instructions).
+  struct Item {
+    int n, h, tile, t0;
+    int64_t slot;
+  };
+  auto locate = [&](uint32_t item) {
+    Item x;
+    x.tile = static_cast<int>(item % kTiles);
+    const uint32_t nh = item / kTiles;
+    x.n = static_cast<int>(nh / static_cast<uint32_t>(p.num_v_heads));
+    x.h = static_cast<int>(nh) - x.n * p.num_v_heads;
+    x.slot = p.state_indices ? p.state_indices[x.n] : x.n;
+    if (x.slot >= p.state_slots) {
+      bad_index();
+      x.slot = -1;
+    }
+    x.t0 = x.n * len;
+    return x;
+  };
+  // The state tile of an item is requested one item ahead (cp.async, L2 only): the copy of the next tile is
+  // in flight while this one is computed and written back, which keeps reads queued at the memory the whole
+  // time instead of only at the start of every CTA.
+  auto prefetch = [&](const Item& x, int stage) {
+    if (x.slot < 0) return;
+    const int row0 = x.tile * BV + warp * 4 + grp;
+    const StateT* sp = static_cast<const StateT*>(p.state) + ((x.slot * p.num_v_heads + x.h) * D + row0) * D + col0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        Piece::copy_async(&s_stage[(stage * R * 4 + r * 4 + j) * 128 + threadIdx.x], sp + (r * 16) * D + j * 32);
+  };
+
+  const T* qb = static_cast<const T*>(p.q);
+  const T* kb = static_cast<const T*>(p.k);
+  const T* vb = static_cast<const T*>(p.v);
+  T* ob = static_cast<T*>(p.o);
+  InterT* ib = static_cast<InterT*>(p.inter);
+  const bool l2norm = (p.flags & QLA_REC_QK_L2NORM) != 0;
+
+  // Rows and gates of a block of steps: warp w requests step first + w while the block in front is computed, and writes what the
+  // CTA needs of it to shared memory behind that block, once for all rows of the tile.
+  uint2 q_raw, k_raw;
+  T v_raw;
+  float a_raw, b_raw, a_log, dt_bias;
+  auto request = [&](const Item& x, int first) {
+    const int step = first + warp;
+    if (step >= len) return;
+    const int64_t t = x.t0 + step, th = t * p.num_v_heads + x.h;
+    const int64_t qk = (t * p.num_k_heads + x.h / (p.num_v_heads / p.num_k_heads)) * D + lane * 4;
+    q_raw = *reinterpret_cast<const uint2*>(qb + qk);
+    k_raw = *reinterpret_cast<const uint2*>(kb + qk);
+    if (BV == 32 || lane < BV) v_raw = vb[th * D + x.tile * BV + lane];
+    a_raw = load_scalar(p.a, p.a_dtype, th);
+    b_raw = load_scalar(p.b, p.a_dtype, th);
+    if (!(p.flags & QLA_REC_A_IS_LOG_DECAY)) {
+      a_log = load_scalar(p.A_log, p.a_log_dtype, x.h);
+      dt_bias = load_scalar(p.dt_bias, p.dt_bias_dtype, x.h);
+    }
+  };
+  auto prepare = [&](const Item& x, int first, StepInputs<R>& in) {
+    if (first + warp >= len) return;
+    F2 q[2], k[2];
+    unpack4<T>(q_raw, q);
+    unpack4<T>(k_raw, k);
+    store4(&in.q[warp][lane * 4], q);
+    store4(&in.k[warp][lane * 4], k);
+    if (BV == 32 || lane < BV) in.v[warp][lane] = Cvt<T>::to_f32(v_raw);
+    // (sums in the order of recurrent_kernel: a state cached in 16 bits is the rounded value of one cached in fp32)
+    __syncwarp();
+    F2 qk2 = 0, qq2 = 0, kk2 = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const ulonglong2 kp = *reinterpret_cast<const ulonglong2*>(&in.k[warp][col0 + 32 * j]);
+      const ulonglong2 qp = *reinterpret_cast<const ulonglong2*>(&in.q[warp][col0 + 32 * j]);
+      qk2 = j == 0 ? mul2(qp.x, kp.x) : fma2(qp.x, kp.x, qk2);
+      qk2 = fma2(qp.y, kp.y, qk2);
+      if (l2norm) {
+        qq2 = fma2(qp.y, qp.y, fma2(qp.x, qp.x, qq2));
+        kk2 = fma2(kp.y, kp.y, fma2(kp.x, kp.x, kk2));
+      }
+    }
+    const float qk = group8_sum(sum2(qk2));
+    float qs = p.scale, ks = 1.f;
+    if (l2norm) {
+      qs *= rsqrtf(group8_sum(sum2(qq2)) + 1e-6f);
+      ks = rsqrtf(group8_sum(sum2(kk2)) + 1e-6f);
+    }
+    float g = a_raw;
+    if (!(p.flags & QLA_REC_A_IS_LOG_DECAY)) {
+      const float y = g + dt_bias, by = p.softplus_beta * y;
+      g = -expf(a_log) * (by <= p.softplus_threshold ? log1pf(expf(by)) / p.softplus_beta : y);
+    }
+    const float decay = expf(g), beta = (p.flags & QLA_REC_B_IS_BETA) ? b_raw : 1.f / (1.f + expf(-b_raw));
+    if (lane == 0) {
+      *reinterpret_cast<float4*>(&in.s[warp].decay) = make_float4(decay, beta, ks, qs);
+      in.s[warp].qk = qk;
+    }
+  };
+
+  Item next = locate(blockIdx.x);  // (the grid is at most total_items)
+  prefetch(next, 0);
+  mm::cp_async_commit();
+  request(next, 0);
+  prepare(next, 0, s_inputs[0]);
+  __syncthreads();
+  int it = 0, buf = 0;
+  for (uint32_t item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
+  const Item cur = next;
+  const bool more = item + gridDim.x < total_items;
+  if (more) {
+    next = locate(item + gridDim.x);
+    prefetch(next, (it + 1) % kRecStages);
+  }
+  mm::cp_async_commit();
+  mm::cp_async_wait<kRecStages - 1>();  // all but the newest group: this item's tile has landed
+
+  const int tile = cur.tile, h = cur.h, n = cur.n;
+  const int64_t sidx = cur.slot;
+  int64_t cidx = -1;
+  if (p.inter != nullptr) {
+    cidx = p.inter_indices ? p.inter_indices[n] : n;
+    if (cidx >= p.inter_slots) {
+      bad_index();
+      cidx = -1;
+    }
+  }
+
+  const int row0 = tile * BV + warp * 4 + grp;  // row of r = 0; r-th row is row0 + 16 r
+
+  F2 S[R][4][2];
+  if (sidx >= 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        Piece::unpack(s_stage[((it % kRecStages) * R * 4 + r * 4 + j) * 128 + threadIdx.x], S[r][j]);
+      }
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        S[r][j][0] = S[r][j][1] = 0;
+  }
+
+  T* orow = ob + (static_cast<int64_t>(cur.t0) * p.num_v_heads + h) * D + row0;
+  InterT* irow = ib + ((cidx * p.inter_steps * p.num_v_heads + h) * D + row0) * D + col0;  // (cidx < 0: not used)
+
+  for (int first = 0; first < len; first += kBlockSteps, buf ^= 1) {
+  // the block behind this one: of this item or the next one's first
+  const bool ends = first + kBlockSteps >= len;
+  if (!ends) request(cur, first + kBlockSteps);
+  else if (more) request(next, 0);
+  const StepInputs<R>& in = s_inputs[buf];
+#pragma unroll 1
+  for (int i = 0, count = min(kBlockSteps, len - first); i < count; ++i) {
+    const int step = first + i;
+    // With the state S before the step (decayed: e^g S) the output is q . (e^g S + delta k) = e^g (q . S) + delta (q . k): both
+    // products with S are formed in one pass and reduced together, before the update.
+    F2 kv[4][2];
+    F2 ak[R][2], aq[R][2];  // k . S, q . S
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(&in.k[i][col0 + 32 * j]);
+      const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(&in.q[i][col0 + 32 * j]);
+      kv[j][0] = k2.x;
+      kv[j][1] = k2.y;
+      const F2 qv[2] = {q2.x, q2.y};
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          ak[r][e] = j == 0 ? mul2(S[r][j][e], kv[j][e]) : fma2(S[r][j][e], kv[j][e], ak[r][e]);
+          aq[r][e] = j == 0 ? mul2(S[r][j][e], qv[e]) : fma2(S[r][j][e], qv[e], aq[r][e]);
+        }
+    }
+    const float4 sc = *reinterpret_cast<const float4*>(&in.s[i].decay);
+    const float decay = sc.x, beta = sc.y, ks = sc.z, qs = sc.w, qk = in.s[i].qk;
+    float dot[R], out[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      dot[r] = sum2(ak[r][0]) + sum2(ak[r][1]);
+      out[r] = sum2(aq[r][0]) + sum2(aq[r][1]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      dot[r] = group8_sum(dot[r]);
+      out[r] = group8_sum(out[r]);
+    }
+    const F2 decay2 = f2(decay, decay);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float delta = fmaf(-(decay * dot[r]), ks, in.v[i][warp * 4 + grp + 16 * r]) * beta * ks;  // times k / |k|: one factor here
+      const F2 delta2 = f2(delta, delta);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) S[r][j][e] = fma2(kv[j][e], delta2, mul2(S[r][j][e], decay2));
+      out[r] = fmaf(delta, qk, decay * out[r]) * qs;
+    }
+    if (sub == 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) orow[16 * r] = Cvt<T>::from_f32(out[r]);
+    }
+    orow += p.num_v_heads * D;
+
+    if (cidx >= 0 && step < p.inter_steps) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store4(irow + (r * 16) * D + j * 32, S[r][j]);
+      irow += static_cast<int64_t>(p.num_v_heads) * D * D;
+    }
+  }
+  if (!ends) prepare(cur, first + kBlockSteps, s_inputs[buf ^ 1]);
+  else if (more) prepare(next, 0, s_inputs[buf ^ 1]);
+  __syncthreads();  // (the other buffer is complete; this one has been read)
+  }  // blocks of steps
 
   if (!(p.flags & QLA_REC_DISABLE_STATE_UPDATE) && sidx >= 0) {
     StateT* sp = static_cast<StateT*>(p.state) + ((sidx * p.num_v_heads + h) * D + row0) * D + col0;
@@ -426,32 +709,39 @@ int resident_ctas(size_t smem, int* out) {
   return QLA_OK;
 }
 
-template <typename T, typename InterT, typename StateT, int R, bool kTree>
+enum Form { kPlain, kTree, kChain, kStep };  // recurrent_kernel without and with parents, recurrent_chain_kernel, recurrent_step_kernel
+template <typename T, typename InterT, typename StateT, int R, Form kForm>
+constexpr auto kernel_of() {
+  if constexpr (kForm == kChain) return &recurrent_chain_kernel<T, InterT, StateT, R>;
+  else if constexpr (kForm == kStep) return &recurrent_step_kernel<T, InterT, StateT, R>;
+  else return &recurrent_kernel<T, InterT, StateT, R, kForm == kTree>;
+}
+template <typename T, typename InterT, typename StateT, int R, Form kForm>
 int resident_tiles(int* out) {
   constexpr size_t smem = kRecStages * R * 4 * 128 * sizeof(typename StatePiece<StateT>::Raw);
-  const int rc = ensure_dynamic_smem<recurrent_kernel<T, InterT, StateT, R, kTree>>(smem);
-  return rc != QLA_OK ? rc : resident_ctas<recurrent_kernel<T, InterT, StateT, R, kTree>>(smem, out);
+  const int rc = ensure_dynamic_smem<kernel_of<T, InterT, StateT, R, kForm>()>(smem);
+  return rc != QLA_OK ? rc : resident_ctas<kernel_of<T, InterT, StateT, R, kForm>()>(smem, out);
 }
 
-template <typename T, typename InterT, typename StateT, int R, bool kTree>
+template <typename T, typename InterT, typename StateT, int R, Form kForm>
 int launch_recurrent_rows(const QlaRecurrentArgs& a, cudaStream_t stream) {
   const int64_t items = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / (16 * R));
   QLA_CHECK_SUPPORTED(items < (int64_t(1) << 31), "too many (sequence, head) pairs");
   constexpr size_t smem = kRecStages * R * 4 * 128 * sizeof(typename StatePiece<StateT>::Raw);
   int resident = 0;
-  const int rc = resident_tiles<T, InterT, StateT, R, kTree>(&resident);
+  const int rc = resident_tiles<T, InterT, StateT, R, kForm>(&resident);
   if (rc != QLA_OK) return rc;
   // one CTA per item while they all fit at once; otherwise as many CTAs as are resident, each walking the
   // items with stride gridDim.x
   const unsigned grid = static_cast<unsigned>(items < resident ? items : resident);
-  QLA_CHECK_CUDA(launch_dependent(recurrent_kernel<T, InterT, StateT, R, kTree>, dim3(grid), dim3(128), smem, stream, a,
+  QLA_CHECK_CUDA(launch_dependent(kernel_of<T, InterT, StateT, R, kForm>(), dim3(grid), dim3(128), smem, stream, a,
                                   static_cast<uint32_t>(items)));
   QLA_CHECK_CUDA(cudaGetLastError());
   return QLA_OK;
 }
 
-template <typename T, typename InterT, typename StateT, bool kTree>
-int launch_recurrent_tree(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
+template <typename T, typename InterT, typename StateT, Form kForm>
+int launch_recurrent_form(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
   // Tiles of 16 rows while they are all resident at once, which spreads a small batch over the most SMs; a second round of
   // them costs the latency of every step again.  With the line at four tiles of 32 rows per SM: 96 heads of 7 tree steps 17.5 us, now
   // 13.2; 112 heads of 4 steps 11.4 -> 9.7; 144 heads of one step 7.0 -> 5.3, with a bf16 pool 6.8 -> 4.8.  (Just above the line it is
@@ -460,29 +750,40 @@ int launch_recurrent_tree(const QlaRecurrentArgs& a, int rows, cudaStream_t stre
     const int64_t tiles = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / 16);
     int resident = 2 * 148;  // (at least: the smallest calls, which are host-bound, do not look it up)
     if (tiles > resident) {
-      const int rc = resident_tiles<T, InterT, StateT, 1, kTree>(&resident);
+      const int rc = resident_tiles<T, InterT, StateT, 1, kForm>(&resident);
       if (rc != QLA_OK) return rc;
     }
     rows = tiles <= resident ? 16 : 32;
     // A tree's tiles of 32 rows with fp32 scratch are resident three per SM, not four: a second round of them that is more than a
     // quarter full takes longer than two rounds of 16 rows.  128 / 136 / 144 / 147 heads of 8 steps, us: 16 rows 22.5 / 23.3 / 23.3 /
     // 23.9, 32 rows 21.3 / 23.5 / 24.9 / 26.0; of 3 steps 11.4 / 11.4 / 11.4 / 11.5 and 11.3 / 11.6 / 12.3 / 12.5.
-    if constexpr (kTree && std::is_same<InterT, float>::value) {
+    if constexpr (kForm == kTree && std::is_same<InterT, float>::value) {
       int resident32 = 0;
       if (rows == 32 && tiles <= 2 * static_cast<int64_t>(resident)) {
-        const int rc = resident_tiles<T, InterT, StateT, 2, kTree>(&resident32);
+        const int rc = resident_tiles<T, InterT, StateT, 2, kForm>(&resident32);
         if (rc != QLA_OK) return rc;
         if (4 * (tiles / 2) > 5 * static_cast<int64_t>(resident32)) rows = 16;
       }
     }
   }
-  return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, kTree>(a, stream)
-                    : launch_recurrent_rows<T, InterT, StateT, 2, kTree>(a, stream);
+  return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, kForm>(a, stream)
+                    : launch_recurrent_rows<T, InterT, StateT, 2, kForm>(a, stream);
 }
 template <typename T, typename InterT, typename StateT>
 int launch_recurrent_state(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
-  return a.parents != nullptr ? launch_recurrent_tree<T, InterT, StateT, true>(a, rows, stream)
-                              : launch_recurrent_tree<T, InterT, StateT, false>(a, rows, stream);
+  // One step: the kernel without the loop, of which five tiles of 32 rows are resident per SM, not four (us, recurrent_kernel /
+  // recurrent_step_kernel, states from HBM, 32 heads: bf16 pools 16 sequences 11.9 / 10.1, 64 37.6 / 30.4, 128 71.0 / 57.0; fp32 pools
+  // 4 6.1 / 5.8, 12 12.2 / 10.7, 24 20.0 / 18.0, 32 24.5 / 23.5, 48 34.8 / 35.0, 64 44.7 / 47.3, 256 163.6 / 187: from about 1200 fp32 heads on HBM is the
+  // bound, and the memory does better with fewer tiles in flight).
+  if (a.tokens_per_seq == 1 && (std::is_same<StateT, __nv_bfloat16>::value || static_cast<int64_t>(a.num_seqs) * a.num_v_heads <= 1024))
+    return launch_recurrent_form<T, InterT, StateT, kStep>(a, rows, stream);
+  if (a.parents != nullptr) return launch_recurrent_form<T, InterT, StateT, kTree>(a, rows, stream);
+  // Several steps, of which every state is cached in 16 bits or none is: instructions are the bound, and the kernel with fewer of them is
+  // the faster one (us, recurrent_kernel / recurrent_chain_kernel, 32 heads: 256 sequences of 4 steps 327 / 270, of 2 207 / 182, 100 of
+  // 8 254 / 226, 16 heads: 33 of 5 26.2 / 24.2).  With fp32 states in the cache HBM is (256 of 4 480 / 481, 16 of 8 50.1 / 51.7), and with one step.
+  if (a.tokens_per_seq > 1 && (a.inter == nullptr || a.inter_dtype == QLA_DT_BF16))
+    return launch_recurrent_form<T, InterT, StateT, kChain>(a, rows, stream);
+  return launch_recurrent_form<T, InterT, StateT, kPlain>(a, rows, stream);
 }
 template <typename T, typename InterT>
 int launch_recurrent(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
