@@ -48,66 +48,65 @@ __device__ __forceinline__ int warm_chunks(const QlaCpPlanArgs& a, int start, in
 
 constexpr int kPlanThreads = 512;
 
-// A state of the caller's (fp32 or bf16, [K][V] or [V][K]) as fp32 [K][V]; no row: zero.  All kPlanThreads threads.
+// A state of the caller's (fp32 or bf16, [K][V] or [V][K]) as fp32 [K][V]; no row: zero.  All kPlanThreads threads of kCopyParts CTAs
+// (blockIdx.z - 1), a quarter each, beside the one that plans.
+constexpr int kCopyParts = 4;
 __device__ __forceinline__ void copy_state(const QlaCpPlanArgs& a, float* dst, int row, int h) {
-  constexpr int kElems = kHeadDim * kHeadDim;
+  constexpr int kElems = kHeadDim * kHeadDim / kCopyParts;  // 32 rows of either
+  const int first = static_cast<int>(blockIdx.z - 1) * kElems;
   if (row < 0) {
     for (int i = threadIdx.x * 4; i < kElems; i += kPlanThreads * 4)
-      *reinterpret_cast<float4*>(dst + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(dst + first + i) = make_float4(0.f, 0.f, 0.f, 0.f);
     return;
   }
-  const int64_t off = (static_cast<int64_t>(row) * a.num_v_heads + h) * kElems;
+  const int64_t off = (static_cast<int64_t>(row) * a.num_v_heads + h) * kHeadDim * kHeadDim + first;
   const float* s32 = static_cast<const float*>(a.h0) + off;
   const __nv_bfloat16* s16 = static_cast<const __nv_bfloat16*>(a.h0) + off;
   const bool b16 = a.h0_dtype == QLA_DT_BF16;
   if (!a.h0_transposed) {
-#pragma unroll 4
-    for (int i = threadIdx.x; i < kElems; i += kPlanThreads) dst[i] = b16 ? __bfloat162float(s16[i]) : s32[i];
+#pragma unroll
+    for (int i = threadIdx.x; i < kElems; i += kPlanThreads) dst[first + i] = b16 ? __bfloat162float(s16[i]) : s32[i];
     return;
   }
-  // transposed through shared memory, 64 source rows at a time: both sides coalesced
-  __shared__ float tile[64][kHeadDim + 1];
-  for (int v0 = 0; v0 < kHeadDim; v0 += 64) {
-    __syncthreads();
-#pragma unroll 4
-    for (int i = threadIdx.x; i < 64 * kHeadDim; i += kPlanThreads)
-      tile[i >> 7][i & 127] = b16 ? __bfloat162float(s16[v0 * kHeadDim + i]) : s32[v0 * kHeadDim + i];
-    __syncthreads();
-#pragma unroll 4
-    for (int i = threadIdx.x; i < 64 * kHeadDim; i += kPlanThreads)
-      dst[(i >> 6) * kHeadDim + v0 + (i & 63)] = tile[i & 63][i >> 6];
-  }
+  // transposed through shared memory, 32 source rows: both sides coalesced
+  __shared__ float tile[32][kHeadDim + 1];
+#pragma unroll
+  for (int i = threadIdx.x; i < kElems; i += kPlanThreads) tile[i >> 7][i & 127] = b16 ? __bfloat162float(s16[i]) : s32[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = threadIdx.x; i < kElems; i += kPlanThreads) dst[(i >> 5) * kHeadDim + (first >> 7) + (i & 31)] = tile[i & 31][i >> 5];
 }
 
-// One CTA per (segment, head): warp 0 finds the warm-up length; all threads write the segment's start state.
+// 1 + kCopyParts CTAs per (segment, head): a warp of the first finds the warm-up length; the others write the segment's start state.
 __global__ void __launch_bounds__(kPlanThreads) cp_plan_kernel(const QlaCpPlanArgs a) {
   grid_dep_wait();    // earlier kernels of the stream have completed (see launch_dependent)
   grid_dep_launch();
   const int seg = blockIdx.x, h = blockIdx.y;
   const int num_heads = a.num_v_heads;
-  if (threadIdx.x < 32) {
-    const int start = a.cu_seqlens[seg], end = a.cu_seqlens[seg + 1];
-    int warm = 0, ml = 0;
-    if (a.seg_next[seg] >= 0 && end > start) {
-      bool reached;
-      warm = warm_chunks(a, start, end, h, &reached);
-      if (!reached) ml = warm;
-    }
-    if (threadIdx.x == 0) {
-      a.warm_limit[seg * num_heads + h] = warm;
-      a.m_limit[seg * num_heads + h] = ml;
-    }
+  if (blockIdx.z != 0) {
+    const int raw = a.seg_start_of[seg];
+    int row = -1;
+    if (raw >= 0 && a.h0 != nullptr) row = a.h0_map != nullptr ? a.h0_map[raw] : raw;
+    copy_state(a, a.cp_h0 + (static_cast<int64_t>(seg) * num_heads + h) * kHeadDim * kHeadDim, row, h);
+    return;
   }
-  if (a.cp_h0 == nullptr) return;
-  const int raw = a.seg_start_of[seg];
-  int row = -1;
-  if (raw >= 0 && a.h0 != nullptr) row = a.h0_map != nullptr ? a.h0_map[raw] : raw;
-  copy_state(a, a.cp_h0 + (static_cast<int64_t>(seg) * num_heads + h) * kHeadDim * kHeadDim, row, h);
+  if (threadIdx.x >= 32) return;
+  const int start = a.cu_seqlens[seg], end = a.cu_seqlens[seg + 1];
+  int warm = 0, ml = 0;
+  if (a.seg_next[seg] >= 0 && end > start) {
+    bool reached;
+    warm = warm_chunks(a, start, end, h, &reached);
+    if (!reached) ml = warm;
+  }
+  if (threadIdx.x == 0) {
+    a.warm_limit[seg * num_heads + h] = warm;
+    a.m_limit[seg * num_heads + h] = ml;
+  }
 }
 
-// The plan with the warm-up folded into the main scan (forward, or reverse for the backward scan): one CTA per
-// (original sequence, head), a warp per segment.  A (sequence, head) in which every segment decays below the threshold needs no state-only pass:
-// the main scan's CTA of segment s simply starts lead[s] = warm(s - 1) chunks early, from a zero state.  If some
+// The plan with the warm-up folded into the main scan (forward, or reverse for the backward scan): 1 + kCopyParts CTAs per
+// (original sequence, head), a warp of the first per segment.  A (sequence, head) in which every segment decays below the threshold needs
+// no state-only pass: the main scan's CTA of segment s simply starts lead[s] = warm(s - 1) chunks early, from a zero state.  If some
 // segment never decays that far the limits are those of cp_plan_kernel (state-only pass, transition matrices,
 // chain) and lead is 0.  Only the row of cp_h0 that starts the sequence is written here.
 __global__ void __launch_bounds__(kPlanThreads) cp_plan_lead_kernel(const QlaCpPlanArgs a) {
@@ -116,6 +115,14 @@ __global__ void __launch_bounds__(kPlanThreads) cp_plan_lead_kernel(const QlaCpP
   const int r = blockIdx.x, h = blockIdx.y;
   const int num_heads = a.num_v_heads;
   const int s0 = a.raw_first_seg[r], s1 = a.raw_first_seg[r + 1];
+  if (blockIdx.z != 0) {
+    // start state of the sequence (backward: the gradient of its final state, into the last segment's row): the
+    // caller's (any dtype / layout, through h0_map) or zero
+    int row = -1;
+    if (a.h0 != nullptr) row = a.h0_map != nullptr ? a.h0_map[r] : r;
+    copy_state(a, a.cp_h0 + (static_cast<int64_t>(a.reverse ? s1 - 1 : s0) * num_heads + h) * kHeadDim * kHeadDim, row, h);
+    return;
+  }
   int any = 0;
   for (int seg = s0 + static_cast<int>(threadIdx.x >> 5); seg < s1; seg += kPlanThreads / 32) {
     const int start = a.cu_seqlens[seg], end = a.cu_seqlens[seg + 1];
@@ -140,11 +147,6 @@ __global__ void __launch_bounds__(kPlanThreads) cp_plan_lead_kernel(const QlaCpP
   __syncthreads();
   if (!any)
     for (int seg = s0 + threadIdx.x; seg < s1; seg += kPlanThreads) a.warm_limit[seg * num_heads + h] = 0;
-  // start state of the sequence (backward: the gradient of its final state, into the last segment's row): the
-  // caller's (any dtype / layout, through h0_map) or zero
-  int row = -1;
-  if (a.h0 != nullptr) row = a.h0_map != nullptr ? a.h0_map[r] : r;
-  copy_state(a, a.cp_h0 + (static_cast<int64_t>(a.reverse ? s1 - 1 : s0) * num_heads + h) * kHeadDim * kHeadDim, row, h);
 }
 
 // The chain  h[next] += M[seg] h[seg]  over the segments of one sequence and head, in order.  A link is a dependent
@@ -290,11 +292,11 @@ extern "C" QLA_API int qla_cp_plan(const QlaCpPlanArgs* a, void* stream) {
   if (a->lead != nullptr) {
     QLA_CHECK_ARG(a->cp_h0 != nullptr && a->raw_first_seg != nullptr && a->num_raw_seqs > 0,
                   "lead needs cp_h0, raw_first_seg and num_raw_seqs");
-    dim3 grid_lead(a->num_raw_seqs, a->num_v_heads);
+    dim3 grid_lead(a->num_raw_seqs, a->num_v_heads, 1 + kCopyParts);
     QLA_CHECK_CUDA(launch_dependent(cp_plan_lead_kernel, grid_lead, dim3(kPlanThreads), 0, static_cast<cudaStream_t>(stream), *a));
     return QLA_OK;
   }
-  dim3 grid(a->num_segments, a->num_v_heads);
+  dim3 grid(a->num_segments, a->num_v_heads, a->cp_h0 != nullptr ? 1 + kCopyParts : 1);
   QLA_CHECK_CUDA(launch_dependent(cp_plan_kernel, grid, dim3(kPlanThreads), 0, static_cast<cudaStream_t>(stream), *a));
   return QLA_OK;
 }
