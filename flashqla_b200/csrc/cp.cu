@@ -152,14 +152,17 @@ __global__ void __launch_bounds__(kPlanThreads) cp_plan_lead_kernel(const QlaCpP
 // The chain  h[next] += M[seg] h[seg]  over the segments of one sequence and head, in order.  A link is a dependent
 // 128 x 128 by 128 x 8 product in fp32: the columns are split over CTAs (8 each), warp w of a CTA has rows 16 w .. 16 w + 15, and a
 // lane every fourth row and 16 of the inner index of each: 4 x 8 sums, two columns per instruction, which the eight lanes
-// of a row then add up in a tree.  A thread's part of M comes straight from global memory (L2), that of the next link
-// while this one is multiplied; the carried columns pass through shared memory in two buffers: one barrier per link.  What
-// bounds it: 64 KB of M per link and CTA, L2 to SM (40 bytes per ns and SM).  36 links of 4 heads take 58 us (59 with split TF32
-// factors on mma.sync, whose error against 64 bits was 2 to 7 times that of fp32; 97 with M through shared memory).
+// of a row then add up in a tree.  M comes by bulk copies into three stages, two links ahead; the carried columns pass through shared
+// memory in two buffers: one barrier per link.  What bounds it: reads of shared memory, 48 of 16 bytes per thread and link.  36 links of
+// 1 / 4 / 8 heads take 53 / 54 / 54 us (59 / 60 / 61 with every thread's part of M straight from L2; 59 with split TF32 factors on
+// mma.sync, whose error against 64 bits was 2 to 7 times that of fp32; 53 / 84 / 165 with the rows split over clusters of four CTAs).
 constexpr int kChainCols = 8;
 constexpr int kChainGroup = 4 * kChainCols + 4;  // floats from four rows of the carried columns to the next four: conflict-free float4
 constexpr int kChainThreads = 256;
 constexpr int kChainFlags = 256;
+constexpr int kChainStages = 3;
+constexpr uint32_t kChainTile = kHeadDim * kHeadDim * 4;
+constexpr size_t kChainSmem = kChainStages * kChainTile;
 
 __device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {  // two fp32 values per instruction
   unsigned long long& r = reinterpret_cast<unsigned long long&>(acc);
@@ -176,6 +179,13 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
   const int s0 = raw_first_seg[r], links = raw_first_seg[r + 1] - s0 - 1;
   __shared__ __align__(16) float s_h[2][kHeadDim / 4 * kChainGroup];  // [buffer][row / 4][row % 4][column]
   __shared__ int flags[kChainFlags];
+  extern __shared__ __align__(128) uint8_t s_m[];  // M of links i, i + 1, i + 2 by turns
+  __shared__ uint64_t full[kChainStages];
+  if (tid == 0) {
+    for (int x = 0; x < kChainStages; ++x) ptx::mbar_init(&full[x], 1);
+    ptx::fence_mbar_init();
+  }
+  uint32_t uses = 0;  // of a stage: bit x, the parity of its next phase
   // link i leads from segment seg_of(i) to seg_of(i + 1)
   auto seg_of = [&](int i) { return reverse ? s0 + links - i : s0 + i; };
   // rows 16 warp + rg + 4 i (i = 0..3), inner indices 32 t + 4 sl .. + 3 (t = 0..3)
@@ -188,19 +198,20 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
   auto carry = [&](int buf, float4 x) {
     *reinterpret_cast<float4*>(&s_h[buf][(row >> 2) * kChainGroup + (row & 3) * kChainCols + col]) = x;
   };
-  using Part = float4[4][4];  // [i][t]
-  auto load_m = [&](int i, Part& part) {
-    const float* m = M + ((static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim + 16 * warp + rg) * kHeadDim + 4 * sl;
-#pragma unroll
-    for (int t = 0; t < 4; ++t)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) part[x][t] = *reinterpret_cast<const float4*>(m + 4 * x * kHeadDim + 32 * t);
+  auto request = [&](int i) {  // thread 0: M of link i (number i % kChainFlags of its batch)
+    const int stage = i % kChainFlags % kChainStages;
+    ptx::mbar_expect_tx(&full[stage], kChainTile);
+    ptx::bulk_load(s_m + stage * kChainTile, M + (static_cast<int64_t>(seg_of(i)) * num_heads + h) * kHeadDim * kHeadDim, kChainTile, &full[stage]);
   };
-  // this thread's four values of the product of `m` and the carried columns in `buf`
-  auto product = [&](const Part& m, int buf) {
+  // this thread's four values of the product of the matrix in `stage` and the carried columns in `buf`
+  auto product = [&](int stage, int buf) {
     float2 acc[4][4] = {};  // [i][pair of columns]
+    const float* part = reinterpret_cast<const float*>(s_m + stage * kChainTile) + (16 * warp + rg) * kHeadDim + 4 * sl;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
+      float4 m[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(part + 4 * i * kHeadDim + 32 * t);
       const float* x = &s_h[buf][(8 * t + sl) * kChainGroup];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -208,7 +219,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
         const float2 xs[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float mv = e == 0 ? m[i][t].x : e == 1 ? m[i][t].y : e == 2 ? m[i][t].z : m[i][t].w;
+          const float mv = e == 0 ? m[i].x : e == 1 ? m[i].y : e == 2 ? m[i].z : m[i].w;
 #pragma unroll
           for (int c = 0; c < 4; ++c) fma2(acc[i][c], make_float2(mv, mv), xs[c]);
         }
@@ -230,7 +241,6 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
     for (int c = 0; c < 2; ++c) out[c] = add(b0 ? z[2 + c] : z[c], b0 ? z[c] : z[2 + c], 1);
     return make_float4(out[0].x, out[0].y, out[1].x, out[1].y);
   };
-  Part parts[2];  // of this link and the next, by turns
   int buf = 0;
   for (int b0 = 0; b0 < links; b0 += kChainFlags) {
     const int nb = min(kChainFlags, links - b0);
@@ -241,38 +251,27 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
     if (__syncthreads_or(mine) == 0) continue;
     bool have_h = false;
     float4 add = make_float4(0.f, 0.f, 0.f, 0.f);  // the next state as it is: what the product is added to
-    if (flags[0] != 0) {
-      load_m(b0, parts[0]);
-      add = *state_of(b0 + 1);
-    }
-    // link i with its matrix in `m`; the next link's is on its way to `m_next` when it returns
-    auto link = [&](int i, Part& m, Part& m_next) {
-      const bool next = i + 1 < nb && flags[i + 1] != 0;
-      if (flags[i] == 0) {  // (uniform)
-        have_h = false;
-        if (next) {
-          load_m(b0 + i + 1, m_next);
-          add = *state_of(b0 + i + 2);
-        }
-        return;
-      }
-      if (!have_h) carry(buf, *state_of(b0 + i));
-      have_h = true;
+    if (flags[0] != 0) add = *state_of(b0 + 1);
+    if (tid == 0)
+      for (int x = 0; x < kChainStages - 1 && x < nb; ++x)
+        if (flags[x] != 0) request(b0 + x);
+    for (int i = 0; i < nb; ++i) {
+      const bool next = i + 1 < nb && flags[i + 1] != 0, work = flags[i] != 0;  // (uniform)
+      if (work && !have_h) carry(buf, *state_of(b0 + i));
+      have_h = work;
       float4 out = add;
-      if (next) {
-        load_m(b0 + i + 1, m_next);
-        add = *state_of(b0 + i + 2);
-      }
-      __syncthreads();  // the carried columns are complete
-      const float4 x = product(m, buf);
+      if (next) add = *state_of(b0 + i + 2);
+      __syncthreads();  // the carried columns are complete, and the matrix of the link before has been read
+      if (tid == 0 && i + kChainStages - 1 < nb && flags[i + kChainStages - 1] != 0) request(b0 + i + kChainStages - 1);
+      if (!work) continue;
+      const int stage = i % kChainStages;
+      if (!ptx::mbar_try_wait(&full[stage], (uses >> stage) & 1) && !ptx::mbar_wait_slow(&full[stage], (uses >> stage) & 1, nullptr, 0)) return;
+      uses ^= 1u << stage;
+      const float4 x = product(stage, buf);
       out.x += x.x; out.y += x.y; out.z += x.z; out.w += x.w;
       buf ^= 1;
       carry(buf, out);
       *state_of(b0 + i + 1) = out;
-    };
-    for (int i = 0; i < nb; i += 2) {
-      link(i, parts[0], parts[1]);
-      if (i + 1 < nb) link(i + 1, parts[1], parts[0]);
     }
     // (a link behind this batch reads the state written last, each value by the thread that wrote it)
   }
@@ -306,7 +305,9 @@ extern "C" QLA_API int qla_cp_chain(const QlaCpChainArgs* a, void* stream) {
   QLA_CHECK_ARG(a != nullptr && a->h0 && a->M && a->m_limit && a->raw_first_seg, "NULL pointer in QlaCpChainArgs");
   QLA_CHECK_ARG(a->num_raw_seqs > 0 && a->num_v_heads > 0, "bad sizes");
   dim3 grid(kHeadDim / kChainCols, a->num_v_heads, a->num_raw_seqs);
-  QLA_CHECK_CUDA(launch_dependent(cp_chain_kernel, grid, dim3(kChainThreads), 0, static_cast<cudaStream_t>(stream), a->h0, a->M,
+  const int rc = ensure_dynamic_smem<cp_chain_kernel>(kChainSmem);
+  if (rc != QLA_OK) return rc;
+  QLA_CHECK_CUDA(launch_dependent(cp_chain_kernel, grid, dim3(kChainThreads), kChainSmem, static_cast<cudaStream_t>(stream), a->h0, a->M,
                                   a->m_limit, a->raw_first_seg, a->num_v_heads, a->reverse));
   return QLA_OK;
 }
