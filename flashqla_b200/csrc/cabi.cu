@@ -70,7 +70,7 @@ namespace qla {
 void launch_info_chunk_fwd_kernel(bool aux, bool w_in_scan, int*, size_t*);
 void launch_info_bwd_scan_kernel(int*, size_t*);
 void launch_info_bwd_chunk_kernel(int*, size_t*);
-void launch_info_kkt_solve_kernel(int*, size_t*);
+void launch_info_kkt_solve_kernel(bool over, int*, size_t*);
 void launch_info_recurrent_kernel(int*, size_t*);
 }  // namespace qla
 
@@ -85,7 +85,8 @@ extern "C" QLA_API int qla_kernel_launch_info(const char* kernel, int32_t* block
   else if (name == "chunk_fwd_kernel:w_in_scan") launch_info_chunk_fwd_kernel(false, true, &block, &smem);
   else if (name == "bwd_scan_kernel") launch_info_bwd_scan_kernel(&block, &smem);
   else if (name == "bwd_chunk_kernel") launch_info_bwd_chunk_kernel(&block, &smem);
-  else if (name == "kkt_solve_kernel") launch_info_kkt_solve_kernel(&block, &smem);
+  else if (name == "kkt_solve_kernel") launch_info_kkt_solve_kernel(false, &block, &smem);
+  else if (name == "kkt_solve_kernel:over") launch_info_kkt_solve_kernel(true, &block, &smem);
   else if (name == "recurrent_kernel" || name == "recurrent_chain_kernel" || name == "recurrent_step_kernel") launch_info_recurrent_kernel(&block, &smem);
   else {
     set_last_error("unknown kernel '%s'", kernel);

@@ -91,10 +91,10 @@ struct Area {
                                         // kW: later columns 64..127 of Wt
   static constexpr uint32_t kN = kX + 6 * kBlock * 4;  // 4 blocks N20, N21, N30, N31 as fragments [s][lane] float4, TF32
   static constexpr uint32_t kBytes = kX + 11264;
-  static constexpr size_t kSmem = 32768 + 2 * kBytes;
+  static constexpr size_t kSmem = 32768 + 2 * kBytes, kSmemOver = 2 * kBytes;  // (kOver: the K tile lies where the areas are)
   static_assert(kN + 4096 <= kBytes && kBytes % 1024 == 0, "shared-memory map");
 };
-constexpr int kCtasPerSm = 3;
+constexpr int kCtasPerSm = 3, kCtasPerSmOver = 4;
 constexpr int kKktThreads = 128;
 
 // Fragments of a block, one array for all uses: value e of the pair [s][h] of lane 4 g + c is element (g + 8 h, 8 s + 2 c + e), which
@@ -225,8 +225,12 @@ __device__ __forceinline__ void chunk_sync(int ci) {  // the two warps that own 
 }
 
 // kW: A and w are written.  Otherwise A diag(beta) and -A diag(beta gamma), for a scan that forms Wt from it.
-template <typename T, bool kW>
-__global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(const __grid_constant__ CUtensorMap tm_k,
+// kOver (not with kW or the norms, which read the K tile later): an item's K tile lies where the two chunks' areas are, which nothing uses before
+// K K^T.  The next item's K comes when both chunks are through with this one, which exposes its latency (about 1 us of 6 to 12), and four
+// CTAs are resident instead of three: 32768 tokens of 16 / 32 heads 114 -> 105 us, 540 k packed tokens of 8 / 8 heads 510-524 -> 482 (with five, 91
+// registers, 133 and 600).
+template <typename T, bool kW, bool kOver>
+__global__ void __launch_bounds__(kKktThreads, kOver ? kCtasPerSmOver : kCtasPerSm) kkt_solve_kernel(const __grid_constant__ CUtensorMap tm_k,
                                                                                    const __grid_constant__ CUtensorMap tm_q,
                                                                                    const __grid_constant__ CUtensorMap tm_a,
                                                                                    const __grid_constant__ CUtensorMap tm_w,
@@ -284,7 +288,8 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
   extern __shared__ __align__(1024) uint8_t smem[];  // (the compiler pads what is in front of it to that alignment)
   using M = Area;
   constexpr int kTmemColumns = kW ? 128 : 64;  // K K^T, and Wt over it
-  uint8_t *sK = smem, *area = smem + 32768 + ci * M::kBytes;
+  static_assert(!kOver || !kW, "Wt is formed from the K tile");
+  uint8_t *sK = smem, *area = smem + (kOver ? 0 : 32768) + ci * M::kBytes;
   float* sX = reinterpret_cast<float*>(area + M::kX);
   float* sN = reinterpret_cast<float*>(area + M::kN);
   // exponents (log2) of L: -L[c][d] = -sign(beta_c) (k_c . k_d) 2^(row[c] + col[d]); the sign is that of beta
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
   __shared__ uint64_t bar_k, bar_q, bar_kk[2], bar_w[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ unsigned k_released;  // times that a chunk was through with what the K tile holds
-  const bool norm = p.rnorm != nullptr;
+  const bool norm = !kOver && p.rnorm != nullptr;
 
   auto load_k = [&](const Item& x) {
     ptx::mbar_expect_tx(&bar_k, 32768);
@@ -437,6 +442,8 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
   };
   // One thread per chunk says when the chunk is through with K (after its last product); the second one to do so loads the next
   // item's.  With the norms the Q tile visits the same memory in between, and each chunk says so a second time.
+  // kOver: both chunks' products have read the K tile
+  auto cta_sync = [&]() { asm volatile("bar.sync 3, 128;" ::: "memory"); };
   const bool q_first = kW && norm && cur.split == 0 && item == blockIdx.x, q_norms = norm && cur.split == 0 && !q_first;
   auto release_k = [&]() {
     unsigned before;
@@ -490,6 +497,9 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
     if (part == 0) {
       locate_next();
       ptx::mbar_wait_addr(a_k, turn);  // (or two such items in a row would release the tile under the other chunk)
+    }
+    if (kOver) cta_sync();
+    if (part == 0) {
       if (lane == 0) release_k();
       if (more) {
         fetch_gates(nxt, nxt.hv0);
@@ -513,7 +523,7 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
     ptx::umma_ss_k64_lanes<2, 2>(tmem, d_k + (16384 >> 4), d_k + (16384 >> 4) + ci * (8192 >> 4), idesc, low_off, high_off, true, a_kk);
   } else {
     locate_next();
-    if (lane == 0) ptx::tma_store_wait_read();  // the last store has read its tiles
+    if (!kOver && lane == 0) ptx::tma_store_wait_read();  // the last store has read its tiles
   }
   // In-kernel L2 norm of q and k (reference: l2norm before the kernels, flash_qla/utils/math.py:14-21 via
   // chunk/__init__.py:332-334): 1/sqrt(|row|^2 + eps), a row per thread.  Everything downstream uses the RAW tiles and
@@ -538,6 +548,7 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
   chunk_sync(ci);
   ptx::mbar_wait_addr(a_kk, kk_turn);
   kk_turn ^= 1;
+  if (kOver) cta_sync();
   ptx::tc_fence_after_sync();
   uint32_t kk_own[kW ? 3 : 1][8], kk_left[kW ? 4 : 1][8];
   const uint32_t high = quad + (16u << 16);
@@ -550,7 +561,7 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
       for (int x = 0; x < 4; ++x) ptx::tmem_ld_frag2(((x >> 1) ? high : quad) + 16 * (x & 1), kk_left[kW ? x : 0]);
     }
     ptx::tmem_wait_ld();
-  } else if (part == 0 && lane == 0) {
+  } else if (!kOver && part == 0 && lane == 0) {
     release_k();
   }
 #pragma unroll 1
@@ -558,10 +569,12 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
     const Gates& gt = s_gates[ci][buf % kGateBuffers];
     const bool last = hv + 1 == hv1;
     if (part == 0 && (!last || more)) fetch_gates(last ? nxt : cur, last ? nxt.hv0 : hv + 1);
-    auto next_gates = [&]() {
-      if (part != 0 || (last && !more)) return;
-      activate(last ? nxt : cur, last ? nxt.hv0 : hv + 1);
-      if (!last || !norm) publish(s_gates[ci][(buf ^ 1) % kGateBuffers]);
+    // (not kW: activated early too, while the other warp forms N of four blocks more, but made public when this head's gates have been read)
+    auto activate_next = [&]() {
+      if (part == 0 && (!last || more)) activate(last ? nxt : cur, last ? nxt.hv0 : hv + 1);
+    };
+    auto publish_next = [&]() {
+      if (part == 0 && (last ? more && !norm : true)) publish(s_gates[ci][(buf ^ 1) % kGateBuffers]);
     };
     if (hv > hv0) {  // the store of the previous head has read its tiles
       if (part == 0 && lane == 0) ptx::tma_store_wait_read();
@@ -678,8 +691,9 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
         product_3xtf32(y, d1, t);
         store_n(own + 2 * kBlock, y, lm);
         emit<T, !kW>(av[2], aw_tile + lm.tile(R + 1, R), y, bg, beta, lane);
-        zero_above(area + M::kAw);
-        if (kW) next_gates();
+        if (kW || hv == hv0) zero_above(area + M::kAw);
+        activate_next();
+        if (kW) publish_next();
       }
       chunk_sync(ci);
       // ---- 3: column block m = part of the lower left quarter, X[2:4][m] = X[2:4][2:4] (N[2:4][0:2] X[0:2][m])
@@ -734,7 +748,8 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
         }
         *reinterpret_cast<uint4*>(area + M::kAw + ptx::sw128_offset(row, j >> 3)) = make_uint4(aw[0], aw[1], aw[2], aw[3]);
       }
-      next_gates();
+      activate_next();
+      publish_next();
     }
     ptx::fence_proxy_async_smem();
     ptx::tc_fence_before_sync();
@@ -755,7 +770,7 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
         ptx::tma_store_commit();
       }
       __syncwarp();
-      next_gates();
+      publish_next();
     }
     if (!kW || p.A_in == nullptr) {
       const int R = 2 * part;
@@ -823,6 +838,11 @@ __global__ void __launch_bounds__(kKktThreads, kCtasPerSm) kkt_solve_kernel(cons
             *reinterpret_cast<const uint4*>(area + M::kAw + (x & 8) * 1024 + ptx::sw128_offset(x >> 4, x & 7));
     }
   }
+  if (kOver) {  // the areas are free for the next K when both chunks say so (their writes are fenced above)
+    if (part == 0 && lane == 0) ptx::tma_store_wait_read();
+    chunk_sync(ci);
+    if (part == 0 && lane == 0) release_k();
+  }
   }  // valid
   if (kW && valid > 0 && q_norms) finish_q(sK);
   }  // items
@@ -871,13 +891,13 @@ int launch_chunk_tables(const int32_t* cu, int n, int32_t* pair_offsets, int32_t
   return QLA_OK;
 }
 
-template <typename T, bool kW>
+template <typename T, bool kW, bool kOver = false>
 static int launch_kkt(const KktParams& p, const CUtensorMap& tm_k, const CUtensorMap& tm_q, const CUtensorMap& tm_a, const CUtensorMap& tm_w, unsigned grid,
                       cudaStream_t stream) {
-  constexpr size_t smem = Area::kSmem;
-  const int rc = ensure_dynamic_smem<kkt_solve_kernel<T, kW>>(smem);
+  constexpr size_t smem = kOver ? Area::kSmemOver : Area::kSmem;
+  const int rc = ensure_dynamic_smem<kkt_solve_kernel<T, kW, kOver>>(smem);
   if (rc != QLA_OK) return rc;
-  QLA_CHECK_CUDA(launch_dependent(kkt_solve_kernel<T, kW>, dim3(grid), dim3(kKktThreads), smem, stream, tm_k, tm_q, tm_a, tm_w, p));
+  QLA_CHECK_CUDA(launch_dependent(kkt_solve_kernel<T, kW, kOver>, dim3(grid), dim3(kKktThreads), smem, stream, tm_k, tm_q, tm_a, tm_w, p));
   QLA_CHECK_CUDA(cudaGetLastError());
   return QLA_OK;
 }
@@ -901,7 +921,8 @@ int launch_kkt_solve(const KktParams& params, const void* k, const void* q, int6
   int slots = 0, dev = 0;
   QLA_CHECK_CUDA(cudaGetDevice(&dev));
   QLA_CHECK_CUDA(cudaDeviceGetAttribute(&slots, cudaDevAttrMultiProcessorCount, dev));
-  slots *= kCtasPerSm;
+  const bool over = !with_w && p.rnorm == nullptr;
+  slots *= over ? kCtasPerSmOver : kCtasPerSm;
   // Work items: the v-heads of a k-head stay together, which reads K once, unless the rounds of resident CTAs come out shorter
   // with fewer heads per item.  Getting an item under way costs about as much as 0.6 heads.
   double best = 0;
@@ -918,14 +939,18 @@ int launch_kkt_solve(const KktParams& params, const void* k, const void* q, int6
   QLA_CHECK_SUPPORTED(items < (int64_t(1) << 31), "too many chunks and heads");
   p.num_pairs = pairs_upper;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(items, slots));
-  if (is_bf16) return with_w ? launch_kkt<__nv_bfloat16, true>(p, tm_k, tm_q, tm_a, tm_w, grid, stream)
-                             : launch_kkt<__nv_bfloat16, false>(p, tm_k, tm_q, tm_a, tm_w, grid, stream);
-  return with_w ? launch_kkt<__half, true>(p, tm_k, tm_q, tm_a, tm_w, grid, stream) : launch_kkt<__half, false>(p, tm_k, tm_q, tm_a, tm_w, grid, stream);
+#define QLA_LAUNCH_KKT(T)                                                                              \
+  return with_w  ? launch_kkt<T, true>(p, tm_k, tm_q, tm_a, tm_w, grid, stream)                        \
+         : over  ? launch_kkt<T, false, true>(p, tm_k, tm_q, tm_a, tm_w, grid, stream)                 \
+                 : launch_kkt<T, false>(p, tm_k, tm_q, tm_a, tm_w, grid, stream)
+  if (is_bf16) QLA_LAUNCH_KKT(__nv_bfloat16);
+  QLA_LAUNCH_KKT(__half);
+#undef QLA_LAUNCH_KKT
 }
 
-void launch_info_kkt_solve_kernel(int* block_threads, size_t* dynamic_smem_bytes) {
+void launch_info_kkt_solve_kernel(bool over, int* block_threads, size_t* dynamic_smem_bytes) {
   *block_threads = kKktThreads;
-  *dynamic_smem_bytes = Area::kSmem;
+  *dynamic_smem_bytes = over ? Area::kSmemOver : Area::kSmem;
 }
 
 }  // namespace qla

@@ -54,18 +54,21 @@ _CHUNK_FWD = dict(
     tensor_maps="A (:w_in_scan: also w): 3-D (64, heads, tokens), box 64 x 1 x 64; q, k, v, w, o, v_new: 4-D (64 columns, heads, tokens, "
                 "2 halves), box 64 x 1 x 64 x 2; h: the same over rows of [chunks * Hv * 128, 128]; 16-bit elements, 128B swizzle; any "
                 "map for what a launch does not use")
+# kkt_solve_kernel<T, kW, kOver>: plain, and :over (kOver: operands of w for a scan that forms it, no norms of q and k)
+_KKT = dict(
+    block=128, dynamic_smem=71680, cluster=1,
+    grid="min(items, 3 * SMs), persistent; items = (pairs of 64-token chunks) * Hk * head_splits",
+    params=[_TMAP + " k", _TMAP + " q", _TMAP + " A", _TMAP + " w",
+            "KktParams (by value; the launcher sets num_pairs (equal lengths), heads_per_cta and head_splits = "
+            "ceil(Hv / Hk / heads_per_cta))"],
+    tensor_maps="k, q, w: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 128 (w: 64) x 2; A, and w of the form with "
+                "kW = 0: 3-D (64, heads, tokens), box 64 x 1 x 64; 16-bit elements, 128B swizzle")
 KERNEL_RULES = {
     "chunk_fwd_kernel": dict(_CHUNK_FWD, dynamic_smem=197632),
     "chunk_fwd_kernel:aux": dict(_CHUNK_FWD, dynamic_smem=214016),
     "chunk_fwd_kernel:w_in_scan": dict(_CHUNK_FWD, dynamic_smem=222208),
-    "kkt_solve_kernel": dict(
-        block=128, dynamic_smem=71680, cluster=1,
-        grid="min(items, 3 * SMs), persistent; items = (pairs of 64-token chunks) * Hk * head_splits",
-        params=[_TMAP + " k", _TMAP + " q", _TMAP + " A", _TMAP + " w",
-                "KktParams (by value; the launcher sets num_pairs (equal lengths), heads_per_cta and head_splits = "
-                "ceil(Hv / Hk / heads_per_cta))"],
-        tensor_maps="k, q, w: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 128 (w: 64) x 2; A, and w of the form with "
-                    "kW = 0: 3-D (64, heads, tokens), box 64 x 1 x 64; 16-bit elements, 128B swizzle"),
+    "kkt_solve_kernel": _KKT,
+    "kkt_solve_kernel:over": dict(_KKT, dynamic_smem=38912, grid=_KKT["grid"].replace("3 * SMs", "4 * SMs")),
     "bwd_scan_kernel": dict(
         block=512, dynamic_smem=214016, cluster=1, grid="num_seqs * Hv (twice that for a dual state-only launch)",
         params=[_TMAP + " q", _TMAP + " k", _TMAP + " dO", _TMAP + " w", _TMAP + " dh (store)", _TMAP + " du (store)",
@@ -92,6 +95,11 @@ def _chunk_fwd_form(mangled: str) -> str:
     return ":aux" if flags[1] == "1" else ":w_in_scan" if flags[5] == "1" else ""
 
 
+def _kkt_form(mangled: str) -> str:
+    """Suffix of the rule of an instantiation: kkt_solve_kernel<T, kW, kOver>."""
+    return ":over" if re.search(r"kkt_solve_kernelI\w+?Lb[01]ELb1E", mangled) else ""
+
+
 def _kernel_entries(directory: Path) -> list:
     """Per-kernel entries from what the build recorded (``kernels.ptxas.json``: the compiler's own report)."""
     rec = Path(directory) / "kernels.ptxas.json"
@@ -103,6 +111,8 @@ def _kernel_entries(directory: Path) -> list:
             base = next((n for n in KERNEL_RULES if n in k["mangled"]), None)
             if base == "chunk_fwd_kernel":
                 base += _chunk_fwd_form(k["mangled"])
+            elif base == "kkt_solve_kernel":
+                base += _kkt_form(k["mangled"])
             rule = KERNEL_RULES.get(base, {})
             entries.append({
                 "export_name": k["mangled"], "kernel_name": base or k["mangled"], "source": src,
