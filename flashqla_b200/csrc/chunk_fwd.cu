@@ -125,11 +125,23 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&x);
 }
 
+// two neighbouring registers of a tensor-memory load as a pair
+__device__ __forceinline__ F2 pair(uint32_t a, uint32_t b) { return f2(__uint_as_float(a), __uint_as_float(b)); }
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(F2 x) {
+  const float2 y = unpack(x);
+  return pack2<T>(y.x, y.y);
+}
+
 // Gated RMS norm of an output tile (two 128B-swizzled [64][64] halves at shared address `so`), in place: rows first + 16 y +
 // 0..7 (y = 0..3) by the four warps that call it, 16 threads per row with eight values each; `z` is the gate row of the
 // tile's first token, `stride` elements from token to token.  The gate is requested before the tile is waited for.  With the
 // four output warps doing all rows a chunk took 3.0 us (1.4 without the norm) and 777 tokens of 32 heads 46 us of scan; with
 // the Pg warps doing half 39.5, with the Pg warps doing all 44.  One copy of the code for both callers.
+// A chunk's norm is bound by instruction issue beside the other roles (2000 of its 2950 cycles; the rest is the latency of the
+// gate), not by how many warps share it.  Pairs of values per instruction and the gate as z * (1 / (1 + 2^(-z log2 e))) without
+// the scaling of tiny operands that a division brings: 777 tokens of 32 heads 45.3 -> 43.9 us of scan, 32768 tokens of 2 / 4 heads
+// 57.7 -> 53.9 (with the pairs in the chain below).  Four rows at once, or the gate held a chunk ahead, were slower (more code).
 template <typename T>
 static __device__ __noinline__ bool norm_rows(uint32_t so, const T* z, int stride, const float* weight, float eps, int valid,
                                               int first, uint32_t bar, uint32_t parity) {
@@ -147,18 +159,21 @@ static __device__ __noinline__ bool norm_rows(uint32_t so, const T* z, int strid
   uint32_t cell = so + (tl & 8) * 1024 + ptx::sw128_offset(row0, tl & 7);
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass, cell += 4096) {  // two rows at a time: half the code, and code is what is short here
-    uint4 raw[2];
+    F2 x[2][4];
     float ss[2];
 #pragma unroll
-    for (int y = 0; y < 2; ++y)
-      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(raw[y].x), "=r"(raw[y].y), "=r"(raw[y].z), "=r"(raw[y].w)
-                   : "r"(cell + 2048u * y) : "memory");
-#pragma unroll
     for (int y = 0; y < 2; ++y) {
-      const T* e = reinterpret_cast<const T*>(&raw[y]);
-      ss[y] = 0.f;
+      uint4 raw;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w)
+                   : "r"(cell + 2048u * y) : "memory");
+      const T* e = reinterpret_cast<const T*>(&raw);
+      F2 sum = f2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ss[y] = fmaf(Cvt<T>::to_f32(e[i]), Cvt<T>::to_f32(e[i]), ss[y]);
+      for (int i = 0; i < 4; ++i) {
+        x[y][i] = f2(Cvt<T>::to_f32(e[2 * i]), Cvt<T>::to_f32(e[2 * i + 1]));
+        sum = fma2(x[y][i], x[y][i], sum);
+      }
+      ss[y] = unpack(sum).x + unpack(sum).y;
     }
 #pragma unroll
     for (int off = 1; off < 16; off <<= 1)
@@ -167,16 +182,18 @@ static __device__ __noinline__ bool norm_rows(uint32_t so, const T* z, int strid
 #pragma unroll
     for (int y = 0; y < 2; ++y) {
       const float rstd = rsqrtf(ss[y] * (1.f / kHeadDim) + eps);
-      const T* e = reinterpret_cast<const T*>(&raw[y]);
       const T* ze = reinterpret_cast<const T*>(&zr[y]);
-      float x[8];
+      uint32_t out[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float zf = Cvt<T>::to_f32(ze[i]);
-        x[i] = Cvt<T>::to_f32(e[i]) * rstd * wv[i] * __fdividef(zf, 1.f + __expf(-zf));
+      for (int i = 0; i < 4; ++i) {
+        const F2 zf = f2(Cvt<T>::to_f32(ze[2 * i]), Cvt<T>::to_f32(ze[2 * i + 1]));
+        const float2 l = unpack(mul2(zf, f2(-1.4426950408889634f, -1.4426950408889634f)));
+        const F2 silu = mul2(zf, f2(ptx::rcp(1.f + ptx::ex2(l.x)), ptx::rcp(1.f + ptx::ex2(l.y))));
+        const float2 r = unpack(mul2(mul2(mul2(x[y][i], f2(rstd, rstd)), f2(wv[2 * i], wv[2 * i + 1])), silu));
+        out[i] = pack2<T>(r.x, r.y);
       }
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cell + 2048u * y), "r"(pack2<T>(x[0], x[1])), "r"(pack2<T>(x[2], x[3])),
-                   "r"(pack2<T>(x[4], x[5])), "r"(pack2<T>(x[6], x[7])) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cell + 2048u * y), "r"(out[0]), "r"(out[1]),
+                   "r"(out[2]), "r"(out[3]) : "memory");
     }
     zr[0] = zr[2];
     zr[1] = zr[3];
@@ -1104,8 +1121,8 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
           const float4 r4 = *reinterpret_cast<const float4*>(&gs->rho[c0 + j]);
-          vp[j >> 1] = pack2<T>(__uint_as_float(d[j]) * r4.x, __uint_as_float(d[j + 1]) * r4.y);
-          vp[(j >> 1) + 1] = pack2<T>(__uint_as_float(d[j + 2]) * r4.z, __uint_as_float(d[j + 3]) * r4.w);
+          vp[j >> 1] = pack2<T>(mul2(pair(d[j], d[j + 1]), f2(r4.x, r4.y)));
+          vp[(j >> 1) + 1] = pack2<T>(mul2(pair(d[j + 2], d[j + 3]), f2(r4.z, r4.w)));
         }
         ptx::tmem_st16(tm + kColD2 + c0, vp);
         ptx::tmem_wait_st();
@@ -1129,7 +1146,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (!(alive = wait(kSDone, ph))) break;
       ptx::tc_fence_after_sync();
       if (warp == 0) trace(1, i, 4);
-            const bool last = (i + 1 == nproc);
+      const bool last = (i + 1 == nproc);
       if (last) {
         if (write_final) {
 #pragma unroll 1
@@ -1160,11 +1177,16 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::tc_fence_before_sync();
         warp_arrive(&bars[kSbfReady], lane);
         if (warp == 0) trace(1, i, 5);
-          // (b) off the critical path: decay of the fp32 state for the next chunk (needed by MMA3 only)
+        // (b) off the critical path: decay of the fp32 state for the next chunk (needed by MMA3 only).  In pairs: half the
+        // instructions (the output epilogue gained nothing from them, or lost: 540 k packed tokens of 8 / 8 heads 972 -> 978 us)
         if (!(alive = wait(kGate0 + ((i + 1) & 3), ((i + 1) >> 2) & 1))) break;
         const float egl_next = gates_of(i + 1)->egl;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) sf[j] = __float_as_uint(__uint_as_float(sf[j]) * egl_next);
+        for (int j = 0; j < 64; j += 2) {
+          const float2 y = unpack(mul2(pair(sf[j], sf[j + 1]), f2(egl_next, egl_next)));
+          sf[j] = __float_as_uint(y.x);
+          sf[j + 1] = __float_as_uint(y.y);
+        }
         ptx::tmem_st32(tm + kColS + col_half, reinterpret_cast<const uint32_t(&)[32]>(sf[0]));
         ptx::tmem_st32(tm + kColS + col_half + 32, reinterpret_cast<const uint32_t(&)[32]>(sf[32]));
         ptx::tmem_wait_st();

@@ -211,6 +211,11 @@ __device__ __forceinline__ float ex2(float x) {  // 2^x, approximate (the MUFU b
   return y;
 }
 
+__device__ __forceinline__ float rcp(float x) {  // 1 / x, approximate
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float lg2(float x) {  // log2, approximate
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
