@@ -751,8 +751,10 @@ int launch_recurrent_state(const QlaRecurrentArgs& a, int rows, cudaStream_t str
   // One step: the kernel without the loop, of which five tiles of 32 rows are resident per SM, not four (us, recurrent_kernel /
   // recurrent_step_kernel, states from HBM, 32 heads: bf16 pools 16 sequences 11.9 / 10.1, 64 37.6 / 30.4, 128 71.0 / 57.0; fp32 pools
   // 4 6.1 / 5.8, 12 12.2 / 10.7, 24 20.0 / 18.0, 32 24.5 / 23.5, 48 34.8 / 35.0, 64 44.7 / 47.3, 256 163.6 / 187: from about 1200 fp32 heads on HBM is the
-  // bound, and the memory does better with fewer tiles in flight).
-  if (a.tokens_per_seq == 1 && (std::is_same<StateT, __nv_bfloat16>::value || static_cast<int64_t>(a.num_seqs) * a.num_v_heads <= 1024))
+  // bound, and the memory does better with fewer tiles in flight).  Calls of 296 heads with a bf16 pool behind one another take 7.61 with the
+  // general kernel, whose two rounds come out even (592 of 1184 tiles), and 7.75 with this one: bf16 pools come here above 384.
+  const int64_t heads = static_cast<int64_t>(a.num_seqs) * a.num_v_heads;
+  if (a.tokens_per_seq == 1 && (std::is_same<StateT, __nv_bfloat16>::value ? heads > 384 : heads <= 1024))
     return launch_recurrent_form<T, InterT, StateT, kStep>(a, rows, stream);
   if (a.parents != nullptr) return launch_recurrent_form<T, InterT, StateT, kTree>(a, rows, stream);
   // Several steps, of which every state is cached in 16 bits or none is: instructions are the bound, and the kernel with fewer of them is
