@@ -121,7 +121,8 @@ class QlaCpPlanArgs(C.Structure):
 class QlaCpChainArgs(C.Structure):
     _fields_ = [
         ("num_raw_seqs", C.c_int32), ("num_v_heads", C.c_int32), ("h0", C.c_void_p), ("M", C.c_void_p),
-        ("m_limit", C.c_void_p), ("raw_first_seg", C.c_void_p), ("reverse", C.c_int32), ("reserved", C.c_int32),
+        ("m_limit", C.c_void_p), ("raw_first_seg", C.c_void_p), ("reverse", C.c_int32), ("has_status", C.c_int32),
+        ("status", C.c_void_p),
     ]
 
 

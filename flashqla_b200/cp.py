@@ -26,6 +26,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import torch
 
 from . import _cabi
+from .utils import device_status
 
 CHUNK = 64
 MIN_SEG_CHUNKS = 8
@@ -169,7 +170,8 @@ def segment_initial_states(plan: CpPlan, k, v, beta, g_cumsum, A, w, h0, scale, 
                flags=_cabi.CHUNK_STATE_ONLY | _cabi.CHUNK_SKIP_PREPARE, seq_map=d["warm_map"], chunk_limit=warm_limit,
                num_seqs=n_seg, w=w, tables=plan.tables, rnorm=rnorm, dual=(m_limit, d["identity"], M))
     ca = _cabi.QlaCpChainArgs(num_raw_seqs=len(plan.raw_first) - 1, num_v_heads=Hv, h0=cp_h0.data_ptr(),
-                              M=M.data_ptr(), m_limit=m_limit.data_ptr(), raw_first_seg=d["raw_first"].data_ptr())
+                              M=M.data_ptr(), m_limit=m_limit.data_ptr(), raw_first_seg=d["raw_first"].data_ptr(),
+                              has_status=1, status=device_status(dev).data_ptr())
     with torch.cuda.device(dev):
         _cabi.check(lib.qla_cp_chain(ca, stream), "qla_cp_chain")
     return cp_h0, lead

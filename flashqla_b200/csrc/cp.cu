@@ -169,10 +169,24 @@ __device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {  // two 
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
 }
 
+// A warp's wait for the matrix in `stage`, the same verdict for all of it.  Given up, the status word says so (192 + stage as the
+// barrier); the thread that requests the copies then waits for those still on their way, `ahead` links from this one on, or for
+// another while: shared memory stays allocated until they have landed.
+static __device__ __noinline__ bool chain_wait(uint64_t* full, int stage, uint32_t uses, int* status, int ahead, const int* flags) {
+  if (__all_sync(__activemask(), ptx::mbar_wait_polling(&full[stage], (uses >> stage) & 1, status, kStatusBarrierTimeout | ((192 + stage) << 8),
+                                                        ptx::kWaitLimitNs)))
+    return true;
+  for (int x = 0; x < ahead; ++x) {
+    const int s = (stage + x) % kChainStages;
+    if (flags[x] != 0) ptx::mbar_wait_nocall(ptx::smem_u32(&full[s]), (uses >> s) & 1, true);
+  }
+  return false;
+}
+
 __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __restrict__ h0, const float* __restrict__ M,
                                                                     const int32_t* __restrict__ m_limit,
                                                                     const int32_t* __restrict__ raw_first_seg, int num_heads,
-                                                                    int reverse) {
+                                                                    int reverse, int* status) {
   grid_dep_wait();
   grid_dep_launch();
   const int c0 = blockIdx.x * kChainCols, h = blockIdx.y, r = blockIdx.z, tid = threadIdx.x;
@@ -181,11 +195,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
   __shared__ int flags[kChainFlags];
   extern __shared__ __align__(128) uint8_t s_m[];  // M of links i, i + 1, i + 2 by turns
   __shared__ uint64_t full[kChainStages];
-  if (tid == 0) {
-    for (int x = 0; x < kChainStages; ++x) ptx::mbar_init(&full[x], 1);
-    ptx::fence_mbar_init();
-  }
-  uint32_t uses = 0;  // of a stage: bit x, the parity of its next phase
+  uint32_t uses = 0;     // of a stage: bit x, the parity of its next phase
+  bool ready = false;    // the barriers are initialised
+  bool gave_up = false;  // a wait of this warp has
   // link i leads from segment seg_of(i) to seg_of(i + 1)
   auto seg_of = [&](int i) { return reverse ? s0 + links - i : s0 + i; };
   // rows 16 warp + rg + 4 i (i = 0..3), inner indices 32 t + 4 sl .. + 3 (t = 0..3)
@@ -245,16 +257,22 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
   for (int b0 = 0; b0 < links; b0 += kChainFlags) {
     const int nb = min(kChainFlags, links - b0);
     int mine = 0;
-    __syncthreads();
+    if (b0 != 0 && __syncthreads_or(gave_up)) return;
     for (int i = tid; i < nb; i += kChainThreads) mine |= (flags[i] = m_limit[seg_of(b0 + i) * num_heads + h]);
     // the usual case (every segment decays below the threshold) has nothing to chain
     if (__syncthreads_or(mine) == 0) continue;
     bool have_h = false;
     float4 add = make_float4(0.f, 0.f, 0.f, 0.f);  // the next state as it is: what the product is added to
     if (flags[0] != 0) add = *state_of(b0 + 1);
-    if (tid == 0)
+    if (tid == 0) {
+      if (!ready) {
+        for (int x = 0; x < kChainStages; ++x) ptx::mbar_init(&full[x], 1);
+        ptx::fence_mbar_init();
+      }
       for (int x = 0; x < kChainStages - 1 && x < nb; ++x)
         if (flags[x] != 0) request(b0 + x);
+    }
+    ready = true;
     for (int i = 0; i < nb; ++i) {
       const bool next = i + 1 < nb && flags[i + 1] != 0, work = flags[i] != 0;  // (uniform)
       if (work && !have_h) carry(buf, *state_of(b0 + i));
@@ -265,7 +283,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
       if (tid == 0 && i + kChainStages - 1 < nb && flags[i + kChainStages - 1] != 0) request(b0 + i + kChainStages - 1);
       if (!work) continue;
       const int stage = i % kChainStages;
-      if (!ptx::mbar_try_wait(&full[stage], (uses >> stage) & 1) && !ptx::mbar_wait_slow(&full[stage], (uses >> stage) & 1, nullptr, 0)) return;
+      if (!ptx::mbar_try_wait(&full[stage], (uses >> stage) & 1) &&
+          !chain_wait(full, stage, uses, status, tid == 0 ? min(kChainStages, nb - i) : 0, flags + i)) {
+        for (gave_up = true; ++i < nb;) __syncthreads();  // (the other warps' barriers)
+        break;
+      }
       uses ^= 1u << stage;
       const float4 x = product(stage, buf);
       out.x += x.x; out.y += x.y; out.z += x.z; out.w += x.w;
@@ -308,6 +330,6 @@ extern "C" QLA_API int qla_cp_chain(const QlaCpChainArgs* a, void* stream) {
   const int rc = ensure_dynamic_smem<cp_chain_kernel>(kChainSmem);
   if (rc != QLA_OK) return rc;
   QLA_CHECK_CUDA(launch_dependent(cp_chain_kernel, grid, dim3(kChainThreads), kChainSmem, static_cast<cudaStream_t>(stream), a->h0, a->M,
-                                  a->m_limit, a->raw_first_seg, a->num_v_heads, a->reverse));
+                                  a->m_limit, a->raw_first_seg, a->num_v_heads, a->reverse, a->has_status != 0 ? a->status : nullptr));
   return QLA_OK;
 }

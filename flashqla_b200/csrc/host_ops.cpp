@@ -307,6 +307,7 @@ void segment_chain(const Plan& p, const SegmentScratch& s, int64_t Hv, bool reve
   QlaCpChainArgs a{};
   a.num_raw_seqs = p.num_raw; a.num_v_heads = Hv; a.h0 = s.h0.data_ptr<float>(); a.M = s.M.data_ptr<float>();
   a.m_limit = s.m_limit; a.raw_first_seg = ptr<int32_t>(p.raw_first); a.reverse = reverse;
+  a.has_status = 1; a.status = status_word(s.h0.device());
   check(qla_cp_chain(&a, stream), "qla_cp_chain");
 }
 void use_tables(QlaChunkFwdArgs& a, const Tensor& tables) {

@@ -39,6 +39,7 @@ import torch
 
 from . import _cabi, cp
 from .chunk import CHUNK, _launch_fwd, chunk_tables_workspace, new_w
+from .utils import device_status
 
 _SP_PLANS: Dict[Tuple, "SpPlan"] = {}
 
@@ -134,7 +135,8 @@ def slice_summary(q, k, v, g, beta, scale: Optional[float] = None) -> _SliceCont
     prefix[0] = torch.eye(128, dtype=torch.float32, device=dev)
     for buf in (cp_h0, prefix):
         ca = _cabi.QlaCpChainArgs(num_raw_seqs=1, num_v_heads=Hv, h0=buf.data_ptr(), M=M.data_ptr(),
-                                  m_limit=m_limit.data_ptr(), raw_first_seg=d["raw_first"].data_ptr())
+                                  m_limit=m_limit.data_ptr(), raw_first_seg=d["raw_first"].data_ptr(),
+                                  has_status=1, status=device_status(dev).data_ptr())
         with torch.cuda.device(dev):
             _cabi.check(lib.qla_cp_chain(ca, stream), "qla_cp_chain")
     summary = torch.stack((cp_h0[n_seg], prefix[n_seg]))

@@ -424,7 +424,7 @@ QLA_API int qla_cp_plan(const QlaCpPlanArgs* args, void* stream);
  * qla_cp_chain: h0[seg + 1] += M[seg] * h0[seg] for every (segment, head) with m_limit != 0, walking
  * the segments of each original sequence in order.  h0 and M are fp32 [num_segments, Hv, 128, 128]
  * ([K, V] and [K, K]); raw_first_seg [num_raw_seqs + 1] gives the first segment of every original
- * sequence.
+ * sequence.  A wait of the kernel that gives up raises *status; the states behind it are unfinished then.
  */
 typedef struct QlaCpChainArgs {
   int32_t num_raw_seqs;
@@ -434,7 +434,8 @@ typedef struct QlaCpChainArgs {
   const int32_t* m_limit;
   const int32_t* raw_first_seg;
   int32_t reverse;            /* backward: h0[seg - 1] += M[seg] * h0[seg], last segment first  */
-  int32_t reserved;
+  int32_t has_status;         /* 1: `status` is read (0 in callers whose struct ends here)      */
+  int32_t* status;            /* device status word or NULL (see QlaChunkFwdArgs.status)        */
 } QlaCpChainArgs;
 
 QLA_API int qla_cp_chain(const QlaCpChainArgs* args, void* stream);

@@ -45,6 +45,15 @@ def test_struct_layouts_match_header(built_lib):
         assert names == [f[0] for f in cls._fields_], cls.__name__
 
 
+def test_every_launch_can_report(built_lib):
+    """Each argument structure whose kernel waits or checks indices has a status word; the chain's is read only from callers that say
+    that they have it, because its structure ended in front of it before."""
+    from flashqla_b200 import _cabi
+    for cls in (_cabi.QlaRecurrentArgs, _cabi.QlaChunkFwdArgs, _cabi.QlaChunkBwdArgs, _cabi.QlaStateCommitArgs, _cabi.QlaCpChainArgs):
+        assert "status" in {f[0] for f in cls._fields_}, cls.__name__
+    assert [f[0] for f in _cabi.QlaCpChainArgs._fields_][-2:] == ["has_status", "status"]
+
+
 def test_argument_validation_without_gpu(built_lib):
     """Host-side checks of the entry point run before any launch, so they work without a GPU."""
     from flashqla_b200 import _cabi

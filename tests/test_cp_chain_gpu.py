@@ -50,6 +50,31 @@ def chain(h, M):
     return out
 
 
+def test_callers_hand_the_chain_their_status_word(monkeypatch):
+    """The Python callers of the chain (the native one sets it in segment_chain): the device's status word goes with every launch."""
+    from flashqla_b200 import _cabi, chunk, cp, seq_parallel, utils
+    seen = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            f = getattr(real, name)
+            return f if name != "qla_cp_chain" else lambda a, stream: (seen.append((a.has_status, a.status)), f(a, stream))[1]
+
+    real = _cabi.lib()
+    monkeypatch.setattr(_cabi, "lib", Recorder)
+    T, Hv = 4096, 2
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.nn.functional.normalize(torch.randn(1, T, Hv, 128, generator=gen, device="cuda"), dim=-1).bfloat16() for _ in range(3))
+    g, beta = -0.1 * torch.rand(1, T, Hv, generator=gen, device="cuda"), torch.rand(1, T, Hv, generator=gen, device="cuda")
+    ctx = seq_parallel.slice_summary(q, k, v, g, beta)
+    assert len(seen) == 2
+    plan = cp.get_plan([T], Hv, q.device)
+    assert plan.use_cp
+    cp.segment_initial_states(plan, k, v, beta, ctx.tensors[4], ctx.tensors[5], ctx.tensors[6], None, ctx.scale, chunk._launch_fwd)
+    assert seen == [(1, utils.device_status(q.device).data_ptr())] * 3
+    utils.check_device_status()
+
+
 def plain(h, M):
     """The same in the type of ``h``, sums of 128 products one after the other."""
     out = h.clone()
