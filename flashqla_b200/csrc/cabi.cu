@@ -72,6 +72,7 @@ void launch_info_bwd_scan_kernel(int*, size_t*);
 void launch_info_bwd_chunk_kernel(int*, size_t*);
 void launch_info_kkt_solve_kernel(bool over, int*, size_t*);
 void launch_info_recurrent_kernel(int*, size_t*);
+void launch_info_cp_chain_kernel(int*, size_t*);
 }  // namespace qla
 
 extern "C" QLA_API int qla_kernel_launch_info(const char* kernel, int32_t* block_threads, size_t* dynamic_smem_bytes) {
@@ -88,6 +89,7 @@ extern "C" QLA_API int qla_kernel_launch_info(const char* kernel, int32_t* block
   else if (name == "kkt_solve_kernel") launch_info_kkt_solve_kernel(false, &block, &smem);
   else if (name == "kkt_solve_kernel:over") launch_info_kkt_solve_kernel(true, &block, &smem);
   else if (name == "recurrent_kernel" || name == "recurrent_chain_kernel" || name == "recurrent_step_kernel") launch_info_recurrent_kernel(&block, &smem);
+  else if (name == "cp_chain_kernel") launch_info_cp_chain_kernel(&block, &smem);
   else {
     set_last_error("unknown kernel '%s'", kernel);
     return QLA_ERR_INVALID_ARG;

@@ -300,6 +300,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
 }
 
 }  // namespace
+
+void launch_info_cp_chain_kernel(int* block_threads, size_t* dynamic_smem_bytes) {
+  *block_threads = kChainThreads;
+  *dynamic_smem_bytes = kChainSmem;
+}
 }  // namespace qla
 
 extern "C" QLA_API int qla_cp_plan(const QlaCpPlanArgs* a, void* stream) {

@@ -81,6 +81,10 @@ KERNEL_RULES = {
         ["BwdParams (by value)", "int total_items"],
         tensor_maps="q..dO, dq..dv: 4-D (64 columns, heads, tokens, 2 halves), box 64 x 1 x 64 x 2; h, dh: the same over rows of "
                     "[chunks * Hv * 128, 128], box 64 x 1 x 128 x 2; A, du: 3-D, box 64 x 1 x 64 and 64 x 1 x 128; all 128B swizzle"),
+    "cp_chain_kernel": dict(
+        block=256, dynamic_smem=196608, cluster=1, grid="(16, Hv, num_raw_seqs)",
+        params=["float* h0", "const float* M", "const int32_t* m_limit", "const int32_t* raw_first_seg", "int num_heads", "int reverse",
+                "int* status (or NULL)"], tensor_maps=None),
     # recurrent_step_kernel: one token per sequence; recurrent_chain_kernel: tokens_per_seq > 1, no parents; recurrent_kernel: any
     **{name: dict(
         block=128, dynamic_smem=32768, cluster=1, grid="min(N * Hv * (128 / rows), resident CTAs), grid-stride over items",

@@ -461,7 +461,7 @@ QLA_API int qla_selftest_bounded_wait(int32_t* status, uint64_t limit_ns, void* 
  * Launch constants of the library's main kernels ("chunk_fwd_kernel", "chunk_fwd_kernel:aux" (stores h and / or v_new),
  * "chunk_fwd_kernel:w_in_scan" (QLA_CHUNK_W_IN_SCAN), "kkt_solve_kernel", "kkt_solve_kernel:over" (that flag without
  * QLA_CHUNK_QK_L2NORM), "bwd_scan_kernel", "bwd_chunk_kernel",
- * "recurrent_kernel", "recurrent_chain_kernel", "recurrent_step_kernel"): threads per block and dynamic shared-memory bytes, as compiled.
+ * "recurrent_kernel", "recurrent_chain_kernel", "recurrent_step_kernel", "cp_chain_kernel"): threads per block and dynamic shared-memory bytes, as compiled.
  * The manifest written beside the library (and beside the per-kernel cubins) carries the same figures for
  * launchers that load the cubins without the CUDA runtime, the role of the reference's AOT export
  * (flash_qla/compile_sm12x_gdn.py:580-669).

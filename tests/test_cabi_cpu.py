@@ -118,6 +118,20 @@ def test_manifest_lists_every_kernel_with_its_cubin(built_lib):
     assert lib.qla_kernel_launch_info(b"no_such_kernel", ctypes.byref(block), ctypes.byref(smem)) == -1
 
 
+def test_manifest_has_a_rule_for_every_kernel_that_asks_for_shared_memory(built_lib):
+    """A launcher that loads a cubin cannot read a kernel's dynamic shared memory from the compiler's report: every kernel whose limit
+    the library raises (the recurrent ones by kernel_of) has its bytes in the manifest."""
+    import json
+    from flashqla_b200 import build, manifest
+    names = {n for src in build.sources() for n in re.findall(r"ensure_dynamic_smem<(\w+)", src.read_text())}
+    assert {"chunk_fwd_kernel", "cp_chain_kernel", "kernel_of"} <= names
+    names = names - {"kernel_of"} | {"recurrent_kernel", "recurrent_chain_kernel", "recurrent_step_kernel"}
+    m = json.loads((built_lib.parent / manifest.MANIFEST_NAME).read_text())
+    for name in names:
+        entries = [k for k in m["kernels"] if re.search(r"\d%s(I|E)" % name, k["export_name"])]
+        assert entries and all(k["shared"] and k["shared"] + k["static_shared"] <= 227 * 1024 for k in entries), name
+
+
 def test_manifest_gives_every_form_of_the_scan_its_shared_memory(built_lib):
     """chunk_fwd_kernel<T, kStateOnly, kAux, kTrace, kNorm, kState16, kWIn>: the forms with kAux and kWIn use more than the plain one."""
     import json
