@@ -686,6 +686,7 @@ int resident_ctas(size_t smem, int* out) {
   return QLA_OK;
 }
 
+constexpr int kSms = 148;
 enum Form { kPlain, kTree, kChain, kStep };  // recurrent_kernel without and with parents, recurrent_chain_kernel, recurrent_step_kernel
 template <typename T, typename InterT, typename StateT, int R, Form kForm>
 constexpr auto kernel_of() {
@@ -725,7 +726,7 @@ int launch_recurrent_form(const QlaRecurrentArgs& a, int rows, cudaStream_t stre
   // rough: 80 heads of 8 steps with fp32 scratch 14.3 with 16 rows, 14.7 with 32; of 4 steps 9.7 and 9.2; 92 of 8 15.5 and 14.8.)
   if (rows == 0) {
     const int64_t tiles = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / 16);
-    int resident = 2 * 148;  // (at least: the smallest calls, which are host-bound, do not look it up)
+    int resident = 2 * kSms;  // (at least: the smallest calls, which are host-bound, do not look it up)
     if (tiles > resident) {
       const int rc = resident_tiles<T, InterT, StateT, 1, kForm>(&resident);
       if (rc != QLA_OK) return rc;
@@ -746,6 +747,44 @@ int launch_recurrent_form(const QlaRecurrentArgs& a, int rows, cudaStream_t stre
   return rows == 16 ? launch_recurrent_rows<T, InterT, StateT, 1, kForm>(a, stream)
                     : launch_recurrent_rows<T, InterT, StateT, 2, kForm>(a, stream);
 }
+// Several steps, of which every state is cached in 16 bits or none is: instructions are most of the time, and recurrent_chain_kernel has
+// fewer of them (us, recurrent_kernel / recurrent_chain_kernel, 32 heads: 256 sequences of 4 steps 370 / 333, of 8 629 / 579, without a cache
+// 330 / 273 and 558 / 464).  But five tiles of 32 rows are resident per SM, not four, and what a tile costs beside its steps (rows and
+// gates of a block of four steps through shared memory) is paid for each tile and block.  So the rounds decide; us, recurrent_kernel / recurrent_chain_kernel,
+// bf16 cache, states from HBM:
+// - to two and a half tiles of 32 rows per SM the chain kernel, with 16 rows while every SM has one such tile: 16 heads of 4 steps 4.95 / 4.53, 74 heads
+//   8.40 / 7.47, 80 heads of 8 14.5 / 13.2.  But above four steps its second block comes late where the steps are all there is (4 heads of 6
+//   5.4 / 6.1, without a cache of 64 29 / 36), and a second block of one or two steps costs as much as one of four (64 heads of 6 9.5 / 9.7).
+// - to one round of the general kernel that one (96 heads of 4 10.0 / 10.2, 132 of 8 15.7 / 17.1; eight tiles of 16 rows per SM 18.2), to one of the chain
+//   kernel (185 heads) the chain kernel (160 heads of 4 13.4 / 11.3, of 8 19.9 / 17.7).
+// - beyond, the general kernel where its last round is nearly full (288 heads of 4 18.0 / 19.3, 592 of 8 50.7 / 51.9) or, above four steps, has just begun (300 of
+//   8 30.1 / 30.5, 448 of 8 40.6 / 42.3), and with a second block of one or two steps unless the chain kernel has a round less (256 of 5
+//   20.1 / 21.7, 512 of 5 35.7 / 33.8).  With more and more rounds that matters less than the instructions.
+// The lines are rough: around them the two differ by up to 4 %.
+template <typename T, typename InterT, typename StateT>
+int takes_chain(const QlaRecurrentArgs& a, int64_t tiles, bool* chain, int* rows) {
+  const int steps = a.tokens_per_seq;
+  const bool cached = a.inter != nullptr, late = cached && steps > 4, stub = cached && (steps == 5 || steps == 6);
+  if (2 * tiles <= 5 * kSms) {
+    *chain = steps <= 4 || tiles > (stub ? 2 : 1) * kSms;
+    if (*rows == 0) *rows = (*chain ? 2 : 1) * tiles <= kSms ? 16 : 32;
+    return QLA_OK;
+  }
+  if (*rows == 0) *rows = 32;
+  int general = 0, own = 0;
+  int rc = resident_tiles<T, InterT, StateT, 2, kPlain>(&general);
+  if (rc == QLA_OK) rc = resident_tiles<T, InterT, StateT, 2, kChain>(&own);
+  if (rc != QLA_OK) return rc;
+  const int64_t rounds = (tiles + general - 1) / general, fill = 20 * (tiles - (rounds - 1) * general);  // (20ths of a round)
+  const bool fewer = (tiles + own - 1) / own < rounds;
+  if (rounds == 1 || tiles <= own) *chain = rounds > 1;
+  else if (stub && rounds > 4) *chain = rounds > (steps == 5 ? 10 : 7);
+  else if (rounds > (late || steps == 2 ? 4 : 2)) *chain = true;
+  else
+    *chain = (fewer || !stub) && fill >= (!late ? 0 : rounds == 3 ? 3 : 5) * general &&
+             fill <= (steps == 3 || steps == 4 ? 17 : late && !fewer ? 14 : 15) * general;
+  return QLA_OK;
+}
 template <typename T, typename InterT, typename StateT>
 int launch_recurrent_state(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
   // One step: the kernel without the loop, of which five tiles of 32 rows are resident per SM, not four (us, recurrent_kernel /
@@ -757,11 +796,13 @@ int launch_recurrent_state(const QlaRecurrentArgs& a, int rows, cudaStream_t str
   if (a.tokens_per_seq == 1 && (std::is_same<StateT, __nv_bfloat16>::value ? heads > 384 : heads <= 1024))
     return launch_recurrent_form<T, InterT, StateT, kStep>(a, rows, stream);
   if (a.parents != nullptr) return launch_recurrent_form<T, InterT, StateT, kTree>(a, rows, stream);
-  // Several steps, of which every state is cached in 16 bits or none is: instructions are the bound, and the kernel with fewer of them is
-  // the faster one (us, recurrent_kernel / recurrent_chain_kernel, 32 heads: 256 sequences of 4 steps 327 / 270, of 2 207 / 182, 100 of
-  // 8 254 / 226, 16 heads: 33 of 5 26.2 / 24.2).  With fp32 states in the cache HBM is (256 of 4 480 / 481, 16 of 8 50.1 / 51.7), and with one step.
-  if (a.tokens_per_seq > 1 && (a.inter == nullptr || a.inter_dtype == QLA_DT_BF16))
-    return launch_recurrent_form<T, InterT, StateT, kChain>(a, rows, stream);
+  // (with fp32 states in the cache HBM is the bound: 256 sequences of 4 steps 480 / 481 us, 16 of 8 50.1 / 51.7)
+  if (a.tokens_per_seq > 1 && (a.inter == nullptr || a.inter_dtype == QLA_DT_BF16)) {
+    bool chain = false;
+    const int rc = takes_chain<T, InterT, StateT>(a, heads * (kHeadDim / 32), &chain, &rows);
+    if (rc != QLA_OK) return rc;
+    if (chain) return launch_recurrent_form<T, InterT, StateT, kChain>(a, rows, stream);
+  }
   return launch_recurrent_form<T, InterT, StateT, kPlain>(a, rows, stream);
 }
 template <typename T, typename InterT>

@@ -27,6 +27,50 @@ def test_decode_around_the_line(n, pool_dtype):
     assert orc.max_abs(pool.float().cpu(), ref_state) <= (1e-4 if pool_dtype == torch.float32 else 2.0 ** -8)
 
 
+def names_of(call):
+    """Names of the recurrent kernels that ``call`` launches, and what it returns."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        got = call()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events() if "recurrent" in e.name], got
+
+
+# both sides of every line between the two kernels and the two tile heights
+@pytest.mark.parametrize("n, steps, cached, kernel, rows", [
+    (18, 4, True, "chain", 16), (19, 4, True, "chain", 32), (37, 5, True, "general", 16), (38, 5, True, "general", 32), (38, 8, True, "chain", 32),
+    (74, 6, True, "general", 32), (75, 6, True, "chain", 32), (92, 8, True, "chain", 32), (93, 8, True, "general", 32),
+    (132, 6, True, "general", 32), (148, 2, True, "general", 32), (149, 2, True, "chain", 32), (185, 8, True, "chain", 32),
+    (200, 5, True, "general", 32), (288, 4, True, "general", 32), (300, 4, True, "chain", 32), (300, 8, True, "general", 32),
+    (512, 5, True, "chain", 32), (4, 64, False, "general", 16), (80, 9, False, "chain", 32), (112, 4, False, "general", 32), (264, 6, False, "general", 32)])
+def test_chains_on_either_side_of_their_lines(n, steps, cached, kernel, rows):
+    """Several steps, cached in bf16 or not at all: which kernel and tile height a call gets depends on its heads and steps, its bits do not."""
+    import flashqla_b200 as fq
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines depend on the number of SMs")
+    gen = torch.Generator(device="cuda").manual_seed(n + steps)
+    q, k, v = (torch.randn(1, n * steps, 1, 128, generator=gen, device="cuda").bfloat16() for _ in range(3))
+    a, b = (torch.randn(1, n * steps, 1, generator=gen, device="cuda") for _ in range(2))
+    pool = 0.1 * torch.randn(n, 1, 128, 128, generator=gen, device="cuda")
+    zero, slots = torch.zeros(1, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
+
+    def call(block_dv, ragged=False):
+        state, scratch = pool.clone(), torch.zeros(n, steps, 1, 128, 128, dtype=torch.bfloat16, device="cuda") if cached else None
+        kw = dict(intermediate_states_buffer=scratch, intermediate_state_indices=slots) if cached else {}
+        if ragged:  # (always the general kernel)
+            kw["cu_seqlens"] = steps * torch.arange(n + 1, dtype=torch.int32, device="cuda")
+        o = fq.fused_sigmoid_gating_delta_rule_update(zero, a, zero, q, k, v, b, state, slots, block_dv=block_dv, **kw)
+        return [o, state] + ([scratch] if cached else [])
+
+    names, got = names_of(lambda: call(None))
+    expected = f"recurrent_chain_kernel<__nv_bfloat16, {'__nv_bfloat16' if cached else 'float'}, float, {rows // 16}>" if kernel == "chain" else \
+        f"recurrent_kernel<__nv_bfloat16, {'__nv_bfloat16' if cached else 'float'}, float, {rows // 16}, false>"
+    assert len(names) == 1 and expected in names[0].replace("(anonymous namespace)::", ""), names
+    for other in (call(16), call(32), call(None, ragged=True)):
+        assert all(torch.equal(x, y) for x, y in zip(got, other))
+    fq.check_device_status()
+
+
 @pytest.mark.parametrize("n, rows", [(74, 16), (75, 32), (111, 32), (138, 32), (139, 16), (148, 16), (149, 32)])
 def test_trees_with_fp32_scratch(n, rows):
     """32-row tiles of a tree are resident three per SM: with 139 to 148 heads two rounds of 16 rows take less time.  Either height
