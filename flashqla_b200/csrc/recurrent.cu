@@ -785,21 +785,52 @@ int takes_chain(const QlaRecurrentArgs& a, int64_t tiles, bool* chain, int* rows
              fill <= (steps == 3 || steps == 4 ? 17 : late && !fewer ? 14 : 15) * general;
   return QLA_OK;
 }
+// One step: the kernel without the loop, of which five tiles of 32 rows are resident per SM, not four, and seven of 16 (us, recurrent_kernel /
+// recurrent_step_kernel, states from HBM, 32 heads: bf16 pools 16 sequences 11.9 / 10.1, 64 37.6 / 30.4, 128 71.0 / 57.0; fp32 pools
+// 4 6.1 / 5.8, 12 12.2 / 10.7, 24 20.0 / 18.0, 32 24.5 / 23.5, 48 34.8 / 35.0, 64 44.7 / 47.3, 256 163.6 / 187: from about 1200 fp32 heads on HBM is the
+// bound, and the memory does better with fewer tiles in flight).  fp32 pools, states from HBM and in L2:
+// - to seven tiles of 16 rows per SM this one (120 heads 6.70 / 6.57, 5.01 / 4.61), with 32 rows where three and a half of 16 per SM are passed and two
+//   and a half of 32 are not (72 heads, 16 and 32 rows 5.80 / 5.25, 4.49 / 4.04; 96 heads 6.23 / 6.53, 4.50 / 5.01); to one round of the general kernel
+//   that one (140 heads 7.00 / 7.00, 5.06 / 5.23);
+// - beyond this one (160 heads 8.70 / 7.17, 6.54 / 5.29), except where more than two thirds of the general kernel's second round are full (296 heads 11.1 /
+//   11.1, 8.14 / 8.48).
+template <typename T, typename InterT, typename StateT>
+int takes_step(const QlaRecurrentArgs& a, int64_t tiles, bool* step, int* rows) {
+  if (std::is_same<StateT, __nv_bfloat16>::value) {
+    // Calls of 296 heads with a bf16 pool behind one another take 7.61 with the general kernel, whose two rounds come out even (592 of 1184
+    // tiles), and 7.75 with this one: bf16 pools come here above 384.
+    *step = tiles > 4 * 384;
+    return QLA_OK;
+  }
+  *step = tiles <= 4 * 1024;
+  if (!*step) return QLA_OK;
+  if (tiles <= 2 * kSms) {
+    if (*rows == 0) *rows = 4 * tiles > 7 * kSms ? 32 : 16;
+    return QLA_OK;
+  }
+  int general = 0, low = 0;
+  int rc = resident_tiles<T, InterT, StateT, 2, kPlain>(&general);
+  if (rc == QLA_OK) rc = resident_tiles<T, InterT, StateT, 1, kStep>(&low);
+  if (rc != QLA_OK) return rc;
+  if (tiles <= general) *step = 2 * tiles <= low;
+  else *step = 3 * tiles <= 5 * general || tiles > 2 * general;
+  if (*rows == 0 && *step) *rows = 2 * tiles > low || 2 * tiles <= 5 * kSms ? 32 : 16;
+  return QLA_OK;
+}
 template <typename T, typename InterT, typename StateT>
 int launch_recurrent_state(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
-  // One step: the kernel without the loop, of which five tiles of 32 rows are resident per SM, not four (us, recurrent_kernel /
-  // recurrent_step_kernel, states from HBM, 32 heads: bf16 pools 16 sequences 11.9 / 10.1, 64 37.6 / 30.4, 128 71.0 / 57.0; fp32 pools
-  // 4 6.1 / 5.8, 12 12.2 / 10.7, 24 20.0 / 18.0, 32 24.5 / 23.5, 48 34.8 / 35.0, 64 44.7 / 47.3, 256 163.6 / 187: from about 1200 fp32 heads on HBM is the
-  // bound, and the memory does better with fewer tiles in flight).  Calls of 296 heads with a bf16 pool behind one another take 7.61 with the
-  // general kernel, whose two rounds come out even (592 of 1184 tiles), and 7.75 with this one: bf16 pools come here above 384.
-  const int64_t heads = static_cast<int64_t>(a.num_seqs) * a.num_v_heads;
-  if (a.tokens_per_seq == 1 && (std::is_same<StateT, __nv_bfloat16>::value ? heads > 384 : heads <= 1024))
-    return launch_recurrent_form<T, InterT, StateT, kStep>(a, rows, stream);
+  const int64_t tiles = static_cast<int64_t>(a.num_seqs) * a.num_v_heads * (kHeadDim / 32);
+  if (a.tokens_per_seq == 1) {
+    bool step = false;
+    const int rc = takes_step<T, InterT, StateT>(a, tiles, &step, &rows);
+    if (rc != QLA_OK) return rc;
+    if (step) return launch_recurrent_form<T, InterT, StateT, kStep>(a, rows, stream);
+  }
   if (a.parents != nullptr) return launch_recurrent_form<T, InterT, StateT, kTree>(a, rows, stream);
   // (with fp32 states in the cache HBM is the bound: 256 sequences of 4 steps 480 / 481 us, 16 of 8 50.1 / 51.7)
   if (a.tokens_per_seq > 1 && (a.inter == nullptr || a.inter_dtype == QLA_DT_BF16)) {
     bool chain = false;
-    const int rc = takes_chain<T, InterT, StateT>(a, heads * (kHeadDim / 32), &chain, &rows);
+    const int rc = takes_chain<T, InterT, StateT>(a, tiles, &chain, &rows);
     if (rc != QLA_OK) return rc;
     if (chain) return launch_recurrent_form<T, InterT, StateT, kChain>(a, rows, stream);
   }

@@ -65,9 +65,45 @@ def test_chains_on_either_side_of_their_lines(n, steps, cached, kernel, rows):
     names, got = names_of(lambda: call(None))
     expected = f"recurrent_chain_kernel<__nv_bfloat16, {'__nv_bfloat16' if cached else 'float'}, float, {rows // 16}>" if kernel == "chain" else \
         f"recurrent_kernel<__nv_bfloat16, {'__nv_bfloat16' if cached else 'float'}, float, {rows // 16}, false>"
-    assert len(names) == 1 and expected in names[0].replace("(anonymous namespace)::", ""), names
+    assert len(names) == 1 and expected in names[0], names
     for other in (call(16), call(32), call(None, ragged=True)):
         assert all(torch.equal(x, y) for x, y in zip(got, other))
+    fq.check_device_status()
+
+
+@pytest.mark.parametrize("pool_dtype, n, kernel, rows", [
+    (torch.float32, 1, "step", 16), (torch.float32, 64, "step", 16), (torch.float32, 65, "step", 32), (torch.float32, 92, "step", 32),
+    (torch.float32, 93, "step", 16), (torch.float32, 129, "step", 16), (torch.float32, 130, "general", 32), (torch.float32, 148, "general", 32),
+    (torch.float32, 149, "step", 32), (torch.float32, 246, "step", 32), (torch.float32, 247, "general", 32), (torch.float32, 296, "general", 32),
+    (torch.float32, 297, "step", 32), (torch.float32, 1024, "step", 32), (torch.float32, 1025, "general", 32)])
+def test_one_step_on_either_side_of_its_lines(pool_dtype, n, kernel, rows):
+    """One token per sequence: which kernel and tile height a call gets depends on its heads and its pool, its bits do not; with and
+    without a cached state of either type, q, k, v of either type, against single tokens by cu_seqlens, which the general kernel takes."""
+    import flashqla_b200 as fq
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines depend on the number of SMs")
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    zero, slots = torch.zeros(1, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
+    a, b = (torch.randn(1, n, 1, generator=gen, device="cuda") for _ in range(2))
+    pool = (0.1 * torch.randn(n, 1, 128, 128, generator=gen, device="cuda")).to(pool_dtype)
+    for dtype, cache in ((torch.bfloat16, None), (torch.float16, torch.float32), (torch.bfloat16, torch.bfloat16)):
+        q, k, v = (torch.randn(1, n, 1, 128, generator=gen, device="cuda").to(dtype) for _ in range(3))
+
+        def call(block_dv, ragged=False):
+            state, scratch = pool.clone(), torch.zeros(n, 1, 1, 128, 128, dtype=cache or torch.float32, device="cuda")
+            kw = dict(intermediate_states_buffer=scratch, intermediate_state_indices=slots) if cache else {}
+            if ragged:
+                kw["cu_seqlens"] = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+            o = fq.fused_sigmoid_gating_delta_rule_update(zero, a, zero, q, k, v, b, state, slots, block_dv=block_dv, **kw)
+            return o, state, scratch
+
+        names, got = names_of(lambda: call(None))
+        types = ", ".join({torch.bfloat16: "__nv_bfloat16", torch.float16: "__half", torch.float32: "float"}[t]
+                          for t in (dtype, torch.bfloat16 if cache == torch.bfloat16 else torch.float32, pool_dtype))
+        expected = f"recurrent_step_kernel<{types}, {rows // 16}>" if kernel == "step" else f"recurrent_kernel<{types}, {rows // 16}, false>"
+        assert len(names) == 1 and expected in names[0], names
+        for other in (call(16), call(32), call(None, ragged=True)):
+            assert all(torch.equal(x, y) for x, y in zip(got, other))
     fq.check_device_status()
 
 
