@@ -794,15 +794,12 @@ int takes_chain(const QlaRecurrentArgs& a, int64_t tiles, bool* chain, int* rows
 //   that one (140 heads 7.00 / 7.00, 5.06 / 5.23);
 // - beyond this one (160 heads 8.70 / 7.17, 6.54 / 5.29), except where more than two thirds of the general kernel's second round are full (296 heads 11.1 /
 //   11.1, 8.14 / 8.48).
+// bf16 pools the same beyond one round of the general kernel (160 heads 7.55 / 5.76, 6.09 / 4.61; 240 8.70 / 8.19, 7.17 / 6.83; 280 8.92 / 8.62, 7.22 / 7.28;
+// 296 9.13 / 9.00, 7.28 / 7.34; 300 10.8 / 8.9, 8.54 / 7.34; 512 15.3 / 12.7, 12.7 / 10.4); to there the general one (120 heads 5.16 / 5.21, 4.44 / 4.61).
 template <typename T, typename InterT, typename StateT>
 int takes_step(const QlaRecurrentArgs& a, int64_t tiles, bool* step, int* rows) {
-  if (std::is_same<StateT, __nv_bfloat16>::value) {
-    // Calls of 296 heads with a bf16 pool behind one another take 7.61 with the general kernel, whose two rounds come out even (592 of 1184
-    // tiles), and 7.75 with this one: bf16 pools come here above 384.
-    *step = tiles > 4 * 384;
-    return QLA_OK;
-  }
-  *step = tiles <= 4 * 1024;
+  constexpr bool kState16 = std::is_same<StateT, __nv_bfloat16>::value;
+  *step = kState16 ? tiles > 2 * kSms : tiles <= 4 * 1024;
   if (!*step) return QLA_OK;
   if (tiles <= 2 * kSms) {
     if (*rows == 0) *rows = 4 * tiles > 7 * kSms ? 32 : 16;
@@ -812,7 +809,7 @@ int takes_step(const QlaRecurrentArgs& a, int64_t tiles, bool* step, int* rows) 
   int rc = resident_tiles<T, InterT, StateT, 2, kPlain>(&general);
   if (rc == QLA_OK) rc = resident_tiles<T, InterT, StateT, 1, kStep>(&low);
   if (rc != QLA_OK) return rc;
-  if (tiles <= general) *step = 2 * tiles <= low;
+  if (tiles <= general) *step = !kState16 && 2 * tiles <= low;
   else *step = 3 * tiles <= 5 * general || tiles > 2 * general;
   if (*rows == 0 && *step) *rows = 2 * tiles > low || 2 * tiles <= 5 * kSms ? 32 : 16;
   return QLA_OK;

@@ -75,7 +75,9 @@ def test_chains_on_either_side_of_their_lines(n, steps, cached, kernel, rows):
     (torch.float32, 1, "step", 16), (torch.float32, 64, "step", 16), (torch.float32, 65, "step", 32), (torch.float32, 92, "step", 32),
     (torch.float32, 93, "step", 16), (torch.float32, 129, "step", 16), (torch.float32, 130, "general", 32), (torch.float32, 148, "general", 32),
     (torch.float32, 149, "step", 32), (torch.float32, 246, "step", 32), (torch.float32, 247, "general", 32), (torch.float32, 296, "general", 32),
-    (torch.float32, 297, "step", 32), (torch.float32, 1024, "step", 32), (torch.float32, 1025, "general", 32)])
+    (torch.float32, 297, "step", 32), (torch.float32, 1024, "step", 32), (torch.float32, 1025, "general", 32),
+    (torch.bfloat16, 74, "general", 16), (torch.bfloat16, 148, "general", 32), (torch.bfloat16, 149, "step", 32), (torch.bfloat16, 246, "step", 32),
+    (torch.bfloat16, 247, "general", 32), (torch.bfloat16, 296, "general", 32), (torch.bfloat16, 297, "step", 32), (torch.bfloat16, 1025, "step", 32)])
 def test_one_step_on_either_side_of_its_lines(pool_dtype, n, kernel, rows):
     """One token per sequence: which kernel and tile height a call gets depends on its heads and its pool, its bits do not; with and
     without a cached state of either type, q, k, v of either type, against single tokens by cu_seqlens, which the general kernel takes."""
