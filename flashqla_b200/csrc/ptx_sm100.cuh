@@ -77,9 +77,6 @@ __device__ __forceinline__ bool mbar_wait_polling(uint64_t* bar, uint32_t parity
   record_wait_failure(status, code, parity);
   return false;
 }
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, int* status, int code) {
-  return mbar_wait_polling(bar, parity, status, code, kWaitLimitNs);
-}
 
 // One look at a barrier: mbarrier.test_wait never suspends the thread.
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
@@ -95,19 +92,12 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Wait executed by a CONVERGED warp, verdict warp-uniform.  The first poll is inline and not voted on:
+// Wait executed by a CONVERGED warp, verdict warp-uniform (mbar_wait_addr).  The first poll is inline and not voted on:
 // the lanes of a converged warp execute the try_wait as one instruction on one barrier word and see the
 // same answer, so either all of them return here or all of them enter the (non-inlined) polling loop,
 // whose vote makes the verdict uniform even at the edge of the time limit.
-static __device__ __noinline__ bool mbar_wait_warp_slow(uint64_t* bar, uint32_t parity, int* status, int code) {
-  return __all_sync(__activemask(), mbar_wait_slow(bar, parity, status, code)) != 0;
-}
-__device__ __forceinline__ bool mbar_wait_warp_call(uint64_t* bar, uint32_t parity, int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_warp_slow(bar, parity, status, code);
-}
-
-// The same wait for kernels that live from their instruction cache.  All code that a CTA executes per chunk shares
+//
+// It is made for kernels that live from their instruction cache.  All code that a CTA executes per chunk shares
 // the SM's 32 KB instruction cache (beyond it a line costs some 40 cycles, measured with straight-line code; beyond
 // 128 KB twice that), and a wait appears some thirty times in a scan kernel: here a call site is one try_wait on a
 // 32-bit shared address and a two-argument call that is hardly ever taken.  What the slow path reports with
