@@ -202,29 +202,6 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&x);
 }
 
-// Two fp32 values per register pair and instruction.
-using F2 = unsigned long long;
-__device__ __forceinline__ F2 f2(float lo, float hi) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ F2 f2(uint32_t lo, uint32_t hi) { return f2(__uint_as_float(lo), __uint_as_float(hi)); }
-__device__ __forceinline__ float2 unpack(F2 x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
-  return r;
-}
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 template <typename T>
 __device__ __forceinline__ F2 widen(uint32_t raw);  // two 16-bit values
 template <>

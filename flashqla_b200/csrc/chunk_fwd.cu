@@ -125,8 +125,6 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&x);
 }
 
-// two neighbouring registers of a tensor-memory load as a pair
-__device__ __forceinline__ F2 pair(uint32_t a, uint32_t b) { return f2(__uint_as_float(a), __uint_as_float(b)); }
 template <typename T>
 __device__ __forceinline__ uint32_t pack2(F2 x) {
   const float2 y = unpack(x);
@@ -1121,8 +1119,8 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
           const float4 r4 = *reinterpret_cast<const float4*>(&gs->rho[c0 + j]);
-          vp[j >> 1] = pack2<T>(mul2(pair(d[j], d[j + 1]), f2(r4.x, r4.y)));
-          vp[(j >> 1) + 1] = pack2<T>(mul2(pair(d[j + 2], d[j + 3]), f2(r4.z, r4.w)));
+          vp[j >> 1] = pack2<T>(mul2(f2(d[j], d[j + 1]), f2(r4.x, r4.y)));
+          vp[(j >> 1) + 1] = pack2<T>(mul2(f2(d[j + 2], d[j + 3]), f2(r4.z, r4.w)));
         }
         ptx::tmem_st16(tm + kColD2 + c0, vp);
         ptx::tmem_wait_st();
@@ -1183,7 +1181,7 @@ chunk_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const float egl_next = gates_of(i + 1)->egl;
 #pragma unroll
         for (int j = 0; j < 64; j += 2) {
-          const float2 y = unpack(mul2(pair(sf[j], sf[j + 1]), f2(egl_next, egl_next)));
+          const float2 y = unpack(mul2(f2(sf[j], sf[j + 1]), f2(egl_next, egl_next)));
           sf[j] = __float_as_uint(y.x);
           sf[j + 1] = __float_as_uint(y.y);
         }

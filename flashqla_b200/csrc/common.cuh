@@ -126,16 +126,23 @@ struct Cvt<float> {
   static __device__ __forceinline__ float from_f32(float x) { return x; }
 };
 
-// Two fp32 values per register pair and instruction (mul / fma .f32x2), for loops that are bound by instruction issue.
+// Two fp32 values per register pair and instruction (add / mul / fma .f32x2), for loops that are bound by instruction issue.
 using F2 = unsigned long long;
 __device__ __forceinline__ F2 f2(float lo, float hi) {
   F2 r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
   return r;
 }
+__device__ __forceinline__ F2 f2(uint32_t lo, uint32_t hi) { return f2(__uint_as_float(lo), __uint_as_float(hi)); }
+__device__ __forceinline__ void unpack(F2 x, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x)); }
 __device__ __forceinline__ float2 unpack(F2 x) {
   float2 r;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) {

@@ -164,11 +164,6 @@ constexpr int kChainStages = 3;
 constexpr uint32_t kChainTile = kHeadDim * kHeadDim * 4;
 constexpr size_t kChainSmem = kChainStages * kChainTile;
 
-__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {  // two fp32 values per instruction
-  unsigned long long& r = reinterpret_cast<unsigned long long&>(acc);
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
-}
-
 // A warp's wait for the matrix in `stage`, the same verdict for all of it.  Given up, the status word says so (192 + stage as the
 // barrier); the thread that requests the copies then waits for those still on their way, `ahead` links from this one on, or for
 // another while: shared memory stays allocated until they have landed.
@@ -217,7 +212,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
   };
   // this thread's four values of the product of the matrix in `stage` and the carried columns in `buf`
   auto product = [&](int stage, int buf) {
-    float2 acc[4][4] = {};  // [i][pair of columns]
+    F2 acc[4][4] = {};  // [i][pair of columns]
     const float* part = reinterpret_cast<const float*>(s_m + stage * kChainTile) + (16 * warp + rg) * kHeadDim + 4 * sl;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
@@ -227,13 +222,13 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
       const float* x = &s_h[buf][(8 * t + sl) * kChainGroup];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float4 lo = *reinterpret_cast<const float4*>(x + e * kChainCols), hi = *reinterpret_cast<const float4*>(x + e * kChainCols + 4);
-        const float2 xs[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
+        const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(x + e * kChainCols), hi = *reinterpret_cast<const ulonglong2*>(x + e * kChainCols + 4);
+        const F2 xs[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float mv = e == 0 ? m[i].x : e == 1 ? m[i].y : e == 2 ? m[i].z : m[i].w;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) fma2(acc[i][c], make_float2(mv, mv), xs[c]);
+          for (int c = 0; c < 4; ++c) acc[i][c] = fma2(f2(mv, mv), xs[c], acc[i][c]);
         }
       }
     }
@@ -246,7 +241,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) cp_chain_kernel(float* __res
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) y[i][c] = add(b2 ? acc[2 + i][c] : acc[i][c], b2 ? acc[i][c] : acc[2 + i][c], 4);
+      for (int c = 0; c < 4; ++c) y[i][c] = add(unpack(b2 ? acc[2 + i][c] : acc[i][c]), unpack(b2 ? acc[i][c] : acc[2 + i][c]), 4);
 #pragma unroll
     for (int c = 0; c < 4; ++c) z[c] = add(b1 ? y[1][c] : y[0][c], b1 ? y[0][c] : y[1][c], 2);
 #pragma unroll
