@@ -238,7 +238,7 @@ bwd_scan_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   } else if (warp == 9) {
     // =========================================================== MMA issuer (whole warp, converged)
-    const uint32_t id_n64 = ptx::mma_idesc(128, 64, fmt, ptx::kMajorK, ptx::kMajorK);        // MMA0, MMA2
+    const uint32_t id_n64 = ptx::mma_idesc(128, 64, fmt, ptx::kMajorK, ptx::kMajorK);        // MMA2
     const uint32_t id_u = ptx::mma_idesc(128, 64, fmt, ptx::kMajorMN, ptx::kMajorMN);       // MMAu
     const uint32_t id_s = ptx::mma_idesc(128, 128, fmt, ptx::kMajorK, ptx::kMajorMN);       // MMA3
     const uint32_t id_q = ptx::mma_idesc(128, 128, fmt, ptx::kMajorMN, ptx::kMajorMN);      // MMAq

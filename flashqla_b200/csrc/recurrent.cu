@@ -1,12 +1,13 @@
 // Recurrent gated-delta-rule step(s): decode (1 token), spec-decode verify (T draft tokens with a
 // cached state per step), tree verify (a step may restart from the cached state of its parent)
-// and ragged sequences (cu_seqlens).  One kernel covers what the reference spreads over 29
-// generated kernels (flash_qla/ops/gated_delta_rule/recurrent_fused.py:290-6249); the per-token
+// and ragged sequences (cu_seqlens).  Three kernels, the same bits, cover what the reference spreads over 29
+// generated kernels (flash_qla/ops/gated_delta_rule/recurrent_fused.py:290-6249): recurrent_kernel takes every call,
+// recurrent_step_kernel one step, recurrent_chain_kernel several (takes_step, takes_chain say which of those).  The per-token
 // math follows the canonical body at :346-487 and the reload rule of the warp kernels at
-// :5803-5836 (a parent equal to the previous step is not reloaded).  Two forms of it, for one step and for chains that are
-// bound by instructions, give the same bits (launch_recurrent_state says which call takes which).
+// :5803-5836 (a parent equal to the previous step is not reloaded).
 //
-// The op is HBM-bound: every (sequence, v-head) streams a 64 KiB fp32 state in and out.
+// The op is HBM-bound (several steps per state: bound by instruction issue unless fp32 states are cached): every (sequence, v-head)
+// streams a 64 KiB fp32 state in and out.
 // Mapping: the state of one head is [V=128 rows][K=128 floats]; a row is 512 B.  Eight lanes share
 // a row, each lane owning four float4 (columns j*32 + sub*4 .. +3, j = 0..3), so one warp
 // instruction moves four whole rows = 2 KiB, fully coalesced, 128-bit per lane.  A thread keeps R
@@ -720,6 +721,7 @@ int launch_recurrent_rows(const QlaRecurrentArgs& a, cudaStream_t stream) {
 
 template <typename T, typename InterT, typename StateT, Form kForm>
 int launch_recurrent_form(const QlaRecurrentArgs& a, int rows, cudaStream_t stream) {
+  // (recurrent_kernel; the height of the other two comes with the call.)
   // Tiles of 16 rows while they are all resident at once, which spreads a small batch over the most SMs; a second round of
   // them costs the latency of every step again.  With the line at four tiles of 32 rows per SM: 96 heads of 7 tree steps 17.5 us, now
   // 13.2; 112 heads of 4 steps 11.4 -> 9.7; 144 heads of one step 7.0 -> 5.3, with a bf16 pool 6.8 -> 4.8.  (Just above the line it is

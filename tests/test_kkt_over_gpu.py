@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("lens, hk, hv", [
-    # 592 CTAs are resident: 219 pairs of chunks x 4 and x 8 heads, pairs of one chunk beside pairs of two; 700 pairs of one chunk;
+    # 592 CTAs are resident: 225 pairs of chunks x 4 and x 8 heads, pairs of one chunk beside pairs of two; 700 pairs of one chunk;
     # 593 pairs of one head: one CTA has a second item
     ([5000, 63, 64, 130, 9000, 1, 127, 128, 8192, 65, 5313], 4, 4),
     ([5000, 63, 64, 130, 9000, 1, 127, 128, 8192, 65, 5313], 8, 32),
@@ -18,6 +18,9 @@ pytestmark = pytest.mark.gpu
 ])
 def test_bits_of_the_raw_forward(lens, hk, hv, dtype):
     import flashqla_b200 as fq
+    pairs = sum(-(-n // 128) for n in lens)
+    resident = 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert pairs * hk > resident or resident != 592, "every CTA has one item: the K tile is not loaded a second time"
     gen = torch.Generator(device="cuda").manual_seed(len(lens) + hv)
     T = sum(lens)
     q, k, v = (torch.randn(1, T, n, 128, generator=gen, device="cuda") for n in (hk, hk, hv))

@@ -20,7 +20,8 @@ def inputs(n, steps, hk, hv, dtype, seed, l2norm):
     return A_log, a, dt, q, k, v, b, pool, slots
 
 
-# a block of steps is four; 16-row tiles are all resident up to 148 heads, 32-row tiles up to 185
+# a block of steps is four; the chain kernel has all but the call of 148 heads, with 16 rows up to 18 heads; its 32-row tiles are
+# all resident up to 185, and from 186 on its CTAs have a second item
 @pytest.mark.parametrize("l2norm", [False, True])
 @pytest.mark.parametrize("n, steps, hk, hv, dtype", [
     (1, 2, 1, 1, torch.bfloat16), (3, 3, 2, 4, torch.float16), (148, 4, 1, 1, torch.bfloat16), (149, 5, 1, 1, torch.bfloat16),
@@ -57,8 +58,8 @@ def test_chain_equals_the_general_kernel(n, steps, hk, hv, dtype, l2norm):
 @pytest.mark.parametrize("pool_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("l2norm", [False, True])
 def test_one_step_on_either_side_of_the_line(pool_dtype, l2norm):
-    """1024 fp32 heads go to the kernel for one step, 1056 to the general one: what the first 32 sequences get does not depend on it.
-    cu_seqlens of single tokens, which the general kernel takes, give the same as well."""
+    """1024 fp32 heads go to the kernel for one step, 1056 to the general one (bf16 pools: both to the former): what the first 32
+    sequences get does not depend on it.  cu_seqlens of single tokens, which the general kernel takes, give the same as well."""
     import flashqla_b200 as fq
     A_log, a, dt, q, k, v, b, pool, _ = inputs(33, 1, 16, 32, torch.bfloat16, 1, l2norm)
     pool, slots = pool.to(pool_dtype), torch.arange(33, dtype=torch.int32, device="cuda")

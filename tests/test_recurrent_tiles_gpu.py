@@ -1,5 +1,5 @@
-"""Height of the recurrent kernel's tiles: 16 rows while all tiles are resident at once, 32 beyond.  Batches on either side of the
-line (four to six tiles per SM) against the oracle."""
+"""Which of the recurrent op's kernels a call gets and the height of its tiles, 16 or 32 rows: both follow from how many tiles there are
+per SM.  Batches on either side of the lines against the oracle, and against each other bit by bit."""
 import pytest
 import torch
 
