@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(128, R == 2 ? 5 : 8) recurrent_chain_kernel(co
   }  // items
 }
 
-// Resident CTAs of `Fn` on the current device (SMs x CTAs per SM), looked up once per device.
+// Resident CTAs of `Fn` on the current device (SMs x CTAs per SM), looked up once per device; its shared-memory limit is raised then.
 template <auto Fn>
 int resident_ctas(size_t smem, int* out) {
   static int cached[64] = {};
@@ -679,6 +679,8 @@ int resident_ctas(size_t smem, int* out) {
     *out = cached[dev];
     return QLA_OK;
   }
+  const int rc = ensure_dynamic_smem<Fn>(smem);
+  if (rc != QLA_OK) return rc;
   int sms = 0, per_sm = 0;
   QLA_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   QLA_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Fn, 128, smem));
@@ -698,8 +700,7 @@ constexpr auto kernel_of() {
 template <typename T, typename InterT, typename StateT, int R, Form kForm>
 int resident_tiles(int* out) {
   constexpr size_t smem = kRecStages * R * 4 * 128 * sizeof(typename StatePiece<StateT>::Raw);
-  const int rc = ensure_dynamic_smem<kernel_of<T, InterT, StateT, R, kForm>()>(smem);
-  return rc != QLA_OK ? rc : resident_ctas<kernel_of<T, InterT, StateT, R, kForm>()>(smem, out);
+  return resident_ctas<kernel_of<T, InterT, StateT, R, kForm>()>(smem, out);
 }
 
 template <typename T, typename InterT, typename StateT, int R, Form kForm>
